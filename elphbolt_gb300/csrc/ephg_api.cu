@@ -96,6 +96,49 @@ std::vector<int> ws_wrap(const double lvec[9], const double vl[3], double eps) {
   return out;
 }
 
+// The nested cell tables of launch_cells_fourier (rows r: n cells, 3 ints each),
+// packed one after the other; offsets off[0..2].  False: cells repeat or span
+// too large a box, and the sums run as matrix products instead.
+bool cell_tables(const std::vector<int> &r, int n, CellTab &t, std::vector<int> &tab, size_t off[3]) {
+  if (n <= 0) return false;
+  for (int d = 0; d < 3; ++d) {
+    int lo = r[d], hi = r[d];
+    for (int i = 1; i < n; ++i) {
+      lo = std::min(lo, r[3 * i + d]);
+      hi = std::max(hi, r[3 * i + d]);
+    }
+    if ((int64_t)hi - lo > 1023 || lo < -1023 || hi > 1023) return false;
+    t.lo[d] = lo;
+    t.ext[d] = hi - lo + 1;
+  }
+  std::map<std::pair<int, int>, int> pair;
+  std::map<int, int> slot;
+  for (int i = 0; i < n; ++i) {
+    slot.emplace(r[3 * i], 0);
+    pair.emplace(std::make_pair(r[3 * i], r[3 * i + 1]), 0);
+  }
+  int k = 0;
+  for (auto &x : slot) x.second = k++;
+  k = 0;
+  for (auto &x : pair) x.second = k++;
+  t.n1 = (int)slot.size();
+  t.npair = (int)pair.size();
+  off[0] = 0;
+  off[1] = (size_t)t.npair * t.ext[2];
+  off[2] = off[1] + (size_t)t.n1 * t.ext[1];
+  tab.assign(off[2] + t.ext[0], -1);
+  for (int i = 0; i < n; ++i) {
+    const int *R = &r[3 * (size_t)i];
+    const int p = pair[{R[0], R[1]}], s = slot[R[0]];
+    int &cell = tab[off[0] + (size_t)p * t.ext[2] + (R[2] - t.lo[2])];
+    if (cell >= 0) return false;
+    cell = i;
+    tab[off[1] + (size_t)s * t.ext[1] + (R[1] - t.lo[1])] = p;
+    tab[off[2] + (R[0] - t.lo[0])] = s;
+  }
+  return true;
+}
+
 }  // namespace
 
 
@@ -189,7 +232,7 @@ int ephg_destroy(ephg_handle *h) {
   void *ptrs[] = {h->Rk, h->Rq, h->Rg, h->degk, h->degq, h->degg, h->Hext, h->Hbox, h->Dbox, h->graw, h->G64,
                   h->masses, h->pair_off, h->ent_iuc, h->ent_woff, h->wrapR, h->ent_rden,
                   h->rcartq, h->D, h->err, h->kposk, h->kposq, h->polar_G, h->polar_Gcell,
-                  h->polar_born, h->polar_tau, h->polar_Da};
+                  h->polar_born, h->polar_tau, h->polar_Da, h->cellk_tab, h->cellq_tab, h->rdegk};
   // stream-ordered frees back to the library pool, which keeps the memory
   // mapped for the next handle
   for (void *p : ptrs)
@@ -256,6 +299,25 @@ int ephg_create(const ephg_wannier_desc *d, ephg_handle **out) {
       (rc = upload(&h->degq, dq.data(), dq.size(), h->st, &h->resident_bytes)) || (rc = upload(&h->degg, dg.data(), dg.size(), h->st, &h->resident_bytes)) ||
       (rc = upload(&h->masses, d->masses, (size_t)h->nat, h->st, &h->resident_bytes)))
     return bail(rc);
+  {   // the cells of the two Fourier sums of g
+    auto cells = [&](const std::vector<int> &r, int n, CellTab &t, int **dev) -> int {
+      std::vector<int> tab;
+      size_t off[3];
+      if (!cell_tables(r, n, t, tab, off)) return EPHG_OK;
+      const int e = upload(dev, tab.data(), tab.size(), h->st, &h->resident_bytes);
+      if (e) return e;
+      t.tab1 = *dev + off[0];
+      t.tab2 = *dev + off[1];
+      t.tab3 = *dev + off[2];
+      t.ok = true;
+      return EPHG_OK;
+    };
+    std::vector<double> rd(nwsk);
+    for (int r = 0; r < nwsk; ++r) rd[r] = 1.0 / dk[r];
+    if ((rc = cells(rk, nwsk, h->cellk, &h->cellk_tab)) || (rc = cells(rq, nwsq, h->cellq, &h->cellq_tab)) ||
+        (rc = upload(&h->rdegk, rd.data(), rd.size(), h->st, &h->resident_bytes)))
+      return bail(rc);
+  }
   // H(Re) with the velocity companions i*rcart*H (wannier.f90:466-478)
   {
     const size_t nn = (size_t)nw * nw;
@@ -1261,47 +1323,84 @@ int ephg::el_rates_view(ephg_handle *h, const ExecView &x, const ephg_rate_reque
       return WSFAILX(rc);
   }
   if (!split) {
-    double2 *Pk, *gk, *B, *Pq, *Cb;
-    const int64_t kc = std::max<int64_t>(1, std::min<int64_t>(nA, ((int64_t)1 << 31) / (Nn * 16)));
-    const int64_t sc = std::max<int64_t>(1, std::min<int64_t>({(int64_t)nst, (int64_t)32768,
-                                                              ((int64_t)1 << 31) / ((int64_t)nwv * ncol * 16)}));
-    if ((rc = wsget((*x.ws), "a_Pk", (size_t)kc * nwsk, &Pk)) || (rc = wsget((*x.ws), "a_gk", (size_t)kc * Nn, &gk)) ||
-        (rc = wsget((*x.ws), "a_B", (size_t)nwsq * ldb, &B)) || (rc = wsget((*x.ws), "b_Pq", (size_t)nwv * nwsq, &Pq)) ||
+    // Each contraction is a Fourier sum of cells onto mesh points: one dimension at a
+    // time (launch_cells_fourier), or as a matrix product where that takes fewer FP64
+    // instructions (a wedge or a window of few rows; 4 per cell and row).  Both are
+    // bound by the FP64 pipe, so the counts decide: 12^3 and 279 cells, 1,479 rows,
+    // 468 ms as products and 14.7 ms as sums.
+    const bool sepA = cells_fourier_cost(h->cellk, mesh, nA) < 4.0 * nA * nwsk;
+    const bool sepB = cells_fourier_cost(h->cellq, mesh, nwv) < 4.0 * nwv * nwsq;
+    const int64_t per = (int64_t)nw * nw, nper = (int64_t)nb * nwsq;   // columns of one (mode, Rp) block; blocks
+    const int64_t bound = (int64_t)1 << 31;
+    double2 *Pk = nullptr, *t1 = nullptr, *t2 = nullptr, *gk, *B, *Pq = nullptr, *Cb, *phk;
+    int *rowmap = nullptr;
+    const int64_t a1 = cells_t1_rows(h->cellk, mesh), a2 = cells_t2_rows(h->cellk, mesh);
+    const int64_t b1 = cells_t1_rows(h->cellq, mesh), b2 = cells_t2_rows(h->cellq, mesh);
+    // stage A as sums: ra blocks at a time, all rows; as products: kc rows at a time, all blocks
+    const int64_t ra = sepA ? std::max<int64_t>(1, std::min<int64_t>(nper, bound / ((a1 + a2 + nA) * per * 16))) : nper;
+    const int64_t kc = sepA ? nA : std::max<int64_t>(1, std::min<int64_t>(nA, bound / (Nn * 16)));
+    // states per chunk of stage B
+    const int64_t brows = sepB ? b1 + b2 + nwv : nwv;
+    const int64_t sc = std::max<int64_t>(1, std::min<int64_t>({(int64_t)nst, (int64_t)32768, bound / (brows * ncol * 16)}));
+    const int64_t n1 = std::max(sepA ? a1 * ra * per : 0, sepB ? b1 * sc * ncol : 0);
+    const int64_t n2 = std::max(sepA ? a2 * ra * per : 0, sepB ? b2 * sc * ncol : 0);
+    if ((!sepA && (rc = wsget((*x.ws), "a_Pk", (size_t)kc * nwsk, &Pk))) ||
+        (n1 && (rc = wsget((*x.ws), "a_t1", (size_t)n1, &t1))) || (n2 && (rc = wsget((*x.ws), "a_t2", (size_t)n2, &t2))) ||
+        (rc = wsget((*x.ws), "a_gk", (size_t)kc * ra * per, &gk)) || (rc = wsget((*x.ws), "a_B", (size_t)nwsq * ldb, &B)) ||
+        (rc = wsget((*x.ws), "a_phk", (size_t)nA * nwsq, &phk)) || (rc = wsget((*x.ws), "a_map", (size_t)N, &rowmap)) ||
+        (!sepB && (rc = wsget((*x.ws), "b_Pq", (size_t)nwv * nwsq, &Pq))) ||
         (rc = wsget((*x.ws), "b_C", (size_t)nwv * ncol * sc, &Cb)))
       return WSFAILX(rc);
-    for (int64_t i0 = 0; i0 < nA; i0 += kc) {   // stage A over the A-rows
-      int n = (int)std::min<int64_t>(kc, nA - i0);
-      launch_phase_mesh(n, arow + i0, mesh, L, nwsk, h->Rk, h->degk, 0, roots, Pk, nwsk, st);
-      (*x.ta).begin(st);
-      launch_zgemm(n, (int)Nn, nwsk, Pk, nwsk, h->G64, Nn, gk, Nn, st);
-      (*x.ta).end(st);
-      // the rotation writes B columns of states [j0, j1) (grid.y <= 32768 per launch)
-      for (int j0 = first_state[i0], j1 = first_state[i0 + n]; j0 < j1; j0 += 32768) {
-        int je = std::min(j1, j0 + 32768);
-        launch_rotate_states_fp64(j0, je, (int)i0, st_code, nw, nb, nwsq, arow, V, gk, Nn, mesh, L,
-                                  roots, h->Rq, h->degq, B + (int64_t)j0 * ncol, ldb, st);
-        (*x.launches) += 1;
+    launch_phase_mesh(nA, arow, mesh, L, nwsq, h->Rq, h->degq, 1, roots, phk, nwsq, st);
+    (*x.launches) += 1;
+    if (sepA) {
+      launch_row_map(N, nA, arow, rowmap, st);
+      (*x.launches) += 1;
+      for (int64_t r0 = 0; r0 < nper; r0 += ra) {
+        const int64_t nr = std::min<int64_t>(ra, nper - r0);
+        (*x.ta).begin(st);
+        launch_cells_fourier(h->cellk, h->G64 + r0 * per, Nn, h->rdegk, (int)(nr * per), mesh, L, roots, t1, t2, rowmap,
+                             gk, nr * per, st);
+        (*x.ta).end(st);
+        launch_rotate_states_fp64(0, nst, 0, st_code, nw, nb, nwsq, r0, nr, arow, V, gk, nr * per, phk, B, ldb, st);
+        (*x.launches) += 4;
       }
-      (*x.launches) += 2;
+    } else {
+      for (int64_t i0 = 0; i0 < nA; i0 += kc) {
+        const int n = (int)std::min<int64_t>(kc, nA - i0);
+        launch_phase_mesh(n, arow + i0, mesh, L, nwsk, h->Rk, h->degk, 0, roots, Pk, nwsk, st);
+        (*x.ta).begin(st);
+        launch_zgemm(n, (int)Nn, nwsk, Pk, nwsk, h->G64, Nn, gk, Nn, st);
+        (*x.ta).end(st);
+        launch_rotate_states_fp64(first_state[i0], first_state[i0 + n], (int)i0, st_code, nw, nb, nwsq, 0, nper, arow, V,
+                                  gk, Nn, phk, B, ldb, st);
+        (*x.launches) += 3;
+      }
     }
     CK(cudaEventRecord(ev.e[2], st));
     // ---- stage B + C: Rp Fourier against e^{2 pi i k'.Rp}, then the epilogue ----
-    launch_phase_mesh(nwv, widx, mesh, L, nwsq, h->Rq, nullptr, 0, roots, Pq, nwsq, st);
+    if (sepB) launch_row_map(N, nwv, widx, rowmap, st);
+    else launch_phase_mesh(nwv, widx, mesh, L, nwsq, h->Rq, nullptr, 0, roots, Pq, nwsq, st);
     (*x.launches) += 1;
     for (int64_t j0 = 0; j0 < nst; j0 += sc) {
       int ns = (int)std::min<int64_t>(sc, nst - j0);
       (*x.tb).begin(st);
-      launch_zgemm(nwv, ns * ncol, nwsq, Pq, nwsq, B + j0 * ncol, ldb, Cb, (int64_t)ns * ncol, st);
+      if (sepB)
+        launch_cells_fourier(h->cellq, B + j0 * ncol, ldb, nullptr, ns * ncol, mesh, L, roots, t1, t2, rowmap, Cb,
+                             (int64_t)ns * ncol, st);
+      else
+        launch_zgemm(nwv, ns * ncol, nwsq, Pq, nwsq, B + j0 * ncol, ldb, Cb, (int64_t)ns * ncol, st);
       (*x.tb).end(st);
+      (*x.launches) += sepB ? 3 : 1;
       launch_epilogue_fp64(nwv, (int)j0, (int)j0 + ns, Cb, (int64_t)ns * ncol, rp, ed, partial, nblk, st);
-      for (int p = 1; p < nsets; ++p) {   // the same GEMM output under the other parameter sets
+      for (int p = 1; p < nsets; ++p) {   // the same sums under the other parameter sets
         EpiData ep = ed;
         ep.bose = rs.bose[p];
         launch_epilogue_fp64(nwv, (int)j0, (int)j0 + ns, Cb, (int64_t)ns * ncol, rs.rp[p], ep, rs.partial[p], nblk,
                              st);
         (*x.launches) += 1;
       }
-      (*x.launches) += 2;
+      (*x.launches) += 1;
     }
   } else {
     rc = tc::split_rates_stage(h->split, *x.ws, st, h->G64, h->nwsk, nwsq, Nn, nw, nb, nwv, nst,

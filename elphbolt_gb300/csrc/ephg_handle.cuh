@@ -27,6 +27,10 @@ struct ephg_handle {
   int hlo[3] = {0, 0, 0}, hext[3] = {1, 1, 1};
   double2 *Dbox = nullptr;   // mass-normalised D terms on the box of wrapped cell vectors [dlo, dlo + dext)
   int dlo[3] = {0, 0, 0}, dext[3] = {1, 1, 1};
+  // the cells of g's two Fourier sums as nested tables (the FP64 rate path), and 1 / deg(Re)
+  ephg::CellTab cellk, cellq;
+  int *cellk_tab = nullptr, *cellq_tab = nullptr;
+  double *rdegk = nullptr;
   double2 *graw = nullptr;   // epmatwp order (i,j,Re,s,Rp)
   double2 *G64 = nullptr;    // stage-A matrix [Re][Nn]
   double *masses = nullptr;

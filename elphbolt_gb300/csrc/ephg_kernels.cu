@@ -4,8 +4,9 @@
 // eigensolver, the FP64 complex GEMM used by the plain drop-in, and the
 // per-(k', state) epilogue that forms |g|^2, X+- and the RTA rate partials.
 // Each kernel names the reference lines it restates.
-#include <mutex>
+#include <algorithm>
 #include <cstdio>
+#include <mutex>
 
 #include "ephg_kernels.cuh"
 
@@ -103,6 +104,155 @@ void launch_mesh_fourier(const double2 *box, const int lo[3], const int ext[3], 
   // along R1: [r1][v3 v2][e] -> [v3 v2][v1][e], rows in muxed mesh order
   k_dft1<true><<<(unsigned)((n3 + 255) / 256), 256, 0, st>>>(n3, ext[0], mesh[1] * mesh[2], mesh[0], nn, lo[0],
                                                              L / mesh[0], L, roots, t2, out);
+}
+
+// ---- the same for many columns at once: the contractions of the FP64 rate path ----
+// Both contractions of the rate path are Fourier sums of cells onto mesh points
+// (stage A: g(Re,Rp) over Re for every column of g; stage B: the state operand
+// over Rp).  As matrix products against the phase matrix they are bound by the
+// FP64 pipe (1.25 TFLOP/s), so what counts is FP64 instructions: one dimension
+// at a time needs ~25x fewer of them (12^3 mesh, 279 cells: 402k complex
+// multiply-adds a column become 25k), and the symmetric range of cells halves
+// them twice more.  With s_r = x_r + x_-r and d_r = x_r - x_-r,
+//   y_v = x_0 + sum_r cos(2 pi v r / m) s_r + i sin(2 pi v r / m) d_r,
+// and y_-v has the same two sums with the second one subtracted: 4 FMA serve two
+// cells and two outputs that take 16 as complex products.
+//
+// One thread owns a column of one line (all of its outputs), so that loads and
+// stores run along the columns and the roots are shared-memory broadcasts; a
+// line's s and d sit in shared memory, [2 h + 1][128 threads].  An FP64
+// instruction of a warp holds the pipe for 16 cycles, so the ~3 shared loads
+// per 4 FMA are hidden at any occupancy of a few warps.  Measured, 12^3, nw 8, nb 6,
+// 279 cells (both contractions): 14.7 ms, 0.95 of the FP64 rate for the instructions
+// counted by cells_fourier_cost; the matrix products took 468 ms at 1.23 TFLOP/s.
+constexpr int CF_THREADS = 128;
+constexpr int CF_MAXM = 1024;                 // mesh points per dimension (shared root table)
+constexpr int CF_SMEM = 160 * 1024;
+
+struct CellDft {
+  int64_t nlines;
+  int B, m, Lm;          // lines (a, b): a = line / B, b = line % B; m outputs; root step L / m
+  int lo, ext, h;        // cell coordinates [lo, lo + ext), h = max |r|
+  const int *tab;        // [a][ext]: input row group or -1
+  int nc, ncb;           // columns, column blocks
+  const double2 *in, *roots;
+  int64_t ldi, ldo;
+  const double *scale;   // per input row group (nullable)
+  const int *rowmap;     // output row of (line, v) (nullable: line m + v)
+  double2 *out;
+};
+
+__global__ void __launch_bounds__(CF_THREADS) k_cells_dft(CellDft g) {
+  extern __shared__ double2 cfs[];
+  double2 *sr = cfs, *sx = cfs + g.m + threadIdx.x;   // sx[u * CF_THREADS]: x_0, then s_r, d_r
+  const int64_t line = blockIdx.x / g.ncb;
+  const int c = (int)(blockIdx.x % g.ncb) * CF_THREADS + threadIdx.x;
+  const int a = (int)(line / g.B), b = (int)(line % g.B);
+  for (int t = threadIdx.x; t < g.m; t += CF_THREADS) sr[t] = g.roots[(int64_t)t * g.Lm];
+  const int *tab = g.tab + (int64_t)a * g.ext;
+  const bool live = c < g.nc;
+  auto fetch = [&](int r) {
+    const int u = r - g.lo;
+    const int t = (live && u >= 0 && u < g.ext) ? tab[u] : -1;
+    if (t < 0) return make_double2(0.0, 0.0);
+    const double2 x = g.in[((int64_t)t * g.B + b) * g.ldi + c];
+    return g.scale ? cscale(x, g.scale[t]) : x;
+  };
+  const double2 x0 = fetch(0);
+#pragma unroll 2
+  for (int r = 1; r <= g.h; ++r) {
+    const double2 p = fetch(r), q = fetch(-r);
+    sx[(2 * r - 1) * CF_THREADS] = cadd(p, q);
+    sx[2 * r * CF_THREADS] = csub(p, q);
+  }
+  __syncthreads();
+  if (!live) return;
+  for (int v = 0; 2 * v <= g.m; ++v) {
+    const int w = (v == 0 || 2 * v == g.m) ? -1 : g.m - v;   // the mirrored output
+    int64_t o1 = line * g.m + v, o2 = w < 0 ? -1 : line * g.m + w;
+    if (g.rowmap) {
+      o1 = g.rowmap[o1];
+      if (o2 >= 0) o2 = g.rowmap[o2];
+      if (o1 < 0 && o2 < 0) continue;
+    }
+    double2 P = x0, Q = make_double2(0.0, 0.0);
+    int idx = 0;
+#pragma unroll 4
+    for (int r = 1; r <= g.h; ++r) {
+      idx += v;
+      if (idx >= g.m) idx -= g.m;
+      const double2 e = sr[idx], s = sx[(2 * r - 1) * CF_THREADS], d = sx[2 * r * CF_THREADS];
+      P.x = fma(e.x, s.x, P.x);
+      P.y = fma(e.x, s.y, P.y);
+      Q.x = fma(e.y, d.x, Q.x);
+      Q.y = fma(e.y, d.y, Q.y);
+    }
+    if (o1 >= 0) g.out[o1 * g.ldo + c] = make_double2(P.x - Q.y, P.y + Q.x);
+    if (o2 >= 0) g.out[o2 * g.ldo + c] = make_double2(P.x + Q.y, P.y - Q.x);
+  }
+}
+
+static int cells_h(const CellTab &t, int d) { return std::max(0, std::max(-t.lo[d], t.lo[d] + t.ext[d] - 1)); }
+
+static size_t cells_smem(const CellTab &t, int d, int m) {
+  return sizeof(double2) * ((size_t)m + (size_t)(2 * cells_h(t, d) + 1) * CF_THREADS);
+}
+
+double cells_fourier_cost(const CellTab &t, const int mesh[3], int64_t rows) {
+  if (!t.ok) return INFINITY;
+  for (int d = 0; d < 3; ++d)
+    if (mesh[d] > CF_MAXM || cells_smem(t, d, mesh[d]) > (size_t)CF_SMEM) return INFINITY;
+  auto line = [&](int d) {   // a line's instructions: 4 h + 4 per output pair, 4 h to form s and d
+    const double h = cells_h(t, d);
+    return (mesh[d] / 2 + 1) * (4 * h + 4) + 4 * h;
+  };
+  const double full = (double)mesh[0] * mesh[1] * mesh[2];
+  return t.npair * line(2) + (double)t.n1 * mesh[2] * line(1) +
+         (double)mesh[1] * mesh[2] * line(0) * std::min(1.0, 2.0 * rows / full);
+}
+
+void launch_cells_fourier(const CellTab &t, const double2 *in, int64_t ldi, const double *scale, int nc,
+                          const int mesh[3], int L, const double2 *roots, double2 *t1, double2 *t2,
+                          const int *rowmap, double2 *out, int64_t ldo, cudaStream_t st) {
+  if (nc <= 0) return;
+  static std::once_flag attr_once;   // once per process: changing a kernel attribute can wait for queued work
+  std::call_once(attr_once,
+                 [] { cudaFuncSetAttribute(k_cells_dft, cudaFuncAttributeMaxDynamicSharedMemorySize, CF_SMEM); });
+  auto pass = [&](int d, int64_t A, int B, const int *tab, const double2 *src, int64_t ls, const double *sc,
+                  const int *map, double2 *dst, int64_t ld) {
+    CellDft g;
+    g.nlines = A * B;
+    g.B = B;
+    g.m = mesh[d];
+    g.Lm = L / mesh[d];
+    g.lo = t.lo[d];
+    g.ext = t.ext[d];
+    g.h = cells_h(t, d);
+    g.tab = tab;
+    g.nc = nc;
+    g.ncb = (nc + CF_THREADS - 1) / CF_THREADS;
+    g.in = src;
+    g.roots = roots;
+    g.ldi = ls;
+    g.ldo = ld;
+    g.scale = sc;
+    g.rowmap = map;
+    g.out = dst;
+    k_cells_dft<<<(unsigned)(g.nlines * g.ncb), CF_THREADS, cells_smem(t, d, mesh[d]), st>>>(g);
+  };
+  pass(2, t.npair, 1, t.tab1, in, ldi, scale, nullptr, t1, nc);                    // [pair][v3]
+  pass(1, t.n1, mesh[2], t.tab2, t1, nc, nullptr, nullptr, t2, nc);                // [r1][v3][v2]
+  pass(0, 1, mesh[1] * mesh[2], t.tab3, t2, nc, nullptr, rowmap, out, ldo);        // [v3 v2][v1]: muxed mesh rows
+}
+
+__global__ void k_row_map(int nrows, const int *rows, int *rowmap) {
+  const int i = blockIdx.x * blockDim.x + threadIdx.x;
+  if (i < nrows) rowmap[rows[i]] = i;
+}
+
+void launch_row_map(int N, int nrows, const int *rows, int *rowmap, cudaStream_t st) {
+  cudaMemsetAsync(rowmap, 0xFF, (size_t)N * sizeof(int), st);
+  if (nrows > 0) k_row_map<<<(nrows + 255) / 256, 256, 0, st>>>(nrows, rows, rowmap);
 }
 
 // expi(twopi * dot_product(k, R)) / deg, misc.f90:588 with wannier.f90:467,1097
@@ -945,42 +1095,38 @@ void launch_iota(int n, int *out, cudaStream_t st) {
 
 // Stage A rotation over the initial band (the U_k half of wannier.f90:960-978),
 // with the k-half of the Rp phase, conj(e^{2 pi i k.Rp})/phwsdeg(Rp), folded in
-// so that the Rp Fourier of all states is one GEMM against e^{2 pi i k'.Rp}.
-__global__ void k_rotate_states_fp64(int j0, int j1, int i0, const int *st_code, int nw, int nb,
-                                     int nws, const int *widx, const double2 *U,
-                                     const double2 *gk, int64_t ldgk, int m1, int m2, int m3,
-                                     int L, const double2 *roots, const int *Rq,
-                                     const double *degq, double2 *B, int64_t ldb) {
+// so that the Rp Fourier of all states is one sum against e^{2 pi i k'.Rp}.
+// FP64-pipe bound: nw complex multiply-adds and one multiply per output, every
+// lane with an output of its own and the phases from a table (their index
+// arithmetic and FP64 divisions per output had cost as much as the rotation):
+// 12^3, nw 8, nb 6, 1,679 states: 1.34 ms (2.96 before; 1.2 at the FP64 rate).
+__global__ void __launch_bounds__(128) k_rotate_states_fp64(int j0, int i0, const int *st_code, int nw, int nb,
+                                                            int nws, int64_t blk0, int64_t nblk, const int *widx,
+                                                            const double2 *U, const double2 *gk, int64_t ldgk,
+                                                            const double2 *phk, double2 *B, int64_t ldb) {
   const int j = j0 + blockIdx.y;
-  const int rp = blockIdx.x;
-  if (j >= j1) return;
+  const int64_t o = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
+  if (o >= nblk * nw) return;
   const int code = st_code[j];
   const int i = code / nw, m = code % nw;
-  const int p = widx[i];
-  const int mesh[3] = {m1, m2, m3};
-  double2 ph = roots[phase_index(p, mesh, L, Rq[3 * rp], Rq[3 * rp + 1], Rq[3 * rp + 2])];
-  ph = make_double2(ph.x / degq[rp], -ph.y / degq[rp]);
-  const double2 *Uk = U + ((size_t)p * nw + m) * nw;
-  const double2 *g = gk + (int64_t)(i - i0) * ldgk;
-  const int ncol = nw * nb;
-  for (int c = threadIdx.x; c < ncol; c += blockDim.x) {
-    int np = c % nw, s = c / nw;
-    double2 acc = make_double2(0.0, 0.0);
-    for (int mp = 0; mp < nw; ++mp)
-      cfma(acc, Uk[mp], g[np + nw * (mp + (int64_t)nw * (s + (int64_t)nb * rp))]);
-    B[(int64_t)rp * ldb + (int64_t)(j - j0) * ncol + c] = cmul(ph, acc);
-  }
+  const int64_t u = o / nw;
+  const int np = (int)(o - u * nw);
+  const int rp = (int)((blk0 + u) / nb), s = (int)((blk0 + u) % nb);
+  const double2 *Uk = U + ((size_t)widx[i] * nw + m) * nw;
+  const double2 *g = gk + (int64_t)(i - i0) * ldgk + np + (int64_t)nw * nw * u;
+  double2 acc = make_double2(0.0, 0.0);
+  for (int mp = 0; mp < nw; ++mp) cfma(acc, Uk[mp], g[nw * mp]);
+  B[(int64_t)rp * ldb + (int64_t)j * nw * nb + np + nw * s] = cmul(phk[(int64_t)i * nws + rp], acc);
 }
 
-void launch_rotate_states_fp64(int j0, int j1, int i0, const int *st_code, int nw, int nb,
-                               int nws, const int *widx, const double2 *U, const double2 *gk,
-                               int64_t ldgk, const int mesh[3], int L, const double2 *roots,
-                               const int *Rq, const double *degq, double2 *B, int64_t ldb,
-                               cudaStream_t st) {
-  if (j1 <= j0) return;
-  dim3 grid(nws, j1 - j0);
-  k_rotate_states_fp64<<<grid, 64, 0, st>>>(j0, j1, i0, st_code, nw, nb, nws, widx, U, gk, ldgk,
-                                            mesh[0], mesh[1], mesh[2], L, roots, Rq, degq, B, ldb);
+void launch_rotate_states_fp64(int j0, int j1, int i0, const int *st_code, int nw, int nb, int nws, int64_t blk0,
+                               int64_t nblk, const int *widx, const double2 *U, const double2 *gk, int64_t ldgk,
+                               const double2 *phk, double2 *B, int64_t ldb, cudaStream_t st) {
+  for (; j0 < j1; j0 += 32768) {   // grid.y
+    dim3 grid((unsigned)((nblk * nw + 127) / 128), std::min(j1 - j0, 32768));
+    k_rotate_states_fp64<<<grid, 128, 0, st>>>(j0, i0, st_code, nw, nb, nws, blk0, nblk, widx, U, gk, ldgk, phk, B,
+                                               ldb);
+  }
 }
 
 __global__ void k_bose(int n, const double *om, double T, double *bose) {

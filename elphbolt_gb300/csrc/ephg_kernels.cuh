@@ -22,6 +22,29 @@ void launch_phase_frac(int nrows, const double *kv, int nR, const int *R, const 
 void launch_mesh_fourier(const double2 *box, const int lo[3], const int ext[3], int nn, const int mesh[3], int L,
                          const double2 *roots, double2 *t1, double2 *t2, double2 *out, cudaStream_t st);
 
+// ---- Fourier sum of many columns over integer cells, one dimension at a time ----
+// The cells of a Wigner-Seitz set as nested index tables (device): tab1 [npair][ext3]
+// the cell of (R1, R2 of the pair, R3) or -1; tab2 [n1][ext2] the pair of (R1, R2)
+// or -1; tab3 [ext1] the R1 slot or -1.  ok: every cell is distinct and the tables fit.
+struct CellTab {
+  bool ok = false;
+  int lo[3] = {0, 0, 0}, ext[3] = {1, 1, 1};
+  int npair = 0, n1 = 0;
+  const int *tab1 = nullptr, *tab2 = nullptr, *tab3 = nullptr;
+};
+// FP64 operations per column of launch_cells_fourier, in multiply-adds; infinity where it cannot run
+double cells_fourier_cost(const CellTab &t, const int mesh[3], int64_t rows);
+// work rows (double2 per column) of t1 and t2
+inline int64_t cells_t1_rows(const CellTab &t, const int mesh[3]) { return (int64_t)t.npair * mesh[2]; }
+inline int64_t cells_t2_rows(const CellTab &t, const int mesh[3]) { return (int64_t)t.n1 * mesh[1] * mesh[2]; }
+// out[rowmap[p]][c] = sum_cells e^{2 pi i k_p.R} scale[cell] in[cell][c], c < nc, for the mesh
+// points p with rowmap[p] >= 0; in rows at stride ldi, out rows at stride ldo; scale nullable.
+void launch_cells_fourier(const CellTab &t, const double2 *in, int64_t ldi, const double *scale, int nc,
+                          const int mesh[3], int L, const double2 *roots, double2 *t1, double2 *t2,
+                          const int *rowmap, double2 *out, int64_t ldo, cudaStream_t st);
+// rowmap[p] = i for p = rows[i], -1 elsewhere (N mesh points)
+void launch_row_map(int N, int nrows, const int *rows, int *rowmap, cudaStream_t st);
+
 // ---- FP64 complex GEMM: C[M][N] = A[M][K] * B[K][N], row-major ----
 void launch_zgemm(int M, int N, int K, const double2 *A, int64_t lda, const double2 *B,
                   int64_t ldb, double2 *C, int64_t ldc, cudaStream_t st);
@@ -118,13 +141,12 @@ void launch_window_flags(int N, int nw, const double *ens, double enref, double 
 void launch_state_flags(int nwv, int nw, const int *widx, const double *ens, double enref,
                         double fsthick, int *flag, int *nin_k, cudaStream_t st);
 void launch_iota(int n, int *out, cudaStream_t st);
-// Stage A rotation: B[Rp][c] (ldb) for states j in [j0,j1) of k-chunk [i0, i0+kc):
-// B = conj(e^{2 pi i k.Rp})/deg(Rp) * sum_m' U_k[m][m'] gk(n',m',s',Rp)
-void launch_rotate_states_fp64(int j0, int j1, int i0, const int *st_code, int nw, int nb,
-                               int nws, const int *widx, const double2 *U, const double2 *gk,
-                               int64_t ldgk, const int mesh[3], int L, const double2 *roots,
-                               const int *Rq, const double *degq, double2 *B, int64_t ldb,
-                               cudaStream_t st);
+// Stage A rotation: B[Rp][c] (ldb) for states j in [j0,j1) of k-chunk [i0, i0+kc) and the
+// (mode, cell) blocks s + nb Rp in [blk0, blk0 + nblk) that gk holds (nw nw values each):
+// B = phk[k][Rp] * sum_m' U_k[m][m'] gk(n',m',s',Rp), phk = conj(e^{2 pi i k.Rp})/deg(Rp) (row stride nws)
+void launch_rotate_states_fp64(int j0, int j1, int i0, const int *st_code, int nw, int nb, int nws, int64_t blk0,
+                               int64_t nblk, const int *widx, const double2 *U, const double2 *gk, int64_t ldgk,
+                               const double2 *phk, double2 *B, int64_t ldb, cudaStream_t st);
 struct EpiData {
   const int *widx;      // window (k' row) -> mesh index
   const int *st_code;   // state -> i*nw + m, i the state's k row (an A-row)
