@@ -901,62 +901,6 @@ int ephg_kq_index(ephg_handle *h, const int64_t mesh[3], int64_t nk, const int64
 // ------------------------------------------------------------- rates
 namespace {
 
-// form_triangles / form_tetrahedra_3d + fill (delta.f90:494-646,648-788) on the
-// host: integer set-up of the simplices of the window mesh, uploaded once per
-// request.  Output layouts: map (nwv, maxc, 2), count (nwv), evals (ns, nw, nv).
-void build_simplices(int kind, const int mesh[3], const std::vector<int> &widx,
-                     const std::vector<double> &ens_w, int nw, std::vector<int> &map,
-                     std::vector<int> &count, std::vector<double> &sev, int &nsimplex, int &maxc,
-                     int &nv) {
-  const int nk = (int)widx.size();
-  const int per = kind == 1 ? 2 : 6;
-  nv = kind == 1 ? 3 : 4;
-  maxc = kind == 1 ? 6 : 24;
-  nsimplex = per * nk;
-  static const int tri[2][3] = {{1, 2, 3}, {1, 3, 4}};
-  static const int tet[6][4] = {{1, 2, 3, 6}, {1, 3, 5, 6}, {3, 5, 6, 7}, {3, 6, 7, 8}, {3, 4, 6, 8}, {2, 3, 4, 6}};
-  std::vector<int> simplex((size_t)nsimplex * nv, 0);
-  map.assign((size_t)nk * maxc * 2, 0);
-  count.assign(nk, 0);
-  // widx is sorted ascending (0-based mesh index) = indexlist - 1
-  auto find = [&](int mux1) -> int {   // binsearch (misc.f90:738), 1-based or -1
-    auto it = std::lower_bound(widx.begin(), widx.end(), mux1 - 1);
-    if (it != widx.end() && *it == mux1 - 1) return (int)(it - widx.begin()) + 1;
-    return -1;
-  };
-  int cnt = 1;
-  for (int ik = 0; ik < nk; ++ik) {
-    int p = widx[ik];
-    int i = p % mesh[0] + 1, j = (p / mesh[0]) % mesh[1] + 1, k = p / (mesh[0] * mesh[1]) + 1;
-    int ip1 = i == mesh[0] ? 1 : i + 1, jp1 = j == mesh[1] ? 1 : j + 1, kp1 = k == mesh[2] ? 1 : k + 1;
-    int sc[8][3] = {{i, j, k}, {ip1, j, k}, {i, jp1, k}, {ip1, jp1, k},
-                    {i, j, kp1}, {ip1, j, kp1}, {i, jp1, kp1}, {ip1, jp1, kp1}};
-    for (int tk = 0; tk < per; ++tk) {
-      for (int tl = 0; tl < nv; ++tl) {
-        int a = (kind == 1 ? tri[tk][tl] : tet[tk][tl]) - 1;
-        int mux = ((sc[a][2] - 1) * mesh[1] + (sc[a][1] - 1)) * mesh[0] + sc[a][0];
-        int tmp = find(mux);
-        simplex[(size_t)(cnt - 1) * nv + tl] = tmp;
-        if (tmp > 0) {
-          int c = ++count[tmp - 1];
-          map[((size_t)(tmp - 1) * maxc + (c - 1)) * 2] = cnt;
-          map[((size_t)(tmp - 1) * maxc + (c - 1)) * 2 + 1] = tl + 1;
-        }
-      }
-      cnt++;
-    }
-  }
-  sev.assign((size_t)nsimplex * nw * nv, 0.0);
-  for (int it = 0; it < nsimplex; ++it) {
-    for (int iv = 0; iv < nv; ++iv) {
-      int aux = simplex[(size_t)it * nv + iv];
-      if (aux > 0)
-        for (int ib = 0; ib < nw; ++ib) sev[((size_t)it * nw + ib) * nv + iv] = ens_w[(size_t)(aux - 1) * nw + ib];
-    }
-    for (int ib = 0; ib < nw; ++ib) std::sort(&sev[((size_t)it * nw + ib) * nv], &sev[((size_t)it * nw + ib) * nv] + nv);
-  }
-}
-
 struct EvTimer {
   cudaEvent_t e[6];
   EvTimer() { for (auto &x : e) cudaEventCreate(&x); }
@@ -1153,25 +1097,18 @@ int ephg::el_rates_view(ephg_handle *h, const ExecView &x, const ephg_rate_reque
   // blocks, electron.f90:553-577), in window order ----
   int nA = nwv;
   const int *arow = widx;
-  int *awin = nullptr;
   std::vector<int> arow_h;
   if (ibz) {
     std::vector<int> rep_h(N);
     CK(cudaMemcpyAsync(rep_h.data(), rep, (size_t)N * sizeof(int), cudaMemcpyDeviceToHost, st));
     CK(cudaStreamSynchronize(st));
-    std::vector<int> awin_h;
     for (int i = 0; i < nwv; ++i)
-      if (rep_h[widx_h[i]] == widx_h[i]) {
-        awin_h.push_back(i);
-        arow_h.push_back(widx_h[i]);
-      }
+      if (rep_h[widx_h[i]] == widx_h[i]) arow_h.push_back(widx_h[i]);
     nA = (int)arow_h.size();
     int *arow_d, *ninA;
-    if ((rc = wsget((*x.ws), "r_arow", (size_t)nA, &arow_d)) || (rc = wsget((*x.ws), "r_awin", (size_t)nA, &awin)) ||
-        (rc = wsget((*x.ws), "r_ninA", (size_t)nA, &ninA)))
+    if ((rc = wsget((*x.ws), "r_arow", (size_t)nA, &arow_d)) || (rc = wsget((*x.ws), "r_ninA", (size_t)nA, &ninA)))
       return WSFAILX(rc);
     CK(cudaMemcpyAsync(arow_d, arow_h.data(), (size_t)nA * sizeof(int), cudaMemcpyHostToDevice, st));
-    CK(cudaMemcpyAsync(awin, awin_h.data(), (size_t)nA * sizeof(int), cudaMemcpyHostToDevice, st));
     arow = arow_d;
     launch_state_flags(nA, nw, arow, ens, req->enref, req->fsthick, sflag, ninA, st);
   }
@@ -1188,34 +1125,8 @@ int ephg::el_rates_view(ephg_handle *h, const ExecView &x, const ephg_rate_reque
   if (!ibz) arow_h = widx_h;
   code_h.resize(nst);
   CK(cudaMemcpyAsync(code_h.data(), st_code, nst * sizeof(int), cudaMemcpyDeviceToHost, st));
-  // simplices for triangle / tetrahedron deltas
   EpiData ed;
   memset(&ed, 0, sizeof ed);
-  if (req->delta_kind != 0) {
-    std::vector<double> ens_all((size_t)N * nw), ens_w((size_t)nwv * nw);
-    CK(cudaMemcpyAsync(ens_all.data(), ens, (size_t)N * nw * sizeof(double), cudaMemcpyDeviceToHost, st));
-    CK(cudaStreamSynchronize(st));
-    for (int i = 0; i < nwv; ++i)
-      for (int b = 0; b < nw; ++b) ens_w[(size_t)i * nw + b] = ens_all[(size_t)widx_h[i] * nw + b];
-    std::vector<int> map, count;
-    std::vector<double> sev;
-    int ns, maxc, nvx;
-    build_simplices((int)req->delta_kind, mesh, widx_h, ens_w, nw, map, count, sev, ns, maxc, nvx);
-    int *dmap, *dcount;
-    double *dsev;
-    if ((rc = wsget((*x.ws), "r_smap", map.size(), &dmap)) || (rc = wsget((*x.ws), "r_scount", count.size(), &dcount)) ||
-        (rc = wsget((*x.ws), "r_sev", sev.size(), &dsev)))
-      return WSFAILX(rc);
-    CK(cudaMemcpyAsync(dmap, map.data(), map.size() * sizeof(int), cudaMemcpyHostToDevice, st));
-    CK(cudaMemcpyAsync(dcount, count.data(), count.size() * sizeof(int), cudaMemcpyHostToDevice, st));
-    CK(cudaMemcpyAsync(dsev, sev.data(), sev.size() * sizeof(double), cudaMemcpyHostToDevice, st));
-    ed.smap = dmap;
-    ed.scount = dcount;
-    ed.sevals = dsev;
-    ed.nsimplex = ns;
-    ed.maxc = maxc;
-    ed.nvx = nvx;
-  }
   CK(cudaStreamSynchronize(st));
   std::vector<int> first_state(nA + 1, nst);
   for (int j = nst - 1; j >= 0; --j) first_state[code_h[j] / nw] = j;
@@ -1272,7 +1183,6 @@ int ephg::el_rates_view(ephg_handle *h, const ExecView &x, const ephg_rate_reque
   rp.const_tp = 2.0 * 3.141592653589793 / hbar_eVps;
   ed.widx = widx;
   ed.sidx = arow;
-  ed.swin = awin;
   ed.st_code = st_code;
   ed.cum = cum;
   ed.ens = ens;
@@ -1307,8 +1217,39 @@ int ephg::el_rates_view(ephg_handle *h, const ExecView &x, const ephg_rate_reque
     ed.phr = phr;
     ed.ph_scale = ph->spindeg;
   }
-  int nblk = (nwv + 127) / 128;                 // k'-row blocks of the rate partials
-  const int nblk_max = std::max((nwv + 15) / 16, (nwv + 255) / 256 * 8);
+  // FP64 epilogues (the FP64 form; the simplex deltas of both): final states, mode
+  // tables of every parameter set and the deltas' tables
+  if (!split || req->delta_kind != 0) {
+    int2 *fin;
+    if ((rc = wsget((*x.ws), "e_fin", (size_t)nin, &fin))) return WSFAILX(rc);
+    launch_final_states(nwv, nw, widx, ens, req->enref, req->fsthick, cum, fin, st);
+    for (int p = 0; p < nsets; ++p) {
+      double4 *mt;
+      if ((rc = wsget((*x.ws), ("e_mt" + std::to_string(p)).c_str(), (size_t)N * nb, &mt))) return WSFAILX(rc);
+      launch_mode_tab(N * nb, om, p ? rs.bose[p] : bose, p ? sets->reqs[p].T : req->T, rp.const_tp, mt, st);
+      rs.mt[p] = mt;
+    }
+    ed.fin = fin;
+    ed.nin = nin;
+    ed.mt = rs.mt[0];
+    (*x.launches) += 1 + nsets;
+    if (req->delta_kind != 0) {
+      SimplexTab &t = ed.sx;
+      int *map;
+      t.stride = req->delta_kind == 1 ? 18 : SX_MAX;
+      const size_t ne = (size_t)nin * t.stride;
+      if ((rc = wsget((*x.ws), "e_sxn", (size_t)nin, &t.n)) || (rc = wsget((*x.ws), "e_sxk", ne, &t.key)) ||
+          (rc = wsget((*x.ws), "e_sxb", ne, &t.b)) || (rc = wsget((*x.ws), "e_sxl", ne, &t.lo)) ||
+          (rc = wsget((*x.ws), "e_sxh", ne, &t.hi)) || (rc = wsget((*x.ws), "a_map", (size_t)N, &map)))
+        return WSFAILX(rc);
+      launch_row_map(N, nwv, widx, map, st);
+      launch_simplex_tab((int)req->delta_kind, mesh, nin, fin, widx, map, ens, nw, t, st);
+      (*x.launches) += 2;
+    }
+    CKL();
+  }
+  int nblk = epf_blocks(nin);                   // blocks of the rate partials
+  const int nblk_max = std::max(nblk, (nwv + 255) / 256 * 8);
   double *partial;
   if ((rc = wsget((*x.ws), "r_partial", (size_t)nst * nblk_max, &partial))) return WSFAILX(rc);
   rs.rp[0] = rp;
@@ -1362,7 +1303,8 @@ int ephg::el_rates_view(ephg_handle *h, const ExecView &x, const ephg_rate_reque
         launch_cells_fourier(h->cellk, h->G64 + r0 * per, Nn, h->rdegk, (int)(nr * per), mesh, L, roots, t1, t2, rowmap,
                              gk, nr * per, st);
         (*x.ta).end(st);
-        launch_rotate_states_fp64(0, nst, 0, st_code, nw, nb, nwsq, r0, nr, arow, V, gk, nr * per, phk, B, ldb, st);
+        launch_rotate_states_fp64(0, nst, 0, st_code, nw, nb, nwsq, r0, nr, arow, V, gk, nr * per, phk, B, ldb,
+                                  (int)sc, nst, st);
         (*x.launches) += 4;
       }
     } else {
@@ -1373,7 +1315,7 @@ int ephg::el_rates_view(ephg_handle *h, const ExecView &x, const ephg_rate_reque
         launch_zgemm(n, (int)Nn, nwsk, Pk, nwsk, h->G64, Nn, gk, Nn, st);
         (*x.ta).end(st);
         launch_rotate_states_fp64(first_state[i0], first_state[i0 + n], (int)i0, st_code, nw, nb, nwsq, 0, nper, arow, V,
-                                  gk, Nn, phk, B, ldb, st);
+                                  gk, Nn, phk, B, ldb, (int)sc, nst, st);
         (*x.launches) += 3;
       }
     }
@@ -1392,12 +1334,17 @@ int ephg::el_rates_view(ephg_handle *h, const ExecView &x, const ephg_rate_reque
         launch_zgemm(nwv, ns * ncol, nwsq, Pq, nwsq, B + j0 * ncol, ldb, Cb, (int64_t)ns * ncol, st);
       (*x.tb).end(st);
       (*x.launches) += sepB ? 3 : 1;
-      launch_epilogue_fp64(nwv, (int)j0, (int)j0 + ns, Cb, (int64_t)ns * ncol, rp, ed, partial, nblk, st);
+      FinalIn in;
+      in.z = Cb;
+      in.ldc = (int64_t)ns * ncol;
+      in.xs = ns;
+      in.js = 1;
+      launch_epilogue_final((int)j0, (int)j0 + ns, in, rp, ed, partial, nblk, st);
       for (int p = 1; p < nsets; ++p) {   // the same sums under the other parameter sets
         EpiData ep = ed;
         ep.bose = rs.bose[p];
-        launch_epilogue_fp64(nwv, (int)j0, (int)j0 + ns, Cb, (int64_t)ns * ncol, rs.rp[p], ep, rs.partial[p], nblk,
-                             st);
+        ep.mt = rs.mt[p];
+        launch_epilogue_final((int)j0, (int)j0 + ns, in, rs.rp[p], ep, rs.partial[p], nblk, st);
         (*x.launches) += 1;
       }
       (*x.launches) += 1;

@@ -1096,36 +1096,77 @@ void launch_iota(int n, int *out, cudaStream_t st) {
 // Stage A rotation over the initial band (the U_k half of wannier.f90:960-978),
 // with the k-half of the Rp phase, conj(e^{2 pi i k.Rp})/phwsdeg(Rp), folded in
 // so that the Rp Fourier of all states is one sum against e^{2 pi i k'.Rp}.
-// FP64-pipe bound: nw complex multiply-adds and one multiply per output, every
-// lane with an output of its own and the phases from a table (their index
-// arithmetic and FP64 divisions per output had cost as much as the rotation):
-// 12^3, nw 8, nb 6, 1,679 states: 1.34 ms (2.96 before; 1.2 at the FP64 rate).
-__global__ void __launch_bounds__(128) k_rotate_states_fp64(int j0, int i0, const int *st_code, int nw, int nb,
-                                                            int nws, int64_t blk0, int64_t nblk, const int *widx,
-                                                            const double2 *U, const double2 *gk, int64_t ldgk,
-                                                            const double2 *phk, double2 *B, int64_t ldb) {
-  const int j = j0 + blockIdx.y;
-  const int64_t o = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
-  if (o >= nblk * nw) return;
-  const int code = st_code[j];
-  const int i = code / nw, m = code % nw;
-  const int64_t u = o / nw;
-  const int np = (int)(o - u * nw);
+// FP64-pipe bound: nw complex multiply-adds and one multiply per output, the
+// phases from a table.  Lanes are states, so that the stores run along the states
+// (the epilogue's lanes); each warp stages its states' nw x nw blocks through
+// shared memory in whole rows, ROT64_V values of each state at a time.
+// 12^3, nw 8, nb 6, 279 cells, 1,679 states: 1.74 ms (1.1 at the FP64 rate; 2.96 with
+// per-output phase arithmetic, 2.63 with each lane reading its own block).
+constexpr int ROT64_THREADS = 64, ROT64_V = 32;
+
+// NW: bands fixed at compile time (the sums then stay in registers), or 0
+template <int NW>
+__global__ void __launch_bounds__(ROT64_THREADS) k_rotate_states_fp64(int j0, int j1, int i0, const int *st_code,
+                                                                      int nw_, int nb, int nws, int64_t blk0,
+                                                                      const int *widx,
+                                                                      const double2 *U, const double2 *gk,
+                                                                      int64_t ldgk, const double2 *phk, double2 *B,
+                                                                      int64_t ldb, int sc, int nst) {
+  __shared__ double2 sg[ROT64_THREADS * (ROT64_V + 1)];
+  constexpr int AW = NW ? NW : 32;
+  const int nw = NW ? NW : nw_;
+  const int lane = threadIdx.x & 31, wj = j0 + blockIdx.x * ROT64_THREADS + (threadIdx.x & ~31);
+  const int j = wj + lane;
+  const bool live = j < j1;
+  const int code = live ? st_code[j] : 0;
+  const int i = live ? code / nw : i0, m = code % nw;
+  const int64_t u = blockIdx.y;
   const int rp = (int)((blk0 + u) / nb), s = (int)((blk0 + u) % nb);
   const double2 *Uk = U + ((size_t)widx[i] * nw + m) * nw;
-  const double2 *g = gk + (int64_t)(i - i0) * ldgk + np + (int64_t)nw * nw * u;
-  double2 acc = make_double2(0.0, 0.0);
-  for (int mp = 0; mp < nw; ++mp) cfma(acc, Uk[mp], g[nw * mp]);
-  B[(int64_t)rp * ldb + (int64_t)j * nw * nb + np + nw * s] = cmul(phk[(int64_t)i * nws + rp], acc);
+  const double2 *g = gk + (int64_t)nw * nw * u;
+  double2 *tile = sg + (threadIdx.x & ~31) * (ROT64_V + 1);
+  const int mpc = ROT64_V / nw, nv = min(32, j1 - wj);   // initial bands per pass; the warp's states
+  double2 acc[AW];
+#pragma unroll
+  for (int np = 0; np < AW; ++np) acc[np] = make_double2(0.0, 0.0);
+  for (int mp0 = 0; mp0 < nw; mp0 += mpc) {
+    const int nm = min(mpc, nw - mp0), n = nw * nm;
+    __syncwarp();
+    for (int t = 0; t < nv; ++t) {   // state t's values, contiguous in gk
+      const double2 *src = g + (int64_t)(__shfl_sync(0xffffffffu, i, t) - i0) * ldgk + nw * mp0;
+      for (int v = lane; v < n; v += 32) tile[t * (ROT64_V + 1) + v] = src[v];
+    }
+    __syncwarp();
+    if (live)
+      for (int mp = 0; mp < nm; ++mp) {
+        const double2 um = Uk[mp0 + mp], *row = tile + lane * (ROT64_V + 1) + nw * mp;
+#pragma unroll
+        for (int np = 0; np < AW; ++np)
+          if (np < nw) cfma(acc[np], um, row[np]);
+      }
+  }
+  if (!live) return;
+  const double2 ph = phk[(int64_t)i * nws + rp];
+  // columns of a chunk of sc states: [n' + nw s'][state]
+  const int jc = j / sc * sc, ns = min(sc, nst - jc);
+  double2 *out = B + (int64_t)rp * ldb + (int64_t)jc * nw * nb + (int64_t)nw * s * ns + (j - jc);
+#pragma unroll
+  for (int np = 0; np < AW; ++np)
+    if (np < nw) out[(int64_t)np * ns] = cmul(ph, acc[np]);
 }
 
 void launch_rotate_states_fp64(int j0, int j1, int i0, const int *st_code, int nw, int nb, int nws, int64_t blk0,
                                int64_t nblk, const int *widx, const double2 *U, const double2 *gk, int64_t ldgk,
-                               const double2 *phk, double2 *B, int64_t ldb, cudaStream_t st) {
-  for (; j0 < j1; j0 += 32768) {   // grid.y
-    dim3 grid((unsigned)((nblk * nw + 127) / 128), std::min(j1 - j0, 32768));
-    k_rotate_states_fp64<<<grid, 128, 0, st>>>(j0, i0, st_code, nw, nb, nws, blk0, nblk, widx, U, gk, ldgk, phk, B,
-                                               ldb);
+                               const double2 *phk, double2 *B, int64_t ldb, int sc, int nst, cudaStream_t st) {
+  if (j1 <= j0) return;
+  for (int64_t b = 0; b < nblk; b += 32768) {   // grid.y
+    dim3 grid((j1 - j0 + ROT64_THREADS - 1) / ROT64_THREADS, (unsigned)std::min<int64_t>(nblk - b, 32768));
+    auto go = [&](auto k) {
+      k<<<grid, ROT64_THREADS, 0, st>>>(j0, j1, i0, st_code, nw, nb, nws, blk0 + b, widx, U, gk + b * nw * nw, ldgk, phk,
+                                        B, ldb, sc, nst);
+    };
+    nw == 4 ? go(k_rotate_states_fp64<4>) : nw == 8 ? go(k_rotate_states_fp64<8>)
+    : nw == 16 ? go(k_rotate_states_fp64<16>) : go(k_rotate_states_fp64<0>);
   }
 }
 
@@ -1142,238 +1183,405 @@ void launch_bose(int N, int nb, const double *om, double T, double *bose, cudaSt
   k_bose<<<(n + 255) / 256, 256, 0, st>>>(n, om, T, bose);
 }
 
-// ----------------------------------------------------------- deltas
-__device__ inline double fermi(double e, double mu, double T) {
-  return 1.0 / (exp((e - mu) / kB / T) + 1.0);     // misc.f90:1001-1009
-}
+// ------------------------------------------------- simplex deltas as tables
+// The triangle and tetrahedron deltas (delta.f90:790-881, 61-225) of one final
+// state (k', n) are functions of the energy alone: over the up to 24 tetrahedra
+// (6 triangles) that share the corner k', each contributes a product of linear
+// factors between its sorted vertex energies.  Between consecutive vertex
+// energies of all of them the sum is one cubic, so a table of (breakpoint,
+// cubic) replaces 24 range tests and formulas with five to seven FP64 divisions
+// each: an evaluation is a binary search and ten FP64 operations.
+//
+// The cubic of (b_i-1, b_i] is kept in Bernstein form, coefficients over
+// (e - b_i-1) and (b_i - e): they are the formulas' blossoms, sums of products
+// of factors of one sign, so the tails keep their relative accuracy, as in the
+// formulas themselves.  Vertex energies of corners outside the window are zero,
+// as the reference leaves them (delta.f90:494-646); equal energies give
+// intervals of no width, which are never looked up, so the formulas' special
+// cases for them need no counterpart.
+struct SimplexEntry {
+  double e[4];      // sorted vertex energies
+  double c1[4];     // first range: x_1 x_1 (or x_1) times sum_i c1_i x_i, x_i = e_i - e
+  double c3[4];     // last range: the same with the last vertex
+  double m[5];      // middle range of a tetrahedron: S^2 (m0 a + m1 b) + Q^2 (m2 b + m3 a) + m4 x_label S Q
+  int label;        // 0-based vertex label; -1: no simplex (its cell is outside the window)
+};
 
-// delta_fn_triang, delta.f90:790-881 (ik 0-based window index, ib 0-based)
-__device__ double delta_triang(double e, int ik, int ib, const RateParams &rp, const EpiData &d) {
-  double acc = 0.0;
-  int num = d.scount[ik];
-  for (int itk = 0; itk < num; ++itk) {
-    int it = d.smap[((size_t)ik * d.maxc + itk) * 2] - 1;
-    int iv = d.smap[((size_t)ik * d.maxc + itk) * 2 + 1];
-    const double *ev = d.sevals + (((size_t)it * rp.nw + ib) * 3);
-    double e1 = ev[0], e2 = ev[1], e3 = ev[2];
-    bool c1 = e <= e1, c2 = e1 < e && e <= e2, c3 = e2 < e && e <= e3, c4 = e3 < e;
-    if (c1 || c4) continue;
-    double E12 = (e - e2) / (e1 - e2), E21 = (e - e1) / (e2 - e1), E13 = (e - e3) / (e1 - e3);
-    double E31 = (e - e1) / (e3 - e1), E23 = (e - e3) / (e2 - e3), E32 = (e - e2) / (e3 - e2);
-    double tmp = 0.0;
-    if (iv == 1) tmp = c2 ? E21 * (E12 + E13) / (e3 - e1) : (c3 ? E23 * E13 / (e3 - e1) : 0.0);
-    else if (iv == 2) tmp = c2 ? E21 * E21 / (e3 - e1) : (c3 ? E23 * E23 / (e3 - e1) : 0.0);
-    else if (iv == 3) tmp = c2 ? E21 * E31 / (e3 - e1) : (c3 ? E23 * (E31 + E32) / (e3 - e1) : 0.0);
-    acc += tmp;
-  }
-  if (acc < 1.0e-12) acc = 0.0;
-  return acc / (double)(2 * (int64_t)rp.N);
-}
+// corners of a mesh cell used by the simplices, and the simplices as corner lists (delta.f90)
+__constant__ int kTri[2][3] = {{1, 2, 3}, {1, 3, 4}};
+__constant__ int kTet[6][4] = {{1, 2, 3, 6}, {1, 3, 5, 6}, {3, 5, 6, 7}, {3, 6, 7, 8}, {3, 4, 6, 8}, {2, 3, 4, 6}};
 
-// delta_fn_tetra, delta.f90:61-225
-__device__ double delta_tetra(double e, int ik, int ib, const RateParams &rp, const EpiData &d) {
-  double acc = 0.0, tmp = 0.0;
-  int num = d.scount[ik];
-  for (int itk = 0; itk < num; ++itk) {
-    int it = d.smap[((size_t)ik * d.maxc + itk) * 2] - 1;
-    int iv = d.smap[((size_t)ik * d.maxc + itk) * 2 + 1];
-    const double *ev = d.sevals + (((size_t)it * rp.nw + ib) * 4);
-    double e1 = ev[0], e2 = ev[1], e3 = ev[2], e4 = ev[3];
-    double e1e = e1 - e, e2e = e2 - e, e3e = e3 - e, e4e = e4 - e;
-    double e21 = e2 - e1, e31 = e3 - e1, e41 = e4 - e1, e32 = e3 - e2, e42 = e4 - e2, e43 = e4 - e3;
-    bool c1 = e1 <= e && e <= e2, c2 = e2 <= e && e <= e3, c3 = e3 <= e && e <= e4;
-    if (e < e1 || e > e4) continue;
-    switch (iv) {
-      case 1:
-        if (c1) { tmp = (e2e / e21 + e3e / e31 + e4e / e41) * (e1e * e1e) / e41 / e31 / e21; if (e1 == e2) tmp = 0.0; }
-        else if (c2) {
-          tmp = -0.5 * (e3e / (e31 * e31) * (e3e * e2e / e42 / e32 + e4e * e1e / e41 / e42 + e3e * e1e / e32 / e41) +
-                        e4e / (e41 * e41) * (e4e * e1e / e42 / e31 + e4e * e2e / e42 / e32 + e3e * e1e / e31 / e32));
-          if (e2 == e3) tmp = -0.5 * (e4e * e1e / e41 / e42 + e1e / e41 + e4e / (e41 * e41) * (e4e * e1e / e42 / e31 + e4e / e42 + e1e / e31));
-        } else if (c3) { tmp = (e4e * e4e * e4e) / (e41 * e41) / e42 / e43; if (e3 == e4) tmp = (e4e * e4e) / (e41 * e41) / e42; }
-        break;
-      case 2:
-        if (c1) { tmp = -(e1e * e1e * e1e) / (e21 * e21) / e31 / e41; if (e1 == e2) tmp = 0.0; }
-        else if (c2) {
-          tmp = -0.5 * (e3e / (e32 * e32) * (e3e * e2e / e42 / e31 + e4e * e2e / e42 / e41 + e3e * e1e / e31 / e41) +
-                        e4e / (e42 * e42) * (e3e * e2e / e32 / e31 + e4e * e1e / e41 / e31 + e4e * e2e / e32 / e41));
-          if (e2 == e3) tmp = -0.5 * (0.0 + e4e / e42 / e41 + 0.0 + e4e / (e42 * e42) * (0.0 + e4e * e1e / e41 / e31 + 1.0));
-        } else if (c3) { tmp = (e4e * e4e * e4e) / e41 / (e42 * e42) / e43; if (e3 == e4) tmp = 0.0; }
-        break;
-      case 3:
-        if (c1) { tmp = -(e1e * e1e * e1e) / e21 / (e31 * e31) / e41; if (e1 == e2) tmp = 0.0; }
-        else if (c2) {
-          tmp = 0.5 * (e2e / (e32 * e32) * (e3e * e2e / e42 / e31 + e4e * e2e / e42 / e41 + e3e * e1e / e31 / e41) +
-                       e1e / (e31 * e31) * (e3e * e2e / e42 / e32 + e4e * e1e / e41 / e42 + e3e * e1e / e32 / e41));
-          if (e2 == e3) tmp = 0.5 * (0.0 + e4e / e42 / e41 + e1e / e31 / e41 + e1e / (e31 * e31) * (0.0 + e4e * e1e / e41 / e42 + e1e / e41));
-        } else if (c3) { tmp = (e4e * e4e * e4e) / e41 / e42 / (e43 * e43); if (e3 == e4) tmp = 0.0; }
-        break;
-      case 4:
-        if (c1) { tmp = -(e1e * e1e * e1e) / e21 / e31 / (e41 * e41); if (e1 == e2) tmp = 0.0; }
-        else if (c2) {
-          tmp = 0.5 * (e2e / (e42 * e42) * (e3e * e2e / e32 / e31 + e4e * e1e / e41 / e31 + e4e * e2e / e32 / e41) +
-                       e1e / (e41 * e41) * (e4e * e1e / e42 / e31 + e4e * e2e / e42 / e32 + e3e * e1e / e31 / e32));
-          if (e2 == e3) tmp = 0.5 * (0.0 + e1e / (e41 * e41) * (e4e * e1e / e42 / e31 + e4e / e42 + e1e / e31));
-        } else if (c3) { tmp = -(e3e / e43 + e2e / e42 + e1e / e41) * (e4e * e4e) / e41 / e42 / e43; if (e3 == e4) tmp = 0.0; }
-        break;
+__device__ void simplex_coefs(int kind, SimplexEntry &t) {
+  const double *e = t.e;
+  const int v = t.label;
+  for (int i = 0; i < 4; ++i) t.c1[i] = t.c3[i] = 0.0;
+  for (int i = 0; i < 5; ++i) t.m[i] = 0.0;
+  const double r21 = 1.0 / (e[1] - e[0]), r31 = 1.0 / (e[2] - e[0]), r32 = 1.0 / (e[2] - e[1]);
+  if (kind == 1) {
+    if (v == 0) {
+      t.c1[1] = -r21 * r21 * r31;
+      t.c1[2] = -r31 * r21 * r31;
+      t.c3[2] = r32 * r31 * r31;
+    } else if (v == 1) {
+      t.c1[0] = r21 * r21 * r31;
+      t.c3[2] = r32 * r32 * r31;
+    } else {
+      t.c1[0] = r21 * r31 * r31;
+      t.c3[0] = -r31 * r32 * r31;
+      t.c3[1] = -r32 * r32 * r31;
     }
-    if (e1 == e2 && e1 == e3 && e1 == e4 && e == e1) tmp = 0.25;
-    acc += tmp;
+    return;
   }
-  if (acc < 1.0e-12) acc = 0.0;
-  return acc / (double)(6 * (int64_t)rp.N);
+  const double r41 = 1.0 / (e[3] - e[0]), r42 = 1.0 / (e[3] - e[1]), r43 = 1.0 / (e[3] - e[2]);
+  const double k1 = r21 * r31 * r41, k3 = r41 * r42 * r43;
+  if (v == 0) {
+    t.c1[1] = r21 * k1;
+    t.c1[2] = r31 * k1;
+    t.c1[3] = r41 * k1;
+    t.c3[3] = k3 * r41;
+    t.m[0] = -0.5 * r31 * r31 * r42 * r32;
+    t.m[1] = -0.5 * r31 * r31 * r32 * r41;
+    t.m[2] = -0.5 * r41 * r41 * r42 * r31;
+    t.m[3] = -0.5 * r41 * r41 * r42 * r32;
+    t.m[4] = -0.5 * (r31 * r31 * r41 * r42 + r41 * r41 * r31 * r32);
+  } else if (v == 1) {
+    t.c1[0] = -k1 * r21;
+    t.c3[3] = k3 * r42;
+    t.m[0] = -0.5 * r32 * r32 * r42 * r31;
+    t.m[1] = -0.5 * r32 * r32 * r31 * r41;
+    t.m[2] = -0.5 * r42 * r42 * r41 * r31;
+    t.m[3] = -0.5 * r42 * r42 * r32 * r41;
+    t.m[4] = -0.5 * (r32 * r32 * r42 * r41 + r42 * r42 * r32 * r31);
+  } else if (v == 2) {
+    t.c1[0] = -k1 * r31;
+    t.c3[3] = k3 * r43;
+    t.m[0] = 0.5 * r32 * r32 * r42 * r31;
+    t.m[1] = 0.5 * r32 * r32 * r42 * r41;
+    t.m[2] = 0.5 * r31 * r31 * r41 * r42;
+    t.m[3] = 0.5 * r31 * r31 * r32 * r41;
+    t.m[4] = 0.5 * (r32 * r32 * r31 * r41 + r31 * r31 * r42 * r32);
+  } else {
+    t.c1[0] = -k1 * r41;
+    t.c3[0] = -r41 * k3;
+    t.c3[1] = -r42 * k3;
+    t.c3[2] = -r43 * k3;
+    t.m[0] = 0.5 * r42 * r42 * r32 * r31;
+    t.m[1] = 0.5 * r42 * r42 * r32 * r41;
+    t.m[2] = 0.5 * r41 * r41 * r42 * r31;
+    t.m[3] = 0.5 * r41 * r41 * r31 * r32;
+    t.m[4] = 0.5 * (r42 * r42 * r41 * r31 + r41 * r41 * r42 * r32);
+  }
 }
 
-__device__ inline double delta_eval(double e, int ikp, int n, double eps_kn, const RateParams &rp,
-                                    const EpiData &d) {
-  if (rp.delta_kind == 0) {
-    double x = (e - eps_kn) / rp.sigma;
-    return (1.0 / sqrt(TWOPI)) / rp.sigma * exp(-0.5 * x * x) * rp.inv_nk;
-  }
-  if (rp.delta_kind == 1) return delta_triang(e, ikp, n, rp, d);
-  return delta_tetra(e, ikp, n, rp, d);
+// beta += the Bernstein coefficients (times the binomials) of a product of three
+// linear factors given by their values at the two ends
+__device__ __forceinline__ void blossom(double *beta, double x0, double x1, double y0, double y1, double z0, double z1) {
+  const double p = x0 * y0, q = x1 * y1, r = fma(x0, y1, x1 * y0);
+  beta[0] = fma(p, z0, beta[0]);
+  beta[1] = fma(r, z0, fma(p, z1, beta[1]));
+  beta[2] = fma(r, z1, fma(q, z0, beta[2]));
+  beta[3] = fma(q, z1, beta[3]);
 }
 
-// Per (k', initial state) epilogue: the k' rotation, the phonon mix, |g|^2
-// (wannier.f90:937-1009), X+- (interactions.f90:2278-2332, 2353) and the
-// per-pair partial of the RTA rate (interactions.f90:3012-3034).  With the
-// phonon side requested, also Y of the same vertex (interactions.f90:1857-1870,
-// 1897: the (k, m, k + q, n, s) vertex of phonon state (q, s) is the (k, m, k', n,
-// s) vertex here, q = k' - k) added into the phonon state's rate.
-// Gv(x) returns the complex Rp-Fourier sum G(n' + nw*s') of the pair.
-template <typename GV>
-__device__ void pair_epilogue(int ip, int j, GV Gv, const RateParams &rp, const EpiData &d,
-                              double &out) {
+// One block per final state: its simplices from the 8 (4) mesh cells that have k'
+// as a corner, their vertex energies ranked, one thread per interval.  FP64 bound
+// (~60 operations per interval and simplex that covers it).
+constexpr int SX_THREADS = 96;
+
+__global__ void __launch_bounds__(SX_THREADS) k_simplex_tab(int kind, int m1, int m2, int m3, const int2 *fin,
+                                                            const int *widx, const int *rowmap, const double *ens,
+                                                            int nw, SimplexTab t) {
+  __shared__ SimplexEntry en[24];
+  __shared__ double bp[SX_MAX];
+  __shared__ int nbp;
+  const int f = blockIdx.x, tid = threadIdx.x;
+  const int nv = kind == 1 ? 3 : 4, per = kind == 1 ? 2 : 6, ne = nv * per;
+  const int2 fs = fin[f];
+  const int p = widx[fs.x];
+  const int mesh[3] = {m1, m2, m3};
+  if (tid == 0) nbp = 0;
+  if (tid < ne) {   // simplex tid / nv of the cell whose corner (tid % nv) is k'
+    const int tk = tid / nv, tl = tid % nv;
+    auto corner = [&](int l) { return (kind == 1 ? kTri[tk][l] : kTet[tk][l]) - 1; };
+    const int a = corner(tl);
+    const int pc[3] = {p % m1, (p / m1) % m2, p / (m1 * m2)};
+    int o[3];
+    for (int d = 0; d < 3; ++d) {   // the cell's origin: k' minus the corner's offset
+      o[d] = pc[d] - ((a >> d) & 1);
+      if (o[d] < 0) o[d] += mesh[d];
+    }
+    SimplexEntry x;
+    x.label = rowmap[o[0] + m1 * (o[1] + m2 * o[2])] >= 0 ? tl : -1;
+    if (x.label >= 0) {
+      for (int l = 0; l < nv; ++l) {
+        int c[3];
+        for (int d = 0; d < 3; ++d) {
+          c[d] = o[d] + ((corner(l) >> d) & 1);
+          if (c[d] >= mesh[d]) c[d] -= mesh[d];
+        }
+        const int mux = c[0] + m1 * (c[1] + m2 * c[2]);
+        x.e[l] = rowmap[mux] >= 0 ? ens[(size_t)mux * nw + fs.y] : 0.0;
+      }
+      for (int u = 1; u < nv; ++u)
+        for (int w = u; w > 0 && x.e[w] < x.e[w - 1]; --w) {
+          const double y = x.e[w];
+          x.e[w] = x.e[w - 1];
+          x.e[w - 1] = y;
+        }
+      if (kind == 1) x.e[3] = x.e[2];
+      simplex_coefs(kind, x);
+    }
+    en[tid] = x;
+  }
+  __syncthreads();
+  // rank the vertex energies
+  for (int u = tid; u < nv * ne; u += SX_THREADS) {
+    const SimplexEntry &x = en[u / nv];
+    if (x.label < 0) continue;
+    const double e = x.e[u % nv];
+    int rank = 0;
+    for (int w = 0; w < nv * ne; ++w) {
+      const SimplexEntry &y = en[w / nv];
+      if (y.label < 0) continue;
+      const double ye = y.e[w % nv];
+      rank += (ye < e) || (ye == e && w < u);
+    }
+    bp[rank] = e;
+    atomicAdd(&nbp, 1);
+  }
+  __syncthreads();
+  const int n = nbp;
+  if (tid == 0) t.n[f] = n;
+  for (int i = tid; i < n; i += SX_THREADS) {
+    const double b1 = bp[i], b0 = i ? bp[i - 1] : b1, w = b1 - b0;
+    double beta[4] = {0.0, 0.0, 0.0, 0.0};
+    if (w > 0.0)
+      for (int u = 0; u < ne; ++u) {
+        const SimplexEntry &x = en[u];
+        if (x.label < 0 || b0 < x.e[0] || b1 > x.e[nv - 1]) continue;
+        double l[4], r[4];
+#pragma unroll
+        for (int c = 0; c < 4; ++c) {
+          l[c] = x.e[c] - b0;
+          r[c] = x.e[c] - b1;
+        }
+        const bool first = b1 <= x.e[1], last = b0 >= x.e[nv - 2];
+        if (first || last) {
+          const double *k = first ? x.c1 : x.c3;
+          const double zl = k[0] * l[0] + k[1] * l[1] + k[2] * l[2] + k[3] * l[3];
+          const double zr = k[0] * r[0] + k[1] * r[1] + k[2] * r[2] + k[3] * r[3];
+          const double xl = first ? l[0] : l[nv - 1], xr = first ? r[0] : r[nv - 1];
+          if (kind == 1) blossom(beta, xl, xr, 1.0, 1.0, zl, zr);
+          else blossom(beta, xl, xr, xl, xr, zl, zr);
+        } else {
+          const bool lo = x.label < 2;
+          const double Sl = lo ? l[2] : l[1], Sr = lo ? r[2] : r[1], Ql = lo ? l[3] : l[0], Qr = lo ? r[3] : r[0];
+          const double al = lo ? l[1] : l[2], ar = lo ? r[1] : r[2], bl = lo ? l[0] : l[3], br = lo ? r[0] : r[3];
+          blossom(beta, Sl, Sr, Sl, Sr, x.m[0] * al + x.m[1] * bl, x.m[0] * ar + x.m[1] * br);
+          blossom(beta, Ql, Qr, Ql, Qr, x.m[2] * bl + x.m[3] * al, x.m[2] * br + x.m[3] * ar);
+          blossom(beta, Sl, Sr, Ql, Qr, x.m[4] * l[x.label], x.m[4] * r[x.label]);
+        }
+      }
+    const double rw = w > 0.0 ? 1.0 / w : 0.0, r3 = rw * rw * rw;
+    const size_t at = (size_t)f * t.stride + i;
+    t.key[at] = (float)b1;
+    t.b[at] = b1;
+    t.lo[at] = make_double2(beta[0] * r3, beta[1] * r3);
+    t.hi[at] = make_double2(beta[2] * r3, beta[3] * r3);
+  }
+}
+
+void launch_simplex_tab(int kind, const int mesh[3], int nin, const int2 *fin, const int *widx, const int *rowmap,
+                        const double *ens, int nw, const SimplexTab &t, cudaStream_t st) {
+  if (nin > 0)
+    k_simplex_tab<<<nin, SX_THREADS, 0, st>>>(kind, mesh[0], mesh[1], mesh[2], fin, widx, rowmap, ens, nw, t);
+}
+
+// the delta of final state f at energy e, before the 1 / (simplices per cell N)
+__device__ __forceinline__ double simplex_delta(const SimplexTab &t, int f, double e) {
+  const int n = t.n[f];
+  const size_t at = (size_t)f * t.stride;
+  const float *key = t.key + at;
+  const double *b = t.b + at;
+  // the first breakpoint >= e: found on the breakpoints rounded to FP32 (rounding is
+  // monotone, so that one is at or before it), then settled in FP64
+  const float ef = (float)e;
+  int lo = 0, hi = n;
+  while (lo < hi) {
+    const int mid = (lo + hi) >> 1;
+    if (key[mid] < ef) lo = mid + 1; else hi = mid;
+  }
+  while (lo < n && b[lo] < e) ++lo;
+  if (lo == 0 || lo == n) return 0.0;
+  const double u = e - b[lo - 1], v = b[lo] - e;
+  const double2 p = t.lo[at + lo], q = t.hi[at + lo];
+  const double acc = fma(fma(p.x, v, p.y * u), v * v, fma(q.x, v, q.y * u) * (u * u));
+  return acc < 1.0e-12 ? 0.0 : acc;
+}
+
+// ------------------------------------------------------- FP64 rate epilogue
+// Window bands of the window k' as a list of final states (k', n), in order
+__global__ void k_final_states(int nwv, int nw, const int *widx, const double *ens, double enref, double fsthick,
+                               const int *cum, int2 *fin) {
+  const int ip = blockIdx.x * blockDim.x + threadIdx.x;
+  if (ip >= nwv) return;
+  int f = cum[ip];
+  for (int n = 0; n < nw; ++n)
+    if (fabs(ens[(size_t)widx[ip] * nw + n] - enref) <= fsthick) fin[f++] = make_int2(ip, n);
+}
+
+void launch_final_states(int nwv, int nw, const int *widx, const double *ens, double enref, double fsthick,
+                         const int *cum, int2 *fin, cudaStream_t st) {
+  k_final_states<<<(nwv + 127) / 128, 128, 0, st>>>(nwv, nw, widx, ens, enref, fsthick, cum, fin);
+}
+
+// Per (q, s): omega, 2 pi / hbar g2unitfactor / (2 omega) (0 below 0.5 meV), n(omega), e^(omega / kT)
+__global__ void k_mode_tab(int n, const double *om, const double *bose, double T, double const_tp, double4 *mt) {
+  const int i = blockIdx.x * blockDim.x + threadIdx.x;
+  if (i >= n) return;
+  const double o = om[i];
+  mt[i] = make_double4(o, o >= 0.5e-3 ? const_tp * (0.5 / o * g2unitfactor) : 0.0, bose[i], exp(o / kB / T));
+}
+
+void launch_mode_tab(int n, const double *om, const double *bose, double T, double const_tp, double4 *mt,
+                     cudaStream_t st) {
+  k_mode_tab<<<(n + 127) / 128, 128, 0, st>>>(n, om, bose, T, const_tp, mt);
+}
+
+// Vertices of (initial state j, final state f): the k' rotation, the phonon mix,
+// |g|^2 (wannier.f90:937-1009), X+- (interactions.f90:2278-2332, 2353) and the RTA
+// rate (interactions.f90:3012-3034).  With the phonon side requested, also Y of
+// the same vertex (interactions.f90:1857-1870, 1897: the (k, m, k + q, n, s) vertex
+// of phonon state (q, s) is the (k, m, k', n, s) vertex here, q = k' - k) added
+// into the phonon state's rate.
+//
+// Bound by the FP64 pipe (16 cycles per warp instruction on an SM), so the split
+// keeps every lane on a vertex of its own and every FP64 instruction on the
+// result: a thread is one initial state and walks EPF_F final states, which are
+// the same for the whole block.  There is no divergence over the window bands,
+// U_k' and the delta's table are read by broadcast, the sum over final states
+// stays in the thread (compensated), and the occupations need no exponential:
+// f(E + w) = 1 / (1 + e^x e^v) and 1 - f(E - w) = 1 / (1 + e^-x e^v), x = (E - mu) / kT
+// per state, v = w / kT per mode.  12^3, nw 8, nb 6 (2.8 M pairs): 5.06 ms (3.9 at the
+// FP64 rate for its ~850 instructions a pair); one thread per (k', state) with a loop
+// over the bands took 15.1 ms.  Tetrahedra, 10x12x11 (1.8 M pairs): 3.1 ms + 0.32 ms for
+// the tables; with every simplex's formula at every vertex 511 ms.
+constexpr int EPF_THREADS = 128;
+
+template <bool F32>
+__device__ __forceinline__ double2 epf_load(const FinalIn &c, int64_t off) {
+  if (F32) return make_double2((double)c.re[off], (double)c.im[off]);
+  return c.z[off];
+}
+
+template <bool F32, bool SIMPLEX, bool PH>
+__global__ void __launch_bounds__(EPF_THREADS) k_epilogue_final(int j0, int ns, FinalIn c, RateParams rp, EpiData d,
+                                                                double *partial, int nblk) {
+  const int jl = blockIdx.x * EPF_THREADS + threadIdx.x;
+  if (jl >= ns) return;
+  const int j = j0 + jl;
   const int nw = rp.nw, nb = rp.nb;
   const int code = d.st_code[j];
-  const int i = code / nw, m = code % nw;
-  const int p = d.sidx[i], pp = d.widx[ip];
-  const int iw = d.swin ? d.swin[i] : i;   // the state's k in the window (simplices)
+  const int p = d.sidx[code / nw], m = code % nw;
   const double E = d.ens[(size_t)p * nw + m];
-  int a1 = p % rp.mesh[0], a2 = (p / rp.mesh[0]) % rp.mesh[1], a3 = p / (rp.mesh[0] * rp.mesh[1]);
-  int b1 = pp % rp.mesh[0], b2 = (pp / rp.mesh[0]) % rp.mesh[1], b3 = pp / (rp.mesh[0] * rp.mesh[1]);
-  int q = (int)(floormod(b1 - a1, rp.mesh[0]) +
-                rp.mesh[0] * (floormod(b2 - a2, rp.mesh[1]) + rp.mesh[1] * floormod(b3 - a3, rp.mesh[2])));
-  double acc = 0.0;
-  int rank_n = 0;
-  const bool ph = d.phr || d.yv;
-  const double fermi1 = ph ? fermi(E, rp.chempot, rp.T) : 0.0;
-  for (int n = 0; n < nw; ++n) {
-    double eps = d.ens[(size_t)pp * nw + n];
-    if (fabs(eps - rp.enref) > rp.fsthick) continue;
-    const double2 *Ukp = d.U + ((size_t)pp * nw + n) * nw;
+  const double kT = kB * rp.T, x = (E - rp.chempot) / kT;
+  const double ex = exp(x), emx = exp(-x);
+  const double f1 = 1.0 / (ex + 1.0);
+  const double isig = SIMPLEX ? 0.0 : 1.0 / rp.sigma;
+  const double dnorm = SIMPLEX ? rp.inv_nk / (rp.delta_kind == 1 ? 2.0 : 6.0)
+                               : (1.0 / sqrt(TWOPI)) / rp.sigma * rp.inv_nk;
+  const int a1 = p % rp.mesh[0], a2 = (p / rp.mesh[0]) % rp.mesh[1], a3 = p / (rp.mesh[0] * rp.mesh[1]);
+  const double2 *Uk = d.U + ((size_t)p * nw + m) * nw;
+  double sum = 0.0, comp = 0.0;
+  const int fe = min(d.nin, (int)(blockIdx.y + 1) * EPF_F);
+  for (int f = blockIdx.y * EPF_F; f < fe; ++f) {
+    const int2 fs = d.fin[f];
+    const int pp = d.widx[fs.x];
+    const double eps = d.ens[(size_t)pp * nw + fs.y];
+    const double2 *Ukp = d.U + ((size_t)pp * nw + fs.y) * nw;
+    int q1 = pp % rp.mesh[0] - a1, q2 = (pp / rp.mesh[0]) % rp.mesh[1] - a2, q3 = pp / (rp.mesh[0] * rp.mesh[1]) - a3;
+    q1 += q1 < 0 ? rp.mesh[0] : 0;
+    q2 += q2 < 0 ? rp.mesh[1] : 0;
+    q3 += q3 < 0 ? rp.mesh[2] : 0;
+    const int q = q1 + rp.mesh[0] * (q2 + rp.mesh[1] * q3);
+    const int64_t base = (int64_t)fs.x * c.ldc + jl * c.js;
     double2 h[32];
     for (int s = 0; s < nb; ++s) {
       double2 a = make_double2(0.0, 0.0);
-      for (int np = 0; np < nw; ++np) cfma_cj(a, Ukp[np], Gv(np + nw * s));
+      for (int np = 0; np < nw; ++np) cfma_cj(a, Ukp[np], epf_load<F32>(c, base + (np + nw * s) * c.xs));
       h[s] = a;
     }
     double2 unm = make_double2(0.0, 0.0);   // dot_product(el_evec_kp, el_evec_k), polar crystals
-    if (d.glp) {
-      const double2 *Uk = d.U + ((size_t)p * nw + m) * nw;
-      for (int c = 0; c < nw; ++c) cfma_cj(unm, Ukp[c], Uk[c]);
-    }
+    if (d.glp)
+      for (int n = 0; n < nw; ++n) cfma_cj(unm, Ukp[n], Uk[n]);
+    double acc = 0.0;
     for (int s = 0; s < nb; ++s) {
-      double om = d.om[(size_t)q * nb + s];
-      double2 gsum = make_double2(0.0, 0.0);
-      const double2 *u = d.u + ((size_t)q * nb + s) * nb;
-      for (int sp = 0; sp < nb; ++sp) cfma(gsum, u[sp], h[sp]);
-      if (d.glp) cfma(gsum, d.glp[(size_t)q * nb + s], unm);   // long-range term (wannier.f90:998-1006)
-      double g2 = (om == 0.0) ? 0.0 : 0.5 * (gsum.x * gsum.x + gsum.y * gsum.y) / om * g2unitfactor;
-      double bose = d.bose[(size_t)q * nb + s];
+      const int qs = q * nb + s;
+      const double4 mt = d.mt[qs];   // omega, prefactor, n, e^v
+      double2 g = make_double2(0.0, 0.0);
+      const double2 *u = d.u + (size_t)qs * nb;
+      for (int sp = 0; sp < nb; ++sp) cfma(g, u[sp], h[sp]);
+      if (d.glp) cfma(g, d.glp[qs], unm);   // long-range term (wannier.f90:998-1006)
+      const double gg = fma(g.x, g.x, g.y * g.y);
       double xp = 0.0, xm = 0.0, y = 0.0;
-      if (om >= 0.5e-3) {
-        double fp = fermi(E + om, rp.chempot, rp.T);
-        double fm = fermi(E - om, rp.chempot, rp.T);
-        double dp = delta_eval(E + om, ip, n, eps, rp, d);
-        double dm = delta_eval(E - om, ip, n, eps, rp, d);
-        xp = rp.const_tp * (g2 * (bose + fp) * dp);
-        xm = rp.const_tp * (g2 * (1.0 + bose - fm) * dm);
-        if (ph) {
-          // Y: delta(E' - omega) at the initial electron (k, m), interactions.f90:1862
-          const double invboseplus1 = 1.0 / (1.0 + bose);
-          const double dy = delta_eval(eps - om, iw, m, E, rp, d);
-          y = rp.const_tp * (g2 * (fermi1 * (1.0 - fp) * invboseplus1) * dy);
+      if (mt.y != 0.0) {
+        double dp, dm;
+        if (SIMPLEX) {
+          dp = simplex_delta(d.sx, f, E + mt.x) * dnorm;
+          dm = simplex_delta(d.sx, f, E - mt.x) * dnorm;
+        } else {
+          const double tp = ((E + mt.x) - eps) * isig, tm = ((E - mt.x) - eps) * isig;
+          dp = dnorm * exp(-0.5 * tp * tp);
+          dm = dnorm * exp(-0.5 * tm * tm);
+        }
+        double A = fma(ex, mt.w, 1.0), B = fma(emx, mt.w, 1.0);
+        if (mt.w > 1e260) {   // omega / kT > 600: the factors may leave FP64's range one by one
+          const double v = mt.x / kT;
+          A = 1.0 + exp(x + v);
+          B = 1.0 + exp(v - x);
+        }
+        const double gc = gg * mt.y, fp = 1.0 / A;
+        xp = gc * (mt.z + fp) * dp;
+        xm = gc * (mt.z + 1.0 / B) * dm;
+        if (PH) {
+          // Y: delta(E' - omega) at the initial electron (k, m), interactions.f90:1862; the Gaussian is even
+          const double dy = SIMPLEX ? simplex_delta(d.sx, j, eps - mt.x) * dnorm : dp;
+          y = gc * (f1 * (1.0 - fp) / (1.0 + mt.z)) * dy;
           if (d.phr && y != 0.0) atomicAdd(d.phr + q + (size_t)rp.N * s, d.ph_scale * y);
         }
       }
       acc += xp + xm;
       if (d.g2) {
-        int64_t off = (int64_t)j * d.per_state + ((int64_t)d.cum[ip] + rank_n) * nb + s;
+        const int64_t off = (int64_t)j * d.per_state + (int64_t)f * nb + s;
         if (off < d.cap) {
-          d.g2[off] = g2;
+          d.g2[off] = mt.x == 0.0 ? 0.0 : 0.5 * gg / mt.x * g2unitfactor;
           if (d.xp) d.xp[off] = xp;
           if (d.xm) d.xm[off] = xm;
           if (d.yv) d.yv[off] = y;
         }
       }
     }
-    rank_n++;
+    const double t = sum + acc;   // compensated (Neumaier)
+    comp += (fabs(sum) >= fabs(acc)) ? (sum - t) + acc : (acc - t) + sum;
+    sum = t;
   }
-  out = acc;
+  partial[(size_t)j * nblk + blockIdx.y] = sum + comp;
 }
 
-// Block-deterministic partial: threads along k' for one state, then a fixed
-// order compensated (Neumaier) sum by thread 0.
-__device__ void block_partial(double v, double *partial, int j, int nblk) {
-  __shared__ double sv[128];
-  sv[threadIdx.x] = v;
-  __syncthreads();
-  if (threadIdx.x == 0) {
-    double s = 0.0, c = 0.0;
-    for (int t = 0; t < (int)blockDim.x; ++t) {
-      double x = sv[t], tt = s + x;
-      c += (fabs(s) >= fabs(x)) ? (s - tt) + x : (x - tt) + s;
-      s = tt;
-    }
-    partial[(size_t)j * nblk + blockIdx.x] = s + c;
+void launch_epilogue_final(int j0, int j1, const FinalIn &c, const RateParams &rp, const EpiData &d, double *partial,
+                           int nblk, cudaStream_t st) {
+  const int ns = j1 - j0;
+  if (ns <= 0 || d.nin <= 0) return;
+  dim3 grid((ns + EPF_THREADS - 1) / EPF_THREADS, (d.nin + EPF_F - 1) / EPF_F);
+  const bool ph = d.phr || d.yv, simplex = rp.delta_kind != 0;
+  auto go = [&](auto k) { k<<<grid, EPF_THREADS, 0, st>>>(j0, ns, c, rp, d, partial, nblk); };
+  if (c.z) {
+    if (simplex) ph ? go(k_epilogue_final<false, true, true>) : go(k_epilogue_final<false, true, false>);
+    else ph ? go(k_epilogue_final<false, false, true>) : go(k_epilogue_final<false, false, false>);
+  } else {
+    if (simplex) ph ? go(k_epilogue_final<true, true, true>) : go(k_epilogue_final<true, true, false>);
+    else ph ? go(k_epilogue_final<true, false, true>) : go(k_epilogue_final<true, false, false>);
   }
-}
-
-__global__ void __launch_bounds__(128) k_epilogue_fp64(int nwv, int j0, const double2 *C,
-                                                       int64_t ldc, RateParams rp, EpiData d,
-                                                       double *partial, int nblk) {
-  const int ip = blockIdx.x * blockDim.x + threadIdx.x;
-  const int j = j0 + blockIdx.y;
-  const int ncol = rp.nw * rp.nb;
-  double v = 0.0;
-  if (ip < nwv) {
-    const double2 *row = C + (int64_t)ip * ldc + (int64_t)(j - j0) * ncol;
-    pair_epilogue(ip, j, [&](int x) { return row[x]; }, rp, d, v);
-  }
-  block_partial(v, partial, j, nblk);
-}
-
-void launch_epilogue_fp64(int nwv, int j0, int j1, const double2 *C, int64_t ldc,
-                          const RateParams &rp, const EpiData &d, double *partial, int nblk,
-                          cudaStream_t st) {
-  if (j1 <= j0) return;
-  dim3 grid(nblk, j1 - j0);
-  k_epilogue_fp64<<<grid, 128, 0, st>>>(nwv, j0, C, ldc, rp, d, partial, nblk);
-}
-
-__global__ void __launch_bounds__(128) k_epilogue_fp32(int nwv, int j0, const float *Cr,
-                                                       const float *Ci, int64_t ldc,
-                                                       RateParams rp, EpiData d,
-                                                       double *partial, int nblk) {
-  const int ip = blockIdx.x * blockDim.x + threadIdx.x;
-  const int j = j0 + blockIdx.y;
-  const int ncol = rp.nw * rp.nb;
-  double v = 0.0;
-  if (ip < nwv) {
-    const int64_t base = (int64_t)ip * ldc + (int64_t)(j - j0) * ncol;
-    pair_epilogue(ip, j, [&](int x) { return make_double2((double)Cr[base + x], (double)Ci[base + x]); },
-                  rp, d, v);
-  }
-  block_partial(v, partial, j, nblk);
-}
-
-void launch_epilogue_fp32(int nwv, int j0, int j1, const float *Cr, const float *Ci,
-                          int64_t ldc, const RateParams &rp, const EpiData &d, double *partial,
-                          int nblk, cudaStream_t st) {
-  if (j1 <= j0) return;
-  dim3 grid(nblk, j1 - j0);
-  k_epilogue_fp32<<<grid, 128, 0, st>>>(nwv, j0, Cr, Ci, ldc, rp, d, partial, nblk);
 }
 
 // rates(ik, m) = compensated sum of the block partials in block order

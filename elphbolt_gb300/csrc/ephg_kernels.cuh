@@ -143,15 +143,26 @@ void launch_state_flags(int nwv, int nw, const int *widx, const double *ens, dou
 void launch_iota(int n, int *out, cudaStream_t st);
 // Stage A rotation: B[Rp][c] (ldb) for states j in [j0,j1) of k-chunk [i0, i0+kc) and the
 // (mode, cell) blocks s + nb Rp in [blk0, blk0 + nblk) that gk holds (nw nw values each):
-// B = phk[k][Rp] * sum_m' U_k[m][m'] gk(n',m',s',Rp), phk = conj(e^{2 pi i k.Rp})/deg(Rp) (row stride nws)
+// B = phk[k][Rp] * sum_m' U_k[m][m'] gk(n',m',s',Rp), phk = conj(e^{2 pi i k.Rp})/deg(Rp) (row stride nws).
+// Columns: chunks of sc states (the last one shorter), within a chunk [n' + nw s'][state].
 void launch_rotate_states_fp64(int j0, int j1, int i0, const int *st_code, int nw, int nb, int nws, int64_t blk0,
                                int64_t nblk, const int *widx, const double2 *U, const double2 *gk, int64_t ldgk,
-                               const double2 *phk, double2 *B, int64_t ldb, cudaStream_t st);
+                               const double2 *phk, double2 *B, int64_t ldb, int sc, int nst, cudaStream_t st);
+// Triangle / tetrahedron deltas of the final states as tables (launch_simplex_tab):
+// per final state the sorted breakpoints b (key: rounded to FP32) and for each the
+// Bernstein coefficients (lo, hi) of the interval that ends there.
+constexpr int SX_MAX = 96;
+struct SimplexTab {
+  int stride;           // entries per final state: 96, or 18 for triangles
+  int *n;
+  float *key;
+  double *b;
+  double2 *lo, *hi;
+};
 struct EpiData {
   const int *widx;      // window (k' row) -> mesh index
   const int *st_code;   // state -> i*nw + m, i the state's k row (an A-row)
   const int *sidx;      // A-row (the k of initial states) -> mesh index
-  const int *swin;      // A-row -> window index (simplices); null: the identity
   const int *cum;       // window k' -> first (k',n) final-state rank
   const double *ens;    // [p][b] eV
   const double2 *U;     // [p][b][c]
@@ -160,11 +171,12 @@ struct EpiData {
   const double2 *u;     // [q][s][c] evec/sqrt(M)
   const float2 *uf;     // same in fp32
   const double *bose;   // [q][s]
-  // triangle / tetrahedron delta data (window-k indexed, 0-based)
-  const int *smap;      // (nwv, maxc, 2): simplex, vertex(1-based)
-  const int *scount;    // (nwv)
-  const double *sevals; // (nsimplex, nw, nv) sorted vertex energies
-  int nsimplex, maxc, nvx;
+  // FP64 epilogue: the final states (window k' row, band), the (q, s) table of
+  // launch_mode_tab and, for the triangle / tetrahedron deltas, theirs
+  const int2 *fin;
+  int nin;
+  const double4 *mt;
+  SimplexTab sx;
   int64_t per_state;    // vertices per initial state
   double *g2, *xp, *xm; // optional vertex lists
   int64_t cap;
@@ -188,15 +200,30 @@ struct RateSets {
   int n;
   RateParams rp[MAX_SETS];
   double *bose[MAX_SETS];      // [q][s] per set (set 0: EpiData.bose)
+  const double4 *mt[MAX_SETS]; // FP64 epilogue: [q][s] per set (set 0: EpiData.mt)
   double *partial[MAX_SETS];   // [j][iblk] per set (set 0: the caller's partial)
 };
-// per (k', state) epilogue on an FP64 C chunk: rates partial sums [j][iblk]
-void launch_epilogue_fp64(int nwv, int j0, int j1, const double2 *C, int64_t ldc,
-                          const RateParams &rp, const EpiData &d, double *partial,
-                          int nblk, cudaStream_t st);
-void launch_epilogue_fp32(int nwv, int j0, int j1, const float *Cr, const float *Ci,
-                          int64_t ldc, const RateParams &rp, const EpiData &d, double *partial,
-                          int nblk, cudaStream_t st);
+// Final states of the window rows in order: fin[cum[ip] + rank] = (ip, band)
+void launch_final_states(int nwv, int nw, const int *widx, const double *ens, double enref, double fsthick,
+                         const int *cum, int2 *fin, cudaStream_t st);
+// The simplex tables of nin final states (kind 1 triangles, 2 tetrahedra); rowmap: mesh point -> window row or -1
+void launch_simplex_tab(int kind, const int mesh[3], int nin, const int2 *fin, const int *widx, const int *rowmap,
+                        const double *ens, int nw, const SimplexTab &t, cudaStream_t st);
+// mt[q][s] = (omega, 2 pi / hbar g2unitfactor / (2 omega) or 0 below 0.5 meV, n, e^(omega / kT))
+void launch_mode_tab(int n, const double *om, const double *bose, double T, double const_tp, double4 *mt,
+                     cudaStream_t st);
+// FP64 epilogue over the states [j0, j1): the Rp sums G(x = n' + nw s') of (window row ip,
+// state j) at ip ldc + x xs + (j - j0) js, in FP64 (z) or as FP32 planes (re, im).  Rate
+// partials [j][block of EPF_F final states].
+constexpr int EPF_F = 16;
+inline int epf_blocks(int nin) { return (nin + EPF_F - 1) / EPF_F; }
+struct FinalIn {
+  const double2 *z = nullptr;
+  const float *re = nullptr, *im = nullptr;
+  int64_t ldc = 0, xs = 1, js = 0;
+};
+void launch_epilogue_final(int j0, int j1, const FinalIn &c, const RateParams &rp, const EpiData &d, double *partial,
+                           int nblk, cudaStream_t st);
 void launch_bose(int N, int nb, const double *om, double T, double *bose, cudaStream_t st);
 void launch_rate_final(int nst, int nblk, const double *partial, const int *st_code, int nw,
                        int N, double *rates_f, cudaStream_t st);

@@ -2679,6 +2679,7 @@ static int split_rates_generic(SplitOperands &s, Workspace &ws, cudaStream_t st,
     EpiData ed = eds, ed_in = eds_in;
     if (set) {
       ed.bose = ed_in.bose = sets->bose[set];
+      ed.mt = ed_in.mt = sets->mt[set];
       ed.g2 = ed.xp = ed.xm = ed.yv = ed_in.g2 = ed_in.xp = ed_in.xm = ed_in.yv = nullptr;
       ed.phr = ed_in.phr = nullptr;
     }
@@ -2719,7 +2720,13 @@ static int split_rates_generic(SplitOperands &s, Workspace &ws, cudaStream_t st,
                                                          partial, nblk);
       TCK(cudaGetLastError());
     } else {
-      launch_epilogue_fp32(nwv, (int)j0, (int)j0 + ns, CBr, CBi, NpC, rp, ed_in, partial, nblk, st);
+      FinalIn in;
+      in.re = CBr;
+      in.im = CBi;
+      in.ldc = NpC;
+      in.js = ncol;
+      launch_epilogue_final((int)j0, (int)j0 + ns, in, rp, ed_in, partial, nblk, st);
+      TCK(cudaGetLastError());
     }
     *launches += 1;
     }
@@ -2928,8 +2935,11 @@ int split_rates_stage(SplitOperands &s, Workspace &ws, cudaStream_t st, const do
   // The fused path packs mesh coordinates in 10 bits each.
   const bool fast86 = (nw == 8 && nb == 6 && rp.delta_kind == 0 && mesh[0] <= 1024 && mesh[1] <= 1024 &&
                        mesh[2] <= 1024);
-  // rate partials per state: one per 32-row block of the fused kernel, one per 128 k' rows otherwise
-  const int nblk = fast86 ? (int)(rup(nwv, 2 * BM) / 32) : (nwv + EPI_ROWS - 1) / EPI_ROWS;
+  // rate partials per state: one per 32-row block of the fused kernel, one per block of
+  // final states with the simplex deltas' FP64 epilogue, one per 128 k' rows otherwise
+  const int nblk = fast86              ? (int)(rup(nwv, 2 * BM) / 32)
+                   : rp.delta_kind != 0 ? epf_blocks(ed_in.nin)
+                                        : (nwv + EPI_ROWS - 1) / EPI_ROWS;
   if (nblk > nblk_max) return tfail(1, "rate partial buffer too small");
   *nblk_used = nblk;
   int rc;

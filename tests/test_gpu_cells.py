@@ -1,5 +1,5 @@
-"""The FP64 rate path's Fourier sums over cells, one dimension at a time, against
-the oracle: meshes of one, two, odd and uneven points per dimension (mirrored
+"""The FP64 rate path's Fourier sums over cells, one dimension at a time, and the
+tabulated simplex deltas, against the oracle: meshes of one, two, odd and uneven points per dimension (mirrored
 outputs v and m - v, the unpaired v = 0 and v = m / 2), cell ranges that are not
 symmetric about zero, more cells than mesh points, and windows so narrow that
 the contractions run as matrix products.  Rates within 1e-10 relative, the FP64
@@ -52,3 +52,28 @@ def test_fp64_rates(oracle_lib, kind, mesh, window):
     m = ref["rates"] > 0
     assert np.all(out["rates"][~m] == 0)
     assert np.max(np.abs(out["rates"][m] - ref["rates"][m]) / ref["rates"][m], initial=0.0) <= 1e-10
+
+
+@pytest.mark.parametrize("delta", [1, 2])
+@pytest.mark.parametrize("mesh", [(1, 1, 7), (2, 3, 5), (6, 2, 1), (5, 4, 3)])
+def test_simplex_rates(oracle_lib, mesh, delta):
+    """Triangle / tetrahedron deltas on meshes whose cells wrap onto themselves (a
+    corner then appears several times in one simplex), windows that cut simplices
+    (corners outside count as zero energy) and the phonon side, whose delta sits
+    at the initial state."""
+    from elphbolt_gb300.build import build
+    from elphbolt_gb300.wannier import Wannier
+    build()
+    wd = crystal("odd")
+    O = oracle_lib.Wannier(wd)
+    e = np.sort(O.el_wann(S.mesh_kvecs(mesh))[0].ravel())
+    mu = float(e[len(e) // 2]) + 0.01
+    W = Wannier(wd)
+    for window in (4.0, 0.7):
+        req = S.RateRequest(mesh=mesh, enref=mu, fsthick=window, chempot=mu, T=300.0, delta_kind=delta)
+        ref = O.el_rates(req)["rates"]
+        refp = O.ph_rates(req, spindeg=2)["rates_phe"]
+        out = W.ph_rates(req, precision=_lib.PREC_FP64, electrons=True)
+        for a, b in ((out["rates"], ref), (out["rates_phe"], refp)):
+            assert np.max(np.abs(a - b)) <= 1e-10 * np.max(np.abs(b), initial=0.0)
+    W.deallocate_wannier()
