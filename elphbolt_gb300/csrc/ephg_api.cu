@@ -19,6 +19,7 @@
 #include "ephg_ws.cuh"
 #include "ephg_handle.cuh"
 #include "ephg_sym.cuh"
+#include "ephg_xgemm.cuh"
 
 using namespace ephg;
 
@@ -232,7 +233,7 @@ int ephg_destroy(ephg_handle *h) {
   void *ptrs[] = {h->Rk, h->Rq, h->Rg, h->degk, h->degq, h->degg, h->Hext, h->Hbox, h->Dbox, h->graw, h->G64,
                   h->masses, h->pair_off, h->ent_iuc, h->ent_woff, h->wrapR, h->ent_rden,
                   h->rcartq, h->D, h->err, h->kposk, h->kposq, h->polar_G, h->polar_Gcell,
-                  h->polar_born, h->polar_tau, h->polar_Da, h->cellk_tab, h->cellq_tab, h->rdegk};
+                  h->polar_born, h->polar_tau, h->polar_Da, h->cellk_tab, h->cellq_tab, h->rdegk, h->exp_H.e, h->exp_G.e, h->exp_raw.e};
   // stream-ordered frees back to the library pool, which keeps the memory
   // mapped for the next handle
   for (void *p : ptrs)
@@ -712,11 +713,15 @@ int ephg_el_wann(ephg_handle *h, int64_t nk, const double *kvecs, double *energi
   }
   CK(cudaMemcpyAsync(kv, kvecs, (size_t)nk * 3 * sizeof(double), cudaMemcpyHostToDevice, h->st));
   launch_phase_frac((int)nk, kv, nwsk, h->Rk, h->degk, P, nwsk, h->st);
-  launch_zgemm((int)nk, ncol, nwsk, P, nwsk, h->Hext, 4 * (int64_t)nn, C, ncol, h->st);
+  const int *ce;
+  if ((rc = resident_colexp(h->exp_H, 4 * (int64_t)nn, nwsk, h->Hext, 4 * (int64_t)nn, &h->resident_bytes, h->st, &ce)))
+    return fail(rc, "el_wann: column exponents");
+  if ((rc = launch_xgemm(h->ws, (int)nk, ncol, nwsk, P, nwsk, h->Hext, 4 * (int64_t)nn, ce, C, ncol, h->err, h->st)))
+    return WSFAIL(rc);
   launch_heig((int)nk, nw, C, ncol, w, V, h->err, h->st);
   launch_el_post((int)nk, nw, w, V, C, ncol, with_vel, sc, ens, with_vel ? vel : nullptr,
                  evecs ? ev : nullptr, nullptr, h->st);
-  h->launches += 4;
+  h->launches += 5;
   CKL();
   CK(cudaMemcpyAsync(energies, ens, (size_t)nk * nw * sizeof(double), cudaMemcpyDeviceToHost, h->st));
   if (evecs) CK(cudaMemcpyAsync(evecs, ev, (size_t)nk * nn * sizeof(double2), cudaMemcpyDeviceToHost, h->st));
@@ -773,6 +778,9 @@ int ephg_gkRp(ephg_handle *h, int64_t nk, const double *kvecs, double *gmixed) {
   if ((rc = wsget(h->ws, "gk_kv", (size_t)chunk * 3, &kv)) || (rc = wsget(h->ws, "gk_P", (size_t)chunk * nwsk, &P)) ||
       (rc = wsget(h->ws, "gk_C", (size_t)chunk * h->Nn, &C)))
     return WSFAIL(rc);
+  const int *ce;
+  if ((rc = resident_colexp(h->exp_G, h->Nn, nwsk, h->G64, h->Nn, &h->resident_bytes, h->st, &ce)))
+    return fail(rc, "gkRp: column exponents");
   std::vector<double> kc((size_t)chunk * 3);
   for (int64_t k0 = 0; k0 < nk; k0 += chunk) {
     int64_t n = std::min(chunk, nk - k0);
@@ -780,8 +788,9 @@ int ephg_gkRp(ephg_handle *h, int64_t nk, const double *kvecs, double *gmixed) {
       for (int64_t i = 0; i < n; ++i) kc[i + n * c] = kvecs[(k0 + i) + nk * c];
     CK(cudaMemcpyAsync(kv, kc.data(), (size_t)n * 3 * sizeof(double), cudaMemcpyHostToDevice, h->st));
     launch_phase_frac((int)n, kv, nwsk, h->Rk, h->degk, P, nwsk, h->st);
-    launch_zgemm((int)n, (int)h->Nn, nwsk, P, nwsk, h->G64, h->Nn, C, h->Nn, h->st);
-    h->launches += 2;
+    if ((rc = launch_xgemm(h->ws, (int)n, h->Nn, nwsk, P, nwsk, h->G64, h->Nn, ce, C, h->Nn, h->err, h->st)))
+      return WSFAIL(rc);
+    h->launches += 3;
     CKL();
     CK(cudaMemcpyAsync(gmixed + 2 * k0 * h->Nn, C, (size_t)n * h->Nn * sizeof(double2),
                        cudaMemcpyDeviceToHost, h->st));
@@ -803,6 +812,9 @@ int ephg_gReq(ephg_handle *h, int64_t nq, const double *qvecs, double *gmixed) {
   if ((rc = wsget(h->ws, "gq_qv", (size_t)chunk * 3, &qv)) || (rc = wsget(h->ws, "gq_P", (size_t)chunk * nwsg, &P)) ||
       (rc = wsget(h->ws, "gq_C", (size_t)chunk * per, &C)) || (rc = wsget(h->ws, "gq_O", (size_t)chunk * per, &O)))
     return WSFAIL(rc);
+  const int *ce;
+  if ((rc = resident_colexp(h->exp_raw, per, nwsg, h->graw, per, &h->resident_bytes, h->st, &ce)))
+    return fail(rc, "gReq: column exponents");
   std::vector<double> qc((size_t)chunk * 3);
   for (int64_t q0 = 0; q0 < nq; q0 += chunk) {
     int64_t n = std::min(chunk, nq - q0);
@@ -811,9 +823,10 @@ int ephg_gReq(ephg_handle *h, int64_t nq, const double *qvecs, double *gmixed) {
     CK(cudaMemcpyAsync(qv, qc.data(), (size_t)n * 3 * sizeof(double), cudaMemcpyHostToDevice, h->st));
     // sum_Rp e^{2 pi i q.Rp}/gwsdeg * g(i,j,Re,s,Rp): rows of the raw array are Rp
     launch_phase_frac((int)n, qv, nwsg, h->Rg, h->degg, P, nwsg, h->st);
-    launch_zgemm((int)n, (int)per, nwsg, P, nwsg, h->graw, per, C, per, h->st);
+    if ((rc = launch_xgemm(h->ws, (int)n, per, nwsg, P, nwsg, h->graw, per, ce, C, per, h->err, h->st)))
+      return WSFAIL(rc);
     launch_permute_greq((int)n, nw, nb, nwsk, C, O, h->st);
-    h->launches += 3;
+    h->launches += 4;
     CKL();
     CK(cudaMemcpyAsync(gmixed + 2 * q0 * per, O, (size_t)n * per * sizeof(double2),
                        cudaMemcpyDeviceToHost, h->st));
@@ -835,24 +848,50 @@ int ephg_g2(ephg_handle *h, int64_t wannspace, int64_t nv, const double *kvecs,
     if (gm_index[v] < 1 || gm_index[v] > ngm) return fail(EPHG_ERR_ARG, "g2: gm_index out of range");
   const int nw = h->nw, nb = h->nb;
   const int nws = wannspace == EPHG_WANNSPACE_PH ? h->nwsg : h->nwsk;
-  const int64_t gstride = (int64_t)nw * nw * nb * nws;
+  const int64_t per = (int64_t)nw * nw * nb, gstride = per * nws;
+  // vertices grouped by their block, as chunks of rows that share one; pieces of whole
+  // chunks whose phases, cell sums and digits fit bounded buffers
+  std::vector<int64_t> at(ngm + 1, 0);
+  for (int64_t v = 0; v < nv; ++v) at[gm_index[v]]++;
+  for (int64_t b = 0; b < ngm; ++b) at[b + 1] += at[b];
+  std::vector<int> perm(nv);
+  for (int64_t v = 0; v < nv; ++v) perm[at[gm_index[v] - 1]++] = (int)v;
+  const int64_t most = std::max<int64_t>(XG_CHUNK, ((int64_t)1 << 28) / (16 * per));   // rows per piece
+  std::vector<int4> chunks;
+  std::vector<std::pair<int64_t, int64_t>> piece;   // first row, first chunk
+  for (int64_t r = 0; r < nv;) {
+    const int64_t b = gm_index[perm[r]];
+    int64_t e = r + 1;
+    while (e < nv && e - r < XG_CHUNK && gm_index[perm[e]] == b) ++e;
+    if (piece.empty() || e - piece.back().first > most || (int64_t)chunks.size() - piece.back().second >= 1024)
+      piece.push_back({r, (int64_t)chunks.size()});
+    chunks.push_back(make_int4((int)(r - piece.back().first), (int)(e - r), (int)(b - 1), 0));
+    r = e;
+  }
+  piece.push_back({nv, (int64_t)chunks.size()});
+  int64_t rows = 0;
+  for (size_t p = 0; p + 1 < piece.size(); ++p) rows = std::max(rows, piece[p + 1].first - piece[p].first);
   double *qv, *en, *out;
-  double2 *ek, *ekp, *eq, *gm;
-  int64_t *gi;
+  double2 *ek, *ekp, *eq, *gm, *P, *G;
+  int *pd;
+  int4 *cd;
   int rc;
   if ((rc = wsget(h->ws, "g2_qv", (size_t)nv * 3, &qv)) || (rc = wsget(h->ws, "g2_en", (size_t)nv, &en)) ||
       (rc = wsget(h->ws, "g2_out", (size_t)nv, &out)) || (rc = wsget(h->ws, "g2_ek", (size_t)nv * nw, &ek)) ||
       (rc = wsget(h->ws, "g2_ekp", (size_t)nv * nw, &ekp)) || (rc = wsget(h->ws, "g2_eq", (size_t)nv * nb, &eq)) ||
-      (rc = wsget(h->ws, "g2_gm", (size_t)ngm * gstride, &gm)) || (rc = wsget(h->ws, "g2_gi", (size_t)nv, &gi)))
+      (rc = wsget(h->ws, "g2_gm", (size_t)ngm * gstride, &gm)) || (rc = wsget(h->ws, "g2_perm", (size_t)nv, &pd)) ||
+      (rc = wsget(h->ws, "g2_chunks", chunks.size(), &cd)) || (rc = wsget(h->ws, "g2_P", (size_t)(rows * nws), &P)) ||
+      (rc = wsget(h->ws, "g2_G", (size_t)(rows * per), &G)))
     return WSFAIL(rc);
   const double *kq = wannspace == EPHG_WANNSPACE_PH ? qvecs : kvecs;
+  CK(cudaMemcpyAsync(gm, gmixed, (size_t)ngm * gstride * sizeof(double2), cudaMemcpyHostToDevice, h->st));
   CK(cudaMemcpyAsync(qv, kq, (size_t)nv * 3 * sizeof(double), cudaMemcpyHostToDevice, h->st));
   CK(cudaMemcpyAsync(en, ph_en, (size_t)nv * sizeof(double), cudaMemcpyHostToDevice, h->st));
   CK(cudaMemcpyAsync(ek, el_evec_k, (size_t)nv * nw * sizeof(double2), cudaMemcpyHostToDevice, h->st));
   CK(cudaMemcpyAsync(ekp, el_evec_kp, (size_t)nv * nw * sizeof(double2), cudaMemcpyHostToDevice, h->st));
   CK(cudaMemcpyAsync(eq, ph_evec_q, (size_t)nv * nb * sizeof(double2), cudaMemcpyHostToDevice, h->st));
-  CK(cudaMemcpyAsync(gm, gmixed, (size_t)ngm * gstride * sizeof(double2), cudaMemcpyHostToDevice, h->st));
-  CK(cudaMemcpyAsync(gi, gm_index, (size_t)nv * sizeof(int64_t), cudaMemcpyHostToDevice, h->st));
+  CK(cudaMemcpyAsync(pd, perm.data(), (size_t)nv * sizeof(int), cudaMemcpyHostToDevice, h->st));
+  CK(cudaMemcpyAsync(cd, chunks.data(), chunks.size() * sizeof(int4), cudaMemcpyHostToDevice, h->st));
   const int *R = wannspace == EPHG_WANNSPACE_PH ? h->Rq : h->Rk;
   const double *deg = wannspace == EPHG_WANNSPACE_PH ? h->degq : h->degk;
   double2 *Lv = nullptr;
@@ -866,9 +905,18 @@ int ephg_g2(ephg_handle *h, int64_t wannspace, int64_t nv, const double *kvecs,
     launch_polar_q(h->polar, (int)nv, nullptr, nullptr, qp, nullptr, nullptr, Lv, h->st);
     h->launches += 1;
   }
-  launch_g2_batch((int)nv, nw, nb, nws, qv, R, deg, ek, ekp, eq, en, h->masses, gm, gi, gstride,
-                  Lv, out, h->st);
-  h->launches += 1;
+  const int *ce;
+  if ((rc = xgemm_colexp(h->ws, ngm, per, nws, gm, gstride, &ce, h->st))) return WSFAIL(rc);
+  for (size_t p = 0; p + 1 < piece.size(); ++p) {
+    const int64_t r0 = piece[p].first, c0 = piece[p].second;
+    const int n = (int)(piece[p + 1].first - r0);
+    launch_phase_list(n, qv, nv, pd + r0, nws, R, deg, P, h->st);
+    if ((rc = launch_xgemm_chunks(h->ws, cd + c0, (int)(piece[p + 1].second - c0), n, per, nws, P, nws, gm, gstride, ce,
+                                  G, per, h->err, h->st)))
+      return WSFAIL(rc);
+    launch_g2_vertices(n, pd + r0, nv, nw, nb, G, ek, ekp, eq, en, h->masses, Lv, out, h->st);
+    h->launches += 5;
+  }
   CKL();
   CK(cudaMemcpyAsync(g2_out, out, (size_t)nv * sizeof(double), cudaMemcpyDeviceToHost, h->st));
   return ephg::api_check_err(h);
@@ -1224,7 +1272,7 @@ int ephg::el_rates_view(ephg_handle *h, const ExecView &x, const ephg_rate_reque
     if ((rc = wsget((*x.ws), "e_fin", (size_t)nin, &fin))) return WSFAILX(rc);
     launch_final_states(nwv, nw, widx, ens, req->enref, req->fsthick, cum, fin, st);
     for (int p = 0; p < nsets; ++p) {
-      double4 *mt;
+      ModeRec *mt;
       if ((rc = wsget((*x.ws), ("e_mt" + std::to_string(p)).c_str(), (size_t)N * nb, &mt))) return WSFAILX(rc);
       launch_mode_tab(N * nb, om, p ? rs.bose[p] : bose, p ? sets->reqs[p].T : req->T, rp.const_tp, mt, st);
       rs.mt[p] = mt;
@@ -1308,11 +1356,14 @@ int ephg::el_rates_view(ephg_handle *h, const ExecView &x, const ephg_rate_reque
         (*x.launches) += 4;
       }
     } else {
+      const int *ce;
+      if ((rc = resident_colexp(h->exp_G, Nn, nwsk, h->G64, Nn, &h->resident_bytes, st, &ce)))
+        return fail(rc, "el_rates: column exponents");
       for (int64_t i0 = 0; i0 < nA; i0 += kc) {
         const int n = (int)std::min<int64_t>(kc, nA - i0);
         launch_phase_mesh(n, arow + i0, mesh, L, nwsk, h->Rk, h->degk, 0, roots, Pk, nwsk, st);
         (*x.ta).begin(st);
-        launch_zgemm(n, (int)Nn, nwsk, Pk, nwsk, h->G64, Nn, gk, Nn, st);
+        if ((rc = launch_xgemm(*x.ws, n, Nn, nwsk, Pk, nwsk, h->G64, Nn, ce, gk, Nn, x.err, st))) return WSFAILX(rc);
         (*x.ta).end(st);
         launch_rotate_states_fp64(first_state[i0], first_state[i0 + n], (int)i0, st_code, nw, nb, nwsq, 0, nper, arow, V,
                                   gk, Nn, phk, B, ldb, (int)sc, nst, st);
@@ -1327,13 +1378,15 @@ int ephg::el_rates_view(ephg_handle *h, const ExecView &x, const ephg_rate_reque
     for (int64_t j0 = 0; j0 < nst; j0 += sc) {
       int ns = (int)std::min<int64_t>(sc, nst - j0);
       (*x.tb).begin(st);
-      if (sepB)
+      if (sepB) {
         launch_cells_fourier(h->cellq, B + j0 * ncol, ldb, nullptr, ns * ncol, mesh, L, roots, t1, t2, rowmap, Cb,
                              (int64_t)ns * ncol, st);
-      else
-        launch_zgemm(nwv, ns * ncol, nwsq, Pq, nwsq, B + j0 * ncol, ldb, Cb, (int64_t)ns * ncol, st);
+      } else if ((rc = launch_xgemm(*x.ws, nwv, (int64_t)ns * ncol, nwsq, Pq, nwsq, B + j0 * ncol, ldb, nullptr, Cb,
+                                    (int64_t)ns * ncol, x.err, st))) {
+        return WSFAILX(rc);
+      }
       (*x.tb).end(st);
-      (*x.launches) += sepB ? 3 : 1;
+      (*x.launches) += 3;
       FinalIn in;
       in.z = Cb;
       in.ldc = (int64_t)ns * ncol;

@@ -7,6 +7,7 @@
 #include "ephg_kernels.cuh"
 #include "ephg_tc.cuh"
 #include "ephg_ws.cuh"
+#include "ephg_xgemm.cuh"
 
 // Resident Wannier data of one crystal on one device, its stream, workspace
 // and error word.
@@ -31,6 +32,8 @@ struct ephg_handle {
   ephg::CellTab cellk, cellq;
   int *cellk_tab = nullptr, *cellq_tab = nullptr;
   double *rdegk = nullptr;
+  // column exponents of the resident right-hand sides of launch_xgemm (lazy): Hext, G64, graw
+  ephg::ColExp exp_H, exp_G, exp_raw;
   double2 *graw = nullptr;   // epmatwp order (i,j,Re,s,Rp)
   double2 *G64 = nullptr;    // stage-A matrix [Re][Nn]
   double *masses = nullptr;

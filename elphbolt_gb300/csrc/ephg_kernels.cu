@@ -278,11 +278,32 @@ void launch_phase_frac(int nrows, const double *kv, int nR, const int *R, const 
   k_phase_frac<<<(unsigned)((n + 255) / 256), 256, 0, st>>>(nrows, kv, nR, R, deg, out, ldo);
 }
 
+// the same for the vectors perm[row] of a list (column stride ldk)
+__global__ void k_phase_list(int nrows, const double *kv, int64_t ldk, const int *perm, int nR, const int *R,
+                             const double *deg, double2 *out) {
+  int64_t idx = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
+  if (idx >= (int64_t)nrows * nR) return;
+  const int row = (int)(idx / nR), r = (int)(idx % nR);
+  const int64_t k = perm[row];
+  double dot = kv[k] * (double)R[3 * r];
+  dot += kv[k + ldk] * (double)R[3 * r + 1];
+  dot += kv[k + 2 * ldk] * (double)R[3 * r + 2];
+  double s, c;
+  sincos(TWOPI * dot, &s, &c);
+  out[idx] = make_double2(c / deg[r], s / deg[r]);
+}
+
+void launch_phase_list(int nrows, const double *kv, int64_t ldk, const int *perm, int nR, const int *R,
+                       const double *deg, double2 *out, cudaStream_t st) {
+  const int64_t n = (int64_t)nrows * nR;
+  if (n > 0) k_phase_list<<<(unsigned)((n + 255) / 256), 256, 0, st>>>(nrows, kv, ldk, perm, nR, R, deg, out);
+}
+
 // ============================================================ FP64 GEMM
-// C[M][N] = A[M][K] * B[K][N], complex double, row-major.  64x64 tile per
-// 256-thread block, 4x4 complex outputs per thread; FP64-FMA bound on GB300.
-// 32-row tiles: the H(k) assembly (N = 64 columns) then spreads over ~3 waves of
-// the 152 SMs instead of 1.4, which an FP64-bound kernel pays for in full.
+// C[M][N] = A[M][K] * B[K][N], complex double, row-major.  32x64 tile per 256-thread
+// block, 2x4 complex outputs per thread; FP64-FMA bound on GB300.  For the call that
+// may not allocate; every other product runs on the tensor cores (launch_xgemm), which
+// needs a buffer for its digits.
 constexpr int ZBM = 32, ZBN = 64, ZBK = 8, ZRM = ZBM / 16;
 
 __global__ void __launch_bounds__(256) k_zgemm(int M, int N, int K, const double2 *__restrict__ A,
@@ -958,43 +979,34 @@ void launch_permute_greq(int nq, int nw, int nb, int nwsk, const double2 *in, do
 }
 
 // ============================================================= g2 batch
-// One warp per vertex: the reference's g2 (wannier.f90:903-1011, non-polar).
-__global__ void k_g2_batch(int nv, int nw, int nb, int nws, const double *qv, const int *R,
-                           const double *deg, const double2 *ek, const double2 *ekp,
-                           const double2 *eq, const double *ph_en, const double *masses,
-                           const double2 *gm, const int64_t *gm_index, int64_t gm_stride,
-                           const double2 *Lv, double *g2) {
+// |g|^2 of the vertices of a list (wannier.f90:903-1011) from their cell sums
+// G(n', m', s') = sum_R e^{2 pi i q.R} / deg gmixed(n', m', s', R), which come from one product
+// per right-hand side (launch_xgemm_chunks): one warp per vertex rotates them by the
+// electrons and the mode, lanes along (n', s').  row v of G is vertex perm[v].
+// The sum over cells comes first because it is linear in the given blocks: the
+// rotation then runs once per vertex instead of once per vertex and cell.
+__global__ void __launch_bounds__(128) k_g2_vertices(int nv, const int *perm, int64_t ld, int nw, int nb,
+                                                     const double2 *G, const double2 *ek, const double2 *ekp,
+                                                     const double2 *eq, const double *ph_en, const double *masses,
+                                                     const double2 *Lv, double *g2) {
   const int lane = threadIdx.x & 31;
-  const int v = blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5);
-  if (v >= nv) return;
-  double en = ph_en[v];
-  if (en == 0.0) { if (lane == 0) g2[v] = 0.0; return; }
-  const double2 *g = gm + (gm_index[v] - 1) * gm_stride;
+  const int row = blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5);
+  if (row >= nv) return;
+  const int64_t v = perm[row];
+  const double en = ph_en[v];
+  if (en == 0.0) {
+    if (lane == 0) g2[v] = 0.0;
+    return;
+  }
+  const double2 *g = G + (int64_t)row * nw * nw * nb;
   double2 gb = make_double2(0.0, 0.0);
-  for (int iws = lane; iws < nws; iws += 32) {
-    double2 ukgu = make_double2(0.0, 0.0);
-    for (int sp = 0; sp < nb; ++sp) {
-      double2 caux = make_double2(0.0, 0.0);
-      for (int np = 0; np < nw; ++np) {
-        double2 ckp = ekp[v + (int64_t)nv * np];
-        for (int mp = 0; mp < nw; ++mp) {
-          // overlap(mp,np) = conj(U_k'(np)) * U_k(mp)
-          double2 ov = cmul(cconj(ckp), ek[v + (int64_t)nv * mp]);
-          cfma(caux, ov, g[np + nw * (mp + (int64_t)nw * (sp + (int64_t)nb * iws))]);
-        }
-      }
-      double2 u = eq[v + (int64_t)nv * sp];
-      u = make_double2(u.x / sqrt(masses[sp / 3]), u.y / sqrt(masses[sp / 3]));
-      cfma(ukgu, u, caux);
-    }
-    double dot = qv[v] * (double)R[3 * iws];
-    dot += qv[v + nv] * (double)R[3 * iws + 1];
-    dot += qv[v + 2 * (int64_t)nv] * (double)R[3 * iws + 2];
-    double2 ph;
-    sincos(TWOPI * dot, &ph.y, &ph.x);
-    ph.x /= deg[iws];
-    ph.y /= deg[iws];
-    cfma(gb, ph, ukgu);
+  for (int o = lane; o < nw * nb; o += 32) {
+    const int np = o % nw, sp = o / nw;
+    double2 h = make_double2(0.0, 0.0);
+    for (int mp = 0; mp < nw; ++mp) cfma(h, ek[v + ld * mp], g[np + nw * (mp + (int64_t)nw * sp)]);
+    // conj(U_k'(n')) u(s') / sqrt(M)
+    const double rm = 1.0 / sqrt(masses[sp / 3]);
+    cfma(gb, cmul(cconj(ekp[v + ld * np]), cscale(eq[v + ld * sp], rm)), h);
   }
 #pragma unroll
   for (int o = 16; o > 0; o >>= 1) {
@@ -1005,25 +1017,21 @@ __global__ void k_g2_batch(int nv, int nw, int nb, int nws, const double *qv, co
     if (Lv) {   // polar: + long_range_prefac(q, u) * dot_product(el_evec_kp, el_evec_k) (wannier.f90:998-1006)
       double2 gl = make_double2(0.0, 0.0), unm = make_double2(0.0, 0.0);
       for (int sp = 0; sp < nb; ++sp) {
-        double2 u = eq[v + (int64_t)nv * sp];
+        double2 u = eq[v + ld * sp];
         u = make_double2(u.x / sqrt(masses[sp / 3]), u.y / sqrt(masses[sp / 3]));
         cfma(gl, Lv[(size_t)v * nb + sp], u);
       }
-      for (int c = 0; c < nw; ++c) cfma_cj(unm, ekp[v + (int64_t)nv * c], ek[v + (int64_t)nv * c]);
+      for (int c = 0; c < nw; ++c) cfma_cj(unm, ekp[v + ld * c], ek[v + ld * c]);
       cfma(gb, gl, unm);
     }
     g2[v] = 0.5 * (gb.x * gb.x + gb.y * gb.y) / en * g2unitfactor;
   }
 }
 
-void launch_g2_batch(int nv, int nw, int nb, int nws, const double *qv, const int *R,
-                     const double *deg, const double2 *ek, const double2 *ekp,
-                     const double2 *eq, const double *ph_en, const double *masses,
-                     const double2 *gm, const int64_t *gm_index, int64_t gm_stride,
-                     const double2 *Lv, double *g2, cudaStream_t st) {
-  if (nv <= 0) return;
-  k_g2_batch<<<(nv + 3) / 4, 128, 0, st>>>(nv, nw, nb, nws, qv, R, deg, ek, ekp, eq, ph_en,
-                                           masses, gm, gm_index, gm_stride, Lv, g2);
+void launch_g2_vertices(int nv, const int *perm, int64_t ld, int nw, int nb, const double2 *G, const double2 *ek,
+                        const double2 *ekp, const double2 *eq, const double *ph_en, const double *masses,
+                        const double2 *Lv, double *g2, cudaStream_t st) {
+  if (nv > 0) k_g2_vertices<<<(nv + 3) / 4, 128, 0, st>>>(nv, perm, ld, nw, nb, G, ek, ekp, eq, ph_en, masses, Lv, g2);
 }
 
 // ============================================================ q indices
@@ -1435,15 +1443,14 @@ void launch_final_states(int nwv, int nw, const int *widx, const double *ens, do
   k_final_states<<<(nwv + 127) / 128, 128, 0, st>>>(nwv, nw, widx, ens, enref, fsthick, cum, fin);
 }
 
-// Per (q, s): omega, 2 pi / hbar g2unitfactor / (2 omega) (0 below 0.5 meV), n(omega), e^(omega / kT)
-__global__ void k_mode_tab(int n, const double *om, const double *bose, double T, double const_tp, double4 *mt) {
+__global__ void k_mode_tab(int n, const double *om, const double *bose, double T, double const_tp, ModeRec *mt) {
   const int i = blockIdx.x * blockDim.x + threadIdx.x;
   if (i >= n) return;
   const double o = om[i];
-  mt[i] = make_double4(o, o >= 0.5e-3 ? const_tp * (0.5 / o * g2unitfactor) : 0.0, bose[i], exp(o / kB / T));
+  mt[i] = ModeRec{o, o >= 0.5e-3 ? const_tp * (0.5 / o * g2unitfactor) : 0.0, bose[i], exp(o / kB / T)};
 }
 
-void launch_mode_tab(int n, const double *om, const double *bose, double T, double const_tp, double4 *mt,
+void launch_mode_tab(int n, const double *om, const double *bose, double T, double const_tp, ModeRec *mt,
                      cudaStream_t st) {
   k_mode_tab<<<(n + 127) / 128, 128, 0, st>>>(n, om, bose, T, const_tp, mt);
 }
@@ -1517,36 +1524,36 @@ __global__ void __launch_bounds__(EPF_THREADS) k_epilogue_final(int j0, int ns, 
     double acc = 0.0;
     for (int s = 0; s < nb; ++s) {
       const int qs = q * nb + s;
-      const double4 mt = d.mt[qs];   // omega, prefactor, n, e^v
+      const ModeRec mt = d.mt[qs];
       double2 g = make_double2(0.0, 0.0);
       const double2 *u = d.u + (size_t)qs * nb;
       for (int sp = 0; sp < nb; ++sp) cfma(g, u[sp], h[sp]);
       if (d.glp) cfma(g, d.glp[qs], unm);   // long-range term (wannier.f90:998-1006)
       const double gg = fma(g.x, g.x, g.y * g.y);
       double xp = 0.0, xm = 0.0, y = 0.0;
-      if (mt.y != 0.0) {
+      if (mt.cx != 0.0) {
         double dp, dm;
         if (SIMPLEX) {
-          dp = simplex_delta(d.sx, f, E + mt.x) * dnorm;
-          dm = simplex_delta(d.sx, f, E - mt.x) * dnorm;
+          dp = simplex_delta(d.sx, f, E + mt.om) * dnorm;
+          dm = simplex_delta(d.sx, f, E - mt.om) * dnorm;
         } else {
-          const double tp = ((E + mt.x) - eps) * isig, tm = ((E - mt.x) - eps) * isig;
+          const double tp = ((E + mt.om) - eps) * isig, tm = ((E - mt.om) - eps) * isig;
           dp = dnorm * exp(-0.5 * tp * tp);
           dm = dnorm * exp(-0.5 * tm * tm);
         }
-        double A = fma(ex, mt.w, 1.0), B = fma(emx, mt.w, 1.0);
-        if (mt.w > 1e260) {   // omega / kT > 600: the factors may leave FP64's range one by one
-          const double v = mt.x / kT;
+        double A = fma(ex, mt.ev, 1.0), B = fma(emx, mt.ev, 1.0);
+        if (mt.ev > 1e260) {   // omega / kT > 600: the factors may leave FP64's range one by one
+          const double v = mt.om / kT;
           A = 1.0 + exp(x + v);
           B = 1.0 + exp(v - x);
         }
-        const double gc = gg * mt.y, fp = 1.0 / A;
-        xp = gc * (mt.z + fp) * dp;
-        xm = gc * (mt.z + 1.0 / B) * dm;
+        const double gc = gg * mt.cx, fp = 1.0 / A;
+        xp = gc * (mt.bose + fp) * dp;
+        xm = gc * (mt.bose + 1.0 / B) * dm;
         if (PH) {
           // Y: delta(E' - omega) at the initial electron (k, m), interactions.f90:1862; the Gaussian is even
-          const double dy = SIMPLEX ? simplex_delta(d.sx, j, eps - mt.x) * dnorm : dp;
-          y = gc * (f1 * (1.0 - fp) / (1.0 + mt.z)) * dy;
+          const double dy = SIMPLEX ? simplex_delta(d.sx, j, eps - mt.om) * dnorm : dp;
+          y = gc * (f1 * (1.0 - fp) / (1.0 + mt.bose)) * dy;
           if (d.phr && y != 0.0) atomicAdd(d.phr + q + (size_t)rp.N * s, d.ph_scale * y);
         }
       }
@@ -1554,7 +1561,7 @@ __global__ void __launch_bounds__(EPF_THREADS) k_epilogue_final(int j0, int ns, 
       if (d.g2) {
         const int64_t off = (int64_t)j * d.per_state + (int64_t)f * nb + s;
         if (off < d.cap) {
-          d.g2[off] = mt.x == 0.0 ? 0.0 : 0.5 * gg / mt.x * g2unitfactor;
+          d.g2[off] = mt.om == 0.0 ? 0.0 : 0.5 * gg / mt.om * g2unitfactor;
           if (d.xp) d.xp[off] = xp;
           if (d.xm) d.xm[off] = xm;
           if (d.yv) d.yv[off] = y;

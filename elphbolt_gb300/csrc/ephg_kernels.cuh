@@ -14,6 +14,9 @@ void launch_phase_mesh(int nrows, const int *rowp, const int mesh[3], int L, int
 // same for arbitrary fractional k: kv (nrows,3) column-major as the reference
 void launch_phase_frac(int nrows, const double *kv, int nR, const int *R, const double *deg,
                        double2 *out, int64_t ldo, cudaStream_t st);
+// the same for the vectors perm[0..nrows) of kv (column stride ldk), / deg; rows of nR
+void launch_phase_list(int nrows, const double *kv, int64_t ldk, const int *perm, int nR, const int *R,
+                       const double *deg, double2 *out, cudaStream_t st);
 
 // out[p][e] = sum_R e^{2 pi i k_p.R} X(R)[e] for every point p of the mesh (muxed
 // order), X given on the box of cell coordinates [lo, lo + ext) per dimension
@@ -94,13 +97,12 @@ void launch_permute_gwann(int nw, int nb, int nwsk, int nwsg, const double2 *raw
 void launch_permute_greq(int nq, int nw, int nb, int nwsk, const double2 *in, double2 *out,
                          cudaStream_t st);
 
-// ---- g2 batched (wannier.f90:903-1011) ----
-// Lv (nv, nb), nullable: the polar long-range vector of each vertex's q (launch_polar_q)
-void launch_g2_batch(int nv, int nw, int nb, int nws, const double *qv, const int *R,
-                     const double *deg, const double2 *ek, const double2 *ekp,
-                     const double2 *eq, const double *ph_en, const double *masses,
-                     const double2 *gm, const int64_t *gm_index, int64_t gm_stride,
-                     const double2 *Lv, double *g2, cudaStream_t st);
+// ---- g2 of a vertex list (wannier.f90:903-1011) ----
+// G (nv rows of nw nw nb): the cell sums of vertices perm[0..nv); the vertex arrays' column
+// stride is ld.  Lv (ld, nb), nullable: the polar long-range vector of each vertex's q
+void launch_g2_vertices(int nv, const int *perm, int64_t ld, int nw, int nb, const double2 *G, const double2 *ek,
+                        const double2 *ekp, const double2 *eq, const double *ph_en, const double *masses,
+                        const double2 *Lv, double *g2, cudaStream_t st);
 
 // ---- polar long-range terms (wannier.f90:784-901, 1013-1071) ----
 // Crystal data of a polar crystal on the device (ephg_set_polar).  The Ewald
@@ -148,6 +150,10 @@ void launch_iota(int n, int *out, cudaStream_t st);
 void launch_rotate_states_fp64(int j0, int j1, int i0, const int *st_code, int nw, int nb, int nws, int64_t blk0,
                                int64_t nblk, const int *widx, const double2 *U, const double2 *gk, int64_t ldgk,
                                const double2 *phk, double2 *B, int64_t ldb, int sc, int nst, cudaStream_t st);
+// Per (q, s), FP64 epilogue: omega, 2 pi / hbar g2unitfactor / (2 omega) (0 below 0.5 meV), n(omega), e^(omega / kT)
+struct alignas(16) ModeRec {
+  double om, cx, bose, ev;
+};
 // Triangle / tetrahedron deltas of the final states as tables (launch_simplex_tab):
 // per final state the sorted breakpoints b (key: rounded to FP32) and for each the
 // Bernstein coefficients (lo, hi) of the interval that ends there.
@@ -175,7 +181,7 @@ struct EpiData {
   // launch_mode_tab and, for the triangle / tetrahedron deltas, theirs
   const int2 *fin;
   int nin;
-  const double4 *mt;
+  const ModeRec *mt;
   SimplexTab sx;
   int64_t per_state;    // vertices per initial state
   double *g2, *xp, *xm; // optional vertex lists
@@ -200,7 +206,7 @@ struct RateSets {
   int n;
   RateParams rp[MAX_SETS];
   double *bose[MAX_SETS];      // [q][s] per set (set 0: EpiData.bose)
-  const double4 *mt[MAX_SETS]; // FP64 epilogue: [q][s] per set (set 0: EpiData.mt)
+  const ModeRec *mt[MAX_SETS]; // FP64 epilogue: [q][s] per set (set 0: EpiData.mt)
   double *partial[MAX_SETS];   // [j][iblk] per set (set 0: the caller's partial)
 };
 // Final states of the window rows in order: fin[cum[ip] + rank] = (ip, band)
@@ -209,8 +215,8 @@ void launch_final_states(int nwv, int nw, const int *widx, const double *ens, do
 // The simplex tables of nin final states (kind 1 triangles, 2 tetrahedra); rowmap: mesh point -> window row or -1
 void launch_simplex_tab(int kind, const int mesh[3], int nin, const int2 *fin, const int *widx, const int *rowmap,
                         const double *ens, int nw, const SimplexTab &t, cudaStream_t st);
-// mt[q][s] = (omega, 2 pi / hbar g2unitfactor / (2 omega) or 0 below 0.5 meV, n, e^(omega / kT))
-void launch_mode_tab(int n, const double *om, const double *bose, double T, double const_tp, double4 *mt,
+// the mode table of n (q, s)
+void launch_mode_tab(int n, const double *om, const double *bose, double T, double const_tp, ModeRec *mt,
                      cudaStream_t st);
 // FP64 epilogue over the states [j0, j1): the Rp sums G(x = n' + nw s') of (window row ip,
 // state j) at ip ldc + x xs + (j - j0) js, in FP64 (z) or as FP32 planes (re, im).  Rate

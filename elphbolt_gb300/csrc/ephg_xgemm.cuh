@@ -1,0 +1,35 @@
+// ephg_xgemm.cuh - FP64 complex products on the tensor cores by exact splitting.
+#pragma once
+#include <mutex>
+
+#include "ephg_ws.cuh"
+
+namespace ephg {
+
+// Column exponents of a right-hand side kept with its owner (the handle's resident
+// operands): built on first use, then read by every product with it.
+struct ColExp {
+  int *e = nullptr;
+  std::mutex mu;
+};
+
+// C[M][N] = A[M][K] B[K][N], complex FP64, row-major, |A| <= 1 (phases).  cexp: B's column
+// exponents (nullable: formed per call in ws).  err: device error word of the bounded waits.
+// Returns 0, or an EPHG_ERR code with ws.msg set.
+int launch_xgemm(Workspace &ws, int M, int64_t N, int K, const double2 *A, int64_t lda, const double2 *B, int64_t ldb,
+                 const int *cexp, double2 *C, int64_t ldc, int *err, cudaStream_t st);
+// Rows of A against several right-hand sides in one launch: chunk c (device) is (first row, rows
+// <= XG_CHUNK, right-hand side); right-hand side b is B + b bstride, [K][N] at stride N.
+// cexp: the nrhs x N exponents of xgemm_colexp.
+constexpr int XG_CHUNK = 32;
+int xgemm_colexp(Workspace &ws, int64_t nrhs, int64_t N, int K, const double2 *B, int64_t bstride, const int **cexp,
+                 cudaStream_t st);
+int launch_xgemm_chunks(Workspace &ws, const int4 *chunks, int nchunks, int rows, int64_t N, int K, const double2 *A,
+                        int64_t lda, const double2 *B, int64_t bstride, const int *cexp, double2 *C, int64_t ldc,
+                        int *err, cudaStream_t st);
+// The exponents of a resident operand B[K][N], built once (allocated from the library pool on st
+// and complete when this returns); *bytes grows by what was allocated.
+int resident_colexp(ColExp &x, int64_t N, int K, const double2 *B, int64_t ldb, int64_t *bytes, cudaStream_t st,
+                    const int **out);
+
+}  // namespace ephg
