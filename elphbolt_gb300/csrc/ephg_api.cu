@@ -231,9 +231,9 @@ int ephg_trim_memory(void) {
 int ephg_destroy(ephg_handle *h) {
   if (!h) return EPHG_OK;
   void *ptrs[] = {h->Rk, h->Rq, h->Rg, h->degk, h->degq, h->degg, h->Hext, h->Hbox, h->Dbox, h->graw, h->G64,
-                  h->masses, h->pair_off, h->ent_iuc, h->ent_woff, h->wrapR, h->ent_rden,
-                  h->rcartq, h->D, h->err, h->kposk, h->kposq, h->polar_G, h->polar_Gcell,
-                  h->polar_born, h->polar_tau, h->polar_Da, h->cellk_tab, h->cellq_tab, h->rdegk, h->exp_H.e, h->exp_G.e, h->exp_raw.e};
+                  h->masses, h->Dcell, h->RD, h->err, h->kposk, h->kposq, h->polar_G, h->polar_Gcell,
+                  h->polar_born, h->polar_tau, h->polar_Da, h->polar_Gf, h->cellk_tab, h->cellq_tab, h->rdegk, h->exp_H.e, h->exp_G.e, h->exp_raw.e,
+                  h->exp_D.e};
   // stream-ordered frees back to the library pool, which keeps the memory
   // mapped for the next handle
   for (void *p : ptrs)
@@ -300,6 +300,15 @@ int ephg_create(const ephg_wannier_desc *d, ephg_handle **out) {
       (rc = upload(&h->degq, dq.data(), dq.size(), h->st, &h->resident_bytes)) || (rc = upload(&h->degg, dg.data(), dg.size(), h->st, &h->resident_bytes)) ||
       (rc = upload(&h->masses, d->masses, (size_t)h->nat, h->st, &h->resident_bytes)))
     return bail(rc);
+  for (int c = 0; c < 3; ++c) {   // range of the Rp coordinates
+    int lo = nwsq > 0 ? rq[c] : 0, hi = lo;
+    for (int r = 0; r < nwsq; ++r) {
+      lo = std::min(lo, rq[3 * r + c]);
+      hi = std::max(hi, rq[3 * r + c]);
+    }
+    h->qlo[c] = lo;
+    h->qext[c] = hi - lo + 1;
+  }
   {   // the cells of the two Fourier sums of g
     auto cells = [&](const std::vector<int> &r, int n, CellTab &t, int **dev) -> int {
       std::vector<int> tab;
@@ -369,104 +378,89 @@ int ephg_create(const ephg_wannier_desc *d, ephg_handle **out) {
     h->resident_bytes += (int64_t)(n * sizeof(double2));
     launch_permute_gwann(nw, nb, nwsk, nwsq, h->graw, h->G64, h->st);
   }
-  // phonon terms: for each atom pair and WS cell, the shortest wraps
+  // Phonon terms.  D(q) is one Fourier sum per element over the wrapped vectors R':
+  // X_ab(R') = massnorm_ab sum of D(iuc)_ab / (deg nwrap) over the (pair(a, b), iuc) whose
+  // shortest wraps include R', and its q derivatives the sums of i rcart(iuc) times the
+  // same terms.  On a mesh X runs on the box of R' (launch_mesh_fourier), at arbitrary
+  // q the distinct R' are the cells of one product (ph_wann).
   {
-    std::vector<int> pair_off(h->nat * h->nat + 1, 0), ent_iuc, ent_woff(1, 0), wrapR;
-    std::vector<double> ent_rden;
-    for (int jat = 0; jat < h->nat; ++jat)
-      for (int iat = 0; iat < h->nat; ++iat) {
-        int pair = iat + h->nat * jat;
-        pair_off[pair] = (int)ent_iuc.size();
+    const int nat = h->nat, ne = nb * nb;
+    struct Wrap {
+      int r[3];
+      double rden;
+    };
+    std::vector<Wrap> wraps;
+    std::vector<int> woff(1, 0);   // wraps of entry (pair = iat + nat jat, iuc), in that order
+    for (int jat = 0; jat < nat; ++jat)
+      for (int iat = 0; iat < nat; ++iat)
         for (int iuc = 0; iuc < nwsq; ++iuc) {
           double dist[3];
           for (int c = 0; c < 3; ++c)
-            dist[c] = ((double)rq[3 * iuc + c] - d->basis[c + 3 * iat] + d->basis[c + 3 * jat]) /
-                      (double)h->cq[c];
-          std::vector<int> w = ws_wrap(h->lattvecs, dist, 1.0e-6);
-          int nwrap = (int)w.size() / 3;
-          ent_iuc.push_back(iuc);
-          ent_rden.push_back(1.0 / (double)(d->phwsdeg[iuc] * nwrap));
-          for (int iw = 0; iw < nwrap; ++iw)
-            for (int c = 0; c < 3; ++c) wrapR.push_back(rq[3 * iuc + c] + w[3 * iw + c] * h->cq[c]);
-          ent_woff.push_back((int)wrapR.size() / 3);
+            dist[c] = ((double)rq[3 * iuc + c] - d->basis[c + 3 * iat] + d->basis[c + 3 * jat]) / (double)h->cq[c];
+          const std::vector<int> w = ws_wrap(h->lattvecs, dist, 1.0e-6);
+          const int nwrap = (int)w.size() / 3;
+          for (int iw = 0; iw < nwrap; ++iw) {
+            Wrap x;
+            for (int c = 0; c < 3; ++c) x.r[c] = rq[3 * iuc + c] + w[3 * iw + c] * h->cq[c];
+            x.rden = 1.0 / (double)(d->phwsdeg[iuc] * nwrap);
+            wraps.push_back(x);
+          }
+          woff.push_back((int)wraps.size());
         }
+    for (int c = 0; c < 3; ++c) {
+      int lo = wraps.empty() ? 0 : wraps[0].r[c], hi = lo;
+      for (const Wrap &x : wraps) {
+        lo = std::min(lo, x.r[c]);
+        hi = std::max(hi, x.r[c]);
       }
-    // pair_off must be monotone over the pair index order used by the kernel
-    {
-      std::vector<int> off(h->nat * h->nat + 1);
-      int cur = 0;
-      for (int p = 0; p < h->nat * h->nat; ++p) {
-        off[p] = cur;
-        cur += nwsq;
-      }
-      off[h->nat * h->nat] = cur;
-      // entries were appended in jat-major order, identical to pair = iat + nat*jat
-      pair_off = off;
+      h->dlo[c] = lo;
+      h->dext[c] = hi - lo + 1;
     }
-    std::vector<double> rcq((size_t)nwsq * 3);
-    for (int r = 0; r < nwsq; ++r)
-      for (int i = 0; i < 3; ++i)
-        rcq[r + (size_t)nwsq * i] = h->lattvecs[i] * rq[3 * r] + h->lattvecs[i + 3] * rq[3 * r + 1] +
-                                    h->lattvecs[i + 6] * rq[3 * r + 2];
-    if ((rc = upload(&h->pair_off, pair_off.data(), pair_off.size(), h->st, &h->resident_bytes)) ||
-        (rc = upload(&h->ent_iuc, ent_iuc.data(), ent_iuc.size(), h->st, &h->resident_bytes)) ||
-        (rc = upload(&h->ent_woff, ent_woff.data(), ent_woff.size(), h->st, &h->resident_bytes)) ||
-        (rc = upload(&h->wrapR, wrapR.data(), wrapR.size(), h->st, &h->resident_bytes)) ||
-        (rc = upload(&h->ent_rden, ent_rden.data(), ent_rden.size(), h->st, &h->resident_bytes)) ||
-        (rc = upload(&h->rcartq, rcq.data(), rcq.size(), h->st, &h->resident_bytes)) ||
-        (rc = upload(&h->D, (const double2 *)d->Dphwann, (size_t)nwsq * nb * nb, h->st, &h->resident_bytes)))
-      return bail(rc);
-    // D(q) on a mesh as one Fourier sum per element over the wrapped vectors R':
-    // X_ab(R') = massnorm_ab sum of rden D(iuc)_ab over the (pair(a, b), iuc)
-    // entries whose wraps include R' (k_dbuild's sum, regrouped)
-    {
-      const int ne = nb * nb;
-      int lo3[3] = {0, 0, 0}, hi3[3] = {0, 0, 0};
-      const int nwr = (int)(wrapR.size() / 3);
-      for (int c = 0; c < 3; ++c) {
-        lo3[c] = hi3[c] = nwr > 0 ? wrapR[c] : 0;
-        for (int i = 0; i < nwr; ++i) {
-          lo3[c] = std::min(lo3[c], wrapR[3 * i + c]);
-          hi3[c] = std::max(hi3[c], wrapR[3 * i + c]);
-        }
-        h->dlo[c] = lo3[c];
-        h->dext[c] = hi3[c] - lo3[c] + 1;
+    const size_t nbox = (size_t)h->dext[0] * h->dext[1] * h->dext[2];
+    if (nbox > ((size_t)1 << 22)) return bail(fail(EPHG_ERR_ARG, "phonon cells span too large a box"));
+    auto box = [&](const Wrap &x) {
+      return ((size_t)(x.r[0] - h->dlo[0]) * h->dext[1] + (x.r[1] - h->dlo[1])) * h->dext[2] + (x.r[2] - h->dlo[2]);
+    };
+    std::vector<int> slot(nbox, -1), cells;   // distinct R', in box order
+    for (const Wrap &x : wraps) slot[box(x)] = 0;
+    for (size_t b = 0; b < nbox; ++b)
+      if (slot[b] == 0) {
+        slot[b] = h->nD++;
+        cells.insert(cells.end(), {(int)(b / ((size_t)h->dext[1] * h->dext[2])) + h->dlo[0],
+                                   (int)(b / h->dext[2] % h->dext[1]) + h->dlo[1], (int)(b % h->dext[2]) + h->dlo[2]});
       }
-      const size_t nbox = (size_t)h->dext[0] * h->dext[1] * h->dext[2];
-      if (nbox > ((size_t)1 << 22)) return bail(fail(EPHG_ERR_ARG, "phonon cells span too large a box"));
-      std::vector<double2> xb(nbox * ne, make_double2(0.0, 0.0));
-      const double2 *Dw = (const double2 *)d->Dphwann;
-      for (int e = 0; e < ne; ++e) {
-        const int a = e % nb, b = e / nb;
-        const int pair = (a / 3) + h->nat * (b / 3);
-        const double massnorm = 1.0 / std::sqrt(d->masses[a / 3] * d->masses[b / 3]) * Ryd2amu;
-        for (int iuc = 0; iuc < nwsq; ++iuc) {
-          const int en = pair * nwsq + iuc;   // entries (pair, cell) in cell order
-          const double2 dv = Dw[iuc + (size_t)nwsq * (a + (size_t)nb * b)];
-          const double f = ent_rden[en] * massnorm;
-          for (int wv = ent_woff[en]; wv < ent_woff[en + 1]; ++wv) {
-            const size_t cell =
-                ((size_t)(wrapR[3 * wv] - lo3[0]) * h->dext[1] + (wrapR[3 * wv + 1] - lo3[1])) * h->dext[2] +
-                (wrapR[3 * wv + 2] - lo3[2]);
-            xb[cell * ne + e].x += f * dv.x;
-            xb[cell * ne + e].y += f * dv.y;
+    std::vector<double2> xb(nbox * ne, make_double2(0.0, 0.0)), xc((size_t)h->nD * 4 * ne, make_double2(0.0, 0.0));
+    const double2 *Dw = (const double2 *)d->Dphwann;
+    for (int e = 0; e < ne; ++e) {
+      const int a = e % nb, b = e / nb;
+      const int pair = (a / 3) + nat * (b / 3);
+      const double massnorm = 1.0 / std::sqrt(d->masses[a / 3] * d->masses[b / 3]) * Ryd2amu;
+      for (int iuc = 0; iuc < nwsq; ++iuc) {
+        const int en = pair * nwsq + iuc;
+        const double2 dv = Dw[iuc + (size_t)nwsq * (a + (size_t)nb * b)];
+        double rc3[3];
+        for (int i = 0; i < 3; ++i)
+          rc3[i] = h->lattvecs[i] * rq[3 * iuc] + h->lattvecs[i + 3] * rq[3 * iuc + 1] + h->lattvecs[i + 6] * rq[3 * iuc + 2];
+        for (int wv = woff[en]; wv < woff[en + 1]; ++wv) {
+          const double f = wraps[wv].rden * massnorm;
+          const double2 t = make_double2(f * dv.x, f * dv.y);
+          const size_t at = box(wraps[wv]);
+          double2 *x = &xb[at * ne + e], *y = &xc[(size_t)slot[at] * 4 * ne + e];
+          x->x += t.x;
+          x->y += t.y;
+          y->x += t.x;
+          y->y += t.y;
+          for (int i = 0; i < 3; ++i) {
+            y[(1 + i) * ne].x -= rc3[i] * t.y;
+            y[(1 + i) * ne].y += rc3[i] * t.x;
           }
         }
       }
-      if ((rc = upload(&h->Dbox, xb.data(), xb.size(), h->st, &h->resident_bytes))) return bail(rc);
     }
-    h->terms.npair = h->nat * h->nat;
-    h->terms.pair_off = h->pair_off;
-    h->terms.ent_iuc = h->ent_iuc;
-    h->terms.ent_woff = h->ent_woff;
-    h->terms.wrapR = h->wrapR;
-    h->terms.ent_rden = h->ent_rden;
-    h->terms.D = h->D;
-    h->terms.rcart = h->rcartq;
-    h->terms.masses = h->masses;
-    h->terms.nwsq = nwsq;
-    h->terms.nb = nb;
-    h->terms.nat = h->nat;
+    if ((rc = upload(&h->Dbox, xb.data(), xb.size(), h->st, &h->resident_bytes)) ||
+        (rc = upload(&h->Dcell, xc.data(), xc.size(), h->st, &h->resident_bytes)) ||
+        (rc = upload(&h->RD, cells.data(), cells.size(), h->st, &h->resident_bytes)))
+      return bail(rc);
   }
   // contraction order of the split form: cells by decreasing |R| (ties by index),
   // so that the decaying Wannier-space terms are summed smallest first
@@ -508,11 +502,12 @@ int ephg_set_polar(ephg_handle *h, const double *epsilon, const double *born) {
   if (!h) return fail(EPHG_ERR_ARG, "set_polar: bad arguments");
   if (epsilon && !born) return fail(EPHG_ERR_ARG, "set_polar: born effective charges are required");
   for (void *p : {(void *)h->polar_G, (void *)h->polar_Gcell, (void *)h->polar_born, (void *)h->polar_tau,
-                  (void *)h->polar_Da})
+                  (void *)h->polar_Da, (void *)h->polar_Gf})
     if (p) cudaFreeAsync(p, h->st);
   CK(cudaStreamSynchronize(h->st));
   h->polar_G = h->polar_Gcell = h->polar_born = h->polar_tau = nullptr;
   h->polar_Da = nullptr;
+  h->polar_Gf = nullptr;
   h->polar_on = false;
   if (!epsilon) return EPHG_OK;   // non-polar
   const double bohr2nm = 0.052917721092, pi = 4.0 * atan(1.0), twopi = 2.0 * pi;   // params.f90
@@ -572,7 +567,9 @@ int ephg_set_polar(ephg_handle *h, const double *epsilon, const double *born) {
   P.Mcell = (int)(Gc.size() / 3);
   P.masses = h->masses;
   int rc;
-  if ((rc = upload(&h->polar_G, G.data(), G.size(), h->st)) ||
+  std::vector<float> Gf(G.begin(), G.end());
+  Gf.insert(Gf.end(), Gc.begin(), Gc.end());
+  if ((rc = upload(&h->polar_Gf, Gf.data(), Gf.size(), h->st)) || (rc = upload(&h->polar_G, G.data(), G.size(), h->st)) ||
       (rc = upload(&h->polar_Gcell, Gc.data(), Gc.size(), h->st)) ||
       (rc = upload(&h->polar_born, born, 9 * (size_t)nat, h->st)) ||
       (rc = upload(&h->polar_tau, tau.data(), tau.size(), h->st)))
@@ -580,6 +577,8 @@ int ephg_set_polar(ephg_handle *h, const double *epsilon, const double *born) {
   CK(pool_alloc((void **)&h->polar_Da, (size_t)nb * nb * sizeof(double2), h->st));
   P.G = h->polar_G;
   P.Gcell = h->polar_Gcell;
+  P.Gf = h->polar_Gf;
+  P.Gcellf = h->polar_Gf + G.size();
   P.born = h->polar_born;
   P.tau = h->polar_tau;
   launch_polar_da(P, h->polar_Da, h->st);
@@ -712,9 +711,9 @@ int ephg_el_wann(ephg_handle *h, int64_t nk, const double *kvecs, double *energi
     CK(cudaMemcpyAsync(sc, scissor, nw * sizeof(double), cudaMemcpyHostToDevice, h->st));
   }
   CK(cudaMemcpyAsync(kv, kvecs, (size_t)nk * 3 * sizeof(double), cudaMemcpyHostToDevice, h->st));
-  launch_phase_frac((int)nk, kv, nwsk, h->Rk, h->degk, P, nwsk, h->st);
+  launch_phase_cells((int)nk, kv, nk, nullptr, nwsk, h->Rk, h->degk, h->hlo, h->hext, P, nwsk, h->st);
   const int *ce;
-  if ((rc = resident_colexp(h->exp_H, 4 * (int64_t)nn, nwsk, h->Hext, 4 * (int64_t)nn, &h->resident_bytes, h->st, &ce)))
+  if ((rc = resident_colexp(h->exp_H, 1, 4 * (int64_t)nn, nwsk, h->Hext, 0, &h->resident_bytes, h->st, &ce)))
     return fail(rc, "el_wann: column exponents");
   if ((rc = launch_xgemm(h->ws, (int)nk, ncol, nwsk, P, nwsk, h->Hext, 4 * (int64_t)nn, ce, C, ncol, h->err, h->st)))
     return WSFAIL(rc);
@@ -740,22 +739,35 @@ int ephg_ph_wann(ephg_handle *h, int64_t nq, const double *qvecs, double *energi
   const int nb = h->nb;
   const size_t nn = (size_t)nb * nb;
   const int with_vel = velocities != nullptr;
+  const int ncol = (with_vel ? 4 : 1) * (int)nn;   // D(q), then its three derivatives
+  const int64_t qb = std::max<int64_t>(1, std::min<int64_t>(nq, ((int64_t)1 << 28) / (16 * std::max(1, h->nD))));
   double *qv, *w, *ens, *vel;
-  double2 *Dq, *dDq, *V, *ev;
+  double2 *P, *Dq, *V, *ev;
   int rc;
-  if ((rc = wsget(h->ws, "ph_qv", (size_t)nq * 3, &qv)) || (rc = wsget(h->ws, "ph_D", (size_t)nq * nn, &Dq)) ||
-      (rc = wsget(h->ws, "ph_dD", with_vel ? (size_t)nq * 3 * nn : 1, &dDq)) ||
+  if ((rc = wsget(h->ws, "ph_qv", (size_t)nq * 3, &qv)) || (rc = wsget(h->ws, "ph_D", (size_t)nq * ncol, &Dq)) ||
+      (rc = wsget(h->ws, "ph_P", (size_t)qb * h->nD, &P)) ||
       (rc = wsget(h->ws, "ph_w", (size_t)nq * nb, &w)) || (rc = wsget(h->ws, "ph_V", (size_t)nq * nn, &V)) ||
       (rc = wsget(h->ws, "ph_e", (size_t)nq * nb, &ens)) ||
       (rc = wsget(h->ws, "ph_vel", with_vel ? (size_t)nq * nb * 3 : 1, &vel)) ||
       (rc = wsget(h->ws, "ph_ev", evecs ? (size_t)nq * nn : 1, &ev)))
     return WSFAIL(rc);
+  const int *ce;
+  if ((rc = resident_colexp(h->exp_D, 1, 4 * (int64_t)nn, h->nD, h->Dcell, 0, &h->resident_bytes, h->st, &ce)))
+    return fail(rc, "ph_wann: column exponents");
   CK(cudaMemcpyAsync(qv, qvecs, (size_t)nq * 3 * sizeof(double), cudaMemcpyHostToDevice, h->st));
-  launch_dbuild((int)nq, nullptr, nullptr, 1, nullptr, qv, h->terms, with_vel, Dq, dDq, h->st);
+  for (int64_t q0 = 0; q0 < nq; q0 += qb) {
+    const int n = (int)std::min(qb, nq - q0);
+    launch_phase_cells(n, qv + q0, nq, nullptr, h->nD, h->RD, nullptr, h->dlo, h->dext, P, h->nD, h->st);
+    if ((rc = launch_xgemm(h->ws, n, ncol, h->nD, P, h->nD, h->Dcell, 4 * (int64_t)nn, ce, Dq + q0 * ncol, ncol, h->err,
+                           h->st)))
+      return WSFAIL(rc);
+    h->launches += 3;
+  }
+  double2 *dDq = Dq + nn;
   if (h->polar_on)   // non-analytic correction (wannier.f90:684-705)
-    launch_polar_q(h->polar, (int)nq, nullptr, nullptr, qv, Dq, with_vel ? dDq : nullptr, nullptr, h->st);
-  launch_heig((int)nq, nb, Dq, nn, w, V, h->err, h->st);
-  launch_ph_post((int)nq, nb, nullptr, qv, w, V, dDq, with_vel, h->masses, ens,
+    launch_polar_q(h->polar, (int)nq, nullptr, nullptr, qv, Dq, with_vel ? dDq : nullptr, ncol, nullptr, h->st);
+  launch_heig((int)nq, nb, Dq, ncol, w, V, h->err, h->st);
+  launch_ph_post((int)nq, nb, nullptr, qv, w, V, dDq, ncol, with_vel, h->masses, ens,
                  evecs ? ev : nullptr, with_vel ? vel : nullptr, nullptr, nullptr, nullptr, h->err,
                  h->st);
   h->launches += 3;
@@ -779,7 +791,7 @@ int ephg_gkRp(ephg_handle *h, int64_t nk, const double *kvecs, double *gmixed) {
       (rc = wsget(h->ws, "gk_C", (size_t)chunk * h->Nn, &C)))
     return WSFAIL(rc);
   const int *ce;
-  if ((rc = resident_colexp(h->exp_G, h->Nn, nwsk, h->G64, h->Nn, &h->resident_bytes, h->st, &ce)))
+  if ((rc = resident_colexp(h->exp_G, 1, h->Nn, nwsk, h->G64, 0, &h->resident_bytes, h->st, &ce)))
     return fail(rc, "gkRp: column exponents");
   std::vector<double> kc((size_t)chunk * 3);
   for (int64_t k0 = 0; k0 < nk; k0 += chunk) {
@@ -787,7 +799,7 @@ int ephg_gkRp(ephg_handle *h, int64_t nk, const double *kvecs, double *gmixed) {
     for (int c = 0; c < 3; ++c)
       for (int64_t i = 0; i < n; ++i) kc[i + n * c] = kvecs[(k0 + i) + nk * c];
     CK(cudaMemcpyAsync(kv, kc.data(), (size_t)n * 3 * sizeof(double), cudaMemcpyHostToDevice, h->st));
-    launch_phase_frac((int)n, kv, nwsk, h->Rk, h->degk, P, nwsk, h->st);
+    launch_phase_cells((int)n, kv, n, nullptr, nwsk, h->Rk, h->degk, h->hlo, h->hext, P, nwsk, h->st);
     if ((rc = launch_xgemm(h->ws, (int)n, h->Nn, nwsk, P, nwsk, h->G64, h->Nn, ce, C, h->Nn, h->err, h->st)))
       return WSFAIL(rc);
     h->launches += 3;
@@ -813,7 +825,7 @@ int ephg_gReq(ephg_handle *h, int64_t nq, const double *qvecs, double *gmixed) {
       (rc = wsget(h->ws, "gq_C", (size_t)chunk * per, &C)) || (rc = wsget(h->ws, "gq_O", (size_t)chunk * per, &O)))
     return WSFAIL(rc);
   const int *ce;
-  if ((rc = resident_colexp(h->exp_raw, per, nwsg, h->graw, per, &h->resident_bytes, h->st, &ce)))
+  if ((rc = resident_colexp(h->exp_raw, 1, per, nwsg, h->graw, 0, &h->resident_bytes, h->st, &ce)))
     return fail(rc, "gReq: column exponents");
   std::vector<double> qc((size_t)chunk * 3);
   for (int64_t q0 = 0; q0 < nq; q0 += chunk) {
@@ -822,7 +834,7 @@ int ephg_gReq(ephg_handle *h, int64_t nq, const double *qvecs, double *gmixed) {
       for (int64_t i = 0; i < n; ++i) qc[i + n * c] = qvecs[(q0 + i) + nq * c];
     CK(cudaMemcpyAsync(qv, qc.data(), (size_t)n * 3 * sizeof(double), cudaMemcpyHostToDevice, h->st));
     // sum_Rp e^{2 pi i q.Rp}/gwsdeg * g(i,j,Re,s,Rp): rows of the raw array are Rp
-    launch_phase_frac((int)n, qv, nwsg, h->Rg, h->degg, P, nwsg, h->st);
+    launch_phase_cells((int)n, qv, n, nullptr, nwsg, h->Rg, h->degg, h->qlo, h->qext, P, nwsg, h->st);
     if ((rc = launch_xgemm(h->ws, (int)n, per, nwsg, P, nwsg, h->graw, per, ce, C, per, h->err, h->st)))
       return WSFAIL(rc);
     launch_permute_greq((int)n, nw, nb, nwsk, C, O, h->st);
@@ -902,7 +914,7 @@ int ephg_g2(ephg_handle *h, int64_t wannspace, int64_t nv, const double *kvecs,
       CK(cudaMemcpyAsync(qp, qvecs, (size_t)nv * 3 * sizeof(double), cudaMemcpyHostToDevice, h->st));
     }
     if ((rc = wsget(h->ws, "g2_L", (size_t)nv * nb, &Lv))) return WSFAIL(rc);
-    launch_polar_q(h->polar, (int)nv, nullptr, nullptr, qp, nullptr, nullptr, Lv, h->st);
+    launch_polar_q(h->polar, (int)nv, nullptr, nullptr, qp, nullptr, nullptr, 0, Lv, h->st);
     h->launches += 1;
   }
   const int *ce;
@@ -910,9 +922,10 @@ int ephg_g2(ephg_handle *h, int64_t wannspace, int64_t nv, const double *kvecs,
   for (size_t p = 0; p + 1 < piece.size(); ++p) {
     const int64_t r0 = piece[p].first, c0 = piece[p].second;
     const int n = (int)(piece[p + 1].first - r0);
-    launch_phase_list(n, qv, nv, pd + r0, nws, R, deg, P, h->st);
-    if ((rc = launch_xgemm_chunks(h->ws, cd + c0, (int)(piece[p + 1].second - c0), n, per, nws, P, nws, gm, gstride, ce,
-                                  G, per, h->err, h->st)))
+    launch_phase_cells(n, qv, nv, pd + r0, nws, R, deg, wannspace == EPHG_WANNSPACE_PH ? h->qlo : h->hlo,
+                       wannspace == EPHG_WANNSPACE_PH ? h->qext : h->hext, P, nws, h->st);
+    if ((rc = launch_xgemm_chunks(h->ws, cd + c0, (int)(piece[p + 1].second - c0), n, per, nws, P, nws, gm, per, gstride,
+                                  ce, G, per, h->err, h->st)))
       return WSFAIL(rc);
     launch_g2_vertices(n, pd + r0, nv, nw, nb, G, ek, ekp, eq, en, h->masses, Lv, out, h->st);
     h->launches += 5;
@@ -1111,13 +1124,13 @@ int ephg::el_rates_view(ephg_handle *h, const ExecView &x, const ephg_rate_reque
     if ((rc = wsget((*x.ws), "r_Lq", (size_t)N * nb, &Lq)) || (rc = wsget((*x.ws), "r_glp", (size_t)N * nb, &glp)) ||
         (split && (rc = wsget((*x.ws), "r_glpf", (size_t)N * nb, &glpf))))
       return WSFAILX(rc);
-    launch_polar_q(h->polar, N, iota, mesh, nullptr, Dq, nullptr, Lq, st);
+    launch_polar_q(h->polar, N, iota, mesh, nullptr, Dq, nullptr, (int64_t)nb * nb, Lq, st);
     (*x.launches) += 1;
   }
   launch_heig(N, nb, Dq, (int64_t)nb * nb, wq, Vq, x.err, st);
   float2 *uf = nullptr;
   if (split && (rc = wsget((*x.ws), "r_uf", (size_t)N * nb * nb, &uf))) return WSFAILX(rc);
-  launch_ph_post(N, nb, iota, nullptr, wq, Vq, nullptr, 0, h->masses, nullptr, nullptr, nullptr, om,
+  launch_ph_post(N, nb, iota, nullptr, wq, Vq, nullptr, 0, 0, h->masses, nullptr, nullptr, nullptr, om,
                  u, uf, x.err, st);
   launch_bose(N, nb, om, req->T, bose, st);
   RateSets rs;
@@ -1357,7 +1370,7 @@ int ephg::el_rates_view(ephg_handle *h, const ExecView &x, const ephg_rate_reque
       }
     } else {
       const int *ce;
-      if ((rc = resident_colexp(h->exp_G, Nn, nwsk, h->G64, Nn, &h->resident_bytes, st, &ce)))
+      if ((rc = resident_colexp(h->exp_G, 1, Nn, nwsk, h->G64, 0, &h->resident_bytes, st, &ce)))
         return fail(rc, "el_rates: column exponents");
       for (int64_t i0 = 0; i0 < nA; i0 += kc) {
         const int n = (int)std::min<int64_t>(kc, nA - i0);

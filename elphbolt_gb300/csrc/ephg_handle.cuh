@@ -32,16 +32,17 @@ struct ephg_handle {
   ephg::CellTab cellk, cellq;
   int *cellk_tab = nullptr, *cellq_tab = nullptr;
   double *rdegk = nullptr;
-  // column exponents of the resident right-hand sides of launch_xgemm (lazy): Hext, G64, graw
-  ephg::ColExp exp_H, exp_G, exp_raw;
+  // column exponents of the resident right-hand sides of launch_xgemm (lazy): Hext, G64, graw, Dcell
+  ephg::ColExp exp_H, exp_G, exp_raw, exp_D;
   double2 *graw = nullptr;   // epmatwp order (i,j,Re,s,Rp)
   double2 *G64 = nullptr;    // stage-A matrix [Re][Nn]
   double *masses = nullptr;
-  // phonon wrap terms
-  int *pair_off = nullptr, *ent_iuc = nullptr, *ent_woff = nullptr, *wrapR = nullptr;
-  double *ent_rden = nullptr, *rcartq = nullptr;
-  double2 *D = nullptr;
-  ephg::PhTerms terms;
+  // phonons at arbitrary q: the nD distinct wrapped cell vectors RD and their terms
+  // Dcell [nD][4 nb nb] (mass-normalised D, then its three q derivatives)
+  int nD = 0;
+  int *RD = nullptr;
+  double2 *Dcell = nullptr;
+  int qlo[3] = {0, 0, 0}, qext[3] = {1, 1, 1};   // range of the Rp coordinates
   int *kposk = nullptr, *kposq = nullptr;   // split-form contraction order (far cells first)
   int *err = nullptr;        // device error word
   ephg::Workspace ws;
@@ -54,6 +55,7 @@ struct ephg_handle {
   bool polar_on = false;
   ephg::PolarDev polar;
   double *polar_G = nullptr, *polar_Gcell = nullptr, *polar_born = nullptr, *polar_tau = nullptr;
+  float *polar_Gf = nullptr;   // polar_G then polar_Gcell in FP32
   double2 *polar_Da = nullptr;
   // crystal symmetry (ephg_set_symmetry): real-space rotations (3,3,n), crystal coordinates
   std::vector<int64_t> sym_rot;

@@ -278,25 +278,71 @@ void launch_phase_frac(int nrows, const double *kv, int nR, const int *R, const 
   k_phase_frac<<<(unsigned)((n + 255) / 256), 256, 0, st>>>(nrows, kv, nR, R, deg, out, ldo);
 }
 
-// the same for the vectors perm[row] of a list (column stride ldk)
+// The same for many rows (row r the vector perm[r], r itself if perm is null; kv's column
+// stride ldk), from tables of e^{2 pi i k_d n} over the cells' range (lo, ext) of each dimension:
+// two complex products per cell instead of an FP64 sincos of ~40 operations, and the
+// angles are rounded per dimension and exactly reduced.  A block takes ROWS rows: four
+// where there are many, one where the call waits for a few.
+// 4,001 rows of 165 cells: 36 us (63 with a sincos and two divisions per cell).
+constexpr int PC_TAB = 128, PC_THREADS = 128;
+
+template <int ROWS>
+__global__ void __launch_bounds__(PC_THREADS) k_phase_cells(int nrows, const double *kv, int64_t ldk, const int *perm,
+                                                            int nR, const int *R, const double *deg, int lo0, int lo1,
+                                                            int lo2, int e0, int e1, int e2, double2 *out,
+                                                            int64_t ldo) {
+  constexpr int T = PC_THREADS / ROWS;   // threads of a row
+  __shared__ double2 tabs[ROWS][PC_TAB];
+  const int lane = threadIdx.x % T, w = threadIdx.x / T;
+  const int row = blockIdx.x * ROWS + w;
+  const bool live = row < nrows;
+  double2 *tab = tabs[w];
+  if (live) {
+    const int64_t k = perm ? perm[row] : row;
+    const double k0 = kv[k], k1 = kv[k + ldk], k2 = kv[k + 2 * ldk];
+    for (int i = lane; i < e0 + e1 + e2; i += T) {
+      const double x = i < e0 ? k0 * (lo0 + i) : i < e0 + e1 ? k1 * (lo1 + i - e0) : k2 * (lo2 + i - e0 - e1);
+      sincospi(2.0 * x, &tab[i].y, &tab[i].x);
+    }
+  }
+  __syncthreads();
+  if (!live) return;
+  for (int r = lane; r < nR; r += T) {
+    double2 v = cmul(cmul(tab[R[3 * r] - lo0], tab[e0 + R[3 * r + 1] - lo1]), tab[e0 + e1 + R[3 * r + 2] - lo2]);
+    if (deg) v = cscale(v, 1.0 / deg[r]);
+    out[(int64_t)row * ldo + r] = v;
+  }
+}
+
+// ranges too long for the tables
 __global__ void k_phase_list(int nrows, const double *kv, int64_t ldk, const int *perm, int nR, const int *R,
-                             const double *deg, double2 *out) {
+                             const double *deg, double2 *out, int64_t ldo) {
   int64_t idx = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
   if (idx >= (int64_t)nrows * nR) return;
   const int row = (int)(idx / nR), r = (int)(idx % nR);
-  const int64_t k = perm[row];
+  const int64_t k = perm ? perm[row] : row;
   double dot = kv[k] * (double)R[3 * r];
   dot += kv[k + ldk] * (double)R[3 * r + 1];
   dot += kv[k + 2 * ldk] * (double)R[3 * r + 2];
   double s, c;
   sincos(TWOPI * dot, &s, &c);
-  out[idx] = make_double2(c / deg[r], s / deg[r]);
+  const double d = deg ? deg[r] : 1.0;
+  out[(int64_t)row * ldo + r] = make_double2(c / d, s / d);
 }
 
-void launch_phase_list(int nrows, const double *kv, int64_t ldk, const int *perm, int nR, const int *R,
-                       const double *deg, double2 *out, cudaStream_t st) {
+void launch_phase_cells(int nrows, const double *kv, int64_t ldk, const int *perm, int nR, const int *R,
+                        const double *deg, const int lo[3], const int ext[3], double2 *out, int64_t ldo,
+                        cudaStream_t st) {
   const int64_t n = (int64_t)nrows * nR;
-  if (n > 0) k_phase_list<<<(unsigned)((n + 255) / 256), 256, 0, st>>>(nrows, kv, ldk, perm, nR, R, deg, out);
+  if (n <= 0) return;
+  auto go = [&](auto kernel, int rows) {
+    kernel<<<(nrows + rows - 1) / rows, PC_THREADS, 0, st>>>(nrows, kv, ldk, perm, nR, R, deg, lo[0], lo[1], lo[2],
+                                                             ext[0], ext[1], ext[2], out, ldo);
+  };
+  if (ext[0] + ext[1] + ext[2] <= PC_TAB)
+    nrows > 2048 ? go(k_phase_cells<4>, 4) : go(k_phase_cells<1>, 1);
+  else
+    k_phase_list<<<(unsigned)((n + 255) / 256), 256, 0, st>>>(nrows, kv, ldk, perm, nR, R, deg, out, ldo);
 }
 
 // ============================================================ FP64 GEMM
@@ -751,136 +797,9 @@ void launch_el_post(int nk, int nw, const double *w, const double2 *V, const dou
 }
 
 // ============================================================= phonons
-// D(q) assembly with Wigner-Seitz wrapping (wannier.f90:631-665), mass
-// normalisation (:716-729).  One block per q.  The wrapped phase sum of each
-// (atom pair, WS cell), sum_w e^{2 pi i q.(R + w N_c)} / (deg * nwrap), is
-// formed once into shared memory (chunks of DB_CHUNK cells) and then each
-// thread contracts it with D(R) for its matrix elements.
-constexpr int DB_CHUNK = 64;
-
-__global__ void __launch_bounds__(128) k_dbuild(int nq, const int *qp, int m1, int m2, int m3, int L,
-                                                const double2 *roots, const double *qv, PhTerms t, int with_vel,
-                                                double2 *Dq, double2 *dDq) {
-  extern __shared__ double2 dsm[];   // [npair][DB_CHUNK] phase sums
-  const int q = blockIdx.x;
-  const int nb = t.nb, nwsq = t.nwsq, npair = t.npair;
-  const int mesh[3] = {m1, m2, m3};
-  const int ne = nb * nb;
-  // each thread owns up to DB_U matrix elements (nb <= 32 gives <= 1024 elements)
-  constexpr int DB_U = 8;
-  // without velocities and for nb^2 <= blockDim / 2, the cells of each chunk are
-  // split over nsl thread slices per element; the slices are added in order at the end
-  const int nsl = (!with_vel && 2 * ne <= (int)blockDim.x) ? (int)blockDim.x / ne : 1;
-  double2 acc[DB_U], dacc[DB_U][3];
-  for (int u = 0; u < DB_U; ++u) {
-    acc[u] = make_double2(0.0, 0.0);
-    for (int p = 0; p < 3; ++p) dacc[u][p] = make_double2(0.0, 0.0);
-  }
-  for (int c0 = 0; c0 < nwsq; c0 += DB_CHUNK) {
-    const int nc = min(DB_CHUNK, nwsq - c0);
-    __syncthreads();
-    for (int w = threadIdx.x; w < npair * nc; w += blockDim.x) {
-      const int pair = w / nc, iuc = c0 + w % nc;
-      const int en = t.pair_off[pair] + iuc;     // entries are (pair, cell) in cell order
-      double2 cs = make_double2(0.0, 0.0);
-      for (int wv = t.ent_woff[en]; wv < t.ent_woff[en + 1]; ++wv) {
-        const int *R = t.wrapR + 3 * wv;
-        double2 ph;
-        if (qp) {
-          ph = roots[phase_index(qp[q], mesh, L, R[0], R[1], R[2])];
-        } else {
-          double dot = qv[q] * (double)R[0];
-          dot += qv[q + nq] * (double)R[1];
-          dot += qv[q + 2 * nq] * (double)R[2];
-          sincos(TWOPI * dot, &ph.y, &ph.x);
-        }
-        cs.x += ph.x;
-        cs.y += ph.y;
-      }
-      const double rden = t.ent_rden[en];
-      dsm[pair * DB_CHUNK + (iuc - c0)] = make_double2(cs.x * rden, cs.y * rden);
-    }
-    __syncthreads();
-    if (nsl > 1) {   // small nb: thread = (element, slice of the chunk's cells), 4-FMA complex MACs
-      if (threadIdx.x < nsl * ne) {
-        const int e = threadIdx.x % ne, sl = threadIdx.x / ne;
-        const int a = e % nb, b = e / nb;
-        const int pair = (a / 3) + t.nat * (b / 3);
-        const double2 *Dp = t.D + (int64_t)nwsq * (a + (int64_t)nb * b);
-        double ar = acc[0].x, ai = acc[0].y;
-        for (int k = sl; k < nc; k += nsl) {
-          const double2 ph = dsm[pair * DB_CHUNK + k], dv = Dp[c0 + k];
-          ar = fma(ph.x, dv.x, ar);
-          ar = fma(-ph.y, dv.y, ar);
-          ai = fma(ph.x, dv.y, ai);
-          ai = fma(ph.y, dv.x, ai);
-        }
-        acc[0] = make_double2(ar, ai);
-      }
-      continue;
-    }
-#pragma unroll
-    for (int u = 0; u < DB_U; ++u) {
-      const int e = threadIdx.x + u * blockDim.x;
-      if (e >= ne) break;
-      const int a = e % nb, b = e / nb;
-      const int pair = (a / 3) + t.nat * (b / 3);
-      for (int k = 0; k < nc; ++k) {
-        const int iuc = c0 + k;
-        const double2 term = cmul(dsm[pair * DB_CHUNK + k], t.D[iuc + (int64_t)nwsq * (a + (int64_t)nb * b)]);
-        acc[u] = cadd(acc[u], term);
-        if (with_vel)
-          for (int p = 0; p < 3; ++p) {
-            const double rc = t.rcart[iuc + (int64_t)nwsq * p];
-            dacc[u][p] = cadd(dacc[u][p], make_double2(-rc * term.y, rc * term.x));
-          }
-      }
-    }
-  }
-  if (nsl > 1) {
-    __syncthreads();
-    double2 *part = dsm;   // [nsl][ne] slice sums (nsl * ne <= blockDim = 128 entries)
-    if (threadIdx.x < nsl * ne) part[threadIdx.x] = acc[0];
-    __syncthreads();
-    if (threadIdx.x < ne) {
-      const int e = threadIdx.x, a = e % nb, b = e / nb;
-      double2 sum = part[e];
-      for (int sl = 1; sl < nsl; ++sl) sum = cadd(sum, part[sl * ne + e]);
-      const double massnorm = 1.0 / sqrt(t.masses[a / 3] * t.masses[b / 3]) * Ryd2amu;
-      Dq[(size_t)q * ne + e] = cscale(sum, massnorm);
-    }
-    return;
-  }
-#pragma unroll
-  for (int u = 0; u < DB_U; ++u) {
-    const int e = threadIdx.x + u * blockDim.x;
-    if (e >= ne) break;
-    const int a = e % nb, b = e / nb;
-    const double massnorm = 1.0 / sqrt(t.masses[a / 3] * t.masses[b / 3]) * Ryd2amu;
-    Dq[(size_t)q * ne + e] = cscale(acc[u], massnorm);
-    if (with_vel)
-      for (int p = 0; p < 3; ++p) dDq[((size_t)q * 3 + p) * ne + e] = cscale(dacc[u][p], massnorm);
-  }
-}
-
-void launch_dbuild(int nq, const int *qp, const int mesh[3], int L, const double2 *roots,
-                   const double *qv, const PhTerms &t, int with_vel, double2 *Dq, double2 *dDq,
-                   cudaStream_t st) {
-  if (nq <= 0) return;
-  // phase sums [npair][DB_CHUNK], reused for the slice sums (<= 128 entries)
-  const size_t smem = (size_t)std::max(t.npair * DB_CHUNK, 128) * sizeof(double2);
-  // once per process: changing a kernel attribute can wait for the device's queued work
-  static std::once_flag attr_once;
-  std::call_once(attr_once, [] {
-    cudaFuncSetAttribute(k_dbuild, cudaFuncAttributeMaxDynamicSharedMemorySize, 96 * 1024);
-  });
-  k_dbuild<<<nq, 128, smem, st>>>(nq, qp, mesh ? mesh[0] : 1, mesh ? mesh[1] : 1, mesh ? mesh[2] : 1, L, roots, qv,
-                                  t, with_vel, Dq, dDq);
-}
-
 // ph_wann post-processing (wannier.f90:740-780)
 __global__ void k_ph_post(int nq, int nb, const int *qp, const double *qv, const double *w,
-                          const double2 *V, const double2 *dDq, int with_vel,
+                          const double2 *V, const double2 *dDq, int64_t ldd, int with_vel,
                           const double *masses, double *energies_f, double2 *evecs_f,
                           double *vel_f, double *om_i, double2 *u_i, float2 *u_f, int *err) {
   int idx = blockIdx.x * blockDim.x + threadIdx.x;
@@ -894,7 +813,7 @@ __global__ void k_ph_post(int nq, int nb, const int *qp, const double *qv, const
   double vel[3] = {0.0, 0.0, 0.0};
   if (with_vel) {
     for (int p = 0; p < 3; ++p) {
-      const double2 *dD = dDq + ((size_t)q * 3 + p) * nn;
+      const double2 *dD = dDq + (size_t)q * ldd + p * nn;
       double2 acc = make_double2(0.0, 0.0);
       for (int r = 0; r < nb; ++r) {
         double2 mv = make_double2(0.0, 0.0);
@@ -928,12 +847,12 @@ __global__ void k_ph_post(int nq, int nb, const int *qp, const double *qv, const
 }
 
 void launch_ph_post(int nq, int nb, const int *qp, const double *qv, const double *w,
-                    const double2 *V, const double2 *dDq, int with_vel, const double *masses,
+                    const double2 *V, const double2 *dDq, int64_t ldd, int with_vel, const double *masses,
                     double *energies_f, double2 *evecs_f, double *vel_f, double *om_i,
                     double2 *u_i, float2 *u_f, int *err, cudaStream_t st) {
   int n = nq * nb;
   if (n == 0) return;
-  k_ph_post<<<(n + 127) / 128, 128, 0, st>>>(nq, nb, qp, qv, w, V, dDq, with_vel, masses,
+  k_ph_post<<<(n + 127) / 128, 128, 0, st>>>(nq, nb, qp, qv, w, V, dDq, ldd, with_vel, masses,
                                              energies_f, evecs_f, vel_f, om_i, u_i, u_f, err);
 }
 

@@ -14,9 +14,11 @@ void launch_phase_mesh(int nrows, const int *rowp, const int mesh[3], int L, int
 // same for arbitrary fractional k: kv (nrows,3) column-major as the reference
 void launch_phase_frac(int nrows, const double *kv, int nR, const int *R, const double *deg,
                        double2 *out, int64_t ldo, cudaStream_t st);
-// the same for the vectors perm[0..nrows) of kv (column stride ldk), / deg; rows of nR
-void launch_phase_list(int nrows, const double *kv, int64_t ldk, const int *perm, int nR, const int *R,
-                       const double *deg, double2 *out, cudaStream_t st);
+// The same for the vectors perm[0..nrows) of kv (0..nrows - 1 if null; column stride ldk); lo, ext: the
+// range of the cell coordinates per dimension; deg nullable; out rows at stride ldo
+void launch_phase_cells(int nrows, const double *kv, int64_t ldk, const int *perm, int nR, const int *R,
+                        const double *deg, const int lo[3], const int ext[3], double2 *out, int64_t ldo,
+                        cudaStream_t st);
 
 // out[p][e] = sum_R e^{2 pi i k_p.R} X(R)[e] for every point p of the mesh (muxed
 // order), X given on the box of cell coordinates [lo, lo + ext) per dimension
@@ -65,28 +67,11 @@ void launch_el_post(int nk, int nw, const double *w, const double2 *V, const dou
                     int64_t ldc, int with_vel, const double *scissor, double *energies_f,
                     double *vel_f, double2 *evecs_f, double *ens_i, cudaStream_t st);
 
-struct PhTerms {
-  int npair;            // natoms^2, pair = iat + nat*jat
-  const int *pair_off;  // (npair+1) offsets into the entry list
-  const int *ent_iuc;   // entry -> WS cell
-  const int *ent_woff;  // entry -> first wrap vector (wrap list offsets, nent+1)
-  const int *wrapR;     // wrap vectors R + w*N_c, 3 ints each
-  const double *ent_rden;// 1 / (phwsdeg * nwrap)
-  const double2 *D;     // (nwsq, nb, nb) column-major
-  const double *rcart;  // (nwsq, 3) lattvecs @ R, nm
-  const double *masses; // per atom
-  int nwsq, nb, nat;
-};
-// Build the mass-normalised dynamical matrix D(q) (and dD/dq with vel);
-// mesh mode if qp != nullptr (exact integer phases), else fractional qv (nq,3).
-void launch_dbuild(int nq, const int *qp, const int mesh[3], int L, const double2 *roots,
-                   const double *qv, const PhTerms &t, int with_vel, double2 *Dq, double2 *dDq,
-                   cudaStream_t st);
 // omega, Gamma / negative handling, velocities; outputs in reference layout
 // (energies_f (nq,nb), evecs_f (nq,nb,nb), vel_f (nq,nb,3)) and/or internal
 // (om_i [q][s], u_i [q][s][c] = evec/sqrt(M_c)).
 void launch_ph_post(int nq, int nb, const int *qp, const double *qv, const double *w,
-                    const double2 *V, const double2 *dDq, int with_vel, const double *masses,
+                    const double2 *V, const double2 *dDq, int64_t ldd, int with_vel, const double *masses,
                     double *energies_f, double2 *evecs_f, double *vel_f, double *om_i,
                     double2 *u_i, float2 *u_f, int *err, cudaStream_t st);
 
@@ -113,6 +98,7 @@ struct PolarDev {
   const double *G = nullptr;      // [M][3] box vectors, Cartesian 1/bohr, in the reference's loop order
   const double *Gcell = nullptr;  // [Mcell][3] those of them that can pass the cut for q in the first cell
   int Mcell = 0;
+  const float *Gf = nullptr, *Gcellf = nullptr;   // the same in FP32, for the first test of the cut
   const double *born = nullptr;   // born(x, ipol, at) at x + 3 ipol + 9 at
   const double *tau = nullptr;    // [nat][3] Cartesian basis, bohr
   const double2 *Da = nullptr;    // (nb,nb) column-major: the q-independent sum (before fac)
@@ -122,11 +108,11 @@ struct PolarDev {
   double alph = 0, gmax = 14.0, fac = 0;   // tpiba^2 (1/bohr^2), cut, 8 pi / volume (1/bohr^3)
 };
 // Per q (mesh index qp[q] on `mesh`, else crystal coordinates qv (nq,3)
-// column-major): Dq[q] += massnorm * dyn_l(q) (nullable; layout of
-// launch_dbuild), dDq[q] += massnorm * ddyn_l(q) * bohr2nm (nullable), and
+// column-major): Dq[q] += massnorm * dyn_l(q) (nullable; matrices ldd values apart),
+// dDq[q] += massnorm * ddyn_l(q) * bohr2nm (nullable; three matrices per q, ldd apart), and
 // Lq[q][c] (nullable) with long_range_prefac(q, u) = sum_c Lq[q][c] u[c].
 void launch_polar_q(const PolarDev &P, int nq, const int *qp, const int mesh[3], const double *qv,
-                    double2 *Dq, double2 *dDq, double2 *Lq, cudaStream_t st);
+                    double2 *Dq, double2 *dDq, int64_t ldd, double2 *Lq, cudaStream_t st);
 // The q-independent part of dyn_nonanalytic into Da (nb,nb), once per crystal.
 void launch_polar_da(const PolarDev &P, double2 *Da, cudaStream_t st);
 // glp[q][s] = sum_c Lq[q][c] u[q][s][c] (u = evec / sqrt(M)), and its fp32 copy (nullable)

@@ -12,27 +12,34 @@
 //
 //   sum_k a_k b_k = sum_l 2^(-7 l - 12) S_l,   S_l = sum over i + j = l, k of integers |d| <= 64
 //
-// Levels 0..6 have an accumulator each; |S_l| <= (l + 1) 4096 K stays within 2^24
-// for the XG_KGROUP positions summed at a time (l <= 5 at worst case; l = 6 for any
-// sum that is not of one sign throughout).  Levels 7 and 8 share the last one, at
-// 2^-49 of the result, where rounding no longer counts.  Products beyond level 8
-// (2^-63) are left out.  The result is the exact sum of the products to ~2^-60 of
-// the largest term, rounded once: its error is at or below that of the FP64
+// Levels have an accumulator each (7 and 8 share one where nine do not fit TMEM); |S_l| <= (l + 1) 4096 K stays within 2^24
+// for the XG_KGROUP positions summed at a time for l <= 5; above that (2^-54 of the
+// result) only for sums not of one sign throughout, and an FP32 rounding there no
+// longer counts.  Products beyond level 8 (2^-63) are left out.  The result is the
+// exact sum of the products to ~2^-60 of the largest term, rounded once: its error is at or below that of the FP64
 // multiply-adds it replaces (g(Re,q), 279 cells, against sums of the same phases in
 // extended precision: 5.5e-17 relative; the multiply-adds 7.6e-16).
 //
 // The tall matrix is the M operand: a tile is 128 of its columns, with K running
 // over (cell, re | im), so that one product gives C = A B for up to 32 rows of
-// phases as N = 64 columns (row m: real and imaginary part).  Its digits are
-// formed where they are used: eight warps read the FP64 values (coalesced along
-// the columns, each once per 32 phase rows) and write the nine BF16 planes of
+// phases as columns (row m: real and imaginary part).  A level's accumulator lies
+// beside the next level's, as the phases' digit planes do in shared memory, so one
+// MMA of up to 256 columns takes a digit of the tall operand with several digits of
+// the phases.  The tall operand's digits are
+// formed where they are used: sixteen warps read the FP64 values (coalesced along
+// the columns, each once per chunk of phase rows) and write the nine BF16 planes of
 // a stage in the swizzled layout the MMA reads; HBM sees the FP64 matrix only.
 // The phases' digits are formed once per call and arrive by bulk copies.  Two
-// stages of 108 KB; 45 digit products of 128 x 64 x 32 per stage, bound by the
-// tensor core's shared-memory operand reads (~4,300 cycles a stage).
+// stages of 104 KB; 45 digit products per stage, the tensor core is the bound
+// (about one cycle a column at these widths), the splitting runs beside it.
 //
-// Measured: g(k,Rp) at 25 k, nw 8, nb 6, 279 cells: 0.43 ms (6.70 as FP64 multiply-adds);
-// 200 H(k) with velocities, nw 8: 0.08 ms (0.61).
+// Measured: g(k,Rp) at 25 k, nw 8, nb 6, 279 cells: 0.29 ms (6.70 as FP64 multiply-adds);
+// 200 H(k) with velocities, nw 8: 0.053 ms (0.61); 1,728 D(q) with derivatives, nb 6, 339
+// wrapped cells: 0.072 ms (1.16 in the kernel that summed them in FP64).  On the way: one
+// MMA per digit pair 0.46 ms, descriptors formed in loops 0.49 ms (the issuing thread
+// was the bound), one FP64 drain warp per quadrant 0.32 ms.
+#include <cuda_bf16.h>
+
 #include <algorithm>
 #include <climits>
 
@@ -45,16 +52,20 @@ namespace ephg {
 using namespace tc;
 
 constexpr int XG_D = 9;                                // digits
-constexpr int XG_ROWS = 128, XG_M = 32, XG_N = 64;     // tile columns of B; phase rows, MMA N
+constexpr int XG_ROWS = 128, XG_M = XG_CHUNK;          // tile columns of B; phase rows of a chunk
+constexpr int XG_W = 2 * XG_M;                         // most MMA columns of a level
 constexpr int XG_CELLS = 16, XG_KV = 2 * XG_CELLS;     // cells and K values per stage
 constexpr int XG_KGROUP = 320 / XG_CELLS;              // stages per accumulation: 640 K values
 constexpr int XG_PLANE_B = XG_ROWS * XG_KV * 2;        // 8 KB per digit
-constexpr int XG_PLANE_A = XG_N * XG_KV * 2;           // 4 KB per digit
+constexpr int XG_PLANE_A = XG_W * XG_KV * 2;           // at most 4 KB per digit
 constexpr int XG_STAGE_B = XG_D * XG_PLANE_B, XG_STAGE_A = XG_D * XG_PLANE_A;
-constexpr int XG_STAGE = XG_STAGE_B + XG_STAGE_A;
+constexpr int XG_STAGE = (XG_STAGE_B + XG_STAGE_A + 1023) / 1024 * 1024;
+// accumulators of a level's W columns: level 8 shares the last of eight where nine do not fit TMEM
+__host__ __device__ constexpr int xg_levels(int W) { return XG_D * W <= 512 ? XG_D : XG_D - 1; }
+static_assert(xg_levels(XG_W) * XG_W <= 512, "the levels' accumulators fit TMEM");
 constexpr int XG_STAGES = 2;
 constexpr int XG_SMEM = XG_STAGES * XG_STAGE + 1024 + 256;
-constexpr int XG_CONV = 256, XG_EPI = 128;             // converter and epilogue threads
+constexpr int XG_CONV = 512, XG_EPI = 256;             // converter and epilogue threads
 constexpr int XG_THREADS = 64 + XG_CONV + XG_EPI;
 constexpr int XG_BATCH = 4096;                         // phase rows per launch (bounds the digit buffer)
 constexpr int XG_BAD = INT_MAX;                        // exponent of a column with a non-finite value
@@ -64,23 +75,26 @@ constexpr int XG_BAD = INT_MAX;                        // exponent of a column w
 __device__ __forceinline__ uint64_t xg_fixed(double x, int e) {
   const uint64_t u = (uint64_t)__double_as_longlong(x);
   const int ex = (int)((u >> 52) & 0x7ff);
-  uint64_t m = u & 0xFFFFFFFFFFFFFull;
-  if (ex) m |= 1ull << 52;
-  const int sh = max(ex, 1) - 1013 - e;   // <= 9
-  m = sh >= 0 ? m << sh : (sh > -64 ? m >> -sh : 0);
+  uint64_t m = (u & 0xFFFFFFFFFFFFFull) << 10;
+  if (ex) m |= 1ull << 62;
+  const int sh = 1023 + e - max(ex, 1);   // >= 0
+  m = sh < 64 ? m >> sh : 0;
   constexpr uint64_t BIAS = 0x4081020408102040ull;   // 64 sum_i 128^i, i = 0..8
-  return BIAS + ((u >> 63) ? (uint64_t)0 - m : m);
+  const uint64_t sg = (uint64_t)((int64_t)u >> 63);
+  return BIAS + ((m ^ sg) - sg);
 }
 
-// digits i of two values as a BF16 pair; digit i carries its weight 2^(-7 i - 6)
+// digits I of two values as a BF16 pair, digit i with its weight 2^(-7 i - 6): the fields under the
+// exponent of 128.0 are the numbers 128 + field, exactly (digit 0 reaches +64: field 128, 256.0)
 template <int I>
 __device__ __forceinline__ uint32_t xg_digit2(uint64_t a, uint64_t b) {
-  constexpr uint32_t magic = (uint32_t)(127 + 17 - 7 * I) << 23;   // 2^(17 - 7 I): ulp 2^(-7 I - 6)
-  const uint32_t mask = I == 0 ? 0xFFu : 0x7Fu;                    // digit 0 reaches +64: field 128
-  const float off = __uint_as_float(magic | 64u);
-  const float fa = __uint_as_float(magic | ((uint32_t)(a >> (56 - 7 * I)) & mask)) - off;
-  const float fb = __uint_as_float(magic | ((uint32_t)(b >> (56 - 7 * I)) & mask)) - off;
-  return __byte_perm(__float_as_uint(fa), __float_as_uint(fb), 0x7632);
+  constexpr uint32_t mask = I == 0 ? 0x00FF00FFu : 0x007F007Fu;
+  const uint32_t f = __byte_perm((uint32_t)(a >> (56 - 7 * I)), (uint32_t)(b >> (56 - 7 * I)), 0x5410);
+  const uint32_t n = (f & mask) | 0x43004300u;
+  const float w = __uint_as_float((uint32_t)(127 - 7 * I - 6) << 23);
+  const __nv_bfloat162 w2 = __float2bfloat162_rn(w), o2 = __float2bfloat162_rn(-192.0f * w);
+  __nv_bfloat162 r = __hfma2(*reinterpret_cast<const __nv_bfloat162 *>(&n), w2, o2);
+  return *reinterpret_cast<uint32_t *>(&r);
 }
 
 template <int I>
@@ -117,18 +131,18 @@ __global__ void __launch_bounds__(256) k_col_exp(int64_t N, int K, const double2
 }
 
 // chunk c of up to 32 rows of A: its first row, row count and right-hand side
-__device__ __forceinline__ int4 xg_chunk(const int4 *chunks, int M, int c) {
+__device__ __forceinline__ int4 xg_chunk(const int4 *chunks, int M, int rpc, int c) {
   if (chunks) return chunks[c];
-  return make_int4(c * XG_M, min(XG_M, M - c * XG_M), 0, 0);
+  return make_int4(c * rpc, min(rpc, M - c * rpc), 0, 0);
 }
 
-// The phases' digit tiles [chunk][stage][digit][64 rows][64 B, swizzled]:
+// The phases' digit tiles [chunk][stage][digit][W rows][64 B, swizzled] (4 W threads):
 // MMA row 2 m holds (re, -im) and row 2 m + 1 (im, re) of A[m][cell] along K.
-__global__ void __launch_bounds__(256) k_xg_phases(const int4 *chunks, int M, int K, int kch, const double2 *A,
-                                                   int64_t lda, uint8_t *dig, int *bad) {
+__global__ void __launch_bounds__(256) k_xg_phases(const int4 *chunks, int M, int rpc, int W, int K, int kch,
+                                                   const double2 *A, int64_t lda, uint8_t *dig, int *bad) {
   const int r = threadIdx.x >> 2, q = threadIdx.x & 3;   // MMA row, 16-byte chunk (4 cells)
   const int kc = blockIdx.x, mc = blockIdx.y;
-  const int4 ch = xg_chunk(chunks, M, mc);
+  const int4 ch = xg_chunk(chunks, M, rpc, mc);
   const int m = ch.x + (r >> 1);
   uint64_t v[8];
 #pragma unroll
@@ -136,20 +150,55 @@ __global__ void __launch_bounds__(256) k_xg_phases(const int4 *chunks, int M, in
     const int k = kc * XG_CELLS + 4 * q + c;
     double2 a = make_double2(0.0, 0.0);
     if ((r >> 1) < ch.y && k < K) a = A[(int64_t)m * lda + k];
-    if (!(fabs(a.x) <= 1.0) || !(fabs(a.y) <= 1.0)) {   // not a phase (a non-finite k): the row's results are NaN
-      bad[m] = 1;
-      a = make_double2(0.0, 0.0);
+    // a mean of phases may round to a few units above 1; anything else beyond is no phase
+    // (a non-finite k) and the row's results are NaN
+    constexpr long long ONE = 0x3ff0000000000000ll, ABS = 0x7fffffffffffffffll;
+    const long long ax = __double_as_longlong(a.x) & ABS, ay = __double_as_longlong(a.y) & ABS;
+    if (ax > ONE || ay > ONE) {
+      if (ax > ONE + 64 || ay > ONE + 64) bad[m] = 1;
+      if (ax > ONE) a.x = copysign(1.0, a.x);
+      if (ay > ONE) a.y = copysign(1.0, a.y);
     }
     v[2 * c] = xg_fixed((r & 1) ? a.y : a.x, 0);
     v[2 * c + 1] = xg_fixed((r & 1) ? a.x : -a.y, 0);
   }
-  xg_store<0>(dig + ((size_t)mc * kch + kc) * XG_STAGE_A + xg_swz(r, q), XG_PLANE_A, v);
+  xg_store<0>(dig + ((size_t)mc * kch + kc) * (XG_D * 64 * W) + xg_swz(r, q), 64 * W, v);
+}
+
+// 2^e sum_l 2^(-7 l - 12) S_l, rounded once, in integer arithmetic: eight FP64 operations a value
+// on GB300's FP64 pipe had made the drain a fifth of a tile's time
+__device__ __forceinline__ double xg_value(const int *s, int e) {
+  if (e == XG_BAD) return __longlong_as_double(0x7ff8000000000000ll);
+  const long long hi = (long long)s[0] * (1 << 21) + (long long)s[1] * (1 << 14) + (long long)s[2] * 128 + s[3];
+  const long long lo = (long long)s[4] * (1 << 28) + (long long)s[5] * (1 << 21) + (long long)s[6] * (1 << 14) +
+                       (long long)s[7] * 128 + s[8];
+  constexpr int LB = 35;
+  constexpr uint64_t LM = (1ull << LB) - 1;
+  long long h = hi + (lo >> LB);                     // the sum is 2^-68 (h 2^35 + l), 0 <= l < 2^35
+  uint64_t l = (uint64_t)lo & LM;
+  const bool neg = h < 0;
+  if (neg) {
+    h = ~h + (l == 0);
+    l = (0 - l) & LM;
+  }
+  if (h == 0 && l == 0) return 0.0;
+  // leading bit to bit 63 (z places above where h's bit 63 has it)
+  const int z = h ? __clzll(h) : __clzll((long long)l) + LB;
+  uint64_t m;
+  if (z <= LB) m = ((uint64_t)h << z) | (l >> (LB - z));
+  else m = (h ? (uint64_t)h << z : 0) | (l << (z - LB));
+  const uint64_t m53 = (m >> 11) + ((m >> 10) & 1);  // 53 bits, rounded to nearest
+  const int ex = e + 1052 - z;                       // value m53 2^(ex - 1074)
+  if (ex < 1 || ex > 2044) return (neg ? -1.0 : 1.0) * ldexp((double)m53, ex - 1074);
+  return __longlong_as_double((long long)(((uint64_t)ex << 52) + m53) | (neg ? (long long)0x8000000000000000ull : 0));
 }
 
 struct XgArgs {
   int M, K, kch, mch;
+  int rpc;                      // rows per chunk
   const int4 *chunks;           // null: one right-hand side, rows in order
   int64_t N, ldb, ldc, bstride; // bstride: values between right-hand sides
+  int64_t estride;              // exponents per right-hand side
   int64_t units;                // (tile of B, chunk of A), chunks fastest
   const double2 *B;
   const uint8_t *dig;
@@ -159,7 +208,7 @@ struct XgArgs {
 };
 
 // kind::f16 with BF16 operands, FP32 accumulators, K-major, M = 128
-__device__ __forceinline__ uint32_t idesc_bf16(int n) {
+__device__ constexpr uint32_t idesc_bf16(int n) {
   return (1u << 4) | (1u << 7) | (1u << 10) | ((uint32_t)(n >> 3) << 17) | ((uint32_t)(XG_ROWS >> 4) << 24);
 }
 
@@ -171,6 +220,27 @@ __device__ __forceinline__ void umma_bf16(uint32_t d_tmem, uint64_t a, uint64_t 
       : "memory");
 }
 
+// One K step: digit I of the tall operand with the phases' digits J.., up to 256 columns of
+// adjacent levels per MMA.  All addresses and descriptors are constants off two bases:
+// the issuing thread had been slower than the tensor core with them formed in loops.
+template <int W, int I = 0, int J = 0>
+__device__ __forceinline__ void xg_products(uint32_t tmem, uint64_t b, uint64_t a, uint32_t more) {
+  constexpr int nlev = xg_levels(W);
+  // the phases' digit 8 meets digit 0 only, at 2^-62 of 1: left out (nine accumulators: it starts the last)
+  constexpr int end = I == 0 ? nlev : XG_D - I < nlev - I ? XG_D - I : nlev - I;
+  constexpr int n = end - J < 256 / W ? end - J : 256 / W;
+  umma_bf16(tmem + (I + J) * W, b + I * (XG_PLANE_B >> 4), a + J * (W * 4), idesc_bf16(n * W), I ? 1u : more);
+  if constexpr (J + n < end) {
+    xg_products<W, I, J + n>(tmem, b, a, more);
+  } else if constexpr (I + 1 < nlev) {
+    xg_products<W, I + 1, 0>(tmem, b, a, more);
+  } else if constexpr (nlev < XG_D) {   // level 8 into level 7's accumulator
+#pragma unroll
+    for (int i = 1; i < XG_D; ++i)
+      umma_bf16(tmem + 7 * W, b + i * (XG_PLANE_B >> 4), a + (8 - i) * (W * 4), idesc_bf16(W), 1u);
+  }
+}
+
 __device__ __forceinline__ void bulk_load(void *dst, const void *src, uint32_t bytes, uint64_t *bar) {
   asm volatile(
       "cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];" ::"r"(smem_u32(dst)),
@@ -178,6 +248,7 @@ __device__ __forceinline__ void bulk_load(void *dst, const void *src, uint32_t b
       : "memory");
 }
 
+template <int W>
 __global__ void __launch_bounds__(XG_THREADS, 1) k_xgemm(XgArgs g) {
   extern __shared__ uint8_t smem_raw[];
   uint8_t *smem = (uint8_t *)(((uintptr_t)smem_raw + 1023) & ~(uintptr_t)1023);
@@ -215,11 +286,12 @@ __global__ void __launch_bounds__(XG_THREADS, 1) k_xgemm(XgArgs g) {
       uint32_t phase = 0;
       bool ok = true;
       for (int64_t u = blockIdx.x; u < g.units && ok; u += gridDim.x) {
-        const uint8_t *src = g.dig + (size_t)(u % g.mch) * g.kch * XG_STAGE_A;
+        const uint32_t bytes = XG_D * 64 * W;
+        const uint8_t *src = g.dig + (size_t)(u % g.mch) * g.kch * bytes;
         for (int kc = 0; kc < g.kch; ++kc) {
           if (!mbar_wait(&empty[stage], phase ^ 1, g.err)) { ok = false; break; }
-          mbar_expect_tx(&full[stage], XG_STAGE_A);
-          bulk_load(smem + stage * XG_STAGE + XG_STAGE_B, src + (size_t)kc * XG_STAGE_A, XG_STAGE_A, &full[stage]);
+          mbar_expect_tx(&full[stage], bytes);
+          bulk_load(smem + stage * XG_STAGE + XG_STAGE_B, src + (size_t)kc * bytes, bytes, &full[stage]);
           if (++stage == XG_STAGES) { stage = 0; phase ^= 1; }
         }
       }
@@ -233,8 +305,6 @@ __global__ void __launch_bounds__(XG_THREADS, 1) k_xgemm(XgArgs g) {
       uint32_t phase = 0;
       bool ok = true;
       for (int64_t u = blockIdx.x; u < g.units && ok; u += gridDim.x) {
-        const int mrows = xg_chunk(g.chunks, g.M, (int)(u % g.mch)).y;
-        const uint32_t id = idesc_bf16((2 * mrows + 15) / 16 * 16);
         for (int k0 = 0; k0 < g.kch && ok; k0 += XG_KGROUP, ++it) {
           if (!mbar_wait(tempty, (it & 1) ^ 1, g.err)) { ok = false; break; }
           tc_fence_after();
@@ -244,15 +314,10 @@ __global__ void __launch_bounds__(XG_THREADS, 1) k_xgemm(XgArgs g) {
             tc_fence_after();
             const uint64_t bd = sdesc(smem + stage * XG_STAGE), ad = sdesc(smem + stage * XG_STAGE + XG_STAGE_B);
 #pragma unroll
-            for (int ks = 0; ks < XG_KV / 16; ++ks) {
-              // addresses in the descriptors count 16 bytes
+            for (int ks = 0; ks < XG_KV / 16; ++ks) {   // addresses in the descriptors count 16 bytes
               const uint64_t bk = bd + 2 * ks, ak = ad + 2 * ks;
-#pragma unroll
-              for (int l = 0; l < XG_D; ++l)
-#pragma unroll
-                for (int i = 0; i <= l; ++i)
-                  umma_bf16(tmem + (l < 7 ? l : 7) * XG_N, bk + i * (XG_PLANE_B >> 4), ak + (l - i) * (XG_PLANE_A >> 4),
-                            id, (kc > k0 || ks > 0 || i > 0 || l == 8) ? 1u : 0u);
+              const uint32_t more = (kc > k0 || ks > 0) ? 1u : 0u;
+              xg_products<W>(tmem, bk, ak, more);
             }
             umma_commit(&empty[stage]);
             if (++stage == XG_STAGES) { stage = 0; phase ^= 1; }
@@ -266,88 +331,82 @@ __global__ void __launch_bounds__(XG_THREADS, 1) k_xgemm(XgArgs g) {
         mbar_wait(drain, 0, g.err);
       }
     }
-  } else if (warp < 2 + XG_CONV / 32) {   // ---- converters: B's digits of a stage, two 16-byte chunks per thread
-    const int t = threadIdx.x - 64, r = t & 127, q0 = t >> 7;
+  } else if (warp < 2 + XG_CONV / 32) {   // ---- converters: B's digits of a stage, one 16-byte chunk of each plane per thread
+    const int t = threadIdx.x - 64, r = t & 127, q = t >> 7;
     int stage = 0;
     uint32_t phase = 0;
     bool ok = true;
     for (int64_t u = blockIdx.x; u < g.units && ok; u += gridDim.x) {
       const int64_t n = (u / g.mch) * XG_ROWS + r;
-      const int64_t rhs = xg_chunk(g.chunks, g.M, (int)(u % g.mch)).z;
+      const int64_t rhs = xg_chunk(g.chunks, g.M, g.rpc, (int)(u % g.mch)).z;
       const bool live = n < g.N;
-      int e = live ? g.cexp[rhs * g.N + n] : 0;
+      int e = live ? g.cexp[rhs * g.estride + n] : 0;
       if (e == XG_BAD) e = 1024;   // the results are NaN; any finite digits do
       const double2 *col = g.B + rhs * g.bstride + n;
-      for (int kc = 0; kc < g.kch; ++kc) {
-        double2 x[2][4];
+      double2 next[4];   // the next stage's values are in flight while this one's are split
+      auto fetch = [&](int kc) {
 #pragma unroll
-        for (int h = 0; h < 2; ++h)
-#pragma unroll
-          for (int c = 0; c < 4; ++c) {
-            const int k = kc * XG_CELLS + 4 * (q0 + 2 * h) + c;
-            x[h][c] = live && k < g.K ? col[(int64_t)k * g.ldb] : make_double2(0.0, 0.0);
-          }
-        if (!mbar_wait(&empty[stage], phase ^ 1, g.err)) { ok = false; break; }
-        uint8_t *sb = smem + stage * XG_STAGE;
-#pragma unroll
-        for (int h = 0; h < 2; ++h) {
-          uint64_t v[8];
-#pragma unroll
-          for (int c = 0; c < 4; ++c) {
-            v[2 * c] = xg_fixed(x[h][c].x, e);
-            v[2 * c + 1] = xg_fixed(x[h][c].y, e);
-          }
-          xg_store<0>(sb + xg_swz(r, q0 + 2 * h), XG_PLANE_B, v);
+        for (int c = 0; c < 4; ++c) {
+          const int k = kc * XG_CELLS + 4 * q + c;
+          next[c] = live && k < g.K ? col[(int64_t)k * g.ldb] : make_double2(0.0, 0.0);
         }
+      };
+      fetch(0);
+      for (int kc = 0; kc < g.kch; ++kc) {
+        uint64_t v[8];
+#pragma unroll
+        for (int c = 0; c < 4; ++c) {
+          v[2 * c] = xg_fixed(next[c].x, e);
+          v[2 * c + 1] = xg_fixed(next[c].y, e);
+        }
+        if (kc + 1 < g.kch) fetch(kc + 1);
+        if (!mbar_wait(&empty[stage], phase ^ 1, g.err)) { ok = false; break; }
+        xg_store<0>(smem + stage * XG_STAGE + xg_swz(r, q), XG_PLANE_B, v);
         asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
         mbar_arrive(&full[stage]);
         if (++stage == XG_STAGES) { stage = 0; phase ^= 1; }
       }
     }
-  } else {   // ---- epilogue: warp w reads TMEM lane quadrant w % 4, a thread one column of B
-    const int quad = warp & 3;
+  } else {   // ---- epilogue: warp w reads TMEM lane quadrant w % 4, a thread every other 4 of a column's results
+    const int quad = warp & 3, half = (warp - 2 - XG_CONV / 32) >> 2;
     const uint32_t tr = tmem + ((uint32_t)(quad * 32) << 16);
+    constexpr int nlev = xg_levels(W);
     int it = 0;
     bool ok = true;
     for (int64_t u = blockIdx.x; u < g.units && ok; u += gridDim.x) {
-      const int4 ch = xg_chunk(g.chunks, g.M, (int)(u % g.mch));
+      const int4 ch = xg_chunk(g.chunks, g.M, g.rpc, (int)(u % g.mch));
       const int mrows = ch.y;
       const int64_t n = (u / g.mch) * XG_ROWS + quad * 32 + lane;
       const bool live = n < g.N;
-      const int e = live ? g.cexp[ch.z * g.N + n] : 0;
-      // 2^e as two factors (e may be at either end of FP64's range)
-      const int e1 = e == XG_BAD ? 0 : e / 2, e2 = e == XG_BAD ? 0 : e - e1;
-      double s1 = __hiloint2double((1023 + e1) << 20, 0);
-      const double s2 = __hiloint2double((1023 + e2) << 20, 0);
-      if (e == XG_BAD) s1 = __longlong_as_double(0x7ff8000000000000ll);
+      const int e = live ? g.cexp[ch.z * g.estride + n] : 0;
+      const unsigned badm = __ballot_sync(0xffffffffu, lane < mrows && g.bad[ch.x + lane]);
       for (int k0 = 0; k0 < g.kch; k0 += XG_KGROUP, ++it) {
         if (!mbar_wait(tfull, it & 1, g.err)) { ok = false; break; }
         tc_fence_after();
 #pragma unroll 1
-        for (int c0 = 0; c0 < 2 * mrows; c0 += 8) {
-          uint32_t a[8][8];
+        for (int c0 = 4 * half; c0 < 2 * mrows; c0 += 8) {
+          uint32_t a[XG_D][4];
           __syncwarp();
 #pragma unroll
-          for (int l = 0; l < 8; ++l) tmem_ld8_nowait(tr + l * XG_N + c0, a[l]);
+          for (int l = 0; l < XG_D; ++l) tmem_ld4_nowait(tr + min(l, nlev - 1) * W + c0, a[l]);
           tmem_wait_ld();
 #pragma unroll
-          for (int c = 0; c < 8; c += 2) {
+          for (int c = 0; c < 4; c += 2) {
             double2 z;
 #pragma unroll
             for (int y = 0; y < 2; ++y) {
-              long long s[8];
+              int s[XG_D];
 #pragma unroll
-              for (int l = 0; l < 8; ++l)   // S_l: exact integers but for the last
-                s[l] = (long long)__float2int_rn(__uint_as_float(a[l][c + y]) *
-                                                 __uint_as_float((uint32_t)(127 + 7 * l + 12) << 23));
-              const long long hi = s[0] * (1ll << 21) + s[1] * (1ll << 14) + s[2] * 128 + s[3];
-              const long long lo = s[4] * (1ll << 21) + s[5] * (1ll << 14) + s[6] * 128 + s[7];
-              const double v = fma((double)hi, 0x1p-33, (double)lo * 0x1p-61);
-              (y ? z.y : z.x) = v * s1 * s2;
+              for (int l = 0; l < XG_D; ++l)   // S_l; with eight accumulators the last holds levels 7 and 8
+                s[l] = __float2int_rn(__uint_as_float(a[l][c + y]) *
+                                      __uint_as_float((uint32_t)(127 + 7 * l + 12) << 23));
+              if (nlev < XG_D)
+                s[8] = __float2int_rn(128.0f * (__uint_as_float(a[7][c + y]) * 0x1p61f - (float)s[7]));
+              (y ? z.y : z.x) = xg_value(s, e);
             }
             const int m = ch.x + (c0 + c) / 2;
             if (live && c0 + c < 2 * mrows) {
-              if (g.bad[m]) z.x = z.y = __longlong_as_double(0x7ff8000000000000ll);
+              if (badm >> ((c0 + c) / 2) & 1) z.x = z.y = __longlong_as_double(0x7ff8000000000000ll);
               double2 *o = g.C + (int64_t)m * g.ldc + n;
               if (k0) {
                 const double2 p = *o;
@@ -387,19 +446,19 @@ int xgemm_colexp(Workspace &ws, int64_t nrhs, int64_t N, int K, const double2 *B
   return EPHG_OK;
 }
 
-int resident_colexp(ColExp &x, int64_t N, int K, const double2 *B, int64_t ldb, int64_t *bytes, cudaStream_t st,
-                    const int **out) {
+int resident_colexp(ColExp &x, int64_t nrhs, int64_t N, int K, const double2 *B, int64_t bstride, int64_t *bytes,
+                    cudaStream_t st, const int **out) {
   std::lock_guard<std::mutex> lk(x.mu);
   if (!x.e) {
     int *e = nullptr;
-    if (pool_alloc((void **)&e, (size_t)N * sizeof(int), st) != cudaSuccess) return EPHG_ERR_NOMEM;
-    col_exp(1, N, K, B, ldb, 0, e, st);
+    if (pool_alloc((void **)&e, (size_t)(nrhs * N) * sizeof(int), st) != cudaSuccess) return EPHG_ERR_NOMEM;
+    col_exp(nrhs, N, K, B, N, bstride, e, st);
     if (cudaGetLastError() != cudaSuccess || cudaStreamSynchronize(st) != cudaSuccess) {   // other streams may read it
       cudaFreeAsync(e, st);
       return EPHG_ERR_CUDA;
     }
     x.e = e;
-    if (bytes) *bytes += N * (int64_t)sizeof(int);
+    if (bytes) *bytes += nrhs * N * (int64_t)sizeof(int);
   }
   *out = x.e;
   return EPHG_OK;
@@ -412,15 +471,22 @@ static int xg_sms() {
   return n > 0 ? n : 1;
 }
 
+template <int W>
+static void xg_run(const XgArgs &g, cudaStream_t st) {
+  static std::once_flag attr_once;   // once per process: changing a kernel attribute can wait for queued work
+  std::call_once(attr_once,
+                 [] { cudaFuncSetAttribute(k_xgemm<W>, cudaFuncAttributeMaxDynamicSharedMemorySize, XG_SMEM); });
+  k_xgemm<W><<<(unsigned)std::min<int64_t>(g.units, xg_sms()), XG_THREADS, XG_SMEM, st>>>(g);
+}
+
 // one launch over mch chunks (dig sized for them)
 static void xg_launch(XgArgs &g, const double2 *A, int64_t lda, uint8_t *dig, int *bad, cudaStream_t st) {
-  static std::once_flag attr_once;   // once per process: changing a kernel attribute can wait for queued work
-  std::call_once(attr_once, [] { cudaFuncSetAttribute(k_xgemm, cudaFuncAttributeMaxDynamicSharedMemorySize, XG_SMEM); });
   g.dig = dig;
   g.bad = bad;
   g.units = (g.N + XG_ROWS - 1) / XG_ROWS * g.mch;
-  k_xg_phases<<<dim3(g.kch, g.mch), 256, 0, st>>>(g.chunks, g.M, g.K, g.kch, A, lda, dig, bad);
-  k_xgemm<<<(unsigned)std::min<int64_t>(g.units, xg_sms()), XG_THREADS, XG_SMEM, st>>>(g);
+  const int W = (2 * g.rpc + 15) / 16 * 16;   // MMA columns of a level
+  k_xg_phases<<<dim3(g.kch, g.mch), 4 * W, 0, st>>>(g.chunks, g.M, g.rpc, W, g.K, g.kch, A, lda, dig, bad);
+  W == 16 ? xg_run<16>(g, st) : W == 32 ? xg_run<32>(g, st) : W == 48 ? xg_run<48>(g, st) : xg_run<64>(g, st);
 }
 
 int launch_xgemm(Workspace &ws, int M, int64_t N, int K, const double2 *A, int64_t lda, const double2 *B, int64_t ldb,
@@ -444,6 +510,7 @@ int launch_xgemm(Workspace &ws, int M, int64_t N, int K, const double2 *A, int64
     g.K = K;
     g.kch = kch;
     g.mch = (g.M + XG_M - 1) / XG_M;
+    g.rpc = (g.M + g.mch - 1) / g.mch;   // even chunks
     g.N = N;
     g.ldb = ldb;
     g.ldc = ldc;
@@ -461,8 +528,8 @@ int launch_xgemm(Workspace &ws, int M, int64_t N, int K, const double2 *A, int64
 }
 
 int launch_xgemm_chunks(Workspace &ws, const int4 *chunks, int nchunks, int rows, int64_t N, int K, const double2 *A,
-                        int64_t lda, const double2 *B, int64_t bstride, const int *cexp, double2 *C, int64_t ldc,
-                        int *err, cudaStream_t st) {
+                        int64_t lda, const double2 *B, int64_t ldb, int64_t bstride, const int *cexp, double2 *C,
+                        int64_t ldc, int *err, cudaStream_t st) {
   if (nchunks <= 0) return EPHG_OK;
   const int kch = (K + XG_CELLS - 1) / XG_CELLS;
   uint8_t *dig;
@@ -477,10 +544,12 @@ int launch_xgemm_chunks(Workspace &ws, const int4 *chunks, int nchunks, int rows
   g.K = K;
   g.kch = kch;
   g.mch = nchunks;
+  g.rpc = std::min(rows, XG_CHUNK);
   g.N = N;
-  g.ldb = N;
+  g.ldb = ldb;
   g.ldc = ldc;
   g.bstride = bstride;
+  g.estride = ldb;
   g.B = B;
   g.cexp = cexp;
   g.C = C;

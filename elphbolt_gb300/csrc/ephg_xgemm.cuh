@@ -19,17 +19,17 @@ struct ColExp {
 int launch_xgemm(Workspace &ws, int M, int64_t N, int K, const double2 *A, int64_t lda, const double2 *B, int64_t ldb,
                  const int *cexp, double2 *C, int64_t ldc, int *err, cudaStream_t st);
 // Rows of A against several right-hand sides in one launch: chunk c (device) is (first row, rows
-// <= XG_CHUNK, right-hand side); right-hand side b is B + b bstride, [K][N] at stride N.
-// cexp: the nrhs x N exponents of xgemm_colexp.
+// <= XG_CHUNK, right-hand side); right-hand side b is B + b bstride, [K][N] at row stride ldb.
+// cexp: the exponents of xgemm_colexp, ldb per right-hand side.
 constexpr int XG_CHUNK = 32;
 int xgemm_colexp(Workspace &ws, int64_t nrhs, int64_t N, int K, const double2 *B, int64_t bstride, const int **cexp,
                  cudaStream_t st);
 int launch_xgemm_chunks(Workspace &ws, const int4 *chunks, int nchunks, int rows, int64_t N, int K, const double2 *A,
-                        int64_t lda, const double2 *B, int64_t bstride, const int *cexp, double2 *C, int64_t ldc,
+                        int64_t lda, const double2 *B, int64_t ldb, int64_t bstride, const int *cexp, double2 *C, int64_t ldc,
                         int *err, cudaStream_t st);
-// The exponents of a resident operand B[K][N], built once (allocated from the library pool on st
+// The exponents of a resident operand (nrhs right-hand sides B[K][N] at stride N, bstride apart), built once (allocated from the library pool on st
 // and complete when this returns); *bytes grows by what was allocated.
-int resident_colexp(ColExp &x, int64_t N, int K, const double2 *B, int64_t ldb, int64_t *bytes, cudaStream_t st,
-                    const int **out);
+int resident_colexp(ColExp &x, int64_t nrhs, int64_t N, int K, const double2 *B, int64_t bstride, int64_t *bytes,
+                    cudaStream_t st, const int **out);
 
 }  // namespace ephg

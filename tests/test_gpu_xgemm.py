@@ -4,9 +4,11 @@ counts and cell counts that leave tiles ragged, more cells than one accumulation
 holds, columns of very different magnitude, and non-finite values.
 
 Tolerance, derived: the split sum is exact to ~2^-60 of the largest product and
-rounded once, 2^-53 of the result; the phases of the two sides differ by their own
-rounding, at most 4 units of 2^-53 for |2 pi k.R| <= 80 rad of equal arguments.
-So each element is within 6 2^-53 sum_R |phase_R| |x_R|.
+rounded once, 2^-53 of the result.  The k-points are multiples of 1/64, so k.R is
+exact and the reference's phases are exact to extended precision; the library's
+are products of three table entries of error 2^-53 each, two complex products and
+a scaling, under 9 2^-53 in all.  So each element is within 12 2^-53
+sum_R |phase_R| |x_R|.
 """
 import dataclasses
 
@@ -44,16 +46,14 @@ def crystal(kind):
 
 
 def phases(k, R, deg):
-    d = k[:, 0:1] * R[:, 0]
-    d = d + k[:, 1:2] * R[:, 1]
-    d = d + k[:, 2:3] * R[:, 2]
-    return np.exp(1j * (2 * np.pi * d)) / deg
+    a = (k @ R.T) % 1.0 * (2 * np.longdouble("3.14159265358979323846264338327950288"))   # exact up to the last product
+    return (np.cos(a) + 1j * np.sin(a)) / deg.astype(np.longdouble)
 
 
 def check(out, ph, x):
     """out (n, ...), ph (n, R), x (R, ...)"""
     ref = np.tensordot(ph.astype(np.clongdouble), x.astype(np.clongdouble), axes=(1, 0))
-    tol = 6 * 2.0 ** -53 * np.tensordot(np.abs(ph), np.abs(x.real) + np.abs(x.imag), axes=(1, 0))
+    tol = 12 * 2.0 ** -53 * np.tensordot(np.abs(ph), np.abs(x.real) + np.abs(x.imag), axes=(1, 0))
     d = (out - ref).astype(np.complex128)
     assert np.all(np.abs(d.real) <= tol) and np.all(np.abs(d.imag) <= tol)
 
