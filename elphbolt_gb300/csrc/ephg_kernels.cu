@@ -758,32 +758,36 @@ void launch_heig(int batch, int n, const double2 *A, int64_t stride, double *w, 
 
 // ============================================================ electrons
 // el_wann post-processing (wannier.f90:499-520): energies (eV, + scissor),
-// evecs(k,b,:) = eigenvector b, velocities by Feynman-Hellmann.
-__global__ void k_el_post(int nk, int nw, const double *w, const double2 *V, const double2 *C,
-                          int64_t ldc, int with_vel, const double *scissor, double *energies_f,
-                          double *vel_f, double2 *evecs_f, double *ens_i) {
+// evecs(k,b,:) = eigenvector b, velocities by Feynman-Hellmann.  A thread per band
+// and direction (y = 0 also writes the band's energy and vector) in blocks of one
+// warp: a few hundred k-points then reach most SMs, where one thread per band in
+// blocks of 128 left 200 k-points on 13 of them (45 us; now 17).
+__global__ void __launch_bounds__(32) k_el_post(int nk, int nw, const double *w, const double2 *V, const double2 *C,
+                                                int64_t ldc, const double *scissor, double *energies_f, double *vel_f,
+                                                double2 *evecs_f, double *ens_i) {
   int idx = blockIdx.x * blockDim.x + threadIdx.x;
   if (idx >= nk * nw) return;
   int k = idx / nw, b = idx % nw;
   const size_t nn = (size_t)nw * nw;
-  double e = w[(size_t)k * nw + b] * Ryd2eV;
-  if (scissor) e += scissor[b];
-  if (energies_f) energies_f[k + (int64_t)nk * b] = e;
-  if (ens_i) ens_i[(size_t)k * nw + b] = e;
   const double2 *Vk = V + (size_t)k * nn;
-  if (evecs_f)
-    for (int c = 0; c < nw; ++c) evecs_f[k + (int64_t)nk * (b + (int64_t)nw * c)] = Vk[c + nw * b];
-  if (with_vel && vel_f) {
-    for (int p = 0; p < 3; ++p) {
-      const double2 *dH = C + (int64_t)k * ldc + (size_t)(1 + p) * nn;
-      double2 acc = make_double2(0.0, 0.0);
-      for (int r = 0; r < nw; ++r) {
-        double2 mv = make_double2(0.0, 0.0);
-        for (int c = 0; c < nw; ++c) cfma(mv, dH[r + nw * c], Vk[c + nw * b]);
-        cfma_cj(acc, Vk[r + nw * b], mv);
-      }
-      vel_f[k + (int64_t)nk * (b + (int64_t)nw * p)] = acc.x * Ryd2radTHz;
+  const int p = blockIdx.y;
+  if (p == 0) {
+    double e = w[(size_t)k * nw + b] * Ryd2eV;
+    if (scissor) e += scissor[b];
+    if (energies_f) energies_f[k + (int64_t)nk * b] = e;
+    if (ens_i) ens_i[(size_t)k * nw + b] = e;
+    if (evecs_f)
+      for (int c = 0; c < nw; ++c) evecs_f[k + (int64_t)nk * (b + (int64_t)nw * c)] = Vk[c + nw * b];
+  }
+  if (vel_f) {
+    const double2 *dH = C + (int64_t)k * ldc + (size_t)(1 + p) * nn;
+    double2 acc = make_double2(0.0, 0.0);
+    for (int r = 0; r < nw; ++r) {
+      double2 mv = make_double2(0.0, 0.0);
+      for (int c = 0; c < nw; ++c) cfma(mv, dH[r + nw * c], Vk[c + nw * b]);
+      cfma_cj(acc, Vk[r + nw * b], mv);
     }
+    vel_f[k + (int64_t)nk * (b + (int64_t)nw * p)] = acc.x * Ryd2radTHz;
   }
 }
 
@@ -792,13 +796,13 @@ void launch_el_post(int nk, int nw, const double *w, const double2 *V, const dou
                     double *vel_f, double2 *evecs_f, double *ens_i, cudaStream_t st) {
   int n = nk * nw;
   if (n == 0) return;
-  k_el_post<<<(n + 127) / 128, 128, 0, st>>>(nk, nw, w, V, C, ldc, with_vel, scissor, energies_f,
-                                             vel_f, evecs_f, ens_i);
+  k_el_post<<<dim3((n + 31) / 32, with_vel && vel_f ? 3 : 1), 32, 0, st>>>(nk, nw, w, V, C, ldc, scissor, energies_f,
+                                                                        with_vel ? vel_f : nullptr, evecs_f, ens_i);
 }
 
 // ============================================================= phonons
-// ph_wann post-processing (wannier.f90:740-780)
-__global__ void k_ph_post(int nq, int nb, const int *qp, const double *qv, const double *w,
+// ph_wann post-processing (wannier.f90:740-780); a thread per mode and direction, as k_el_post
+__global__ void __launch_bounds__(32) k_ph_post(int nq, int nb, const int *qp, const double *qv, const double *w,
                           const double2 *V, const double2 *dDq, int64_t ldd, int with_vel,
                           const double *masses, double *energies_f, double2 *evecs_f,
                           double *vel_f, double *om_i, double2 *u_i, float2 *u_f, int *err) {
@@ -810,25 +814,21 @@ __global__ void k_ph_post(int nq, int nb, const int *qp, const double *qv, const
   double e = sqrt(fabs(o2));
   if (o2 < 0.0 || signbit(o2)) e = -e;          // sign(sqrt(abs(w)), w)
   const double2 *Vq = V + (size_t)q * nn;
-  double vel[3] = {0.0, 0.0, 0.0};
-  if (with_vel) {
-    for (int p = 0; p < 3; ++p) {
-      const double2 *dD = dDq + (size_t)q * ldd + p * nn;
-      double2 acc = make_double2(0.0, 0.0);
-      for (int r = 0; r < nb; ++r) {
-        double2 mv = make_double2(0.0, 0.0);
-        for (int c = 0; c < nb; ++c) cfma(mv, dD[r + nb * c], Vq[c + nb * s]);
-        cfma_cj(acc, Vq[r + nb * s], mv);
-      }
-      vel[p] = acc.x / (2.0 * e) * Ryd2radTHz;
+  const int p = blockIdx.y;
+  const bool gamma = qp ? (qp[q] == 0) : (qv[q] == 0.0 && qv[q + nq] == 0.0 && qv[q + 2 * nq] == 0.0);
+  if (with_vel && vel_f) {
+    const double2 *dD = dDq + (size_t)q * ldd + p * nn;
+    double2 acc = make_double2(0.0, 0.0);
+    for (int r = 0; r < nb; ++r) {
+      double2 mv = make_double2(0.0, 0.0);
+      for (int c = 0; c < nb; ++c) cfma(mv, dD[r + nb * c], Vq[c + nb * s]);
+      cfma_cj(acc, Vq[r + nb * s], mv);
     }
+    vel_f[q + (int64_t)nq * (s + (int64_t)nb * p)] = gamma ? 0.0 : acc.x / (2.0 * e) * Ryd2radTHz;
   }
+  if (p) return;
   e *= Ryd2eV;
-  bool gamma = qp ? (qp[q] == 0) : (qv[q] == 0.0 && qv[q + nq] == 0.0 && qv[q + 2 * nq] == 0.0);
-  if (gamma) {
-    if (s < 3) e = 0.0;
-    vel[0] = vel[1] = vel[2] = 0.0;
-  }
+  if (gamma && s < 3) e = 0.0;
   if (e < -0.005) atomicOr(err, DERR_NEG_PHONON);
   else if (e < 0.0 && e > -0.005) e = 0.0;
   if (energies_f) energies_f[q + (int64_t)nq * s] = e;
@@ -842,8 +842,6 @@ __global__ void k_ph_post(int nq, int nb, const int *qp, const double *qv, const
       if (u_i) u_i[((size_t)q * nb + s) * nb + c] = u;
       if (u_f) u_f[((size_t)q * nb + s) * nb + c] = make_float2((float)u.x, (float)u.y);
     }
-  if (with_vel && vel_f)
-    for (int p = 0; p < 3; ++p) vel_f[q + (int64_t)nq * (s + (int64_t)nb * p)] = vel[p];
 }
 
 void launch_ph_post(int nq, int nb, const int *qp, const double *qv, const double *w,
@@ -852,7 +850,7 @@ void launch_ph_post(int nq, int nb, const int *qp, const double *qv, const doubl
                     double2 *u_i, float2 *u_f, int *err, cudaStream_t st) {
   int n = nq * nb;
   if (n == 0) return;
-  k_ph_post<<<(n + 127) / 128, 128, 0, st>>>(nq, nb, qp, qv, w, V, dDq, ldd, with_vel, masses,
+  k_ph_post<<<dim3((n + 31) / 32, with_vel && vel_f ? 3 : 1), 32, 0, st>>>(nq, nb, qp, qv, w, V, dDq, ldd, with_vel, masses,
                                              energies_f, evecs_f, vel_f, om_i, u_i, u_f, err);
 }
 

@@ -153,8 +153,27 @@ struct GemmArgs {
   int64_t ldc;
   int *err;
   int ileave;                // 1: outputs interleaved by 32 rows in groups of 4 columns: (r, c) at
-                             //    (r / 32) ldc 32 + (c / 4) 128 + (r % 32) 4 + c % 4 (ldc a multiple of 4)
+                             //    (r / 32) ldc 32 + (c / 4) 128 + (r % 32) 4 + c % 4 (ldc a multiple of 4);
+                             // 2: in groups of 32 columns (ileave32)
 };
+
+// Element (r, c) of an output interleaved by 32 rows in groups of 32 columns: a drain
+// lane's 16 columns are 64 consecutive bytes and a warp's 32 rows lie in 4 KB, so it
+// writes whole sectors; a reader of one row gets whole 128-byte lines.  Row-major, each store of a
+// warp touched 32 rows 1 MB apart, half a sector each: at 96 K positions the drain
+// took 20,000 of a stage-A tile's 32,000 cycles (nw 16, nb 12, 13^3: stage A's GEMMs
+// 1.60 ms per launch, now 1.05; groups of 16 columns 0.86, but the rotation that reads
+// them 1.34 -> 1.76 instead of 1.41).
+__host__ __device__ __forceinline__ int64_t ileave32(int64_t r, int64_t c, int64_t ldc) {
+  return ((r >> 5) * ldc + (c & ~(int64_t)31)) * 32 + (r & 31) * 32 + (c & 31);
+}
+
+// 32 bytes in one streaming store
+__device__ __forceinline__ void st_cs8(float *p, const float *v) {
+  asm volatile("st.global.cs.v8.f32 [%0], {%1,%2,%3,%4,%5,%6,%7,%8};" ::"l"(p), "f"(v[0]), "f"(v[1]), "f"(v[2]), "f"(v[3]),
+               "f"(v[4]), "f"(v[5]), "f"(v[6]), "f"(v[7])
+               : "memory");
+}
 
 // One output tile as the three roles see it: operand maps, first A / B row of
 // plane 0, K blocks, and the tile's first output element.
@@ -223,6 +242,38 @@ struct GroupGemm {
     return tile_job(&q->tA, &q->tB, q->g, t - q->tile0);
   }
 };
+
+// The MMAs of one stage (d: descriptor of its first plane; addresses count 16 bytes).
+// A operand with two adjacent B planes is one MMA of N = 256 into two adjacent
+// accumulators: every element's chain of products is the one of twelve N = 128
+// MMAs, in their order (the products with -Im need the planes in the other order
+// and stay narrow).  Descriptors are constants off one base.  nw 16, nb 12, 13^3
+// (96 K positions): the GEMMs 5.80 -> 5.71 ms; their drain is the larger part there.
+template <bool NEAR>
+__device__ __forceinline__ void cgemm_stage(uint32_t tmem, uint64_t d, uint32_t more) {
+  constexpr uint32_t IDP = idesc_tf32(false), IDN = idesc_tf32(true), IDW = idesc_tf32_n(false, 2 * BN);
+  constexpr uint32_t P = PLANE_BYTES >> 4;
+  const uint32_t m = tmem, c = tmem + 2 * BN;   // main and correction accumulators (re | im)
+  const uint32_t dm = NEAR ? c : m;
+#pragma unroll
+  for (int ks = 0; ks < BK / 8; ++ks) {
+    const uint64_t k = d + 2 * ks;   // 8 tf32 = 32 B along K inside the swizzle atom
+    const uint64_t Ahr = k, Ahi = k + P, Alr = k + 2 * P, Ali = k + 3 * P;
+    const uint64_t Bhr = k + 4 * P, Bhi = k + 5 * P, Blr = k + 6 * P, Bli = k + 7 * P;
+    const uint32_t acc = ks ? 1u : more;
+    // corrections: hi*lo + lo*hi
+    umma(c, Ahr, Blr, IDW, acc);        // (Ahr Blr | Ahr Bli)
+    umma(c, Alr, Bhr, IDW, 1);          // (Alr Bhr | Alr Bhi)
+    umma(c, Ahi, Bli, IDN, 1);
+    umma(c + BN, Ahi, Blr, IDP, 1);
+    umma(c, Ali, Bhi, IDN, 1);
+    umma(c + BN, Ali, Bhr, IDP, 1);
+    // main: Re = Ar Br - Ai Bi, Im = Ar Bi + Ai Br (hi parts)
+    umma(dm, Ahr, Bhr, IDW, NEAR ? 1u : acc);
+    umma(dm, Ahi, Bhi, IDN, 1);
+    umma(dm + BN, Ahi, Bhr, IDP, 1);
+  }
+}
 
 // Warp-specialised 3xTF32 complex GEMM over the tiles [t0, t1) of a tile
 // space, strided by the grid: warp 0 lane 0 issues TMA loads, warp 1 lane 0
@@ -300,12 +351,11 @@ __device__ __forceinline__ void cgemm_body(const Jobs &jobs, int t0, int t1, int
     }
   } else if (warp == 1) {
     if (lane == 0) {   // ---- MMA issuer
-      constexpr uint32_t IDP = idesc_tf32(false), IDN = idesc_tf32(true);
       int stage = 0;
       uint32_t phase = 0;
       int it = 0;
       bool ok = true;
-      const uint32_t mr = tmem, mi = tmem + BN, cr = tmem + 2 * BN, ci = tmem + 3 * BN;
+      const uint64_t d0 = sdesc(smem);
       for (int t = t0 + blockIdx.x; t < t1 && ok; t += gridDim.x, ++it) {
         const int nkb = jobs(t).nkb;
         if (!mbar_wait(&tempty[0], (it & 1) ^ 1, err)) { ok = false; break; }
@@ -313,35 +363,11 @@ __device__ __forceinline__ void cgemm_body(const Jobs &jobs, int t0, int t1, int
         for (int kb = 0; kb < nkb; ++kb) {
           if (!mbar_wait(&full[stage], phase, err)) { ok = false; break; }
           tc_fence_after();
-          uint8_t *sb = smem + stage * STAGE_BYTES;
-#pragma unroll
-          for (int ks = 0; ks < BK / 8; ++ks) {
-            const int off = ks * 32;   // 8 tf32 = 32 B along K inside the swizzle atom
-            const uint64_t Ahr = sdesc(sb + 0 * PLANE_BYTES + off), Ahi = sdesc(sb + 1 * PLANE_BYTES + off);
-            const uint64_t Alr = sdesc(sb + 2 * PLANE_BYTES + off), Ali = sdesc(sb + 3 * PLANE_BYTES + off);
-            const uint64_t Bhr = sdesc(sb + 4 * PLANE_BYTES + off), Bhi = sdesc(sb + 5 * PLANE_BYTES + off);
-            const uint64_t Blr = sdesc(sb + 6 * PLANE_BYTES + off), Bli = sdesc(sb + 7 * PLANE_BYTES + off);
-            const uint32_t acc = (kb == 0 && ks == 0) ? 0u : 1u;
-            // corrections: hi*lo + lo*hi
-            umma(cr, Ahr, Blr, IDP, acc);
-            umma(cr, Alr, Bhr, IDP, 1);
-            umma(cr, Ahi, Bli, IDN, 1);
-            umma(cr, Ali, Bhi, IDN, 1);
-            umma(ci, Ahr, Bli, IDP, acc);
-            umma(ci, Alr, Bhi, IDP, 1);
-            umma(ci, Ahi, Blr, IDP, 1);
-            umma(ci, Ali, Bhr, IDP, 1);
-            // main: Re = Ar Br - Ai Bi, Im = Ar Bi + Ai Br (hi parts).  The last K
-            // block holds the nearest cells, the largest terms: they go to the
-            // short correction chain instead of the long main chain.
-            const bool nearblk = (kb == nkb - 1) && nkb > 1;
-            const uint32_t dr = nearblk ? cr : mr, di = nearblk ? ci : mi;
-            const uint32_t am = nearblk ? 1u : acc;
-            umma(dr, Ahr, Bhr, IDP, am);
-            umma(dr, Ahi, Bhi, IDN, 1);
-            umma(di, Ahr, Bhi, IDP, am);
-            umma(di, Ahi, Bhr, IDP, 1);
-          }
+          const uint64_t sd = d0 + (uint32_t)(stage * (STAGE_BYTES >> 4));
+          // The last K block holds the nearest cells, the largest terms: their main
+          // products go to the short correction chain instead of the long main chain.
+          if (kb == nkb - 1 && nkb > 1) cgemm_stage<true>(tmem, sd, 1u);
+          else cgemm_stage<false>(tmem, sd, kb ? 1u : 0u);
           umma_commit(&empty[stage]);     // frees the smem stage when these MMAs retire
           if (++stage == STAGES) { stage = 0; phase ^= 1; }
         }
@@ -366,8 +392,8 @@ __device__ __forceinline__ void cgemm_body(const Jobs &jobs, int t0, int t1, int
       const uint32_t tr = tmem + ((uint32_t)(quad * 32) << 16);
       // row-major: the row's 16 columns as float4 stores; interleaved: each group of
       // 4 columns of the warp's 32 rows is 512 consecutive bytes (one float4 per lane)
-      float *cr = j.ileave ? j.Cr + (int64_t)quad * j.ldc * 32 + 4 * lane : j.Cr + (int64_t)row * j.ldc;
-      float *ci = j.ileave ? j.Ci + (int64_t)quad * j.ldc * 32 + 4 * lane : j.Ci + (int64_t)row * j.ldc;
+      const int64_t off = j.ileave ? (int64_t)quad * j.ldc * 32 + (j.ileave == 2 ? 32 : 4) * lane : (int64_t)row * j.ldc;
+      float *cr = j.Cr + off, *ci = j.Ci + off;
 #pragma unroll 1
       for (int c0 = cbeg; c0 < cbeg + CW; c0 += 16) {
         uint32_t ar[16], ai[16], br[16], bi[16];
@@ -383,7 +409,13 @@ __device__ __forceinline__ void cgemm_body(const Jobs &jobs, int t0, int t1, int
           vi[q] = __uint_as_float(ai[q]) + __uint_as_float(bi[q]);
         }
         // streaming stores: the output is read once, later, by another kernel
-        if (j.ileave) {
+        if (j.ileave == 2) {
+          const int64_t o = (int64_t)(c0 & ~31) * 32 + (c0 & 16);
+          st_cs8(cr + o, vr);
+          st_cs8(cr + o + 8, vr + 8);
+          st_cs8(ci + o, vi);
+          st_cs8(ci + o + 8, vi + 8);
+        } else if (j.ileave) {
 #pragma unroll
           for (int q = 0; q < 4; ++q) {
             __stcs((float4 *)(cr + (int64_t)(c0 + 4 * q) * 32),
@@ -768,7 +800,7 @@ __global__ void k_rotate_planes(int j0, int j1, int i0, const int *st_code, int 
   const int p = widx[i];
   const double2 *Uk = U + ((size_t)p * nw + m) * nw;
   const int ncol = nw * nb;
-  const int64_t grow = (int64_t)(i - i0) * ldg;
+  const int64_t grow = i - i0;
   for (int e = blockIdx.x * blockDim.x + threadIdx.x; e < ncol * nws; e += gridDim.x * blockDim.x) {
     const int rp = e % nws, c = e / nws;
     const int np = c % nw, s = c / nw;
@@ -776,7 +808,7 @@ __global__ void k_rotate_planes(int j0, int j1, int i0, const int *st_code, int 
     ph = make_double2(ph.x / degq[rp], -ph.y / degq[rp]);
     double2 acc = make_double2(0.0, 0.0);
     for (int mp = 0; mp < nw; ++mp) {
-      int64_t off = grow + np + nw * (mp + (int64_t)nw * (s + (int64_t)nb * rp));
+      const int64_t off = ileave32(grow, np + nw * (mp + (int64_t)nw * (s + (int64_t)nb * rp)), ldg);
       cfma(acc, Uk[mp], make_double2((double)gr[off], (double)gi[off]));
     }
     const int64_t col = (int64_t)(j - jbase) * ncol + c;
@@ -830,7 +862,6 @@ __global__ void __launch_bounds__(256) k_rotate_k(int i0, const int *first_state
     double2 u = U[((size_t)p * nw + m) * nw + mp];
     sU[t] = make_float2((float)u.x, (float)u.y);
   }
-  const int64_t grow = (int64_t)(i - i0) * ldg;
   const int64_t plane = Np2 * Kp2;
   for (int s0 = 0; s0 < nb; s0 += sch) {
     const int ns = min(sch, nb - s0), pc = nn * ns, nc = nw * ns;
@@ -849,7 +880,7 @@ __global__ void __launch_bounds__(256) k_rotate_k(int i0, const int *first_state
             const int kk = t / pc4, e = 4 * (t - kk * pc4);
             const int rp = kinv[kp0 + kk];
             if (rp >= 0) {
-              const int64_t off = grow + (int64_t)rp * per + nn * s0 + e;
+              const int64_t off = ileave32(i - i0, (int64_t)rp * per + nn * s0 + e, ldg);
               a[u] = __ldg((const float4 *)(gr + off));
               b[u] = __ldg((const float4 *)(gi + off));
             }
@@ -2484,7 +2515,7 @@ static int split_rates_generic(SplitOperands &s, Workspace &ws, cudaStream_t st,
                                                                  degk, kposA, roots, PA, Mp, KpA);
     TCK(cudaGetLastError());
     tA->begin(st);
-    if ((rc = cgemm(PA, Mp, 0, Mp, s.G, NpA, 0, (int)NpA, KpA, CAr, CAi, NpA, err, st, chunk_us, yield, bm)))
+    if ((rc = cgemm(PA, Mp, 0, Mp, s.G, NpA, 0, (int)NpA, KpA, CAr, CAi, NpA, err, st, chunk_us, yield, bm, 2)))
       return rc;
     tA->end(st);
     {
