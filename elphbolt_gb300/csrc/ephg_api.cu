@@ -1255,6 +1255,7 @@ int ephg::el_rates_view(ephg_handle *h, const ExecView &x, const ephg_rate_reque
   ed.glp = glp;
   ed.glpf = glpf;
   ed.per_state = (int64_t)nin * nb;
+  ed.nin = nin;
   double *g2d = nullptr, *xpd = nullptr, *xmd = nullptr, *yd = nullptr, *phr = nullptr;
   int64_t vtot = (int64_t)nst * nin * nb;
   int64_t vcap = std::min<int64_t>(cap, vtot);
@@ -1291,7 +1292,6 @@ int ephg::el_rates_view(ephg_handle *h, const ExecView &x, const ephg_rate_reque
       rs.mt[p] = mt;
     }
     ed.fin = fin;
-    ed.nin = nin;
     ed.mt = rs.mt[0];
     (*x.launches) += 1 + nsets;
     if (req->delta_kind != 0) {

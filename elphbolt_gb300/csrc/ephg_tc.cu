@@ -144,6 +144,18 @@ __device__ __forceinline__ void tmem_ld16_nowait(uint32_t taddr, uint32_t *r) {
 }
 
 // -------------------------------------------------------- the GEMM kernel
+// Stage B with the k' rotation in its drain (nw != 0): instead of the nw nb sums G(n', s') of
+// every (k' row, state), the products h(n, s') = sum_n' conj(U_k'[n][n']) G(n', s') of the
+// row's window bands n are written, H[(state nb + s')][final state], n_window nb values
+// for nw nb.  nw divides the tile's columns (8, 16, 32).
+struct RotOut {
+  int nw = 0;
+  const int4 *row = nullptr;    // per row: mesh index, window-band mask, first final state (mask 0: padding)
+  const float2 *Uf = nullptr;   // [mesh point][band][n']
+  float2 *H = nullptr;
+  int64_t ldh = 0;
+};
+
 struct GemmArgs {
   int mtiles, ntiles, nkb;   // tile counts, K blocks of BK
   int t0, t1;                // tiles [t0, t1) of this launch
@@ -155,6 +167,7 @@ struct GemmArgs {
   int ileave;                // 1: outputs interleaved by 32 rows in groups of 4 columns: (r, c) at
                              //    (r / 32) ldc 32 + (c / 4) 128 + (r % 32) 4 + c % 4 (ldc a multiple of 4);
                              // 2: in groups of 32 columns (ileave32)
+  RotOut rot;
 };
 
 // Element (r, c) of an output interleaved by 32 rows in groups of 32 columns: a drain
@@ -184,6 +197,7 @@ struct TileJob {
   float *Cr, *Ci;
   int64_t ldc;
   int ileave;
+  RotOut rot;   // H at the tile's first (state, s') row
 };
 
 __host__ __device__ __forceinline__ TileJob tile_job(const CUtensorMap *tA, const CUtensorMap *tB, const GemmArgs &g,
@@ -203,6 +217,8 @@ __host__ __device__ __forceinline__ TileJob tile_job(const CUtensorMap *tA, cons
   j.Ci = g.Ci + off;
   j.ldc = g.ldc;
   j.ileave = g.ileave;
+  j.rot = g.rot;
+  if (g.rot.nw) j.rot.H += (int64_t)nt * (BN / g.rot.nw) * g.rot.ldh;
   return j;
 }
 
@@ -273,6 +289,70 @@ __device__ __forceinline__ void cgemm_stage(uint32_t tmem, uint64_t d, uint32_t 
     umma(dm, Ahi, Bhi, IDN, 1);
     umma(dm + BN, Ahi, Bhr, IDP, 1);
   }
+}
+
+// The drain of a tile with the k' rotation: a lane's row ip, its window bands two (nw 32:
+// one) at a time with their U_k' rows in registers, loaded while the tile's MMAs run.  Sums
+// and their order are those of a thread that reads G back (ascending n').  The output
+// is ~nw times smaller, and final states, not rows, are what lanes lie along when it
+// is read.  Returns false if the wait gave up.
+template <int NW>
+__device__ __forceinline__ bool rot_drain(const RotOut &ro, int ip, uint32_t tr, uint64_t *tfull, uint32_t parity,
+                                          int *err) {
+  constexpr int NBP = NW <= 16 ? 2 : 1;   // bands per pass over the accumulators
+  const int4 ri = __ldg(ro.row + ip);
+  unsigned left = (unsigned)ri.y;
+  const int nbw = __popc(left), nbmax = __reduce_max_sync(0xffffffffu, nbw);
+  const float2 *Urow = ro.Uf + (size_t)ri.x * NW * NW;
+  for (int b0 = 0; b0 == 0 || b0 < nbmax; b0 += NBP) {
+    float2 u[NBP][NW];
+#pragma unroll
+    for (int b = 0; b < NBP; ++b) {
+      const int n = left ? __ffs(left) - 1 : 0;
+      left &= left - 1;   // 0 stays 0
+      if (b0 + b < nbw)
+#pragma unroll
+        for (int c = 0; c < NW; c += 2) {
+          const float4 t = __ldg((const float4 *)(Urow + (size_t)n * NW + c));
+          u[b][c] = make_float2(t.x, t.y);
+          u[b][c + 1] = make_float2(t.z, t.w);
+        }
+    }
+    if (b0 == 0) {
+      if (!mbar_wait(tfull, parity, err)) return false;
+      tc_fence_after();
+    }
+    float2 *out = ro.H + ri.z + b0;
+    float2 a[NBP];
+#pragma unroll 1
+    for (int c0 = 0; c0 < BN; c0 += (NW > 16 ? NW : 16)) {
+#pragma unroll
+      for (int cc = 0; cc < (NW > 16 ? NW : 16); cc += 16) {
+        uint32_t ar[16], ai[16], br[16], bi[16];
+        __syncwarp();
+        tmem_ld16_nowait(tr + c0 + cc, ar);
+        tmem_ld16_nowait(tr + BN + c0 + cc, ai);
+        tmem_ld16_nowait(tr + 2 * BN + c0 + cc, br);
+        tmem_ld16_nowait(tr + 3 * BN + c0 + cc, bi);
+        asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
+#pragma unroll
+        for (int q = 0; q < 16; ++q) {
+          const float2 g = make_float2(__uint_as_float(ar[q]) + __uint_as_float(br[q]),
+                                       __uint_as_float(ai[q]) + __uint_as_float(bi[q]));
+          const int c = (cc + q) % NW;
+#pragma unroll
+          for (int b = 0; b < NBP; ++b) {
+            if (c == 0) a[b] = make_float2(0.f, 0.f);
+            if (b0 + b < nbw) {
+              cfmaf_cj(a[b], u[b][c], g);
+              if (c == NW - 1) __stcs(out + (int64_t)((c0 + cc + q) / NW) * ro.ldh + b, a[b]);
+            }
+          }
+        }
+      }
+    }
+  }
+  return true;
 }
 
 // Warp-specialised 3xTF32 complex GEMM over the tiles [t0, t1) of a tile
@@ -382,14 +462,24 @@ __device__ __forceinline__ void cgemm_body(const Jobs &jobs, int t0, int t1, int
   } else {   // ---- epilogue: warp w drains TMEM lane quadrant w % 4, column block (w - 2) / 4
     const int quad = warp & 3;
     constexpr int CW = BN / (GEMM_EPI_WARPS / 4);
+    static_assert(GEMM_EPI_WARPS == 4, "the rotating drain takes all columns of its quadrant");
     const int cbeg = ((warp - 2) >> 2) * CW;
     const int row = quad * 32 + lane;
     int it = 0;
     for (int t = t0 + blockIdx.x; t < t1; t += gridDim.x, ++it) {
       const TileJob j = jobs(t);
+      const uint32_t tr = tmem + ((uint32_t)(quad * 32) << 16);
+      if (j.rot.nw) {
+        const bool ok = j.rot.nw == 8    ? rot_drain<8>(j.rot, j.arow + row, tr, &tfull[0], it & 1, err)
+                        : j.rot.nw == 16 ? rot_drain<16>(j.rot, j.arow + row, tr, &tfull[0], it & 1, err)
+                                         : rot_drain<32>(j.rot, j.arow + row, tr, &tfull[0], it & 1, err);
+        if (!ok) break;
+        tc_fence_before();
+        mbar_arrive(&tempty[0]);
+        continue;
+      }
       if (!mbar_wait(&tfull[0], it & 1, err)) break;
       tc_fence_after();
-      const uint32_t tr = tmem + ((uint32_t)(quad * 32) << 16);
       // row-major: the row's 16 columns as float4 stores; interleaved: each group of
       // 4 columns of the warp's 32 rows is 512 consecutive bytes (one float4 per lane)
       const int64_t off = j.ileave ? (int64_t)quad * j.ldc * 32 + (j.ileave == 2 ? 32 : 4) * lane : (int64_t)row * j.ldc;
@@ -631,12 +721,13 @@ void batcher_stats(const GemmBatcher *b, int64_t *launches, int64_t *problems, i
 // With a batch member the GEMM joins its batcher's next grouped launch.
 static int cgemm(const float *Ap, int64_t Astride, int64_t Aoff, int Mp, const float *Bp, int64_t Bstride,
                  int64_t Boff, int Np, int Kp, float *Cr, float *Ci, int64_t ldc, int *err, cudaStream_t st,
-                 int chunk_us = 0, const Yield &yield = Yield(), const BatchMember *bm = nullptr, int ileave = 0) {
+                 int chunk_us = 0, const Yield &yield = Yield(), const BatchMember *bm = nullptr, int ileave = 0,
+                 const RotOut &rot = RotOut()) {
   if (Mp % BM || Np % BN || Kp % BK || Mp <= 0 || Np <= 0) return tfail(1, "cgemm: shapes not tile multiples");
   if (4 * Astride > INT32_MAX || 4 * Bstride > INT32_MAX) return tfail(1, "cgemm: operand too tall for TMA coords");
   if (bm && bm->gb) {
     GroupProblem p;
-    memset(&p, 0, sizeof p);
+    memset((void *)&p, 0, sizeof p);
     int rc;
     if ((rc = make_map(&p.tA, Ap, Kp, 4 * Astride)) || (rc = make_map(&p.tB, Bp, Kp, 4 * Bstride))) return rc;
     p.g.mtiles = Mp / BM;
@@ -651,6 +742,7 @@ static int cgemm(const float *Ap, int64_t Astride, int64_t Aoff, int Mp, const f
     p.g.ldc = ldc;
     p.g.err = err;
     p.g.ileave = ileave;
+    p.g.rot = rot;
     return bm->gb->submit(bm->id, p, st);
   }
   CUtensorMap ta, tb;
@@ -674,6 +766,7 @@ static int cgemm(const float *Ap, int64_t Astride, int64_t Aoff, int Mp, const f
   g.ldc = ldc;
   g.err = err;
   g.ileave = ileave;
+  g.rot = rot;
   int tiles = g.mtiles * g.ntiles;
   int grid = std::min(tiles, num_sms());
   // chunk_us > 0: launches of about that length (a tile is ~0.4 us per 16 K positions) so
@@ -1341,8 +1434,8 @@ __global__ void __launch_bounds__(EPI_ROWS) k_epilogue_split2(int nwv, int j0, i
   }
 }
 
-// Generic-shape split epilogue without shared-memory staging: one thread per
-// (k' row, state), EPI_ROWS consecutive rows of one state per block.  A thread
+// Split epilogue without shared-memory staging for nw = 24, whose bands the rotating
+// drain's tiles (multiples of 32 columns) would cut: one thread per (k' row, state), EPI_ROWS consecutive rows of one state per block.  A thread
 // reads its row's nw x nb complex Rp sums straight from the GEMM output, which
 // the GEMM wrote interleaved by 32 rows in 4-column groups (GemmArgs::ileave):
 // each float4 load of a warp is 512 consecutive bytes.  NW bands fixed
@@ -1350,9 +1443,9 @@ __global__ void __launch_bounds__(EPI_ROWS) k_epilogue_split2(int nwv, int j0, i
 constexpr int EPR_NB = 18;
 
 template <int NW, int NB>
-__global__ void __launch_bounds__(EPI_ROWS, NW * NB <= 96 ? 4 : 3) k_epilogue_rows(int nwv, int j0, const float *Cr, const float *Ci,
-                                                            int64_t ldc, RateParams rp, EpiData d, QTab qt,
-                                                            double *partial, int nblk) {
+__global__ void __launch_bounds__(EPI_ROWS, 3) k_epilogue_rows(int nwv, int j0, const float *Cr, const float *Ci,
+                                                               int64_t ldc, RateParams rp, EpiData d, QTab qt,
+                                                               double *partial, int nblk) {
   static_assert(NW % 4 == 0, "16-byte row loads");
   __shared__ double wsum[EPI_ROWS / 32];
   const int ip = blockIdx.x * EPI_ROWS + threadIdx.x;
@@ -1440,6 +1533,111 @@ __global__ void __launch_bounds__(EPI_ROWS, NW * NB <= 96 ? 4 : 3) k_epilogue_ro
         }
       }
       rank_n++;
+    }
+    v = (double)acc;
+  }
+  // fixed-order block reduction: warp shuffle tree, then the warp sums in order
+  for (int o = 16; o > 0; o >>= 1) v += __shfl_down_sync(0xffffffffu, v, o);
+  if ((threadIdx.x & 31) == 0) wsum[threadIdx.x >> 5] = v;
+  __syncthreads();
+  if (threadIdx.x == 0) {
+    double sacc = 0.0;
+    for (int w = 0; w < EPI_ROWS / 32; ++w) sacc += wsum[w];
+    partial[(size_t)j * nblk + blockIdx.x] = sacc;
+  }
+}
+
+// Row data of the rotating drain and its epilogue: (mesh index, window-band mask, first final state)
+__global__ void k_rot_rows(int nwv, int Mp, int nw, const int *widx, const double *ens, const int *cum, double enref,
+                           double fsthick, int4 *row) {
+  const int ip = blockIdx.x * blockDim.x + threadIdx.x;
+  if (ip >= Mp) return;
+  int4 r = make_int4(0, 0, 0, 0);
+  if (ip < nwv) {
+    r.x = widx[ip];
+    r.z = cum[ip];
+    unsigned m = 0;
+    for (int n = 0; n < nw; ++n) m |= (unsigned)(fabs(ens[(size_t)r.x * nw + n] - enref) <= fsthick) << n;
+    r.y = (int)m;
+  }
+  row[ip] = r;
+}
+
+// Generic-shape split epilogue over the rotated sums H[(state nb + s')][final state] of the
+// GEMM's drain (RotOut): one thread per (k' row, state), its window bands in turn; a warp's
+// rows read consecutive final states.  The phonon mix, |g|^2, X+- and the row's sum as
+// k_epilogue_rows forms them, to the bit.  nw 16, nb 12, 13^3: 2.56 ms (4.35 reading
+// the unrotated sums).
+template <int NB>
+__global__ void __launch_bounds__(EPI_ROWS, 4) k_epilogue_h(int nwv, int j0, const float2 *H, int64_t ldh,
+                                                            const int4 *row, RateParams rp, EpiData d, QTab qt,
+                                                            double *partial, int nblk) {
+  __shared__ double wsum[EPI_ROWS / 32];
+  const int ip = blockIdx.x * EPI_ROWS + threadIdx.x;
+  const int j = j0 + blockIdx.y;
+  const int nw = rp.nw, nb = rp.nb;
+  double v = 0.0;
+  if (ip < nwv) {
+    const int code = d.st_code[j];
+    const int i = code / nw, m = code % nw;
+    const int4 ri = __ldg(row + ip);
+    const int p = d.sidx[i], pp = ri.x;
+    const double E = d.ens[(size_t)p * nw + m];
+    const float ex = (float)fmin(exp((E - rp.chempot) / (kB * rp.T)), 3.0e38);
+    const double inv_sig = 1.0 / rp.sigma;
+    const float dnorm = (float)((1.0 / sqrt(2.0 * 3.141592653589793)) / rp.sigma * rp.inv_nk);
+    const int a1 = p % rp.mesh[0], a2 = (p / rp.mesh[0]) % rp.mesh[1], a3 = p / (rp.mesh[0] * rp.mesh[1]);
+    const int b1 = pp % rp.mesh[0], b2 = (pp / rp.mesh[0]) % rp.mesh[1], b3 = pp / (rp.mesh[0] * rp.mesh[1]);
+    const int q = (int)(floormod(b1 - a1, rp.mesh[0]) +
+                        rp.mesh[0] * (floormod(b2 - a2, rp.mesh[1]) + rp.mesh[1] * floormod(b3 - a3, rp.mesh[2])));
+    const float2 *hj = H + (int64_t)(j - j0) * nb * ldh + ri.z;
+    const bool ph = d.phr || d.yv;
+    const YOcc yo = y_occ(E, rp.chempot, kB * rp.T);   // also e^-x of the Fermi factors
+    float acc = 0.0f;
+    int rank_n = 0;
+    for (unsigned left = (unsigned)ri.y; left; left &= left - 1, ++rank_n) {
+      const int n = __ffs(left) - 1;
+      const double eps = d.ens[(size_t)pp * nw + n];
+      float2 unm = make_float2(0.f, 0.f);   // <U_k'[n]|U_k[m]>, polar crystals
+      if (d.glpf) {
+        const float2 *Ukp = d.Uf + ((size_t)pp * nw + n) * nw, *Uk = d.Uf + ((size_t)p * nw + m) * nw;
+        for (int c = 0; c < nw; ++c) cfmaf_cj(unm, Ukp[c], Uk[c]);
+      }
+      float2 h[NB];
+#pragma unroll
+      for (int s = 0; s < NB; ++s)
+        if (s < nb) h[s] = __ldg(hj + (int64_t)s * ldh + rank_n);
+      const F2 dn = f2_of((E - eps) * inv_sig);
+#pragma unroll
+      for (int s = 0; s < NB; ++s) {
+        if (s >= nb) break;
+        const int qs = q * nb + s;
+        const float2 *u = d.uf + (size_t)qs * nb;
+        float2 g = make_float2(0.f, 0.f);
+#pragma unroll
+        for (int sp = 0; sp < NB; ++sp)
+          if (sp < nb) cfmaf(g, u[sp], h[sp]);
+        if (d.glpf) cfmaf(g, d.glpf[qs], unm);   // long-range term (wannier.f90:998-1006)
+        const float gg = __fmaf_rn(g.y, g.y, __fmul_rn(g.x, g.x));   // roundings explicit
+        const float g2c = __fmul_rn(gg, qt.cx[qs]);
+        const VtxF f = vtx_factors<true>(dn, ex, yo.emx, qt.wv[qs], qt.bose[qs], dnorm);
+        const float xp = __fmul_rn(__fmul_rn(g2c, f.ap), f.dp * TWO_M64);
+        const float xm = __fmul_rn(__fmul_rn(g2c, f.am), f.dm * TWO_M64);
+        acc = __fadd_rn(acc, __fadd_rn(xp, xm));
+        // Y, scaled by 2^64: the Gaussian is even, so delta(E' - omega - E) is dp
+        const float y = ph ? g2c * f.dp * y_factor(yo, qt.bose[qs]) : 0.f;
+        if (d.phr && y != 0.f) atomicAdd(d.phr + q + (size_t)rp.N * s, d.ph_scale * TWO_M64D * (double)y);
+        if (d.g2) {
+          int64_t off = (int64_t)j * d.per_state + ((int64_t)ri.z + rank_n) * nb + s;
+          if (off < d.cap) {
+            const double om = d.om[qs];
+            d.g2[off] = (om == 0.0) ? 0.0 : 0.5 * (double)gg / om * g2unitfactor;
+            d.xp[off] = xp;
+            d.xm[off] = xm;
+            if (d.yv) d.yv[off] = TWO_M64D * (double)y;
+          }
+        }
+      }
     }
     v = (double)acc;
   }
@@ -2550,15 +2748,26 @@ static int split_rates_generic(SplitOperands &s, Workspace &ws, cudaStream_t st,
   TCK(cudaEventRecord(ev_stage_a, st));
   // stage B: A planes = e^{2 pi i k'.Rp} for the window k'
   const int MpB = (int)rup(nwv, BM);
-  float *PB, *CBr, *CBi;
+  // The Gaussian epilogue works on sums the GEMM's drain has rotated by U_k' where whole
+  // bands fit its tiles; for nw = 24 it reads the output interleaved by 32 rows
+  // (coalesced), elsewhere row-major.
+  const bool gauss = rp.delta_kind == 0 && nb <= EPR_NB;
+  const bool rotated = gauss && (nw == 8 || nw == 16 || nw == 32), rows_kernel = gauss && nw == 24;
+  const int64_t ldh = rup(ed_in.nin, 32);   // final states of the rotated output's rows
+  float *PB, *CBr = nullptr, *CBi = nullptr;
+  RotOut rot;
+  int4 *rrow = nullptr;
   // states per chunk: a multiple of 8 (8 * 48 = 3 * 128 columns) bounded by chunk_bytes of output
-  int64_t sc = chunk_bytes / ((int64_t)MpB * ncol * 8);
+  int64_t sc = chunk_bytes / (rotated ? nb * ldh * 8 : (int64_t)MpB * ncol * 8);
   sc = std::max<int64_t>(8, sc / 8 * 8);
   sc = std::min<int64_t>(sc, rup(nst, 8));
   sc = std::min<int64_t>(sc, 32768);
   const int64_t NpC = rup(sc * ncol, BN);
-  if ((rc = wsget(ws, "tc_PB", (size_t)4 * MpB * KpB, &PB)) || (rc = wsget(ws, "tc_CBr", (size_t)MpB * NpC, &CBr)) ||
-      (rc = wsget(ws, "tc_CBi", (size_t)MpB * NpC, &CBi)))
+  if ((rc = wsget(ws, "tc_PB", (size_t)4 * MpB * KpB, &PB)) ||
+      (!rotated && ((rc = wsget(ws, "tc_CBr", (size_t)MpB * NpC, &CBr)) ||
+                    (rc = wsget(ws, "tc_CBi", (size_t)MpB * NpC, &CBi)))) ||
+      (rotated && ((rc = wsget(ws, "tc_H", (size_t)(NpC / nw * ldh), &rot.H)) ||
+                   (rc = wsget(ws, "tc_rrow", (size_t)MpB, &rrow)))))
     return tfail(6, ws.msg.c_str());
   TCK(cudaMemsetAsync(PB, 0, (size_t)4 * MpB * KpB * sizeof(float), st));
   {
@@ -2572,6 +2781,15 @@ static int split_rates_generic(SplitOperands &s, Workspace &ws, cudaStream_t st,
   EpiData ed = ed_in;
   ed.Uf = et.Uf;
   QTab qt{et.cx, et.bs, et.wv};
+  if (rotated) {
+    k_rot_rows<<<(MpB + 127) / 128, 128, 0, st>>>(nwv, MpB, nw, widx, ed_in.ens, ed_in.cum, rp.enref, rp.fsthick, rrow);
+    TCK(cudaGetLastError());
+    *launches += 1;
+    rot.nw = nw;
+    rot.row = rrow;
+    rot.Uf = et.Uf;
+    rot.ldh = ldh;
+  }
   // the other parameter sets: their mode tables; no vertex lists
   const int nsets = sets ? sets->n : 1;
   QTab qts[MAX_SETS];
@@ -2597,15 +2815,13 @@ static int split_rates_generic(SplitOperands &s, Workspace &ws, cudaStream_t st,
   const RateParams &rp0 = rp;
   double *const partial0 = partial;
   const EpiData eds = ed, eds_in = ed_in;
-  // the row epilogue reads the GEMM output interleaved by 32 rows (coalesced), the others row-major
-  const bool rows_kernel = rp.delta_kind == 0 && nb <= EPR_NB && (nw == 8 || nw == 16 || nw == 24 || nw == 32);
   for (int64_t j0 = 0; j0 < nst; j0 += sc) {
     const int ns = (int)std::min<int64_t>(sc, nst - j0);
     const int Npc = (int)rup((int64_t)ns * ncol, BN);
     tB->begin(st);
     if (j0 > 0) yield();
     if ((rc = cgemm(PB, MpB, 0, MpB, B2, Np2, j0 * ncol, Npc, KpB, CBr, CBi, NpC, err, st, chunk_us, yield, bm,
-                    rows_kernel ? 1 : 0)))
+                    rows_kernel ? 1 : 0, rot)))
       return rc;
     tB->end(st);
     const size_t esm = (size_t)2 * EPI_ROWS * (ncol + 1) * sizeof(float);
@@ -2620,25 +2836,20 @@ static int split_rates_generic(SplitOperands &s, Workspace &ws, cudaStream_t st,
       ed.g2 = ed.xp = ed.xm = ed.yv = ed_in.g2 = ed_in.xp = ed_in.xm = ed_in.yv = nullptr;
       ed.phr = ed_in.phr = nullptr;
     }
-    if (rows_kernel) {
-      dim3 grid(nblk, ns);
-      // NB: the mode arrays' size (6, 12 or 18), the smallest that holds nb
-      auto rows = [&](auto kernel) {
-        kernel<<<grid, EPI_ROWS, 0, st>>>(nwv, (int)j0, CBr, CBi, NpC, rp, ed, qt, partial, nblk);
+    const int nbc = nb <= 6 ? 6 : nb <= 12 ? 12 : 18;   // the mode arrays' size, the smallest that holds nb
+    if (rotated) {
+      auto over_h = [&](auto kernel) {
+        kernel<<<dim3(nblk, ns), EPI_ROWS, 0, st>>>(nwv, (int)j0, rot.H, ldh, rrow, rp, ed, qt, partial, nblk);
       };
-      const int nbc = nb <= 6 ? 6 : nb <= 12 ? 12 : 18;
-#define EPHG_ROWS_NB(NWV)                                                          \
-  (nbc == 6 ? rows(k_epilogue_rows<NWV, 6>) : nbc == 12 ? rows(k_epilogue_rows<NWV, 12>) \
-            : rows(k_epilogue_rows<NWV, 18>))
-      if (nw == 8)
-        EPHG_ROWS_NB(8);
-      else if (nw == 16)
-        EPHG_ROWS_NB(16);
-      else if (nw == 24)
-        EPHG_ROWS_NB(24);
-      else
-        EPHG_ROWS_NB(32);
-#undef EPHG_ROWS_NB
+      nbc == 6 ? over_h(k_epilogue_h<6>) : nbc == 12 ? over_h(k_epilogue_h<12>) : over_h(k_epilogue_h<18>);
+      TCK(cudaGetLastError());
+    } else if (rows_kernel) {
+      auto rows = [&](auto kernel) {
+        kernel<<<dim3(nblk, ns), EPI_ROWS, 0, st>>>(nwv, (int)j0, CBr, CBi, NpC, rp, ed, qt, partial, nblk);
+      };
+      nbc == 6    ? rows(k_epilogue_rows<24, 6>)
+      : nbc == 12 ? rows(k_epilogue_rows<24, 12>)
+                  : rows(k_epilogue_rows<24, 18>);
       TCK(cudaGetLastError());
     } else if (rp.delta_kind == 0 && esm > 200 * 1024) {
       dim3 grid(nblk, ns);
@@ -3038,7 +3249,7 @@ extern "C" int ephg_debug_group_tiles(int np, const int *mtiles, const int *ntil
   std::vector<GroupProblem> tab(np);
   int64_t T = 0;
   for (int i = 0; i < np; ++i) {
-    memset(&tab[i], 0, sizeof(GroupProblem));
+    memset((void *)&tab[i], 0, sizeof(GroupProblem));
     if (mtiles[i] <= 0 || ntiles[i] <= 0) return 1;
     tab[i].g.mtiles = mtiles[i];
     tab[i].g.ntiles = ntiles[i];
