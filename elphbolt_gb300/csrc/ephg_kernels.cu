@@ -412,10 +412,17 @@ void launch_zgemm(int M, int N, int K, const double2 *A, int64_t lda, const doub
 }
 
 // ====================================================== Jacobi eigensolver
-// One warp per Hermitian matrix (n <= 32).  Parallel cyclic Jacobi with the
-// round-robin ordering: n/2 disjoint rotations per step, n-1 steps per sweep
-// (Golub & Van Loan sec. 8.5.4).  Stands in for zheev('V','U') at
-// wannier.f90:489 and :732.
+// Hermitian matrices, n <= 32.  Parallel cyclic Jacobi with the round-robin ordering:
+// n/2 disjoint rotations per step, n-1 steps per sweep (Golub & Van Loan sec. 8.5.4).
+// Stands in for zheev('V','U') at wannier.f90:489 and :732.
+//
+// A block of T threads takes G matrices together.  A warp's FP64 instruction costs the
+// same with 3 active lanes as with 32, and a step has n/2 rotations and n^2/2 element
+// pairs: the lanes are therefore dealt out over the matrices that still have sweeps to
+// do (n = 6, one matrix per warp: 3 and 18 of 32 lanes; half the FP64 instructions are
+// then the rotations').  Every element's arithmetic, and the norms' order, are those of
+// one matrix alone.  Matrices lie in shared memory with an odd leading dimension, which
+// rows and columns alike read without bank conflicts.
 //
 // Mixed precision, because GB300's FP64 rate is a sixtieth of its FP32 rate:
 //  1. FP32 sweeps bring the matrix to near-diagonal form (off-diagonal norm
@@ -442,121 +449,206 @@ __device__ __forceinline__ void rr_pair(int r, int m, int lane, int &p, int &q) 
   q = max(a, b);
 }
 
-// FP32 sweeps on A (float2, column-major n x n) accumulating into Q until the
-// off-diagonal norm is 1e-10 of the total or stalls below 1e-6 of it; P4 / PI:
-// the step's rotations (c, s, e^{i phi}) and pairs.
-__device__ void jacobi_f32(int n, float2 *A, float2 *Q, float4 *P4, int2 *PI, int lane) {
-  const int nn = n * n, m = n + (n & 1), half = m / 2;
-  float prev = INFINITY;
-  for (int sweep = 0; sweep < EIG_MAXSWEEP32; ++sweep) {
-    float off = 0.f, tot = 0.f;
-    for (int idx = lane; idx < nn; idx += 32) {
-      const float2 a = A[idx];
-      const float a2 = a.x * a.x + a.y * a.y;
-      tot += a2;
-      if (idx % n != idx / n) off += a2;
-    }
+// x / d for x d < 2^32, from inv_of(d)
+__device__ __forceinline__ unsigned inv_of(int d) { return d == 1 ? 0u : 0xffffffffu / (unsigned)d + 1u; }
+__device__ __forceinline__ int div_by(int x, unsigned inv) { return inv ? (int)__umulhi((unsigned)x, inv) : x; }
+
+constexpr int EIG_G = 4;       // matrices per block at most
+constexpr int EIG_SMS = 152;   // SMs
+
+// What a block's sweeps share: which matrices are done, their last off-diagonal norms.
+struct EigState {
+  int done[EIG_G];
+  double prev[EIG_G];
+};
+
+// The matrices of a block that still have sweeps to do, four bits each.
+__device__ __forceinline__ int eig_active(const EigState &es, int G, unsigned &map) {
+  int na = 0;
+  map = 0;
+  for (int g = 0; g < G; ++g)
+    if (!es.done[g]) map |= (unsigned)g << (4 * na++);
+  return na;
+}
+
+// Index helpers of a block's items: n, n / 2 pairs (n even; odd n has a dummy player).
+struct EigDims {
+  int n, m, half, ld, size;          // size: doubles2 of one matrix's storage
+  unsigned inv_n, inv_half, inv_hn, inv_nn;
+};
+
+// A rotation's factors from a_pq = (ax, ay), rr = |a_pq| and d = a_qq - a_pp: the lane with
+// `phase` returns e^{i phi} = (ax, ay) / rr, the other (c, t = tan), each with two of the
+// four divisions.
+__device__ __forceinline__ float2 rotation_f32(bool phase, float ax, float ay, float d, float rr) {
+  const float u = (phase ? ax : d) / (phase ? rr : 2.f * rr);   // tau
+  const bool big = fabsf(u) > 1e18f;
+  const float num = phase ? ay : big ? 0.5f : u >= 0.f ? 1.f : -1.f;
+  const float v = num / (phase ? rr : big ? u : fabsf(u) + sqrtf(1.f + u * u));
+  return phase ? make_float2(u, v) : make_float2(rsqrtf(1.f + v * v), v);
+}
+
+// (tot, off) summed over the warp's lanes by a butterfly, the two in opposite halves.
+template <typename F>
+__device__ __forceinline__ void warp_sums(F &tot, F &off, int lane) {
+  F v = lane < 16 ? tot : off;
+  const F w = lane < 16 ? off : tot;
+  v += __shfl_xor_sync(0xffffffffu, w, 16);
 #pragma unroll
-    for (int o = 16; o > 0; o >>= 1) {
-      off += __shfl_xor_sync(0xffffffffu, off, o);
-      tot += __shfl_xor_sync(0xffffffffu, tot, o);
+  for (int o = 8; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
+  tot = __shfl_sync(0xffffffffu, v, 0);
+  off = __shfl_sync(0xffffffffu, v, 16);
+}
+
+// FP32 sweeps on A (float2, column-major) accumulating into Q until the off-diagonal
+// norm is 1e-10 of the total or stalls below 1e-6 of it; P4 / PI: the step's rotations
+// (c, s, e^{i phi}) and pairs.  base: the block's first matrix, dim.size apart.
+template <int T>
+__device__ void jacobi_f32(const EigDims &e, double2 *base, EigState &es, int G, int tid) {
+  const int n = e.n, ld = e.ld, nn = n * n, half = e.half, lane = tid & 31, warp = tid >> 5;
+  auto fA = [&](int g) { return (float2 *)(base + (size_t)g * e.size + 2 * ld * n); };
+  auto fQ = [&](int g) { return (float2 *)(base + (size_t)g * e.size + 2 * ld * n) + ld * n; };
+  auto fP = [&](int g) { return (float4 *)(base + (size_t)g * e.size + 4 * ld * n); };
+  auto fI = [&](int g) { return (int2 *)(base + (size_t)g * e.size + 4 * ld * n + 16); };
+  unsigned map;
+  int na = eig_active(es, G, map);
+  for (int sweep = 0; sweep < EIG_MAXSWEEP32; ++sweep) {
+    for (int a = warp; a < na; a += T / 32) {
+      const int g = (map >> (4 * a)) & 15;
+      const float2 *A = fA(g);
+      float off = 0.f, tot = 0.f;
+      for (int idx = lane; idx < nn; idx += 32) {
+        const int j = div_by(idx, e.inv_n), i = idx - j * n;
+        const float2 v = A[i + ld * j];
+        const float a2 = v.x * v.x + v.y * v.y;
+        tot += a2;
+        if (i != j) off += a2;
+      }
+      warp_sums(tot, off, lane);
+      // done at 1e-10 of the total, or once it stalls near FP32's floor; a
+      // non-finite norm also stops it (Q is then not used)
+      const float prev = (float)es.prev[g];
+      __syncwarp();
+      if (lane == 0) {
+        es.done[g] = !(off > 1e-10f * tot) || (off <= 1e-6f * tot && off > 0.25f * prev);
+        es.prev[g] = off;
+      }
     }
-    // done at 1e-10 of the total, or once it stalls near FP32's floor; a
-    // non-finite norm also stops it (Q is then not used)
-    if (!(off > 1e-10f * tot) || (off <= 1e-6f * tot && off > 0.25f * prev)) return;
-    prev = off;
-    for (int r = 0; r < m - 1; ++r) {
-      if (lane < half) {
+    __syncthreads();
+    na = eig_active(es, G, map);
+    if (na == 0) return;
+    const int cnt = na * half * n, cntv = (cnt + 31) & ~31;
+    for (int r = 0; r < e.m - 1; ++r) {
+      for (int idx = tid; idx < 2 * na * half; idx += T) {
+        const int v = idx >> 1, a = div_by(v, e.inv_half), l = v - a * half, g = (map >> (4 * a)) & 15;
+        const bool phase = idx & 1;
+        const float2 *A = fA(g);
         int p, q;
-        rr_pair(r, m, lane, p, q);
-        float c = 1.f, sn = 0.f, phx = 1.f, phy = 0.f;
+        rr_pair(r, e.m, l, p, q);
+        float2 out = make_float2(1.f, 0.f);
         if (q < n) {
-          const float2 apq = A[p + n * q];
+          const float2 apq = A[p + ld * q];
           const float rr = hypotf(apq.x, apq.y);
-          if (rr > 0.f) {
-            const float tau = (A[q + n * q].x - A[p + n * p].x) / (2.f * rr);
-            const float tf = fabsf(tau) > 1e18f ? 0.5f / tau
-                                                : (tau >= 0.f ? 1.f : -1.f) / (fabsf(tau) + sqrtf(1.f + tau * tau));
-            c = rsqrtf(1.f + tf * tf);
-            sn = tf * c;
-            phx = apq.x / rr;
-            phy = apq.y / rr;
-          }
+          if (rr > 0.f) out = rotation_f32(phase, apq.x, apq.y, A[q + ld * q].x - A[p + ld * p].x, rr);
+          if (rr > 0.f && !phase) out.y *= out.x;   // s = t c
         }
-        P4[lane] = make_float4(c, sn, phx, phy);
-        PI[lane] = make_int2(p, q < n ? q : -1);
+        ((float2 *)(fP(g) + l))[phase] = out;   // (c, s); e^{i phi}
+        if (!phase) fI(g)[l] = make_int2(p, q < n ? q : -1);
       }
-      __syncwarp();
-      // columns: A <- A J, Q <- Q J;  J = [[c, s], [-s e^{-i phi}, c e^{-i phi}]]
-      for (int idx = lane; idx < half * n; idx += 32) {
-        const int k = idx / n, i = idx % n;
-        const int2 pq = PI[k];
+      __syncthreads();
+      // columns: A <- A J;  J = [[c, s], [-s e^{-i phi}, c e^{-i phi}]]
+      for (int idx = tid; idx < cnt; idx += T) {
+        const int a = div_by(idx, e.inv_hn), w = idx - a * half * n, k = div_by(w, e.inv_n), i = w - k * n;
+        const int g = (map >> (4 * a)) & 15;
+        const int2 pq = fI(g)[k];
         if (pq.y < 0) continue;
-        const float4 r4 = P4[k];
-        const float2 aip = A[i + n * pq.x], aiq = A[i + n * pq.y];
-        float2 t = make_float2(r4.z * aiq.x + r4.w * aiq.y, r4.z * aiq.y - r4.w * aiq.x);
-        A[i + n * pq.x] = make_float2(r4.x * aip.x - r4.y * t.x, r4.x * aip.y - r4.y * t.y);
-        A[i + n * pq.y] = make_float2(r4.y * aip.x + r4.x * t.x, r4.y * aip.y + r4.x * t.y);
-        const float2 vip = Q[i + n * pq.x], viq = Q[i + n * pq.y];
-        t = make_float2(r4.z * viq.x + r4.w * viq.y, r4.z * viq.y - r4.w * viq.x);
-        Q[i + n * pq.x] = make_float2(r4.x * vip.x - r4.y * t.x, r4.x * vip.y - r4.y * t.y);
-        Q[i + n * pq.y] = make_float2(r4.y * vip.x + r4.x * t.x, r4.y * vip.y + r4.x * t.y);
+        const float4 r4 = fP(g)[k];
+        float2 *xp = fA(g) + i + ld * pq.x, *xq = fA(g) + i + ld * pq.y;
+        const float2 aip = *xp, aiq = *xq;
+        const float2 t = make_float2(r4.z * aiq.x + r4.w * aiq.y, r4.z * aiq.y - r4.w * aiq.x);
+        *xp = make_float2(r4.x * aip.x - r4.y * t.x, r4.x * aip.y - r4.y * t.y);
+        *xq = make_float2(r4.y * aip.x + r4.x * t.x, r4.y * aip.y + r4.x * t.y);
       }
-      __syncwarp();
-      // rows: A <- J^H A
-      for (int idx = lane; idx < half * n; idx += 32) {
-        const int k = idx / n, jj = idx % n;
-        const int2 pq = PI[k];
+      __syncthreads();
+      // rows: A <- J^H A, its diagonal kept real; Q <- Q J, by other warps
+      for (int idx = tid; idx < cntv + cnt; idx += T) {
+        const bool row = idx < cntv;
+        const int v = row ? idx : idx - cntv;
+        if (v >= cnt) continue;
+        const int a = div_by(v, e.inv_hn), w = v - a * half * n, k = div_by(w, e.inv_n), i = w - k * n;
+        const int g = (map >> (4 * a)) & 15;
+        const int2 pq = fI(g)[k];
         if (pq.y < 0) continue;
-        const float4 r4 = P4[k];
-        const float2 apj = A[pq.x + n * jj], aqj = A[pq.y + n * jj];
-        const float2 t = make_float2(r4.z * aqj.x - r4.w * aqj.y, r4.z * aqj.y + r4.w * aqj.x);
-        A[pq.x + n * jj] = make_float2(r4.x * apj.x - r4.y * t.x, r4.x * apj.y - r4.y * t.y);
-        A[pq.y + n * jj] = make_float2(r4.y * apj.x + r4.x * t.x, r4.y * apj.y + r4.x * t.y);
-      }
-      __syncwarp();
-      if (lane < half) {
-        const int2 pq = PI[lane];
-        if (pq.y >= 0) {
-          A[pq.x + n * pq.x].y = 0.f;   // the diagonal of a Hermitian matrix is real
-          A[pq.y + n * pq.y].y = 0.f;
+        const float4 r4 = fP(g)[k];
+        if (row) {
+          float2 *A = fA(g) + ld * i;
+          const float2 apj = A[pq.x], aqj = A[pq.y];
+          const float2 t = make_float2(r4.z * aqj.x - r4.w * aqj.y, r4.z * aqj.y + r4.w * aqj.x);
+          const float2 np = make_float2(r4.x * apj.x - r4.y * t.x, r4.x * apj.y - r4.y * t.y);
+          const float2 nq = make_float2(r4.y * apj.x + r4.x * t.x, r4.y * apj.y + r4.x * t.y);
+          A[pq.x] = make_float2(np.x, i == pq.x ? 0.f : np.y);
+          A[pq.y] = make_float2(nq.x, i == pq.y ? 0.f : nq.y);
+        } else {
+          float2 *xp = fQ(g) + i + ld * pq.x, *xq = fQ(g) + i + ld * pq.y;
+          const float2 vip = *xp, viq = *xq;
+          const float2 t = make_float2(r4.z * viq.x + r4.w * viq.y, r4.z * viq.y - r4.w * viq.x);
+          *xp = make_float2(r4.x * vip.x - r4.y * t.x, r4.x * vip.y - r4.y * t.y);
+          *xq = make_float2(r4.y * vip.x + r4.x * t.x, r4.y * vip.y + r4.x * t.y);
         }
       }
-      __syncwarp();
+      __syncthreads();
     }
   }
 }
 
-// C = op(X) Y for n x n complex FP64 matrices in shared memory (column-major),
-// op(X) = X^H if XH; one warp.
-template <bool XH>
-__device__ void wmatmul(int n, const double2 *X, const double2 *Y, double2 *C, int lane) {
-  for (int idx = lane; idx < n * n; idx += 32) {
-    const int i = idx % n, jj = idx / n;
+// C = op(X) Y for the block's n x n complex FP64 matrices (X, Y, C: offsets in a matrix's
+// storage), op(X) = X^H if XH.
+template <int T, bool XH>
+__device__ void group_matmul(const EigDims &e, double2 *base, int ng, int X, int Y, int C, int tid) {
+  const int n = e.n, ld = e.ld;
+  for (int idx = tid; idx < ng * n * n; idx += T) {
+    const int g = div_by(idx, e.inv_nn), w = idx - g * n * n, jj = div_by(w, e.inv_n), i = w - jj * n;
+    double2 *M = base + (size_t)g * e.size;
+    const double2 *x = M + X + (XH ? ld * i : i), *y = M + Y + ld * jj;
     double2 acc = make_double2(0.0, 0.0);
     for (int k = 0; k < n; ++k) {
-      if (XH) cfma_cj(acc, X[k + n * i], Y[k + n * jj]);
-      else cfma(acc, X[i + n * k], Y[k + n * jj]);
+      if (XH) cfma_cj(acc, x[k], y[k]);
+      else cfma(acc, x[ld * k], y[k]);
     }
-    C[idx] = acc;
+    M[C + i + ld * jj] = acc;
   }
-  __syncwarp();
+  __syncthreads();
 }
 
-__global__ void k_heig(int batch, int n, const double2 *__restrict__ A, int64_t stride,
-                       double *__restrict__ w, double2 *__restrict__ V, int *err) {
+// Bound by FP64 instructions: one holds an SM sub-partition for 64 cycles.  A rotation's two
+// normalisations therefore run on two lanes, and V <- V J in other warps than A <- J^H A.
+// Against one warp per matrix: 13,824 matrices of n = 8 and of n = 6 2.37 -> 1.44 ms, 2,197
+// of n = 16 and of n = 12 2.64 -> 1.80, 1,728 of n = 6 154 -> 100 us, 200 of n = 8
+// 115 -> 82 (175,000 cycles a matrix: a third in the FP32 sweeps, half in the FP64 ones).
+template <int T>
+__global__ void __launch_bounds__(T) k_heig(int batch, int n, int G, const double2 *__restrict__ A, int64_t stride,
+                                            double *__restrict__ w, double2 *__restrict__ V, int *err) {
   extern __shared__ double2 sm[];
-  const int lane = threadIdx.x & 31, wib = threadIdx.x >> 5, wpb = blockDim.x >> 5;
-  const int mat = blockIdx.x * wpb + wib;
-  const int nn = n * n;
-  double2 *sA = sm + (size_t)wib * (4 * nn + 3 * 16);
-  double2 *sV = sA + nn, *sT = sV + nn, *sT2 = sT + nn;
-  double2 *sP = sT2 + nn;   // per pair: (c, s), (ph.x, ph.y), (p, q) packed
-  float2 *fA = (float2 *)sT, *fQ = fA + nn;   // the FP32 phase, inside sT
-  if (mat >= batch) return;
-  const double2 *Am = A + (size_t)mat * stride;
-  for (int idx = lane; idx < nn; idx += 32) {
-    int i = idx % n, j = idx / n;
+  __shared__ EigState es;
+  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+  const int mat0 = blockIdx.x * G, ng = min(G, batch - mat0), nn = n * n;
+  EigDims e;
+  e.n = n;
+  e.m = n + (n & 1);         // even number of players (dummy = n)
+  e.half = e.m / 2;
+  e.ld = n | 1;
+  e.size = 4 * e.ld * n + 3 * 16;
+  e.inv_n = inv_of(n);
+  e.inv_half = inv_of(e.half);
+  e.inv_hn = inv_of(e.half * n);
+  e.inv_nn = inv_of(nn);
+  const int ld = e.ld, half = e.half;
+  // a matrix's storage: A, V, two temporaries (the FP32 phase inside the first), per
+  // pair (c, s), (ph.x, ph.y), (p, q)
+  const int oV = ld * n, oT = 2 * ld * n, oT2 = 3 * ld * n, oP = 4 * ld * n;
+  for (int idx = tid; idx < ng * nn; idx += T) {
+    const int g = div_by(idx, e.inv_nn), v0 = idx - g * nn, j = div_by(v0, e.inv_n), i = v0 - j * n;
+    const double2 *Am = A + (size_t)(mat0 + g) * stride;
     double2 v;
     if (i < j) {                       // averaged upper triangle (wannier.f90:481-486)
       double2 aij = Am[i + n * j], aji = Am[j + n * i];
@@ -567,84 +659,116 @@ __global__ void k_heig(int batch, int n, const double2 *__restrict__ A, int64_t 
     } else {
       v = make_double2(Am[i + n * i].x, 0.0);
     }
-    sA[idx] = v;
-    fA[idx] = make_float2((float)v.x, (float)v.y);
-    fQ[idx] = make_float2(i == j ? 1.f : 0.f, 0.f);
+    double2 *M = sm + (size_t)g * e.size;
+    M[i + ld * j] = v;
+    float2 *fA = (float2 *)(M + oT), *fQ = fA + ld * n;
+    fA[i + ld * j] = make_float2((float)v.x, (float)v.y);
+    fQ[i + ld * j] = make_float2(i == j ? 1.f : 0.f, 0.f);
   }
-  __syncwarp();
+  if (tid < EIG_G) {
+    es.done[tid] = tid >= ng;
+    es.prev[tid] = INFINITY;
+  }
+  __syncthreads();
   // 1. FP32 sweeps
-  jacobi_f32(n, fA, fQ, (float4 *)sP, (int2 *)((float4 *)sP + 16), lane);
-  bool finite = true;
-  for (int idx = lane; idx < nn; idx += 32) {
-    const float2 q = fQ[idx];
-    finite = finite && isfinite(q.x) && isfinite(q.y);
-    sV[idx] = make_double2((double)q.x, (double)q.y);
+  jacobi_f32<T>(e, sm, es, G, tid);
+  for (int g = warp; g < ng; g += T / 32) {
+    double2 *M = sm + (size_t)g * e.size;
+    const float2 *fQ = (const float2 *)(M + oT) + ld * n;
+    bool finite = true;
+    for (int idx = lane; idx < nn; idx += 32) {
+      const int j = div_by(idx, e.inv_n), o = idx - j * n + ld * j;
+      const float2 q = fQ[o];
+      finite = finite && isfinite(q.x) && isfinite(q.y);
+      M[oV + o] = make_double2((double)q.x, (double)q.y);
+    }
+    if (!__all_sync(0xffffffffu, finite)) {   // FP32 overflowed: the FP64 sweeps start from A itself
+      for (int idx = lane; idx < nn; idx += 32) {
+        const int j = div_by(idx, e.inv_n), i = idx - j * n;
+        M[oV + i + ld * j] = make_double2(i == j ? 1.0 : 0.0, 0.0);
+      }
+    }
   }
-  __syncwarp();
-  if (!__all_sync(0xffffffffu, finite)) {   // FP32 overflowed: the FP64 sweeps start from A itself
-    for (int idx = lane; idx < nn; idx += 32) sV[idx] = make_double2(idx % n == idx / n ? 1.0 : 0.0, 0.0);
-    __syncwarp();
+  __syncthreads();
+  if (tid < EIG_G) {
+    es.done[tid] = tid >= ng;
+    es.prev[tid] = INFINITY;
   }
   // 2. Q unitary to FP64 rounding: X <- X (3I - X^H X) / 2, twice
   for (int it = 0; it < 2; ++it) {
-    wmatmul<true>(n, sV, sV, sT, lane);
-    for (int idx = lane; idx < nn; idx += 32) {
-      const double2 t = sT[idx];
-      sT[idx] = make_double2((idx % n == idx / n ? 3.0 : 0.0) - t.x, -t.y);
+    group_matmul<T, true>(e, sm, ng, oV, oV, oT, tid);
+    for (int idx = tid; idx < ng * nn; idx += T) {
+      const int g = div_by(idx, e.inv_nn), v0 = idx - g * nn, j = div_by(v0, e.inv_n), i = v0 - j * n;
+      double2 &t = sm[(size_t)g * e.size + oT + i + ld * j];
+      t = make_double2((i == j ? 3.0 : 0.0) - t.x, -t.y);
     }
-    __syncwarp();
-    wmatmul<false>(n, sV, sT, sT2, lane);
-    for (int idx = lane; idx < nn; idx += 32) sV[idx] = cscale(sT2[idx], 0.5);
-    __syncwarp();
+    __syncthreads();
+    group_matmul<T, false>(e, sm, ng, oV, oT, oT2, tid);
+    for (int idx = tid; idx < ng * nn; idx += T) {
+      const int g = div_by(idx, e.inv_nn), v0 = idx - g * nn, j = div_by(v0, e.inv_n), o = v0 - j * n + ld * j;
+      double2 *M = sm + (size_t)g * e.size;
+      M[oV + o] = cscale(M[oT2 + o], 0.5);
+    }
+    __syncthreads();
   }
   // 3. B = Q^H A Q, made exactly Hermitian (its rounding is below the FP64 sweeps' floor)
-  wmatmul<false>(n, sA, sV, sT, lane);
-  wmatmul<true>(n, sV, sT, sA, lane);
-  for (int idx = lane; idx < nn; idx += 32) {
-    const int i = idx % n, j = idx / n;
+  group_matmul<T, false>(e, sm, ng, 0, oV, oT, tid);
+  group_matmul<T, true>(e, sm, ng, oV, oT, 0, tid);
+  for (int idx = tid; idx < ng * nn; idx += T) {
+    const int g = div_by(idx, e.inv_nn), v0 = idx - g * nn, j = div_by(v0, e.inv_n), i = v0 - j * n;
+    double2 *M = sm + (size_t)g * e.size;
     if (i < j) {
-      const double2 bij = sA[i + n * j], bji = sA[j + n * i];
+      const double2 bij = M[i + ld * j], bji = M[j + ld * i];
       const double2 v = make_double2(0.5 * (bij.x + bji.x), 0.5 * (bij.y - bji.y));
-      sA[i + n * j] = v;
-      sA[j + n * i] = cconj(v);
+      M[i + ld * j] = v;
+      M[j + ld * i] = cconj(v);
     } else if (i == j) {
-      sA[idx].y = 0.0;
+      M[i + ld * j].y = 0.0;
     }
   }
-  __syncwarp();
+  __syncthreads();
   // 4. FP64 sweeps on B, accumulating into V = Q
-  const int m = n + (n & 1);         // even number of players (dummy = n)
-  const int half = m / 2;
-  bool converged = false;
-  double prev_off = INFINITY;
-  for (int sweep = 0; sweep < EIG_MAXSWEEP; ++sweep) {
-    double off = 0.0, tot = 0.0;
-    for (int idx = lane; idx < nn; idx += 32) {
-      double2 a = sA[idx];
-      double a2 = a.x * a.x + a.y * a.y;
-      tot += a2;
-      if (idx % n != idx / n) off += a2;
+  unsigned map;
+  int na = eig_active(es, G, map);
+  for (int sweep = 0; sweep < EIG_MAXSWEEP && na > 0; ++sweep) {
+    for (int a = warp; a < na; a += T / 32) {
+      const int g = (map >> (4 * a)) & 15;
+      const double2 *M = sm + (size_t)g * e.size;
+      double off = 0.0, tot = 0.0;
+      for (int idx = lane; idx < nn; idx += 32) {
+        const int j = div_by(idx, e.inv_n), i = idx - j * n;
+        double2 v = M[i + ld * j];
+        double a2 = v.x * v.x + v.y * v.y;
+        tot += a2;
+        if (i != j) off += a2;
+      }
+      warp_sums(tot, off, lane);
+      // Converged: the off-diagonal norm is ~7 eps of the matrix norm, or it has
+      // reached the FP64 rounding floor (the rotations leave a_pq at rounding
+      // level rather than zero, so the floor sits near 1e-31..1e-30 of the total
+      // and may not pass the first test): below 1e-26 of the total and no longer
+      // falling by 4x per sweep.
+      const double prev_off = es.prev[g];
+      __syncwarp();
+      if (lane == 0) {
+        es.done[g] = off <= 1e-30 * tot || off == 0.0 || (off <= 1e-26 * tot && off > 0.25 * prev_off);
+        es.prev[g] = off;
+      }
     }
-#pragma unroll
-    for (int o = 16; o > 0; o >>= 1) {
-      off += __shfl_xor_sync(0xffffffffu, off, o);
-      tot += __shfl_xor_sync(0xffffffffu, tot, o);
-    }
-    // Converged: the off-diagonal norm is ~7 eps of the matrix norm, or it has
-    // reached the FP64 rounding floor (the rotations leave a_pq at rounding
-    // level rather than zero, so the floor sits near 1e-31..1e-30 of the total
-    // and may not pass the first test): below 1e-26 of the total and no longer
-    // falling by 4x per sweep.
-    if (off <= 1e-30 * tot || off == 0.0 || (off <= 1e-26 * tot && off > 0.25 * prev_off)) {
-      converged = true;
-      break;
-    }
-    prev_off = off;
-    for (int r = 0; r < m - 1; ++r) {
-      if (lane < half) {
+    __syncthreads();
+    na = eig_active(es, G, map);
+    if (na == 0) break;
+    const int cnt = na * half * n, cntv = (cnt + 31) & ~31;
+    for (int r = 0; r < e.m - 1; ++r) {
+      // Rotations, two lanes each: both find the angle, the even one makes (c, s) unitary to
+      // FP64 rounding, the odd one e^{i phi}; comparisons are on the integer images.
+      for (int idx = tid; idx < 2 * na * half; idx += T) {
+        const int v0 = idx >> 1, a = div_by(v0, e.inv_half), l = v0 - a * half;
+        const bool phase = idx & 1;
+        double2 *M = sm + (size_t)((map >> (4 * a)) & 15) * e.size, *sP = M + oP;
         int p, q;
-        rr_pair(r, m, lane, p, q);
-        double c = 1.0, s = 0.0, phx = 1.0, phy = 0.0;
+        rr_pair(r, e.m, l, p, q);
+        double2 out = make_double2(1.0, 0.0);
         if (q < n) {
           // The rotation angle is computed in FP32 on operands scaled by the
           // power of two of a_pq (GB300's FP64 divide / sqrt are slow); the
@@ -652,108 +776,120 @@ __global__ void k_heig(int batch, int n, const double2 *__restrict__ A, int64_t 
           // similarity transform that leaves a_pq ~ 1e-7 of its value.  Later
           // rotations remove that residual; a_pq is not forced to zero.  With
           // |a_qq - a_pp| > 1e30 |a_pq| the rotation is negligible and skipped.
-          const double2 apq = sA[p + n * q];
-          const double d = sA[q + n * q].x - sA[p + n * p].x;
-          const double mx = fmax(fabs(apq.x), fabs(apq.y));
-          const int ex = ((__double2hiint(mx) >> 20) & 0x7ff) - 1023;
-          if (mx > 0.0 && ex > -1000 && ex < 1000) {
+          const double2 apq = M[p + ld * q];
+          const double d = M[q + ld * q].x - M[p + ld * p].x;
+          const int ex = (max(__double2hiint(apq.x) & 0x7fffffff, __double2hiint(apq.y) & 0x7fffffff) >> 20) - 1023;
+          if (ex > -1000 && ex < 1000) {
             const double sc = __hiloint2double((1023 - ex) << 20, 0);   // 2^-ex: max |a_pq| -> [1, 2)
             const float ax = (float)(apq.x * sc), ay = (float)(apq.y * sc);
             const double dsc = d * sc;
             const float rr = sqrtf(ax * ax + ay * ay);
-            if (fabs(dsc) <= 1e30) {
-              const float tau = (float)dsc / (2.f * rr);
-              const float tf = fabsf(tau) > 1e18f ? 0.5f / tau
-                                                  : (tau >= 0.f ? 1.f : -1.f) / (fabsf(tau) + sqrtf(1.f + tau * tau));
-              double px = (double)(ax / rr), py = (double)(ay / rr);
-              double cc = (double)rsqrtf(1.f + tf * tf);
-              double ss = (double)tf * cc;
-              // two Newton steps of 1/sqrt(r2) from 1: |ph| = 1 and c^2 + s^2 = 1 in FP64
-              double r2 = px * px + py * py, f = 1.5 - 0.5 * r2;
+            if ((__double_as_longlong(dsc) & 0x7fffffffffffffffll) <= __double_as_longlong(1e30)) {
+              const float2 ct = rotation_f32(phase, ax, ay, (float)dsc, rr);
+              const double x = (double)ct.x, y = (double)ct.y * (phase ? 1.0 : x);   // s = t c
+              // two Newton steps of 1/sqrt(r2) from 1: x^2 + y^2 = 1 in FP64
+              const double r2 = x * x + y * y;
+              double f = 1.5 - 0.5 * r2;
               f = f * (1.5 - 0.5 * r2 * f * f);
-              phx = px * f;
-              phy = py * f;
-              r2 = cc * cc + ss * ss;
-              f = 1.5 - 0.5 * r2;
-              f = f * (1.5 - 0.5 * r2 * f * f);
-              c = cc * f;
-              s = ss * f;
+              out = make_double2(x * f, y * f);
             }
           }
         }
-        sP[3 * lane] = make_double2(c, s);
-        sP[3 * lane + 1] = make_double2(phx, phy);
-        sP[3 * lane + 2] = make_double2((double)p, (double)(q < n ? q : -1));
+        sP[3 * l + phase] = out;   // (c, s); e^{i phi}
+        if (!phase) *(int2 *)(sP + 3 * l + 2) = make_int2(p, q < n ? q : -1);
       }
-      __syncwarp();
-      // columns: A <- A J, V <- V J;  J = [[c, s], [-s e^{-i phi}, c e^{-i phi}]]
-      for (int idx = lane; idx < half * n; idx += 32) {
-        int k = idx / n, i = idx % n;
-        int q = (int)sP[3 * k + 2].y;
-        if (q < 0) continue;
-        int p = (int)sP[3 * k + 2].x;
-        double c = sP[3 * k].x, s = sP[3 * k].y;
-        double2 phc = make_double2(sP[3 * k + 1].x, -sP[3 * k + 1].y);
-        double2 aip = sA[i + n * p], aiq = sA[i + n * q];
-        double2 t = cmul(phc, aiq);
-        sA[i + n * p] = make_double2(c * aip.x - s * t.x, c * aip.y - s * t.y);
-        sA[i + n * q] = make_double2(s * aip.x + c * t.x, s * aip.y + c * t.y);
-        double2 vip = sV[i + n * p], viq = sV[i + n * q];
-        t = cmul(phc, viq);
-        sV[i + n * p] = make_double2(c * vip.x - s * t.x, c * vip.y - s * t.y);
-        sV[i + n * q] = make_double2(s * vip.x + c * t.x, s * vip.y + c * t.y);
+      __syncthreads();
+      // columns: A <- A J;  J = [[c, s], [-s e^{-i phi}, c e^{-i phi}]]
+      for (int idx = tid; idx < cnt; idx += T) {
+        const int a = div_by(idx, e.inv_hn), v0 = idx - a * half * n, k = div_by(v0, e.inv_n), i = v0 - k * n;
+        double2 *M = sm + (size_t)((map >> (4 * a)) & 15) * e.size;
+        const double2 *sP = M + oP + 3 * k;
+        const int2 pq = *(const int2 *)(sP + 2);
+        if (pq.y < 0) continue;
+        double2 *xp = M + ld * pq.x + i, *xq = M + ld * pq.y + i;
+        const double c = sP[0].x, s = sP[0].y;
+        const double2 phc = make_double2(sP[1].x, -sP[1].y);
+        const double2 aip = *xp, aiq = *xq;
+        const double2 t = cmul(phc, aiq);
+        *xp = make_double2(c * aip.x - s * t.x, c * aip.y - s * t.y);
+        *xq = make_double2(s * aip.x + c * t.x, s * aip.y + c * t.y);
       }
-      __syncwarp();
-      // rows: A <- J^H A
-      for (int idx = lane; idx < half * n; idx += 32) {
-        int k = idx / n, j = idx % n;
-        int q = (int)sP[3 * k + 2].y;
-        if (q < 0) continue;
-        int p = (int)sP[3 * k + 2].x;
-        double c = sP[3 * k].x, s = sP[3 * k].y;
-        double2 ph = sP[3 * k + 1];
-        double2 apj = sA[p + n * j], aqj = sA[q + n * j];
-        double2 t = cmul(ph, aqj);
-        sA[p + n * j] = make_double2(c * apj.x - s * t.x, c * apj.y - s * t.y);
-        sA[q + n * j] = make_double2(s * apj.x + c * t.x, s * apj.y + c * t.y);
-      }
-      __syncwarp();
-      if (lane < half) {
-        int q = (int)sP[3 * lane + 2].y;
-        if (q >= 0) {
-          int p = (int)sP[3 * lane + 2].x;
-          sA[p + n * p].y = 0.0;   // the diagonal of a Hermitian matrix is real
-          sA[q + n * q].y = 0.0;
+      __syncthreads();
+      // rows: A <- J^H A, its diagonal kept real; V <- V J, by other warps
+      for (int idx = tid; idx < cntv + cnt; idx += T) {
+        const bool row = idx < cntv;
+        const int v = row ? idx : idx - cntv;
+        if (v >= cnt) continue;
+        const int a = div_by(v, e.inv_hn), v0 = v - a * half * n, k = div_by(v0, e.inv_n), i = v0 - k * n;
+        double2 *M = sm + (size_t)((map >> (4 * a)) & 15) * e.size;
+        const double2 *sP = M + oP + 3 * k;
+        const int2 pq = *(const int2 *)(sP + 2);
+        if (pq.y < 0) continue;
+        const double c = sP[0].x, s = sP[0].y;
+        if (row) {
+          const double2 ph = sP[1];
+          M += ld * i;
+          const double2 apj = M[pq.x], aqj = M[pq.y];
+          const double2 t = cmul(ph, aqj);
+          const double2 np = make_double2(c * apj.x - s * t.x, c * apj.y - s * t.y);
+          const double2 nq = make_double2(s * apj.x + c * t.x, s * apj.y + c * t.y);
+          M[pq.x] = make_double2(np.x, i == pq.x ? 0.0 : np.y);
+          M[pq.y] = make_double2(nq.x, i == pq.y ? 0.0 : nq.y);
+        } else {
+          const double2 phc = make_double2(sP[1].x, -sP[1].y);
+          double2 *xp = M + oV + ld * pq.x + i, *xq = M + oV + ld * pq.y + i;
+          const double2 vip = *xp, viq = *xq;
+          const double2 t = cmul(phc, viq);
+          *xp = make_double2(c * vip.x - s * t.x, c * vip.y - s * t.y);
+          *xq = make_double2(s * vip.x + c * t.x, s * vip.y + c * t.y);
         }
       }
-      __syncwarp();
+      __syncthreads();
     }
   }
-  if (!converged && lane == 0) atomicOr(err, DERR_EIG);
+  if (na > 0 && tid == 0) atomicOr(err, DERR_EIG);   // not converged
   // sort ascending by rank (ties by index), write eigenvalues and columns
-  for (int i = lane; i < n; i += 32) {
-    double di = sA[i + n * i].x;
+  for (int idx = tid; idx < ng * n; idx += T) {
+    const int g = div_by(idx, e.inv_n), i = idx - g * n;
+    const double2 *M = sm + (size_t)g * e.size;
+    double di = M[i + ld * i].x;
     int rank = 0;
     for (int j = 0; j < n; ++j) {
-      double dj = sA[j + n * j].x;
+      double dj = M[j + ld * j].x;
       rank += (dj < di) || (dj == di && j < i);
     }
-    w[(size_t)mat * n + rank] = di;
-    for (int c = 0; c < n; ++c) V[(size_t)mat * nn + c + n * rank] = sV[c + n * i];
+    w[(size_t)(mat0 + g) * n + rank] = di;
+    for (int c = 0; c < n; ++c) V[(size_t)(mat0 + g) * nn + c + n * rank] = M[oV + c + ld * i];
   }
+}
+
+template <int T>
+static void heig_run(int batch, int n, int G, const double2 *A, int64_t stride, double *w, double2 *V, int *err,
+                     cudaStream_t st) {
+  // once per process: changing a kernel attribute can wait for the device's queued work
+  static std::once_flag attr_once;
+  std::call_once(attr_once, [] {
+    cudaFuncSetAttribute(k_heig<T>, cudaFuncAttributeMaxDynamicSharedMemorySize, 96 * 1024);
+  });
+  const size_t smem = (size_t)G * (4 * (n | 1) * n + 3 * 16) * sizeof(double2);   // 77 KB at most
+  k_heig<T><<<(batch + G - 1) / G, T, smem, st>>>(batch, n, G, A, stride, w, V, err);
 }
 
 void launch_heig(int batch, int n, const double2 *A, int64_t stride, double *w, double2 *V,
                  int *err, cudaStream_t st) {
   if (batch <= 0) return;
-  int wpb = n <= 8 ? 4 : n <= 16 ? 2 : 1;
-  size_t smem = (size_t)wpb * (4 * n * n + 3 * 16) * sizeof(double2);   // 67 KB at most (n = 32)
-  // once per process: changing a kernel attribute can wait for the device's queued work
-  static std::once_flag attr_once;
-  std::call_once(attr_once, [] {
-    cudaFuncSetAttribute(k_heig, cudaFuncAttributeMaxDynamicSharedMemorySize, 96 * 1024);
-  });
-  k_heig<<<(batch + wpb - 1) / wpb, 32 * wpb, smem, st>>>(batch, n, A, stride, w, V, err);
+  // Small batches are bound by the latency of one matrix, whose phases more warps shorten;
+  // from a few matrices per SM sub-partition on by FP64 instructions, which taking matrices
+  // together saves where one leaves lanes idle.  Microseconds at G = 1 / together:
+  //   512 of n = 8:    90 / 103 (G = 4)      1,728 of n = 6:  133 / 100 (G = 4)
+  //   2,197 of n = 12: 659 / 613 (G = 2)     2,197 of n = 16: 1,190 / 1,242 (G = 2)
+  const bool many = batch >= 8 * EIG_SMS;
+  if (n <= 8) {
+    if (many) heig_run<128>(batch, n, 4, A, stride, w, V, err, st);
+    else heig_run<64>(batch, n, 1, A, stride, w, V, err, st);
+  } else {
+    heig_run<128>(batch, n, n <= 12 && many ? 2 : 1, A, stride, w, V, err, st);
+  }
 }
 
 // ============================================================ electrons
