@@ -111,5 +111,15 @@ __device__ __forceinline__ void tmem_ld8_nowait(uint32_t taddr, uint32_t *r) {
                : "r"(taddr));
 }
 
+// 16 bytes to shared memory without passing through registers; zeros after the first `bytes`.
+__device__ __forceinline__ void cp_async16(void *dst, const void *src, int bytes) {
+  asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"(smem_u32(dst)), "l"(src), "r"(bytes) : "memory");
+}
+__device__ __forceinline__ void cp_async_commit() { asm volatile("cp.async.commit_group;" ::: "memory"); }
+template <int N>
+__device__ __forceinline__ void cp_async_wait() {
+  asm volatile("cp.async.wait_group %0;" ::"n"(N) : "memory");
+}
+
 }  // namespace tc
 }  // namespace ephg

@@ -916,126 +916,145 @@ __global__ void k_rotate_planes(int j0, int j1, int i0, const int *st_code, int 
   }
 }
 
-// Stage-A rotation, one block per window k: the block loads g(k,Rp) for KT
-// contraction positions at a time (coalesced rows of nw*nw values per mode),
-// rotates over the initial band for every in-window state of k, applies the
-// k-half of the Rp phase and writes KT consecutive K positions of each operand
-// row, so that both the reads and the split-plane writes are whole sectors.
-// Modes are taken sch at a time so that the staged g fits shared memory for
-// any nb.  kinv[kp] = Rp cell at contraction position kp (-1 for padding).
+// Stage-A rotation, one block per window k: the block stages g(k,Rp) for ROT_KT
+// contraction positions at a time (a warp each, coalesced rows of nw*nw values per
+// mode, real and imaginary parts apart), rotates over the initial band for every
+// in-window state of k, applies the k-half of the Rp phase and writes ROT_KT
+// consecutive K positions of each operand row, so that both the reads and the
+// split-plane writes are whole sectors.  Modes are taken sch at a time so that the
+// staged g fits shared memory for any nb.  The copies of the next positions (cp.async: no
+// registers, no waiting) run while these are rotated.
+// kinv[kp] = Rp cell at contraction position kp (-1 for padding).
+// Bound by HBM: g(k,Rp) is read once, 2.3 MB per k at nw 16, nb 12.  1,792 k there:
+// 0.83 ms, 5.6 TB/s (1.41 with loads through registers, an index division per load, the phases'
+// FP64 divisions between the barriers and 64 of 256 threads rotating).
 constexpr int ROT_KT = 8;
-static_assert(ROT_KT == 8, "k_rotate_k writes 8 K positions as two float4 per plane");
-constexpr int ROT_SMEM = 160 * 1024;
+constexpr int ROT_THREADS = 32 * ROT_KT;
+constexpr int ROT_PAD = 4;   // floats per staged position: lanes of one row read different banks
+constexpr int ROT_SMEM = 220 * 1024;
 constexpr int ROT_SMEM_TARGET = 72 * 1024;
 
 // shared memory of k_rotate_k for sch modes per pass and nsk <= nw states per row
-static size_t rotate_k_smem(int nw, int sch) {
-  return ((sizeof(float2) * ROT_KT * nw * nw * sch + 15) & ~(size_t)15) + sizeof(float2) * (nw * nw + ROT_KT);
+static size_t rotate_k_smem(int nw, int sch, int Kp2) {
+  return sizeof(float) * 2 * 2 * ROT_KT * (nw * nw * sch + ROT_PAD) + sizeof(float2) * (nw * nw + Kp2);
 }
 
-__global__ void __launch_bounds__(256) k_rotate_k(int i0, const int *first_state, int nw, int nb, int sch,
-                                                  const int *st_code, const int *widx, const double2 *U,
-                                                  const float *gr, const float *gi, int64_t ldg, int m1, int m2,
-                                                  int m3, int L, const double2 *roots, const int *Rq,
-                                                  const double *degq, const int *kinv, int Kp2, float *Bp,
-                                                  int64_t Np2) {
-  extern __shared__ unsigned char rsm[];
+// Rotation of k_rotate_k's staged positions: a thread forms KS of the ROT_KT positions of
+// one operand row, ROT_KT / KS neighbouring lanes the row's whole 32-byte sectors of the
+// four planes; lanes then walk consecutive bands n' (conflict-free shared reads).
+// gr, gi: [ROT_KT][pcp].
+template <int KS>
+__device__ __forceinline__ void rotate_rows(int rows, int nc, int nw, int pcp, const float *gr, const float *gi,
+                                            const float2 *sU, const float2 *sph, float *Bp, int64_t plane, int64_t col0, int ncol,
+                                            int Kp2) {
+  constexpr int KL = ROT_KT / KS;
+  for (int t = threadIdx.x; t < rows * KL; t += blockDim.x) {
+    const int o = t / KL, k0 = (t % KL) * KS;
+    const int c = o % nc, js = o / nc;
+    const int np = c % nw, s = c / nw;
+    float2 acc[KS];
+#pragma unroll
+    for (int kk = 0; kk < KS; ++kk) acc[kk] = make_float2(0.f, 0.f);
+    const int g0 = k0 * pcp + np + nw * nw * s;
+    const float2 *u = sU + js * nw;
+    for (int mp = 0; mp < nw; ++mp) {
+      const float2 um = u[mp];
+#pragma unroll
+      for (int kk = 0; kk < KS; ++kk) {
+        const int o2 = g0 + kk * pcp + nw * mp;
+        cfmaf(acc[kk], um, make_float2(gr[o2], gi[o2]));
+      }
+    }
+    float pl[4][KS];
+#pragma unroll
+    for (int kk = 0; kk < KS; ++kk) {
+      const float2 ph = sph[k0 + kk];
+      float hr, lr, hi, li;
+      split2((double)(ph.x * acc[kk].x - ph.y * acc[kk].y), hr, lr);
+      split2((double)(ph.x * acc[kk].y + ph.y * acc[kk].x), hi, li);
+      pl[0][kk] = hr;
+      pl[1][kk] = hi;
+      pl[2][kk] = lr;
+      pl[3][kk] = li;
+    }
+    float *dst = Bp + (col0 + (int64_t)js * ncol + c) * Kp2 + k0;
+#pragma unroll
+    for (int q = 0; q < 4; ++q) {
+      if (KS == 1) dst[q * plane] = pl[q][0];
+#pragma unroll
+      for (int kk = 0; kk + 1 < KS; kk += 2) *(float2 *)(dst + q * plane + kk) = make_float2(pl[q][kk], pl[q][kk + 1]);
+    }
+  }
+}
+
+__global__ void __launch_bounds__(ROT_THREADS) k_rotate_k(int i0, const int *first_state, int nw, int nb, int sch,
+                                                          const int *st_code, const int *widx, const double2 *U,
+                                                          const float *gr, const float *gi, int64_t ldg, int m1,
+                                                          int m2, int m3, int L, const double2 *roots, const int *Rq,
+                                                          const double *degq, const int *kinv, int Kp2, float *Bp,
+                                                          int64_t Np2) {
+  extern __shared__ __align__(16) float rsm[];
   const int i = i0 + blockIdx.x;
   const int j0 = first_state[i], j1 = first_state[i + 1];
   const int nsk = j1 - j0;
   if (nsk <= 0) return;
   const int p = widx[i];
   const int per = nw * nw * nb, ncol = nw * nb, nn = nw * nw;
-  float2 *sg = (float2 *)rsm;                                   // [ROT_KT][nw * nw * sch]
-  float2 *sU = (float2 *)(rsm + ((sizeof(float2) * ROT_KT * nn * sch + 15) & ~(size_t)15));  // [nsk][nw]
-  float2 *sph = sU + nsk * nw;                                  // [ROT_KT]
+  const int pcm = nn * sch + ROT_PAD, bufsz = 2 * ROT_KT * pcm;   // rsm: [2][re, im][ROT_KT][pcm]
+  float2 *sU = (float2 *)(rsm + 2 * bufsz);                       // [nsk][nw]
+  float2 *sph = sU + nn;                                          // [Kp2]
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const int64_t row = ileave32(i - i0, 0, ldg);
+  const int npos = Kp2 / ROT_KT, npass = (nb + sch - 1) / sch * npos;
+  auto load = [&](int pass) {
+    const int s0 = pass / npos * sch, pc = nn * min(sch, nb - s0);
+    const int rp = kinv[pass % npos * ROT_KT + warp];
+    const int64_t c0 = rp >= 0 ? (int64_t)rp * per + nn * s0 : 0;
+    const int bytes = rp >= 0 ? 16 : 0;   // padding positions: zeros
+    float *dr = rsm + (pass & 1) * bufsz + warp * pcm, *di = dr + ROT_KT * pcm;
+    for (int e = 4 * lane; e < pc; e += 128) {   // 16 bytes: every row offset is a multiple of 4
+      const int64_t c = c0 + e, off = row + ((c & ~(int64_t)31) << 5) + (c & 31);
+      cp_async16(dr + e, gr + off, bytes);
+      cp_async16(di + e, gi + off, bytes);
+    }
+    cp_async_commit();
+  };
+  load(0);
   for (int t = threadIdx.x; t < nsk * nw; t += blockDim.x) {
     int js = t / nw, mp = t % nw;
     int m = st_code[j0 + js] % nw;
     double2 u = U[((size_t)p * nw + m) * nw + mp];
     sU[t] = make_float2((float)u.x, (float)u.y);
   }
-  const int64_t plane = Np2 * Kp2;
-  for (int s0 = 0; s0 < nb; s0 += sch) {
-    const int ns = min(sch, nb - s0), pc = nn * ns, nc = nw * ns;
-    for (int kp0 = 0; kp0 < Kp2; kp0 += ROT_KT) {
-      __syncthreads();
-      // 16-byte loads (4 consecutive values; every row offset is a multiple of 4),
-      // four of them in flight per thread before the shared stores
-      const int pc4 = pc >> 2, tot = ROT_KT * pc4;
-      for (int t0 = threadIdx.x; t0 < tot; t0 += 4 * blockDim.x) {
-        float4 a[4], b[4];
-#pragma unroll
-        for (int u = 0; u < 4; ++u) {
-          const int t = t0 + u * blockDim.x;
-          a[u] = b[u] = make_float4(0.f, 0.f, 0.f, 0.f);
-          if (t < tot) {
-            const int kk = t / pc4, e = 4 * (t - kk * pc4);
-            const int rp = kinv[kp0 + kk];
-            if (rp >= 0) {
-              const int64_t off = ileave32(i - i0, (int64_t)rp * per + nn * s0 + e, ldg);
-              a[u] = __ldg((const float4 *)(gr + off));
-              b[u] = __ldg((const float4 *)(gi + off));
-            }
-          }
-        }
-#pragma unroll
-        for (int u = 0; u < 4; ++u) {
-          const int t = t0 + u * blockDim.x;
-          if (t < tot) {
-            float4 *dst = (float4 *)(sg + 4 * t);
-            dst[0] = make_float4(a[u].x, b[u].x, a[u].y, b[u].y);
-            dst[1] = make_float4(a[u].z, b[u].z, a[u].w, b[u].w);
-          }
-        }
-      }
-      if (threadIdx.x < ROT_KT) {
-        int rp = kinv[kp0 + threadIdx.x];
-        float2 ph = make_float2(0.f, 0.f);
-        if (rp >= 0) {
-          double2 r = roots[phase_idx(p, m1, m2, m3, L, Rq[3 * rp], Rq[3 * rp + 1], Rq[3 * rp + 2])];
-          ph = make_float2((float)(r.x / degq[rp]), (float)(-r.y / degq[rp]));
-        }
-        sph[threadIdx.x] = ph;
-      }
-      __syncthreads();
-      // a thread forms the ROT_KT positions of one operand row: lanes walk
-      // consecutive bands n' (conflict-free shared reads) and each writes whole
-      // 32-byte sectors of the four planes
-      for (int o = threadIdx.x; o < nsk * nc; o += blockDim.x) {
-        const int c = o % nc, js = o / nc;
-        const int np = c % nw, s = c / nw;
-        float2 acc[ROT_KT];
-#pragma unroll
-        for (int kk = 0; kk < ROT_KT; ++kk) acc[kk] = make_float2(0.f, 0.f);
-        const float2 *g = sg + np + nn * s;
-        const float2 *u = sU + js * nw;
-        for (int mp = 0; mp < nw; ++mp) {
-          const float2 um = u[mp];
-#pragma unroll
-          for (int kk = 0; kk < ROT_KT; ++kk) cfmaf(acc[kk], um, g[kk * pc + nw * mp]);
-        }
-        float pl[4][ROT_KT];
-#pragma unroll
-        for (int kk = 0; kk < ROT_KT; ++kk) {
-          const float2 ph = sph[kk];
-          float hr, lr, hi, li;
-          split2((double)(ph.x * acc[kk].x - ph.y * acc[kk].y), hr, lr);
-          split2((double)(ph.x * acc[kk].y + ph.y * acc[kk].x), hi, li);
-          pl[0][kk] = hr;
-          pl[1][kk] = hi;
-          pl[2][kk] = lr;
-          pl[3][kk] = li;
-        }
-        const int64_t col = (int64_t)(j0 + js) * ncol + np + nw * (s0 + s);
-#pragma unroll
-        for (int q = 0; q < 4; ++q) {
-          float4 *dst = (float4 *)(Bp + q * plane + col * Kp2 + kp0);
-          dst[0] = make_float4(pl[q][0], pl[q][1], pl[q][2], pl[q][3]);
-          dst[1] = make_float4(pl[q][4], pl[q][5], pl[q][6], pl[q][7]);
-        }
-      }
+  for (int t = threadIdx.x; t < Kp2; t += blockDim.x) {
+    const int rp = kinv[t];
+    float2 ph = make_float2(0.f, 0.f);
+    if (rp >= 0) {
+      double2 r = roots[phase_idx(p, m1, m2, m3, L, Rq[3 * rp], Rq[3 * rp + 1], Rq[3 * rp + 2])];
+      ph = make_float2((float)(r.x / degq[rp]), (float)(-r.y / degq[rp]));
     }
+    sph[t] = ph;
+  }
+  const int64_t plane = Np2 * Kp2;
+  for (int pass = 0; pass < npass; ++pass) {
+    if (pass + 1 < npass) {
+      load(pass + 1);
+      cp_async_wait<1>();
+    } else {
+      cp_async_wait<0>();
+    }
+    __syncthreads();   // this pass's copies of all warps are in place
+    const int s0 = pass / npos * sch, kp0 = pass % npos * ROT_KT;
+    const int nc = nw * min(sch, nb - s0), rows = nsk * nc;
+    const float *sr = rsm + (pass & 1) * bufsz, *si = sr + ROT_KT * pcm;
+    float *dst = Bp + kp0;
+    const int64_t col0 = (int64_t)j0 * ncol + nw * s0;
+    // as many threads per operand row as keep the block's busy
+    if (8 * rows <= ROT_THREADS) rotate_rows<1>(rows, nc, nw, pcm, sr, si, sU, sph + kp0, dst, plane, col0, ncol, Kp2);
+    else if (4 * rows <= ROT_THREADS) rotate_rows<2>(rows, nc, nw, pcm, sr, si, sU, sph + kp0, dst, plane, col0, ncol, Kp2);
+    else if (2 * rows <= ROT_THREADS) rotate_rows<4>(rows, nc, nw, pcm, sr, si, sU, sph + kp0, dst, plane, col0, ncol, Kp2);
+    else rotate_rows<8>(rows, nc, nw, pcm, sr, si, sU, sph + kp0, dst, plane, col0, ncol, Kp2);
+    __syncthreads();   // the buffer has been read
   }
 }
 
@@ -2717,19 +2736,19 @@ static int split_rates_generic(SplitOperands &s, Workspace &ws, cudaStream_t st,
       return rc;
     tA->end(st);
     {
-      // modes per pass: as many as keep the staged g within ROT_SMEM_TARGET (three
-      // blocks per SM), at least one (up to ROT_SMEM)
+      // modes per pass: as many as keep the staged g within ROT_SMEM_TARGET (three blocks
+      // per SM; one at 110 KB 1.04 times as long at nw 16, 1.05 at nw 24), at least one
       int sch = nb;
-      while (sch > 1 && rotate_k_smem(nw, sch) > (size_t)ROT_SMEM_TARGET) --sch;
-      const size_t sm = rotate_k_smem(nw, sch);
+      while (sch > 1 && rotate_k_smem(nw, sch, KpB) > (size_t)ROT_SMEM_TARGET) --sch;
+      const size_t sm = rotate_k_smem(nw, sch, KpB);
       if (sm <= (size_t)ROT_SMEM && (nw % 2) == 0) {   // 16-byte staging: nw * nw a multiple of 4
         // once per process: changing a kernel attribute can wait for the device's queued work
         static std::once_flag attr_once;
         std::call_once(attr_once, [] {
           cudaFuncSetAttribute(k_rotate_k, cudaFuncAttributeMaxDynamicSharedMemorySize, ROT_SMEM);
         });
-        k_rotate_k<<<n, 256, sm, st>>>((int)i0, fs_d, nw, nb, sch, st_code, arow, U, CAr, CAi, NpA, mesh[0],
-                                      mesh[1], mesh[2], L, roots, Rq, degq, kinvB, KpB, B2, Np2);
+        k_rotate_k<<<n, ROT_THREADS, sm, st>>>((int)i0, fs_d, nw, nb, sch, st_code, arow, U, CAr, CAi, NpA,
+                                              mesh[0], mesh[1], mesh[2], L, roots, Rq, degq, kinvB, KpB, B2, Np2);
         TCK(cudaGetLastError());
         (*launches)++;
       } else {   // large nw*nw*nb: one thread per output element
