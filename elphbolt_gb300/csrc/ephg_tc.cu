@@ -166,19 +166,19 @@ struct GemmArgs {
   int *err;
   int ileave;                // 1: outputs interleaved by 32 rows in groups of 4 columns: (r, c) at
                              //    (r / 32) ldc 32 + (c / 4) 128 + (r % 32) 4 + c % 4 (ldc a multiple of 4);
-                             // 2: in groups of 32 columns (ileave32)
+                             // 2: in groups of 16 columns (ileave16)
   RotOut rot;
 };
 
-// Element (r, c) of an output interleaved by 32 rows in groups of 32 columns: a drain
-// lane's 16 columns are 64 consecutive bytes and a warp's 32 rows lie in 4 KB, so it
-// writes whole sectors; a reader of one row gets whole 128-byte lines.  Row-major, each store of a
-// warp touched 32 rows 1 MB apart, half a sector each: at 96 K positions the drain
-// took 20,000 of a stage-A tile's 32,000 cycles (nw 16, nb 12, 13^3: stage A's GEMMs
-// 1.60 ms per launch, now 1.05; groups of 16 columns 0.86, but the rotation that reads
-// them 1.34 -> 1.76 instead of 1.41).
-__host__ __device__ __forceinline__ int64_t ileave32(int64_t r, int64_t c, int64_t ldc) {
-  return ((r >> 5) * ldc + (c & ~(int64_t)31)) * 32 + (r & 31) * 32 + (c & 31);
+// Element (r, c) of an output interleaved by 32 rows in groups of 16 columns: a drain
+// lane's 16 columns are 64 consecutive bytes and a warp's 32 rows 2 KB, which it writes
+// whole; a reader of one row gets whole sectors.  Row-major, each store of a warp touched
+// 32 rows 1 MB apart, half a sector each: at 96 K positions the drain took 20,000 of a
+// stage-A tile's 32,000 cycles (nw 16, nb 12, 13^3: stage A's GEMMs 1.60 ms per launch,
+// now 0.92; groups of 32 columns 1.05, of which the rotation then reads whole 128-byte
+// lines: 0.83 instead of 0.91 ms per request).
+__host__ __device__ __forceinline__ int64_t ileave16(int64_t r, int64_t c, int64_t ldc) {
+  return ((r >> 5) * ldc + (c & ~(int64_t)15)) * 32 + (r & 31) * 16 + (c & 15);
 }
 
 // 32 bytes in one streaming store
@@ -482,7 +482,7 @@ __device__ __forceinline__ void cgemm_body(const Jobs &jobs, int t0, int t1, int
       tc_fence_after();
       // row-major: the row's 16 columns as float4 stores; interleaved: each group of
       // 4 columns of the warp's 32 rows is 512 consecutive bytes (one float4 per lane)
-      const int64_t off = j.ileave ? (int64_t)quad * j.ldc * 32 + (j.ileave == 2 ? 32 : 4) * lane : (int64_t)row * j.ldc;
+      const int64_t off = j.ileave ? (int64_t)quad * j.ldc * 32 + (j.ileave == 2 ? 16 : 4) * lane : (int64_t)row * j.ldc;
       float *cr = j.Cr + off, *ci = j.Ci + off;
 #pragma unroll 1
       for (int c0 = cbeg; c0 < cbeg + CW; c0 += 16) {
@@ -500,7 +500,7 @@ __device__ __forceinline__ void cgemm_body(const Jobs &jobs, int t0, int t1, int
         }
         // streaming stores: the output is read once, later, by another kernel
         if (j.ileave == 2) {
-          const int64_t o = (int64_t)(c0 & ~31) * 32 + (c0 & 16);
+          const int64_t o = (int64_t)c0 * 32;
           st_cs8(cr + o, vr);
           st_cs8(cr + o + 8, vr + 8);
           st_cs8(ci + o, vi);
@@ -901,7 +901,7 @@ __global__ void k_rotate_planes(int j0, int j1, int i0, const int *st_code, int 
     ph = make_double2(ph.x / degq[rp], -ph.y / degq[rp]);
     double2 acc = make_double2(0.0, 0.0);
     for (int mp = 0; mp < nw; ++mp) {
-      const int64_t off = ileave32(grow, np + nw * (mp + (int64_t)nw * (s + (int64_t)nb * rp)), ldg);
+      const int64_t off = ileave16(grow, np + nw * (mp + (int64_t)nw * (s + (int64_t)nb * rp)), ldg);
       cfma(acc, Uk[mp], make_double2((double)gr[off], (double)gi[off]));
     }
     const int64_t col = (int64_t)(j - jbase) * ncol + c;
@@ -926,7 +926,7 @@ __global__ void k_rotate_planes(int j0, int j1, int i0, const int *st_code, int 
 // registers, no waiting) run while these are rotated.
 // kinv[kp] = Rp cell at contraction position kp (-1 for padding).
 // Bound by HBM: g(k,Rp) is read once, 2.3 MB per k at nw 16, nb 12.  1,792 k there:
-// 0.83 ms, 5.6 TB/s (1.41 with loads through registers, an index division per load, the phases'
+// 0.91 ms, 5.1 TB/s (1.41 with loads through registers, an index division per load, the phases'
 // FP64 divisions between the barriers and 64 of 256 threads rotating).
 constexpr int ROT_KT = 8;
 constexpr int ROT_THREADS = 32 * ROT_KT;
@@ -1004,7 +1004,7 @@ __global__ void __launch_bounds__(ROT_THREADS) k_rotate_k(int i0, const int *fir
   float2 *sU = (float2 *)(rsm + 2 * bufsz);                       // [nsk][nw]
   float2 *sph = sU + nn;                                          // [Kp2]
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  const int64_t row = ileave32(i - i0, 0, ldg);
+  const int64_t row = ileave16(i - i0, 0, ldg);
   const int npos = Kp2 / ROT_KT, npass = (nb + sch - 1) / sch * npos;
   auto load = [&](int pass) {
     const int s0 = pass / npos * sch, pc = nn * min(sch, nb - s0);
@@ -1013,7 +1013,7 @@ __global__ void __launch_bounds__(ROT_THREADS) k_rotate_k(int i0, const int *fir
     const int bytes = rp >= 0 ? 16 : 0;   // padding positions: zeros
     float *dr = rsm + (pass & 1) * bufsz + warp * pcm, *di = dr + ROT_KT * pcm;
     for (int e = 4 * lane; e < pc; e += 128) {   // 16 bytes: every row offset is a multiple of 4
-      const int64_t c = c0 + e, off = row + ((c & ~(int64_t)31) << 5) + (c & 31);
+      const int64_t c = c0 + e, off = row + ((c & ~(int64_t)15) << 5) + (c & 15);
       cp_async16(dr + e, gr + off, bytes);
       cp_async16(di + e, gi + off, bytes);
     }
