@@ -5,8 +5,6 @@
 // z_a(j) = sum_i g_i born(i, j, a) and w(3a+i) = p_a z_a(i), the G + q term of
 // dyn_nonanalytic is a rank-one update
 //   D += f w w^H,   f = e^{-qeq/4alph}/qeq,
-// its derivative along x is M_x + M_x^H with the outer product
-//   M_x += f v_x w^H,   v_x(3a+i) = p_a born(x, i, a) + (i tau_a(x) - dgeg_x (1/4alph + 1/qeq) / 2) w(3a+i),
 // and long_range_prefac is sum_c L(c) u(c), L = i fac conj(sum_g f w).
 //
 // One block per q, bound by the FP64 pipe, so what counts is FP64 instructions on
@@ -17,10 +15,10 @@
 // are tested; the others never contribute.  Fixed order throughout: deterministic
 // sums.
 //
-// With velocities (k_polar_vel) every thread sums outer products, the candidates
-// split over as many slices as the block has threads per matrix element: 1,728 q,
-// 13^3 box: 0.32 ms (1.13 ms with the FP64 test on every box vector, its terms
-// formed in partly filled warps and ~70 operations per element and vector).
+// With velocities (k_polar_vel) the sums' Hermitian halves, the candidates split over as
+// many slices as the block has threads per item: 1,728 q, 13^3 box: 0.18 ms (1.13 ms with
+// the FP64 test on every box vector, its terms formed in partly filled warps and ~70
+// operations per element and vector; 0.32 with the derivative's outer products whole).
 // Without (k_polar) an element is summed by one thread in the loop order, from
 // f p_a conj(p_b) per pair of atoms and z.  The tensor-core rates round the
 // eigenvectors to FP32 in the gauge that the eigensolver leaves them in, which the
@@ -230,35 +228,45 @@ __global__ void __launch_bounds__(PL_THREADS) k_polar(PolarDev P, const double *
   }
 }
 
-// With velocities.  Entry of a candidate: complex vectors of nb values: w, f w (right and
-// left factors), f v_x for x = 0..2.
-constexpr int PV_VECTORS = 5;
+// With velocities.  With r = w w^H of a candidate, the derivative along x of sum f r is
+//   dD_x(i,j) = born(x,i) P(a,j) + conj(born(x,j) P(b,i)) + i (tau_a - tau_b)(x) D(i,j) - 2 W_x(i,j),
+//   P(a,j) = sum f p_a conj(w_j),  W_x = sum f dgeg_x (1/4alph + 1/qeq) / 2 r
+// for i, j of atoms a, b: beside the nat nb sums of P only D and the W_x are summed, which are
+// Hermitian: 12 FP64 operations per candidate on nb (nb + 1) / 2 elements instead of 16 on
+// nb^2, and no vector per direction to prepare.
+// Entry of a candidate (double2): w (nb), f p_a (nat), (f, W_0's weight), (W_1's, W_2's).
+// NU: items per thread (nb (nb + 1) / 2 and nat nb <= NU * PL_THREADS).
+__host__ __device__ inline int pv_entry(int nat) { return 4 * nat + 2; }
 
 template <int NU>
 __global__ void __launch_bounds__(PL_THREADS) k_polar_vel(PolarDev P, const double *G, const float *Gf, int M, int nq,
                                                           const int *qp, int m1, int m2, int m3, const double *qv,
-                                                          int nent, double2 *Dq, double2 *dDq, int64_t ldd,
-                                                          double2 *Lq) {
-  extern __shared__ double2 psm[];   // [nent][vectors][nb]
+                                                          int nent, double2 *Dq, double2 *dDq, int64_t ldd) {
+  extern __shared__ double2 psm[];   // entries; at the end the sums
   __shared__ int list[PL_LIST];
   __shared__ int wcount[PL_THREADS / 32];
-  constexpr int NV = PV_VECTORS;
   const int q = blockIdx.x;
-  const int nat = P.nat, nb = P.nb, ne = nb * nb;
+  const int nat = P.nat, nb = P.nb, ne = nb * nb, nh = nb * (nb + 1) / 2, np = nat * nb, esz = pv_entry(nat);
   const int tid = threadIdx.x;
   double qc[3];
   pl_q(P, q, nq, qp, m1, m2, m3, qv, qc);
-  // thread's elements: el = tid + u PL_THREADS of the nb^2 matrix and nb vector elements, or
-  // (NU = 1) element tid % nel of slice tid / nel
-  const int nel = ne + nb, nsl = NU == 1 ? PL_THREADS / nel : 1;
-  const int slice = NU == 1 ? tid / nel : 0, el0 = NU == 1 ? tid % nel : tid;
-  const bool work = slice < nsl;
-  double2 acc[NU], dacc[NU][3];
+  // Hermitian items (i >= j) and P items, each tid + u PL_THREADS, or (NU = 1) split over
+  // as many slices of the candidates as the block has threads per item
+  const int hsl = NU == 1 ? PL_THREADS / nh : 1, psl = NU == 1 ? PL_THREADS / np : 1;
+  const int hs = NU == 1 ? tid / nh : 0, h0 = NU == 1 ? tid % nh : tid;
+  const int ps = NU == 1 ? tid / np : 0, p0 = NU == 1 ? tid % np : tid;
+  int hi[NU], hj[NU];
+  double2 acc[NU][4], pacc[NU];
 #pragma unroll
   for (int u = 0; u < NU; ++u) {
-    acc[u] = make_double2(0.0, 0.0);
+    const int it = h0 + u * PL_THREADS;
+    int i = 0;
+    while ((i + 1) * (i + 2) / 2 <= it) ++i;
+    hi[u] = hs < hsl && it < nh ? i : -1;
+    hj[u] = it - i * (i + 1) / 2;
+    pacc[u] = make_double2(0.0, 0.0);
 #pragma unroll
-    for (int x = 0; x < 3; ++x) dacc[u][x] = make_double2(0.0, 0.0);
+    for (int x = 0; x < 4; ++x) acc[u][x] = make_double2(0.0, 0.0);
   }
   for (int c0 = 0; c0 < M;) {
     const int nl = pl_candidates(P, Gf, M, qc, c0, list, wcount);
@@ -272,83 +280,95 @@ __global__ void __launch_bounds__(PL_THREADS) k_polar_vel(PolarDev P, const doub
         const double qeq = geg(P.eps, g);
         const bool pass = qeq > 0.0 && qeq / P.alph / 4.0 < P.gmax;
         const double f = pass ? exp(-qeq / P.alph / 4.0) / qeq : 0.0;
-        const double dgc = pass ? 0.5 * (0.25 / P.alph + 1.0 / qeq) : 0.0;
+        const double dgc = pass ? 0.5 * f * (0.25 / P.alph + 1.0 / qeq) : 0.0;
         double dge[3];
         for (int x = 0; x < 3; ++x)
           dge[x] = dgc * ((P.eps[x] + P.eps[3 * x]) * g[0] + (P.eps[x + 3] + P.eps[3 * x + 1]) * g[1] +
                           (P.eps[x + 6] + P.eps[3 * x + 2]) * g[2]);
-        double2 *e = psm + (size_t)tid * NV * nb;
+        double2 *e = psm + (size_t)tid * esz;
         for (int a = 0; a < nat; ++a) {
           double sn, cs;
           sincos(g[0] * P.tau[3 * a] + g[1] * P.tau[3 * a + 1] + g[2] * P.tau[3 * a + 2], &sn, &cs);
           for (int i = 0; i < 3; ++i) {
             const double *Z = P.born + 3 * i + 9 * a;
             const double z = g[0] * Z[0] + g[1] * Z[1] + g[2] * Z[2];
-            const double2 w = make_double2(cs * z, sn * z);
-            e[3 * a + i] = w;
-            e[nb + 3 * a + i] = cscale(w, f);
-            for (int x = 0; x < 3; ++x) {
-              const double t = P.tau[3 * a + x];
-              e[(2 + x) * nb + 3 * a + i] = make_double2(f * (cs * Z[x] - dge[x] * w.x - t * w.y),
-                                                         f * (sn * Z[x] - dge[x] * w.y + t * w.x));
-            }
+            e[3 * a + i] = make_double2(cs * z, sn * z);
           }
+          e[nb + a] = make_double2(f * cs, f * sn);
         }
+        e[nb + nat] = make_double2(f, dge[0]);
+        e[nb + nat + 1] = make_double2(dge[1], dge[2]);
       }
       __syncthreads();
-      if (work)
 #pragma unroll
-        for (int u = 0; u < NU; ++u) {
-          const int el = el0 + u * PL_THREADS;
-          if (el < ne) {
-            const int i = el % nb, j = el / nb;
-            for (int k = slice; k < n; k += nsl) {
-              const double2 *e = psm + (size_t)k * NV * nb;
-              const double2 r = cconj(e[j]);
-              cfma(acc[u], e[nb + i], r);
-#pragma unroll
-              for (int x = 0; x < 3; ++x) cfma(dacc[u][x], e[(2 + x) * nb + i], r);
-            }
-          } else if (el < nel && Lq) {
-            for (int k = slice; k < n; k += nsl) acc[u] = cadd(acc[u], psm[(size_t)k * NV * nb + nb + (el - ne)]);
+      for (int u = 0; u < NU; ++u)
+        if (hi[u] >= 0)
+          for (int k = hs; k < n; k += hsl) {
+            const double2 *e = psm + (size_t)k * esz;
+            const double2 wi = e[hi[u]], wj = e[hj[u]], f0 = e[nb + nat], f1 = e[nb + nat + 1];
+            const double2 r = make_double2(wi.x * wj.x + wi.y * wj.y, wi.y * wj.x - wi.x * wj.y);
+            acc[u][0].x += f0.x * r.x;
+            acc[u][0].y += f0.x * r.y;
+            acc[u][1].x += f0.y * r.x;
+            acc[u][1].y += f0.y * r.y;
+            acc[u][2].x += f1.x * r.x;
+            acc[u][2].y += f1.x * r.y;
+            acc[u][3].x += f1.y * r.x;
+            acc[u][3].y += f1.y * r.y;
           }
-        }
+#pragma unroll
+      for (int u = 0; u < NU; ++u) {
+        const int it = p0 + u * PL_THREADS;
+        if (ps < psl && it < np)
+          for (int k = ps; k < n; k += psl) {
+            const double2 *e = psm + (size_t)k * esz;
+            cfma(pacc[u], e[nb + it / nb], cconj(e[it % nb]));
+          }
+      }
     }
   }
-  // ---- the slices' sums in order; M_x and its transpose meet in shared memory
+  // ---- the slices' sums in order, into the first slice's places
   __syncthreads();
+  double2 *pp = psm + (size_t)hsl * 4 * nh;   // [psl][np], behind [hsl][4][nh]
 #pragma unroll
   for (int u = 0; u < NU; ++u) {
-    const int el = el0 + u * PL_THREADS;
-    if (work && el < nel) {
-      psm[(size_t)(slice * 4) * nel + el] = acc[u];
+    const int it = h0 + u * PL_THREADS, ip = p0 + u * PL_THREADS;
+    if (hi[u] >= 0)
 #pragma unroll
-      for (int x = 0; x < 3; ++x) psm[(size_t)(slice * 4 + 1 + x) * nel + el] = dacc[u][x];
-    }
+      for (int x = 0; x < 4; ++x) psm[(hs * 4 + x) * nh + it] = acc[u][x];
+    if (ps < psl && ip < np) pp[ps * np + ip] = pacc[u];
   }
   __syncthreads();
-  auto sum = [&](int c, int el) {
-    double2 t = psm[(size_t)c * nel + el];
-    for (int sl = 1; sl < nsl; ++sl) t = cadd(t, psm[(size_t)(sl * 4 + c) * nel + el]);
-    return t;
+  for (int t = tid; t < 4 * nh + np; t += PL_THREADS) {
+    double2 *o = t < 4 * nh ? psm + t : pp + (t - 4 * nh);
+    const int n = t < 4 * nh ? hsl : psl, step = t < 4 * nh ? 4 * nh : np;
+    double2 v = *o;
+    for (int sl = 1; sl < n; ++sl) v = cadd(v, o[sl * step]);
+    *o = v;
+  }
+  __syncthreads();
+  auto herm = [&](int x, int i, int j) {
+    const int hi_ = max(i, j), lo = min(i, j);
+    const double2 v = psm[x * nh + hi_ * (hi_ + 1) / 2 + lo];
+    return i >= j ? v : cconj(v);
   };
-  for (int el = tid; el < nel; el += PL_THREADS) {
-    if (el < ne) {
-      const int i = el % nb, j = el / nb;
-      const double mn = 1.0 / sqrt(P.masses[i / 3] * P.masses[j / 3]) * Ryd2amu;
-      if (Dq) {
-        double2 d = sum(0, el);
-        if (P.Da) d = cadd(d, P.Da[el]);
-        double2 &o = Dq[q * ldd + el];
-        o = cadd(o, cscale(d, P.fac * mn));
-      }
-      for (int x = 0; x < 3; ++x) {
-        double2 &o = dDq[q * ldd + x * ne + el];
-        o = cadd(o, cscale(cadd(sum(1 + x, el), cconj(sum(1 + x, j + nb * i))), P.fac * BOHR2NM * mn));
-      }
-    } else if (Lq) {
-      const double2 t = sum(0, el);
-      Lq[(size_t)q * nb + (el - ne)] = make_double2(P.fac * t.y, P.fac * t.x);   // i fac conj(t)
+  for (int el = tid; el < ne; el += PL_THREADS) {
+    const int i = el % nb, j = el / nb, a = i / 3, b = j / 3;
+    const double mn = 1.0 / sqrt(P.masses[a] * P.masses[b]) * Ryd2amu;
+    const double2 d0 = herm(0, i, j);
+    if (Dq) {
+      double2 &o = Dq[q * ldd + el];
+      o = cadd(o, cscale(P.Da ? cadd(d0, P.Da[el]) : d0, P.fac * mn));
+    }
+    const double2 pi = pp[a * nb + j], pj = cconj(pp[b * nb + i]);
+    for (int x = 0; x < 3; ++x) {
+      const double zi = P.born[x + 3 * (i % 3) + 9 * a], zj = P.born[x + 3 * (j % 3) + 9 * b];
+      const double rr = P.tau[3 * a + x] - P.tau[3 * b + x];
+      const double2 w = herm(1 + x, i, j);
+      const double2 d = make_double2(zi * pi.x + zj * pj.x - rr * d0.y - 2.0 * w.x,
+                                     zi * pi.y + zj * pj.y + rr * d0.x - 2.0 * w.y);
+      double2 &o = dDq[q * ldd + x * ne + el];
+      o = cadd(o, cscale(d, P.fac * BOHR2NM * mn));
     }
   }
 }
@@ -385,17 +405,17 @@ static void polar_dispatch(const PolarDev &P, const PolarBox &B, int nq, const i
 
 template <int NU>
 static void polar_vel_run(const PolarDev &P, const PolarBox &B, int nq, const int *qp, const int mesh[3],
-                          const double *qv, double2 *Dq, double2 *dDq, int64_t ldd, double2 *Lq, cudaStream_t st) {
+                          const double *qv, double2 *Dq, double2 *dDq, int64_t ldd, cudaStream_t st) {
   static std::once_flag once;
   std::call_once(once, [] {
-    cudaFuncSetAttribute(k_polar_vel<NU>, cudaFuncAttributeMaxDynamicSharedMemorySize, 2 * PL_SMEM);
+    cudaFuncSetAttribute(k_polar_vel<NU>, cudaFuncAttributeMaxDynamicSharedMemorySize, PL_SMEM);
   });
-  const int nel = P.nb * P.nb + P.nb;
-  const size_t entry = (size_t)PV_VECTORS * P.nb * sizeof(double2);
+  const int nh = P.nb * (P.nb + 1) / 2, np = P.nat * P.nb;
+  const size_t entry = (size_t)pv_entry(P.nat) * sizeof(double2);
   const int nent = pl_entries(entry);
-  const size_t sums = (size_t)(NU == 1 ? PL_THREADS / nel : 1) * 4 * nel * sizeof(double2);
+  const size_t sums = sizeof(double2) * ((NU == 1 ? PL_THREADS / nh : 1) * 4 * nh + (NU == 1 ? PL_THREADS / np : 1) * np);
   k_polar_vel<NU><<<nq, PL_THREADS, std::max(nent * entry, sums), st>>>(
-      P, B.G, B.Gf, B.M, nq, qp, mesh ? mesh[0] : 1, mesh ? mesh[1] : 1, mesh ? mesh[2] : 1, qv, nent, Dq, dDq, ldd, Lq);
+      P, B.G, B.Gf, B.M, nq, qp, mesh ? mesh[0] : 1, mesh ? mesh[1] : 1, mesh ? mesh[2] : 1, qv, nent, Dq, dDq, ldd);
 }
 
 void launch_polar_q(const PolarDev &P, int nq, const int *qp, const int mesh[3], const double *qv, double2 *Dq,
@@ -407,10 +427,9 @@ void launch_polar_q(const PolarDev &P, int nq, const int *qp, const int mesh[3],
     polar_dispatch<false>(P, B, nq, qp, mesh, qv, Dq, ldd, Lq, st);
     return;
   }
-  const int nel = P.nb * P.nb + P.nb;
-  if (nel <= PL_THREADS) polar_vel_run<1>(P, B, nq, qp, mesh, qv, Dq, dDq, ldd, Lq, st);
-  else if (nel <= 3 * PL_THREADS) polar_vel_run<3>(P, B, nq, qp, mesh, qv, Dq, dDq, ldd, Lq, st);
-  else polar_vel_run<9>(P, B, nq, qp, mesh, qv, Dq, dDq, ldd, Lq, st);
+  if (P.nb * (P.nb + 1) / 2 <= PL_THREADS) polar_vel_run<1>(P, B, nq, qp, mesh, qv, Dq, dDq, ldd, st);
+  else polar_vel_run<5>(P, B, nq, qp, mesh, qv, Dq, dDq, ldd, st);
+  if (Lq) polar_dispatch<false>(P, B, nq, qp, mesh, qv, nullptr, ldd, Lq, st);
 }
 
 void launch_polar_da(const PolarDev &P, double2 *Da, cudaStream_t st) {
