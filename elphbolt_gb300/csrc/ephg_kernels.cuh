@@ -54,7 +54,7 @@ void launch_row_map(int N, int nrows, const int *rows, int *rowmap, cudaStream_t
 void launch_zgemm(int M, int N, int K, const double2 *A, int64_t lda, const double2 *B,
                   int64_t ldb, double2 *C, int64_t ldc, cudaStream_t st);
 
-// ---- Hermitian eigensolver (batched, one warp per matrix, n <= 32) ----
+// ---- Hermitian eigensolver (batched, n <= 32) ----
 // A: batch matrices (n,n) column-major at stride n*n, upper triangle forced
 // Hermitian as in wannier.f90:481-486.  w: (batch, n) ascending;
 // V: (batch, n, n) column-major, columns = eigenvectors.
