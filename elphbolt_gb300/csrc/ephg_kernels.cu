@@ -7,7 +7,9 @@
 #include <algorithm>
 #include <cstdio>
 #include <mutex>
+#include <vector>
 
+#include "../../include/ephg_debug.h"
 #include "ephg_kernels.cuh"
 
 namespace ephg {
@@ -1526,8 +1528,6 @@ void launch_mode_tab(int n, const double *om, const double *bose, double T, doub
 // FP64 rate for its ~850 instructions a pair); one thread per (k', state) with a loop
 // over the bands took 15.1 ms.  Tetrahedra, 10x12x11 (1.8 M pairs): 3.1 ms + 0.32 ms for
 // the tables; with every simplex's formula at every vertex 511 ms.
-constexpr int EPF_THREADS = 128;
-
 template <bool F32>
 __device__ __forceinline__ double2 epf_load(const FinalIn &c, int64_t off) {
   if (F32) return make_double2((double)c.re[off], (double)c.im[off]);
@@ -1537,7 +1537,8 @@ __device__ __forceinline__ double2 epf_load(const FinalIn &c, int64_t off) {
 template <bool F32, bool SIMPLEX, bool PH>
 __global__ void __launch_bounds__(EPF_THREADS) k_epilogue_final(int j0, int ns, FinalIn c, RateParams rp, EpiData d,
                                                                 double *partial, int nblk) {
-  const int jl = blockIdx.x * EPF_THREADS + threadIdx.x;
+  const int2 blk = epf_block(blockIdx.x, ns);
+  const int jl = blk.x * EPF_THREADS + threadIdx.x;
   if (jl >= ns) return;
   const int j = j0 + jl;
   const int nw = rp.nw, nb = rp.nb;
@@ -1553,8 +1554,8 @@ __global__ void __launch_bounds__(EPF_THREADS) k_epilogue_final(int j0, int ns, 
   const int a1 = p % rp.mesh[0], a2 = (p / rp.mesh[0]) % rp.mesh[1], a3 = p / (rp.mesh[0] * rp.mesh[1]);
   const double2 *Uk = d.U + ((size_t)p * nw + m) * nw;
   double sum = 0.0, comp = 0.0;
-  const int fe = min(d.nin, (int)(blockIdx.y + 1) * EPF_F);
-  for (int f = blockIdx.y * EPF_F; f < fe; ++f) {
+  const int fe = min(d.nin, (blk.y + 1) * EPF_F);
+  for (int f = blk.y * EPF_F; f < fe; ++f) {
     const int2 fs = d.fin[f];
     const int pp = d.widx[fs.x];
     const double eps = d.ens[(size_t)pp * nw + fs.y];
@@ -1625,14 +1626,14 @@ __global__ void __launch_bounds__(EPF_THREADS) k_epilogue_final(int j0, int ns, 
     comp += (fabs(sum) >= fabs(acc)) ? (sum - t) + acc : (acc - t) + sum;
     sum = t;
   }
-  partial[(size_t)j * nblk + blockIdx.y] = sum + comp;
+  partial[(size_t)j * nblk + blk.y] = sum + comp;
 }
 
 void launch_epilogue_final(int j0, int j1, const FinalIn &c, const RateParams &rp, const EpiData &d, double *partial,
                            int nblk, cudaStream_t st) {
   const int ns = j1 - j0;
   if (ns <= 0 || d.nin <= 0) return;
-  dim3 grid((ns + EPF_THREADS - 1) / EPF_THREADS, (d.nin + EPF_F - 1) / EPF_F);
+  const unsigned grid = (unsigned)epf_grid(ns, d.nin);
   const bool ph = d.phr || d.yv, simplex = rp.delta_kind != 0;
   auto go = [&](auto k) { k<<<grid, EPF_THREADS, 0, st>>>(j0, ns, c, rp, d, partial, nblk); };
   if (c.z) {
@@ -1779,3 +1780,20 @@ int launch_degenerate_average(double *g2, int64_t per, int nin, const int *st_co
 }
 
 }  // namespace ephg
+
+extern "C" int ephg_debug_epilogue_grid(int nstates, int nin, int64_t *grid) {
+  using namespace ephg;
+  if (nstates <= 0 || nin <= 0 || !grid) return EPHG_ERR_ARG;
+  grid[0] = epf_grid(nstates, nin);
+  grid[1] = grid[2] = 1;
+  const int64_t ns = (nstates + EPF_THREADS - 1) / EPF_THREADS, nf = epf_blocks(nin);
+  std::vector<bool> seen((size_t)(ns * nf));
+  for (int64_t b = 0; b < grid[0]; ++b) {
+    const int2 p = epf_block((unsigned)b, nstates);
+    if (p.x < 0 || p.x >= ns || p.y < 0 || p.y >= nf || seen[(size_t)(p.x + ns * p.y)]) return EPHG_ERR_INDEX;
+    seen[(size_t)(p.x + ns * p.y)] = true;
+  }
+  for (bool x : seen)
+    if (!x) return EPHG_ERR_INDEX;
+  return EPHG_OK;
+}

@@ -207,8 +207,16 @@ void launch_mode_tab(int n, const double *om, const double *bose, double T, doub
 // FP64 epilogue over the states [j0, j1): the Rp sums G(x = n' + nw s') of (window row ip,
 // state j) at ip ldc + x xs + (j - j0) js, in FP64 (z) or as FP32 planes (re, im).  Rate
 // partials [j][block of EPF_F final states].
-constexpr int EPF_F = 16;
+constexpr int EPF_F = 16, EPF_THREADS = 128;
 inline int epf_blocks(int nin) { return (nin + EPF_F - 1) / EPF_F; }
+// Its grid is one-dimensional, blocks of EPF_THREADS states fastest: a mesh of 2^24 points has
+// up to 3.3e7 blocks of final states, which the other dimensions (65,535) do not hold.
+inline int64_t epf_grid(int ns, int nin) { return (int64_t)((ns + EPF_THREADS - 1) / EPF_THREADS) * epf_blocks(nin); }
+// (block of states, block of final states) of block b
+__host__ __device__ inline int2 epf_block(unsigned b, int ns) {
+  const unsigned n = (unsigned)(ns + EPF_THREADS - 1) / EPF_THREADS;
+  return make_int2((int)(b % n), (int)(b / n));
+}
 struct FinalIn {
   const double2 *z = nullptr;
   const float *re = nullptr, *im = nullptr;
