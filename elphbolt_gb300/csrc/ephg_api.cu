@@ -232,8 +232,7 @@ int ephg_destroy(ephg_handle *h) {
   if (!h) return EPHG_OK;
   void *ptrs[] = {h->Rk, h->Rq, h->Rg, h->degk, h->degq, h->degg, h->Hext, h->Hbox, h->Dbox, h->graw, h->G64,
                   h->masses, h->Dcell, h->RD, h->err, h->kposk, h->kposq, h->polar_G, h->polar_Gcell,
-                  h->polar_born, h->polar_tau, h->polar_Da, h->polar_Gf, h->cellk_tab, h->cellq_tab, h->rdegk, h->exp_H.e, h->exp_G.e, h->exp_raw.e,
-                  h->exp_D.e};
+                  h->polar_born, h->polar_tau, h->polar_Da, h->polar_Gf, h->cellk_tab, h->cellq_tab, h->rdegk, h->exp_H, h->exp_G, h->exp_raw, h->exp_D};
   // stream-ordered frees back to the library pool, which keeps the memory
   // mapped for the next handle
   for (void *p : ptrs)
@@ -483,6 +482,26 @@ int ephg_create(const ephg_wannier_desc *d, ephg_handle **out) {
     if ((rc = upload(&h->kposk, pk.data(), pk.size(), h->st, &h->resident_bytes)) || (rc = upload(&h->kposq, pq.data(), pq.size(), h->st, &h->resident_bytes)))
       return bail(rc);
   }
+  // column exponents of the operands that launch_xgemm multiplies by: part of the resident data, so
+  // that no request allocates beside its workspace (four bytes a column; one pass over each operand)
+  {
+    const struct {
+      int **e;
+      int64_t n;
+      int K;
+      const double2 *B;
+    } ops[] = {{&h->exp_H, 4 * (int64_t)nw * nw, nwsk, h->Hext},
+               {&h->exp_G, h->Nn, nwsk, h->G64},
+               {&h->exp_raw, (int64_t)nw * nw * nb * nwsk, nwsq, h->graw},
+               {&h->exp_D, 4 * (int64_t)nb * nb, h->nD, h->Dcell}};
+    for (const auto &o : ops) {
+      if (o.n <= 0) continue;
+      if (pool_alloc((void **)o.e, (size_t)o.n * sizeof(int), h->st) != cudaSuccess)
+        return bail(fail(EPHG_ERR_NOMEM, "device allocation of column exponents, %lld bytes", (long long)(4 * o.n)));
+      h->resident_bytes += o.n * (int64_t)sizeof(int);
+      launch_colexp(o.n, o.K, o.B, *o.e, h->st);
+    }
+  }
   if (pool_alloc((void **)&h->err, sizeof(int), h->st) != cudaSuccess)
     return bail(fail(EPHG_ERR_CUDA, "device allocation of the error word"));
   if (cudaMemsetAsync(h->err, 0, sizeof(int), h->st) != cudaSuccess) return bail(fail(EPHG_ERR_CUDA, "memset"));
@@ -712,10 +731,7 @@ int ephg_el_wann(ephg_handle *h, int64_t nk, const double *kvecs, double *energi
   }
   CK(cudaMemcpyAsync(kv, kvecs, (size_t)nk * 3 * sizeof(double), cudaMemcpyHostToDevice, h->st));
   launch_phase_cells((int)nk, kv, nk, nullptr, nwsk, h->Rk, h->degk, h->hlo, h->hext, P, nwsk, h->st);
-  const int *ce;
-  if ((rc = resident_colexp(h->exp_H, 1, 4 * (int64_t)nn, nwsk, h->Hext, 0, &h->resident_bytes, h->st, &ce)))
-    return fail(rc, "el_wann: column exponents");
-  if ((rc = launch_xgemm(h->ws, (int)nk, ncol, nwsk, P, nwsk, h->Hext, 4 * (int64_t)nn, ce, C, ncol, h->err, h->st)))
+  if ((rc = launch_xgemm(h->ws, (int)nk, ncol, nwsk, P, nwsk, h->Hext, 4 * (int64_t)nn, h->exp_H, C, ncol, h->err, h->st)))
     return WSFAIL(rc);
   launch_heig((int)nk, nw, C, ncol, w, V, h->err, h->st);
   launch_el_post((int)nk, nw, w, V, C, ncol, with_vel, sc, ens, with_vel ? vel : nullptr,
@@ -751,15 +767,12 @@ int ephg_ph_wann(ephg_handle *h, int64_t nq, const double *qvecs, double *energi
       (rc = wsget(h->ws, "ph_vel", with_vel ? (size_t)nq * nb * 3 : 1, &vel)) ||
       (rc = wsget(h->ws, "ph_ev", evecs ? (size_t)nq * nn : 1, &ev)))
     return WSFAIL(rc);
-  const int *ce;
-  if ((rc = resident_colexp(h->exp_D, 1, 4 * (int64_t)nn, h->nD, h->Dcell, 0, &h->resident_bytes, h->st, &ce)))
-    return fail(rc, "ph_wann: column exponents");
   CK(cudaMemcpyAsync(qv, qvecs, (size_t)nq * 3 * sizeof(double), cudaMemcpyHostToDevice, h->st));
   for (int64_t q0 = 0; q0 < nq; q0 += qb) {
     const int n = (int)std::min(qb, nq - q0);
     launch_phase_cells(n, qv + q0, nq, nullptr, h->nD, h->RD, nullptr, h->dlo, h->dext, P, h->nD, h->st);
-    if ((rc = launch_xgemm(h->ws, n, ncol, h->nD, P, h->nD, h->Dcell, 4 * (int64_t)nn, ce, Dq + q0 * ncol, ncol, h->err,
-                           h->st)))
+    if ((rc = launch_xgemm(h->ws, n, ncol, h->nD, P, h->nD, h->Dcell, 4 * (int64_t)nn, h->exp_D, Dq + q0 * ncol, ncol,
+                           h->err, h->st)))
       return WSFAIL(rc);
     h->launches += 3;
   }
@@ -790,9 +803,6 @@ int ephg_gkRp(ephg_handle *h, int64_t nk, const double *kvecs, double *gmixed) {
   if ((rc = wsget(h->ws, "gk_kv", (size_t)chunk * 3, &kv)) || (rc = wsget(h->ws, "gk_P", (size_t)chunk * nwsk, &P)) ||
       (rc = wsget(h->ws, "gk_C", (size_t)chunk * h->Nn, &C)))
     return WSFAIL(rc);
-  const int *ce;
-  if ((rc = resident_colexp(h->exp_G, 1, h->Nn, nwsk, h->G64, 0, &h->resident_bytes, h->st, &ce)))
-    return fail(rc, "gkRp: column exponents");
   std::vector<double> kc((size_t)chunk * 3);
   for (int64_t k0 = 0; k0 < nk; k0 += chunk) {
     int64_t n = std::min(chunk, nk - k0);
@@ -800,7 +810,7 @@ int ephg_gkRp(ephg_handle *h, int64_t nk, const double *kvecs, double *gmixed) {
       for (int64_t i = 0; i < n; ++i) kc[i + n * c] = kvecs[(k0 + i) + nk * c];
     CK(cudaMemcpyAsync(kv, kc.data(), (size_t)n * 3 * sizeof(double), cudaMemcpyHostToDevice, h->st));
     launch_phase_cells((int)n, kv, n, nullptr, nwsk, h->Rk, h->degk, h->hlo, h->hext, P, nwsk, h->st);
-    if ((rc = launch_xgemm(h->ws, (int)n, h->Nn, nwsk, P, nwsk, h->G64, h->Nn, ce, C, h->Nn, h->err, h->st)))
+    if ((rc = launch_xgemm(h->ws, (int)n, h->Nn, nwsk, P, nwsk, h->G64, h->Nn, h->exp_G, C, h->Nn, h->err, h->st)))
       return WSFAIL(rc);
     h->launches += 3;
     CKL();
@@ -824,9 +834,6 @@ int ephg_gReq(ephg_handle *h, int64_t nq, const double *qvecs, double *gmixed) {
   if ((rc = wsget(h->ws, "gq_qv", (size_t)chunk * 3, &qv)) || (rc = wsget(h->ws, "gq_P", (size_t)chunk * nwsg, &P)) ||
       (rc = wsget(h->ws, "gq_C", (size_t)chunk * per, &C)) || (rc = wsget(h->ws, "gq_O", (size_t)chunk * per, &O)))
     return WSFAIL(rc);
-  const int *ce;
-  if ((rc = resident_colexp(h->exp_raw, 1, per, nwsg, h->graw, 0, &h->resident_bytes, h->st, &ce)))
-    return fail(rc, "gReq: column exponents");
   std::vector<double> qc((size_t)chunk * 3);
   for (int64_t q0 = 0; q0 < nq; q0 += chunk) {
     int64_t n = std::min(chunk, nq - q0);
@@ -835,7 +842,7 @@ int ephg_gReq(ephg_handle *h, int64_t nq, const double *qvecs, double *gmixed) {
     CK(cudaMemcpyAsync(qv, qc.data(), (size_t)n * 3 * sizeof(double), cudaMemcpyHostToDevice, h->st));
     // sum_Rp e^{2 pi i q.Rp}/gwsdeg * g(i,j,Re,s,Rp): rows of the raw array are Rp
     launch_phase_cells((int)n, qv, n, nullptr, nwsg, h->Rg, h->degg, h->qlo, h->qext, P, nwsg, h->st);
-    if ((rc = launch_xgemm(h->ws, (int)n, per, nwsg, P, nwsg, h->graw, per, ce, C, per, h->err, h->st)))
+    if ((rc = launch_xgemm(h->ws, (int)n, per, nwsg, P, nwsg, h->graw, per, h->exp_raw, C, per, h->err, h->st)))
       return WSFAIL(rc);
     launch_permute_greq((int)n, nw, nb, nwsk, C, O, h->st);
     h->launches += 4;
@@ -1369,14 +1376,11 @@ int ephg::el_rates_view(ephg_handle *h, const ExecView &x, const ephg_rate_reque
         (*x.launches) += 4;
       }
     } else {
-      const int *ce;
-      if ((rc = resident_colexp(h->exp_G, 1, Nn, nwsk, h->G64, 0, &h->resident_bytes, st, &ce)))
-        return fail(rc, "el_rates: column exponents");
       for (int64_t i0 = 0; i0 < nA; i0 += kc) {
         const int n = (int)std::min<int64_t>(kc, nA - i0);
         launch_phase_mesh(n, arow + i0, mesh, L, nwsk, h->Rk, h->degk, 0, roots, Pk, nwsk, st);
         (*x.ta).begin(st);
-        if ((rc = launch_xgemm(*x.ws, n, Nn, nwsk, Pk, nwsk, h->G64, Nn, ce, gk, Nn, x.err, st))) return WSFAILX(rc);
+        if ((rc = launch_xgemm(*x.ws, n, Nn, nwsk, Pk, nwsk, h->G64, Nn, h->exp_G, gk, Nn, x.err, st))) return WSFAILX(rc);
         (*x.ta).end(st);
         launch_rotate_states_fp64(first_state[i0], first_state[i0 + n], (int)i0, st_code, nw, nb, nwsq, 0, nper, arow, V,
                                   gk, Nn, phk, B, ldb, (int)sc, nst, st);

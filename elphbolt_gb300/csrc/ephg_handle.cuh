@@ -32,8 +32,8 @@ struct ephg_handle {
   ephg::CellTab cellk, cellq;
   int *cellk_tab = nullptr, *cellq_tab = nullptr;
   double *rdegk = nullptr;
-  // column exponents of the resident right-hand sides of launch_xgemm (lazy): Hext, G64, graw, Dcell
-  ephg::ColExp exp_H, exp_G, exp_raw, exp_D;
+  // column exponents of the resident right-hand sides of launch_xgemm: Hext, G64, graw, Dcell
+  int *exp_H = nullptr, *exp_G = nullptr, *exp_raw = nullptr, *exp_D = nullptr;
   double2 *graw = nullptr;   // epmatwp order (i,j,Re,s,Rp)
   double2 *G64 = nullptr;    // stage-A matrix [Re][Nn]
   double *masses = nullptr;

@@ -446,22 +446,8 @@ int xgemm_colexp(Workspace &ws, int64_t nrhs, int64_t N, int K, const double2 *B
   return EPHG_OK;
 }
 
-int resident_colexp(ColExp &x, int64_t nrhs, int64_t N, int K, const double2 *B, int64_t bstride, int64_t *bytes,
-                    cudaStream_t st, const int **out) {
-  std::lock_guard<std::mutex> lk(x.mu);
-  if (!x.e) {
-    int *e = nullptr;
-    if (pool_alloc((void **)&e, (size_t)(nrhs * N) * sizeof(int), st) != cudaSuccess) return EPHG_ERR_NOMEM;
-    col_exp(nrhs, N, K, B, N, bstride, e, st);
-    if (cudaGetLastError() != cudaSuccess || cudaStreamSynchronize(st) != cudaSuccess) {   // other streams may read it
-      cudaFreeAsync(e, st);
-      return EPHG_ERR_CUDA;
-    }
-    x.e = e;
-    if (bytes) *bytes += nrhs * N * (int64_t)sizeof(int);
-  }
-  *out = x.e;
-  return EPHG_OK;
+void launch_colexp(int64_t N, int K, const double2 *B, int *e, cudaStream_t st) {
+  col_exp(1, N, K, B, N, 0, e, st);
 }
 
 static int xg_sms() {

@@ -1,17 +1,8 @@
 // ephg_xgemm.cuh - FP64 complex products on the tensor cores by exact splitting.
 #pragma once
-#include <mutex>
-
 #include "ephg_ws.cuh"
 
 namespace ephg {
-
-// Column exponents of a right-hand side kept with its owner (the handle's resident
-// operands): built on first use, then read by every product with it.
-struct ColExp {
-  int *e = nullptr;
-  std::mutex mu;
-};
 
 // C[M][N] = A[M][K] B[K][N], complex FP64, row-major, |A| <= 1 (phases).  cexp: B's column
 // exponents (nullable: formed per call in ws).  err: device error word of the bounded waits.
@@ -27,9 +18,7 @@ int xgemm_colexp(Workspace &ws, int64_t nrhs, int64_t N, int K, const double2 *B
 int launch_xgemm_chunks(Workspace &ws, const int4 *chunks, int nchunks, int rows, int64_t N, int K, const double2 *A,
                         int64_t lda, const double2 *B, int64_t ldb, int64_t bstride, const int *cexp, double2 *C, int64_t ldc,
                         int *err, cudaStream_t st);
-// The exponents of a resident operand (nrhs right-hand sides B[K][N] at stride N, bstride apart), built once (allocated from the library pool on st
-// and complete when this returns); *bytes grows by what was allocated.
-int resident_colexp(ColExp &x, int64_t nrhs, int64_t N, int K, const double2 *B, int64_t bstride, int64_t *bytes,
-                    cudaStream_t st, const int **out);
+// The exponents of an operand B[K][N] that its owner keeps (into e, N values), in stream order.
+void launch_colexp(int64_t N, int K, const double2 *B, int *e, cudaStream_t st);
 
 }  // namespace ephg
