@@ -875,21 +875,30 @@ int ephg_g2(ephg_handle *h, int64_t wannspace, int64_t nv, const double *kvecs,
   for (int64_t b = 0; b < ngm; ++b) at[b + 1] += at[b];
   std::vector<int> perm(nv);
   for (int64_t v = 0; v < nv; ++v) perm[at[gm_index[v] - 1]++] = (int)v;
-  const int64_t most = std::max<int64_t>(XG_CHUNK, ((int64_t)1 << 28) / (16 * per));   // rows per piece
   std::vector<int4> chunks;
-  std::vector<std::pair<int64_t, int64_t>> piece;   // first row, first chunk
+  int most = 1;   // rows of the longest chunk
   for (int64_t r = 0; r < nv;) {
     const int64_t b = gm_index[perm[r]];
     int64_t e = r + 1;
     while (e < nv && e - r < XG_CHUNK && gm_index[perm[e]] == b) ++e;
-    if (piece.empty() || e - piece.back().first > most || (int64_t)chunks.size() - piece.back().second >= 1024)
-      piece.push_back({r, (int64_t)chunks.size()});
-    chunks.push_back(make_int4((int)(r - piece.back().first), (int)(e - r), (int)(b - 1), 0));
+    chunks.push_back(make_int4((int)r, (int)(e - r), (int)(b - 1), 0));
+    most = std::max(most, (int)(e - r));
     r = e;
   }
-  piece.push_back({nv, (int64_t)chunks.size()});
+  // rows of a piece: phases (nws values) and cell sums (per); chunks: digits
+  const int64_t bound = (int64_t)1 << 28;
+  const int64_t row_most = bound / (16 * std::max<int64_t>(per, nws));
+  const int64_t chunk_most = std::min<int64_t>(XG_MAXCHUNKS, bound / xgemm_chunk_bytes(most, nws));
+  std::vector<std::pair<int64_t, int64_t>> piece;   // first row, first chunk
   int64_t rows = 0;
-  for (size_t p = 0; p + 1 < piece.size(); ++p) rows = std::max(rows, piece[p + 1].first - piece[p].first);
+  for (size_t c = 0; c < chunks.size(); ++c) {
+    const int64_t r = chunks[c].x, e = r + chunks[c].y;
+    if (piece.empty() || e - piece.back().first > row_most || (int64_t)c - piece.back().second >= chunk_most)
+      piece.push_back({r, (int64_t)c});
+    chunks[c].x = (int)(r - piece.back().first);
+    rows = std::max(rows, e - piece.back().first);
+  }
+  piece.push_back({nv, (int64_t)chunks.size()});
   double *qv, *en, *out;
   double2 *ek, *ekp, *eq, *gm, *P, *G;
   int *pd;
@@ -931,8 +940,8 @@ int ephg_g2(ephg_handle *h, int64_t wannspace, int64_t nv, const double *kvecs,
     const int n = (int)(piece[p + 1].first - r0);
     launch_phase_cells(n, qv, nv, pd + r0, nws, R, deg, wannspace == EPHG_WANNSPACE_PH ? h->qlo : h->hlo,
                        wannspace == EPHG_WANNSPACE_PH ? h->qext : h->hext, P, nws, h->st);
-    if ((rc = launch_xgemm_chunks(h->ws, cd + c0, (int)(piece[p + 1].second - c0), n, per, nws, P, nws, gm, per, gstride,
-                                  ce, G, per, h->err, h->st)))
+    if ((rc = launch_xgemm_chunks(h->ws, cd + c0, (int)(piece[p + 1].second - c0), most, n, per, nws, P, nws, gm, per,
+                                  gstride, ce, G, per, h->err, h->st)))
       return WSFAIL(rc);
     launch_g2_vertices(n, pd + r0, nv, nw, nb, G, ek, ekp, eq, en, h->masses, Lv, out, h->st);
     h->launches += 5;

@@ -465,12 +465,19 @@ static void xg_run(const XgArgs &g, cudaStream_t st) {
   k_xgemm<W><<<(unsigned)std::min<int64_t>(g.units, xg_sms()), XG_THREADS, XG_SMEM, st>>>(g);
 }
 
+// MMA columns of a level for chunks of up to `rows` rows
+static int xg_width(int rows) { return (2 * rows + 15) / 16 * 16; }
+
+int64_t xgemm_chunk_bytes(int most, int K) {
+  return (int64_t)((K + XG_CELLS - 1) / XG_CELLS) * XG_D * 64 * xg_width(most);
+}
+
 // one launch over mch chunks (dig sized for them)
 static void xg_launch(XgArgs &g, const double2 *A, int64_t lda, uint8_t *dig, int *bad, cudaStream_t st) {
   g.dig = dig;
   g.bad = bad;
   g.units = (g.N + XG_ROWS - 1) / XG_ROWS * g.mch;
-  const int W = (2 * g.rpc + 15) / 16 * 16;   // MMA columns of a level
+  const int W = xg_width(g.rpc);
   k_xg_phases<<<dim3(g.kch, g.mch), 4 * W, 0, st>>>(g.chunks, g.M, g.rpc, W, g.K, g.kch, A, lda, dig, bad);
   W == 16 ? xg_run<16>(g, st) : W == 32 ? xg_run<32>(g, st) : W == 48 ? xg_run<48>(g, st) : xg_run<64>(g, st);
 }
@@ -513,7 +520,7 @@ int launch_xgemm(Workspace &ws, int M, int64_t N, int K, const double2 *A, int64
   return EPHG_OK;
 }
 
-int launch_xgemm_chunks(Workspace &ws, const int4 *chunks, int nchunks, int rows, int64_t N, int K, const double2 *A,
+int launch_xgemm_chunks(Workspace &ws, const int4 *chunks, int nchunks, int most, int rows, int64_t N, int K, const double2 *A,
                         int64_t lda, const double2 *B, int64_t ldb, int64_t bstride, const int *cexp, double2 *C,
                         int64_t ldc, int *err, cudaStream_t st) {
   if (nchunks <= 0) return EPHG_OK;
@@ -521,7 +528,7 @@ int launch_xgemm_chunks(Workspace &ws, const int4 *chunks, int nchunks, int rows
   uint8_t *dig;
   int *bad;
   int rc;
-  if ((rc = wsget(ws, "x_dig", (size_t)nchunks * kch * XG_STAGE_A, &dig)) ||
+  if ((rc = wsget(ws, "x_dig", (size_t)(nchunks * xgemm_chunk_bytes(most, K)), &dig)) ||
       (rc = wsget(ws, "x_bad", (size_t)rows, &bad)))
     return rc;
   cudaMemsetAsync(bad, 0, (size_t)rows * sizeof(int), st);
@@ -530,7 +537,7 @@ int launch_xgemm_chunks(Workspace &ws, const int4 *chunks, int nchunks, int rows
   g.K = K;
   g.kch = kch;
   g.mch = nchunks;
-  g.rpc = std::min(rows, XG_CHUNK);
+  g.rpc = most;
   g.N = N;
   g.ldb = ldb;
   g.ldc = ldc;

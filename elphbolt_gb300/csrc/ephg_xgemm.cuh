@@ -10,12 +10,14 @@ namespace ephg {
 int launch_xgemm(Workspace &ws, int M, int64_t N, int K, const double2 *A, int64_t lda, const double2 *B, int64_t ldb,
                  const int *cexp, double2 *C, int64_t ldc, int *err, cudaStream_t st);
 // Rows of A against several right-hand sides in one launch: chunk c (device) is (first row, rows
-// <= XG_CHUNK, right-hand side); right-hand side b is B + b bstride, [K][N] at row stride ldb.
-// cexp: the exponents of xgemm_colexp, ldb per right-hand side.
-constexpr int XG_CHUNK = 32;
+// <= most <= XG_CHUNK, right-hand side); right-hand side b is B + b bstride, [K][N] at row stride ldb.
+// cexp: the exponents of xgemm_colexp, ldb per right-hand side.  The phases' digits take
+// xgemm_chunk_bytes per chunk; at most XG_MAXCHUNKS chunks.
+constexpr int XG_CHUNK = 32, XG_MAXCHUNKS = 32768;
+int64_t xgemm_chunk_bytes(int most, int K);
 int xgemm_colexp(Workspace &ws, int64_t nrhs, int64_t N, int K, const double2 *B, int64_t bstride, const int **cexp,
                  cudaStream_t st);
-int launch_xgemm_chunks(Workspace &ws, const int4 *chunks, int nchunks, int rows, int64_t N, int K, const double2 *A,
+int launch_xgemm_chunks(Workspace &ws, const int4 *chunks, int nchunks, int most, int rows, int64_t N, int K, const double2 *A,
                         int64_t lda, const double2 *B, int64_t ldb, int64_t bstride, const int *cexp, double2 *C, int64_t ldc,
                         int *err, cudaStream_t st);
 // The exponents of an operand B[K][N] that its owner keeps (into e, N values), in stream order.
