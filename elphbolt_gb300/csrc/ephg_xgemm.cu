@@ -12,10 +12,13 @@
 //
 //   sum_k a_k b_k = sum_l 2^(-7 l - 12) S_l,   S_l = sum over i + j = l, k of integers |d| <= 64
 //
-// Levels have an accumulator each (7 and 8 share one where nine do not fit TMEM); |S_l| <= (l + 1) 4096 K stays within 2^24
+// Levels have an accumulator each, 7 and 8 one together (nine of the widest chunk do not
+// fit TMEM; every chunk width takes the same eight, so that a row's result does not depend
+// on how many rows share its call); |S_l| <= (l + 1) 4096 K stays within 2^24
 // for the XG_KGROUP positions summed at a time for l <= 5; above that (2^-54 of the
 // result) only for sums not of one sign throughout, and an FP32 rounding there no
-// longer counts.  Products beyond level 8 (2^-63) are left out.  The result is the
+// longer counts.  Products beyond level 8 (2^-63), and the tall operand's first digit with
+// the phases' last (2^-62 of one phase), are left out.  The result is the
 // exact sum of the products to ~2^-60 of the largest term, rounded once: its error is at or below that of the FP64
 // multiply-adds it replaces (g(Re,q), 279 cells, against sums of the same phases in
 // extended precision: 5.5e-17 relative; the multiply-adds 7.6e-16).
@@ -30,7 +33,7 @@
 // the columns, each once per chunk of phase rows) and write the nine BF16 planes of
 // a stage in the swizzled layout the MMA reads; HBM sees the FP64 matrix only.
 // The phases' digits are formed once per call and arrive by bulk copies.  Two
-// stages of 104 KB; 45 digit products per stage, the tensor core is the bound
+// stages of 104 KB; 44 digit products per stage, the tensor core is the bound
 // (about one cycle a column at these widths), the splitting runs beside it.
 //
 // Measured: g(k,Rp) at 25 k, nw 8, nb 6, 279 cells: 0.29 ms (6.70 as FP64 multiply-adds);
@@ -51,18 +54,17 @@ namespace ephg {
 
 using namespace tc;
 
-constexpr int XG_D = 9;                                // digits
+constexpr int XG_D = 9, XG_DA = XG_D - 1;              // digits; the phases' last one meets none (below)
 constexpr int XG_ROWS = 128, XG_M = XG_CHUNK;          // tile columns of B; phase rows of a chunk
 constexpr int XG_W = 2 * XG_M;                         // most MMA columns of a level
 constexpr int XG_CELLS = 16, XG_KV = 2 * XG_CELLS;     // cells and K values per stage
 constexpr int XG_KGROUP = 320 / XG_CELLS;              // stages per accumulation: 640 K values
 constexpr int XG_PLANE_B = XG_ROWS * XG_KV * 2;        // 8 KB per digit
 constexpr int XG_PLANE_A = XG_W * XG_KV * 2;           // at most 4 KB per digit
-constexpr int XG_STAGE_B = XG_D * XG_PLANE_B, XG_STAGE_A = XG_D * XG_PLANE_A;
+constexpr int XG_STAGE_B = XG_D * XG_PLANE_B, XG_STAGE_A = XG_DA * XG_PLANE_A;
 constexpr int XG_STAGE = (XG_STAGE_B + XG_STAGE_A + 1023) / 1024 * 1024;
-// accumulators of a level's W columns: level 8 shares the last of eight where nine do not fit TMEM
-__host__ __device__ constexpr int xg_levels(int W) { return XG_D * W <= 512 ? XG_D : XG_D - 1; }
-static_assert(xg_levels(XG_W) * XG_W <= 512, "the levels' accumulators fit TMEM");
+constexpr int XG_LEVELS = XG_D - 1;                    // accumulators of W columns; level 8 shares the last
+static_assert(XG_LEVELS * XG_W <= 512, "the levels' accumulators fit TMEM");
 constexpr int XG_STAGES = 2;
 constexpr int XG_SMEM = XG_STAGES * XG_STAGE + 1024 + 256;
 constexpr int XG_CONV = 512, XG_EPI = 256;             // converter and epilogue threads
@@ -97,12 +99,13 @@ __device__ __forceinline__ uint32_t xg_digit2(uint64_t a, uint64_t b) {
   return *reinterpret_cast<uint32_t *>(&r);
 }
 
-template <int I>
+// the planes of digits I .. D - 1
+template <int D, int I = 0>
 __device__ __forceinline__ void xg_store(uint8_t *p, int plane, const uint64_t *v) {
-  if constexpr (I < XG_D) {
+  if constexpr (I < D) {
     *(uint4 *)(p + I * plane) = make_uint4(xg_digit2<I>(v[0], v[1]), xg_digit2<I>(v[2], v[3]), xg_digit2<I>(v[4], v[5]),
                                            xg_digit2<I>(v[6], v[7]));
-    xg_store<I + 1>(p, plane, v);
+    xg_store<D, I + 1>(p, plane, v);
   }
 }
 
@@ -136,7 +139,7 @@ __device__ __forceinline__ int4 xg_chunk(const int4 *chunks, int M, int rpc, int
   return make_int4(c * rpc, min(rpc, M - c * rpc), 0, 0);
 }
 
-// The phases' digit tiles [chunk][stage][digit][W rows][64 B, swizzled] (4 W threads):
+// The phases' digit tiles [chunk][stage][XG_DA digits][W rows][64 B, swizzled] (4 W threads):
 // MMA row 2 m holds (re, -im) and row 2 m + 1 (im, re) of A[m][cell] along K.
 __global__ void __launch_bounds__(256) k_xg_phases(const int4 *chunks, int M, int rpc, int W, int K, int kch,
                                                    const double2 *A, int64_t lda, uint8_t *dig, int *bad) {
@@ -162,7 +165,7 @@ __global__ void __launch_bounds__(256) k_xg_phases(const int4 *chunks, int M, in
     v[2 * c] = xg_fixed((r & 1) ? a.y : a.x, 0);
     v[2 * c + 1] = xg_fixed((r & 1) ? a.x : -a.y, 0);
   }
-  xg_store<0>(dig + ((size_t)mc * kch + kc) * (XG_D * 64 * W) + xg_swz(r, q), 64 * W, v);
+  xg_store<XG_DA>(dig + ((size_t)mc * kch + kc) * (XG_DA * 64 * W) + xg_swz(r, q), 64 * W, v);
 }
 
 // 2^e sum_l 2^(-7 l - 12) S_l, rounded once, in integer arithmetic: eight FP64 operations a value
@@ -225,16 +228,14 @@ __device__ __forceinline__ void umma_bf16(uint32_t d_tmem, uint64_t a, uint64_t 
 // the issuing thread had been slower than the tensor core with them formed in loops.
 template <int W, int I = 0, int J = 0>
 __device__ __forceinline__ void xg_products(uint32_t tmem, uint64_t b, uint64_t a, uint32_t more) {
-  constexpr int nlev = xg_levels(W);
-  // the phases' digit 8 meets digit 0 only, at 2^-62 of 1: left out (nine accumulators: it starts the last)
-  constexpr int end = I == 0 ? nlev : XG_D - I < nlev - I ? XG_D - I : nlev - I;
+  constexpr int end = XG_LEVELS - I;
   constexpr int n = end - J < 256 / W ? end - J : 256 / W;
   umma_bf16(tmem + (I + J) * W, b + I * (XG_PLANE_B >> 4), a + J * (W * 4), idesc_bf16(n * W), I ? 1u : more);
   if constexpr (J + n < end) {
     xg_products<W, I, J + n>(tmem, b, a, more);
-  } else if constexpr (I + 1 < nlev) {
+  } else if constexpr (I + 1 < XG_LEVELS) {
     xg_products<W, I + 1, 0>(tmem, b, a, more);
-  } else if constexpr (nlev < XG_D) {   // level 8 into level 7's accumulator
+  } else {   // level 8 into level 7's accumulator
 #pragma unroll
     for (int i = 1; i < XG_D; ++i)
       umma_bf16(tmem + 7 * W, b + i * (XG_PLANE_B >> 4), a + (8 - i) * (W * 4), idesc_bf16(W), 1u);
@@ -286,7 +287,7 @@ __global__ void __launch_bounds__(XG_THREADS, 1) k_xgemm(XgArgs g) {
       uint32_t phase = 0;
       bool ok = true;
       for (int64_t u = blockIdx.x; u < g.units && ok; u += gridDim.x) {
-        const uint32_t bytes = XG_D * 64 * W;
+        const uint32_t bytes = XG_DA * 64 * W;
         const uint8_t *src = g.dig + (size_t)(u % g.mch) * g.kch * bytes;
         for (int kc = 0; kc < g.kch; ++kc) {
           if (!mbar_wait(&empty[stage], phase ^ 1, g.err)) { ok = false; break; }
@@ -361,7 +362,7 @@ __global__ void __launch_bounds__(XG_THREADS, 1) k_xgemm(XgArgs g) {
         }
         if (kc + 1 < g.kch) fetch(kc + 1);
         if (!mbar_wait(&empty[stage], phase ^ 1, g.err)) { ok = false; break; }
-        xg_store<0>(smem + stage * XG_STAGE + xg_swz(r, q), XG_PLANE_B, v);
+        xg_store<XG_D>(smem + stage * XG_STAGE + xg_swz(r, q), XG_PLANE_B, v);
         asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
         mbar_arrive(&full[stage]);
         if (++stage == XG_STAGES) { stage = 0; phase ^= 1; }
@@ -370,7 +371,6 @@ __global__ void __launch_bounds__(XG_THREADS, 1) k_xgemm(XgArgs g) {
   } else {   // ---- epilogue: warp w reads TMEM lane quadrant w % 4, a thread every other 4 of a column's results
     const int quad = warp & 3, half = (warp - 2 - XG_CONV / 32) >> 2;
     const uint32_t tr = tmem + ((uint32_t)(quad * 32) << 16);
-    constexpr int nlev = xg_levels(W);
     int it = 0;
     bool ok = true;
     for (int64_t u = blockIdx.x; u < g.units && ok; u += gridDim.x) {
@@ -385,10 +385,10 @@ __global__ void __launch_bounds__(XG_THREADS, 1) k_xgemm(XgArgs g) {
         tc_fence_after();
 #pragma unroll 1
         for (int c0 = 4 * half; c0 < 2 * mrows; c0 += 8) {
-          uint32_t a[XG_D][4];
+          uint32_t a[XG_LEVELS][4];
           __syncwarp();
 #pragma unroll
-          for (int l = 0; l < XG_D; ++l) tmem_ld4_nowait(tr + min(l, nlev - 1) * W + c0, a[l]);
+          for (int l = 0; l < XG_LEVELS; ++l) tmem_ld4_nowait(tr + l * W + c0, a[l]);
           tmem_wait_ld();
 #pragma unroll
           for (int c = 0; c < 4; c += 2) {
@@ -397,11 +397,10 @@ __global__ void __launch_bounds__(XG_THREADS, 1) k_xgemm(XgArgs g) {
             for (int y = 0; y < 2; ++y) {
               int s[XG_D];
 #pragma unroll
-              for (int l = 0; l < XG_D; ++l)   // S_l; with eight accumulators the last holds levels 7 and 8
+              for (int l = 0; l < XG_LEVELS; ++l)   // S_l; the last accumulator holds levels 7 and 8
                 s[l] = __float2int_rn(__uint_as_float(a[l][c + y]) *
                                       __uint_as_float((uint32_t)(127 + 7 * l + 12) << 23));
-              if (nlev < XG_D)
-                s[8] = __float2int_rn(128.0f * (__uint_as_float(a[7][c + y]) * 0x1p61f - (float)s[7]));
+              s[8] = __float2int_rn(128.0f * (__uint_as_float(a[7][c + y]) * 0x1p61f - (float)s[7]));
               (y ? z.y : z.x) = xg_value(s, e);
             }
             const int m = ch.x + (c0 + c) / 2;
@@ -469,7 +468,7 @@ static void xg_run(const XgArgs &g, cudaStream_t st) {
 static int xg_width(int rows) { return (2 * rows + 15) / 16 * 16; }
 
 int64_t xgemm_chunk_bytes(int most, int K) {
-  return (int64_t)((K + XG_CELLS - 1) / XG_CELLS) * XG_D * 64 * xg_width(most);
+  return (int64_t)((K + XG_CELLS - 1) / XG_CELLS) * XG_DA * 64 * xg_width(most);
 }
 
 // one launch over mch chunks (dig sized for them)
