@@ -1297,7 +1297,8 @@ int ephg::el_rates_view(ephg_handle *h, const ExecView &x, const ephg_rate_reque
   }
   // FP64 epilogues (the FP64 form; the simplex deltas of both): final states, mode
   // tables of every parameter set and the deltas' tables
-  if (!split || req->delta_kind != 0) {
+  const bool final_epi = !split || req->delta_kind != 0;
+  if (final_epi) {
     int2 *fin;
     if ((rc = wsget((*x.ws), "e_fin", (size_t)nin, &fin))) return WSFAILX(rc);
     launch_final_states(nwv, nw, widx, ens, req->enref, req->fsthick, cum, fin, st);
@@ -1325,8 +1326,9 @@ int ephg::el_rates_view(ephg_handle *h, const ExecView &x, const ephg_rate_reque
     }
     CKL();
   }
-  int nblk = epf_blocks(nin);                   // blocks of the rate partials
-  const int nblk_max = std::max(nblk, (nwv + 255) / 256 * 8);
+  // blocks of the rate partials: of final states in the FP64 epilogues, else of 32 (fused) or 128 rows
+  const int nblk_max = final_epi ? epf_blocks(nin) : (nwv + 255) / 256 * 8;
+  int nblk = nblk_max;
   double *partial;
   if ((rc = wsget((*x.ws), "r_partial", (size_t)nst * nblk_max, &partial))) return WSFAILX(rc);
   rs.rp[0] = rp;
