@@ -1519,13 +1519,13 @@ void launch_mode_tab(int n, const double *om, const double *bose, double T, doub
 //
 // Bound by the FP64 pipe (16 cycles per warp instruction on an SM), so the split
 // keeps every lane on a vertex of its own and every FP64 instruction on the
-// result: a thread is one initial state and walks EPF_F final states, which are
-// the same for the whole block.  There is no divergence over the window bands,
+// result: a thread is one initial state and walks epf_per(nin) final states, the
+// same ones as its neighbours.  There is no divergence over the window bands,
 // U_k' and the delta's table are read by broadcast, the sum over final states
 // stays in the thread (compensated), and the occupations need no exponential:
 // f(E + w) = 1 / (1 + e^x e^v) and 1 - f(E - w) = 1 / (1 + e^-x e^v), x = (E - mu) / kT
-// per state, v = w / kT per mode.  12^3, nw 8, nb 6 (2.8 M pairs): 5.06 ms (3.9 at the
-// FP64 rate for its ~850 instructions a pair); one thread per (k', state) with a loop
+// per state, v = w / kT per mode.  12^3, nw 8, nb 6 (2.8 M pairs): 4.3 ms (3.9 at the
+// FP64 rate for its ~850 instructions a pair; 5.06 with 16 final states per thread); one thread per (k', state) with a loop
 // over the bands took 15.1 ms.  Tetrahedra, 10x12x11 (1.8 M pairs): 3.1 ms + 0.32 ms for
 // the tables; with every simplex's formula at every vertex 511 ms.
 template <bool F32>
@@ -1537,9 +1537,9 @@ __device__ __forceinline__ double2 epf_load(const FinalIn &c, int64_t off) {
 template <bool F32, bool SIMPLEX, bool PH>
 __global__ void __launch_bounds__(EPF_THREADS) k_epilogue_final(int j0, int ns, FinalIn c, RateParams rp, EpiData d,
                                                                 double *partial, int nblk) {
-  const int2 blk = epf_block(blockIdx.x, ns);
-  const int jl = blk.x * EPF_THREADS + threadIdx.x;
-  if (jl >= ns) return;
+  const int2 it = epf_item((int64_t)blockIdx.x * EPF_THREADS + threadIdx.x, ns);
+  const int jl = it.x, grp = it.y;
+  if (grp >= nblk) return;
   const int j = j0 + jl;
   const int nw = rp.nw, nb = rp.nb;
   const int code = d.st_code[j];
@@ -1554,8 +1554,8 @@ __global__ void __launch_bounds__(EPF_THREADS) k_epilogue_final(int j0, int ns, 
   const int a1 = p % rp.mesh[0], a2 = (p / rp.mesh[0]) % rp.mesh[1], a3 = p / (rp.mesh[0] * rp.mesh[1]);
   const double2 *Uk = d.U + ((size_t)p * nw + m) * nw;
   double sum = 0.0, comp = 0.0;
-  const int fe = min(d.nin, (blk.y + 1) * EPF_F);
-  for (int f = blk.y * EPF_F; f < fe; ++f) {
+  const int f0 = grp * epf_per(d.nin), fe = min(d.nin, f0 + epf_per(d.nin));
+  for (int f = f0; f < fe; ++f) {
     const int2 fs = d.fin[f];
     const int pp = d.widx[fs.x];
     const double eps = d.ens[(size_t)pp * nw + fs.y];
@@ -1626,7 +1626,7 @@ __global__ void __launch_bounds__(EPF_THREADS) k_epilogue_final(int j0, int ns, 
     comp += (fabs(sum) >= fabs(acc)) ? (sum - t) + acc : (acc - t) + sum;
     sum = t;
   }
-  partial[(size_t)j * nblk + blk.y] = sum + comp;
+  partial[(size_t)j * nblk + grp] = sum + comp;
 }
 
 void launch_epilogue_final(int j0, int j1, const FinalIn &c, const RateParams &rp, const EpiData &d, double *partial,
@@ -1786,14 +1786,16 @@ extern "C" int ephg_debug_epilogue_grid(int nstates, int nin, int64_t *grid) {
   if (nstates <= 0 || nin <= 0 || !grid) return EPHG_ERR_ARG;
   grid[0] = epf_grid(nstates, nin);
   grid[1] = grid[2] = 1;
-  const int64_t ns = (nstates + EPF_THREADS - 1) / EPF_THREADS, nf = epf_blocks(nin);
-  std::vector<bool> seen((size_t)(ns * nf));
-  for (int64_t b = 0; b < grid[0]; ++b) {
-    const int2 p = epf_block((unsigned)b, nstates);
-    if (p.x < 0 || p.x >= ns || p.y < 0 || p.y >= nf || seen[(size_t)(p.x + ns * p.y)]) return EPHG_ERR_INDEX;
-    seen[(size_t)(p.x + ns * p.y)] = true;
+  const int64_t ng = epf_blocks(nin);
+  if (ng * epf_per(nin) < nin || (ng - 1) * epf_per(nin) >= nin) return EPHG_ERR_INDEX;
+  std::vector<bool> seen((size_t)(nstates * ng));
+  int64_t left = nstates * ng;
+  for (int64_t t = 0; t < grid[0] * EPF_THREADS; ++t) {
+    const int2 p = epf_item(t, nstates);
+    if (p.y >= ng) continue;
+    if (p.x < 0 || p.x >= nstates || p.y < 0 || seen[(size_t)(p.x + nstates * (int64_t)p.y)]) return EPHG_ERR_INDEX;
+    seen[(size_t)(p.x + nstates * (int64_t)p.y)] = true;
+    --left;
   }
-  for (bool x : seen)
-    if (!x) return EPHG_ERR_INDEX;
-  return EPHG_OK;
+  return left ? EPHG_ERR_INDEX : EPHG_OK;
 }

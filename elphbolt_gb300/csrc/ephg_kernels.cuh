@@ -206,17 +206,25 @@ void launch_mode_tab(int n, const double *om, const double *bose, double T, doub
                      cudaStream_t st);
 // FP64 epilogue over the states [j0, j1): the Rp sums G(x = n' + nw s') of (window row ip,
 // state j) at ip ldc + x xs + (j - j0) js, in FP64 (z) or as FP32 planes (re, im).  Rate
-// partials [j][block of EPF_F final states].
-constexpr int EPF_F = 16, EPF_THREADS = 128;
-inline int epf_blocks(int nin) { return (nin + EPF_F - 1) / EPF_F; }
-// Its grid is one-dimensional, blocks of EPF_THREADS states fastest: a mesh of 2^24 points has
-// up to 3.3e7 blocks of final states, which the other dimensions (65,535) do not hold.
-inline int64_t epf_grid(int ns, int nin) { return (int64_t)((ns + EPF_THREADS - 1) / EPF_THREADS) * epf_blocks(nin); }
-// (block of states, block of final states) of block b
-__host__ __device__ inline int2 epf_block(unsigned b, int ns) {
-  const unsigned n = (unsigned)(ns + EPF_THREADS - 1) / EPF_THREADS;
-  return make_int2((int)(b % n), (int)(b / n));
+// partials [j][group of epf_per(nin) final states].
+constexpr int EPF_THREADS = 128;
+// A thread's final states: one while there are few, so that a request of few states fills the chip
+// and waits for one vertex instead of 16 in a row; more where the partials, added up one after the
+// other per state, would take longer than a further vertex (both grow with nin; about 512
+// partials), at most 16.  Stage C in ms with 1 / 2 / 4 / 16 (one thread per window row and
+// state, its bands in turn, before): nw 4, 36 states 0.07 / 0.09 / 0.14 / 0.48 (0.14); nw 16,
+// 740 states 2.5 / 2.7 / 2.8 / 8.0 (5.7); nw 8, 1,984 states 6.5 / 6.0 / 5.8 / 6.6 (18.4); wedge of 82
+// states with 2,238 final states 0.94 / 0.66 / 0.50 / 0.60 (0.78).
+__host__ __device__ inline int epf_per(int nin) {
+  const int n = (nin + 511) / 512;
+  return n < 1 ? 1 : n > 16 ? 16 : n;
 }
+inline int epf_blocks(int nin) { return (nin + epf_per(nin) - 1) / epf_per(nin); }
+// Its grid is one-dimensional over the (state, group) pairs, states fastest: no lane idles for want
+// of states, and a mesh of 2^24 points has more groups than the other grid dimensions hold (65,535).
+inline int64_t epf_grid(int ns, int nin) { return ((int64_t)ns * epf_blocks(nin) + EPF_THREADS - 1) / EPF_THREADS; }
+// (state, group) of thread t
+__host__ __device__ inline int2 epf_item(int64_t t, int ns) { return make_int2((int)(t % ns), (int)(t / ns)); }
 struct FinalIn {
   const double2 *z = nullptr;
   const float *re = nullptr, *im = nullptr;

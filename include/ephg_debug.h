@@ -68,9 +68,9 @@ int ephg_debug_batcher_selftest(int nmembers, int iters, uint64_t seed, int64_t 
 int ephg_debug_group_tiles(int np, const int *mtiles, const int *ntiles, int *hits);
 
 /* The FP64 rate epilogue's launch over nstates initial and nin final states, on
- * the host: grid[3] receives its dimensions; every block's (states, final
- * states) is formed as the kernel forms it.  Returns EPHG_ERR_INDEX if one lies
- * outside, is taken twice or is left out. */
+ * the host: grid[3] receives its dimensions; every thread's (state, group of
+ * final states) is formed as the kernel forms it.  Returns EPHG_ERR_INDEX if one
+ * lies outside, is taken twice or is left out. */
 int ephg_debug_epilogue_grid(int nstates, int nin, int64_t *grid);
 
 #ifdef __cplusplus
