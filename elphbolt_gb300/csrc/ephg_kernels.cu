@@ -7,6 +7,7 @@
 #include <algorithm>
 #include <cstdio>
 #include <mutex>
+#include <type_traits>
 #include <vector>
 
 #include "../../include/ephg_debug.h"
@@ -1167,8 +1168,12 @@ void launch_iota(int n, int *out, cudaStream_t st) {
 // per-output phase arithmetic, 2.63 with each lane reading its own block).
 constexpr int ROT64_THREADS = 64, ROT64_V = 32;
 
-// NW: bands fixed at compile time (the sums then stay in registers), or 0
-template <int NW>
+// A thread's sums over the initial band, one per final one, stay in registers: CAP of them, the next
+// multiple of 4 from nw on, or nw = CAP known to the compiler (EXACT).  With 32 for every nw
+// the registers and the unrolled tail are paid by all: 9^3, nb 6, 1,200 states, with 32 / with CAP:
+// nw 3 0.33 / 0.11 ms, nw 5 0.49 / 0.18, nw 10 1.07 / 0.50, nw 12 1.34 / 0.55, nw 20 3.11 / 1.35,
+// nw 24 3.89 / 1.83; nw 32 5.57, with nw known 3.56.
+template <int CAP, bool EXACT>
 __global__ void __launch_bounds__(ROT64_THREADS) k_rotate_states_fp64(int j0, int j1, int i0, const int *st_code,
                                                                       int nw_, int nb, int nws, int64_t blk0,
                                                                       const int *widx,
@@ -1176,8 +1181,7 @@ __global__ void __launch_bounds__(ROT64_THREADS) k_rotate_states_fp64(int j0, in
                                                                       int64_t ldgk, const double2 *phk, double2 *B,
                                                                       int64_t ldb, int sc, int nst) {
   __shared__ double2 sg[ROT64_THREADS * (ROT64_V + 1)];
-  constexpr int AW = NW ? NW : 32;
-  const int nw = NW ? NW : nw_;
+  const int nw = EXACT ? CAP : nw_;
   const int lane = threadIdx.x & 31, wj = j0 + blockIdx.x * ROT64_THREADS + (threadIdx.x & ~31);
   const int j = wj + lane;
   const bool live = j < j1;
@@ -1189,9 +1193,9 @@ __global__ void __launch_bounds__(ROT64_THREADS) k_rotate_states_fp64(int j0, in
   const double2 *g = gk + (int64_t)nw * nw * u;
   double2 *tile = sg + (threadIdx.x & ~31) * (ROT64_V + 1);
   const int mpc = ROT64_V / nw, nv = min(32, j1 - wj);   // initial bands per pass; the warp's states
-  double2 acc[AW];
+  double2 acc[CAP];
 #pragma unroll
-  for (int np = 0; np < AW; ++np) acc[np] = make_double2(0.0, 0.0);
+  for (int np = 0; np < CAP; ++np) acc[np] = make_double2(0.0, 0.0);
   for (int mp0 = 0; mp0 < nw; mp0 += mpc) {
     const int nm = min(mpc, nw - mp0), n = nw * nm;
     __syncwarp();
@@ -1204,7 +1208,7 @@ __global__ void __launch_bounds__(ROT64_THREADS) k_rotate_states_fp64(int j0, in
       for (int mp = 0; mp < nm; ++mp) {
         const double2 um = Uk[mp0 + mp], *row = tile + lane * (ROT64_V + 1) + nw * mp;
 #pragma unroll
-        for (int np = 0; np < AW; ++np)
+        for (int np = 0; np < CAP; ++np)
           if (np < nw) cfma(acc[np], um, row[np]);
       }
   }
@@ -1214,7 +1218,7 @@ __global__ void __launch_bounds__(ROT64_THREADS) k_rotate_states_fp64(int j0, in
   const int jc = j / sc * sc, ns = min(sc, nst - jc);
   double2 *out = B + (int64_t)rp * ldb + (int64_t)jc * nw * nb + (int64_t)nw * s * ns + (j - jc);
 #pragma unroll
-  for (int np = 0; np < AW; ++np)
+  for (int np = 0; np < CAP; ++np)
     if (np < nw) out[(int64_t)np * ns] = cmul(ph, acc[np]);
 }
 
@@ -1228,8 +1232,20 @@ void launch_rotate_states_fp64(int j0, int j1, int i0, const int *st_code, int n
       k<<<grid, ROT64_THREADS, 0, st>>>(j0, j1, i0, st_code, nw, nb, nws, blk0 + b, widx, U, gk + b * nw * nw, ldgk, phk,
                                         B, ldb, sc, nst);
     };
-    nw == 4 ? go(k_rotate_states_fp64<4>) : nw == 8 ? go(k_rotate_states_fp64<8>)
-    : nw == 16 ? go(k_rotate_states_fp64<16>) : go(k_rotate_states_fp64<0>);
+    auto upto = [&](auto cap) {
+      constexpr int C = decltype(cap)::value;
+      nw == C ? go(k_rotate_states_fp64<C, true>) : go(k_rotate_states_fp64<C, false>);
+    };
+    switch ((nw + 3) / 4) {
+      case 1: upto(std::integral_constant<int, 4>()); break;
+      case 2: upto(std::integral_constant<int, 8>()); break;
+      case 3: upto(std::integral_constant<int, 12>()); break;
+      case 4: upto(std::integral_constant<int, 16>()); break;
+      case 5: upto(std::integral_constant<int, 20>()); break;
+      case 6: upto(std::integral_constant<int, 24>()); break;
+      case 7: upto(std::integral_constant<int, 28>()); break;
+      default: upto(std::integral_constant<int, 32>()); break;
+    }
   }
 }
 
