@@ -4,8 +4,30 @@
 #include <stdint.h>
 
 #include <cmath>
+#include <mutex>
+#include <set>
 
 namespace ephg {
+
+// Runs f on the first call on each device: kernel attributes belong to the device that is
+// current when they are set, and changing one can wait for the device's queued work.
+class OncePerDevice {
+  std::mutex mu;
+  std::set<int> done;
+
+ public:
+  template <typename F>
+  void operator()(F f) {
+    int dev = 0;
+    cudaGetDevice(&dev);
+    on(dev, f);
+  }
+  template <typename F>
+  void on(int dev, F f) {
+    std::lock_guard<std::mutex> lk(mu);
+    if (done.insert(dev).second) f();
+  }
+};
 
 // ---- constants: src/params.f90:27-57 (same expressions, same doubles) ----
 constexpr double qe = 1.602176634e-19;

@@ -6,7 +6,6 @@
 // Each kernel names the reference lines it restates.
 #include <algorithm>
 #include <cstdio>
-#include <mutex>
 #include <type_traits>
 #include <vector>
 
@@ -218,9 +217,8 @@ void launch_cells_fourier(const CellTab &t, const double2 *in, int64_t ldi, cons
                           const int mesh[3], int L, const double2 *roots, double2 *t1, double2 *t2,
                           const int *rowmap, double2 *out, int64_t ldo, cudaStream_t st) {
   if (nc <= 0) return;
-  static std::once_flag attr_once;   // once per process: changing a kernel attribute can wait for queued work
-  std::call_once(attr_once,
-                 [] { cudaFuncSetAttribute(k_cells_dft, cudaFuncAttributeMaxDynamicSharedMemorySize, CF_SMEM); });
+  static OncePerDevice attr;
+  attr([] { cudaFuncSetAttribute(k_cells_dft, cudaFuncAttributeMaxDynamicSharedMemorySize, CF_SMEM); });
   auto pass = [&](int d, int64_t A, int B, const int *tab, const double2 *src, int64_t ls, const double *sc,
                   const int *map, double2 *dst, int64_t ld) {
     CellDft g;
@@ -869,11 +867,8 @@ __global__ void __launch_bounds__(T) k_heig(int batch, int n, int G, const doubl
 template <int T>
 static void heig_run(int batch, int n, int G, const double2 *A, int64_t stride, double *w, double2 *V, int *err,
                      cudaStream_t st) {
-  // once per process: changing a kernel attribute can wait for the device's queued work
-  static std::once_flag attr_once;
-  std::call_once(attr_once, [] {
-    cudaFuncSetAttribute(k_heig<T>, cudaFuncAttributeMaxDynamicSharedMemorySize, 96 * 1024);
-  });
+  static OncePerDevice attr;
+  attr([] { cudaFuncSetAttribute(k_heig<T>, cudaFuncAttributeMaxDynamicSharedMemorySize, 96 * 1024); });
   const size_t smem = (size_t)G * (4 * (n | 1) * n + 3 * 16) * sizeof(double2);   // 77 KB at most
   k_heig<T><<<(batch + G - 1) / G, T, smem, st>>>(batch, n, G, A, stride, w, V, err);
 }
@@ -1814,4 +1809,14 @@ extern "C" int ephg_debug_epilogue_grid(int nstates, int nin, int64_t *grid) {
     --left;
   }
   return left ? EPHG_ERR_INDEX : EPHG_OK;
+}
+
+extern "C" int ephg_debug_once_per_device(int n, const int *devices, int *ran) {
+  if (n <= 0 || !devices || !ran) return EPHG_ERR_ARG;
+  ephg::OncePerDevice once;
+  for (int i = 0; i < n; ++i) {
+    ran[i] = 0;
+    once.on(devices[i], [&] { ran[i] = 1; });
+  }
+  return EPHG_OK;
 }

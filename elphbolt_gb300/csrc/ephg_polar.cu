@@ -25,7 +25,6 @@
 // last bit of D decides where an off-diagonal element is all rounding: sums in
 // another order move those rates by 1e-7, so here the order stays the loop's.
 #include <algorithm>
-#include <mutex>
 
 #include "ephg_common.cuh"
 #include "ephg_kernels.cuh"
@@ -383,11 +382,8 @@ struct PolarBox {
 template <int NU, bool DA>
 static void polar_run(const PolarDev &P, const PolarBox &B, int nq, const int *qp, const int mesh[3], const double *qv,
                       double2 *Dq, int64_t ldd, double2 *Lq, cudaStream_t st) {
-  // once per process: changing a kernel attribute can wait for the device's queued work
-  static std::once_flag once;
-  std::call_once(once, [] {
-    cudaFuncSetAttribute(k_polar<NU, DA>, cudaFuncAttributeMaxDynamicSharedMemorySize, PL_SMEM);
-  });
+  static OncePerDevice attr;
+  attr([] { cudaFuncSetAttribute(k_polar<NU, DA>, cudaFuncAttributeMaxDynamicSharedMemorySize, PL_SMEM); });
   const size_t entry = pl_entry_doubles(P.nat, DA) * sizeof(double);
   const int nent = pl_entries(entry);
   k_polar<NU, DA><<<nq, PL_THREADS, nent * entry, st>>>(P, B.G, B.Gf, B.M, nq, qp, mesh ? mesh[0] : 1,
@@ -406,10 +402,8 @@ static void polar_dispatch(const PolarDev &P, const PolarBox &B, int nq, const i
 template <int NU>
 static void polar_vel_run(const PolarDev &P, const PolarBox &B, int nq, const int *qp, const int mesh[3],
                           const double *qv, double2 *Dq, double2 *dDq, int64_t ldd, cudaStream_t st) {
-  static std::once_flag once;
-  std::call_once(once, [] {
-    cudaFuncSetAttribute(k_polar_vel<NU>, cudaFuncAttributeMaxDynamicSharedMemorySize, PL_SMEM);
-  });
+  static OncePerDevice attr;
+  attr([] { cudaFuncSetAttribute(k_polar_vel<NU>, cudaFuncAttributeMaxDynamicSharedMemorySize, PL_SMEM); });
   const int nh = P.nb * (P.nb + 1) / 2, np = P.nat * P.nb;
   const size_t entry = (size_t)pv_entry(P.nat) * sizeof(double2);
   const int nent = pl_entries(entry);

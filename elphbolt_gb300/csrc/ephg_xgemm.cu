@@ -458,9 +458,8 @@ static int xg_sms() {
 
 template <int W>
 static void xg_run(const XgArgs &g, cudaStream_t st) {
-  static std::once_flag attr_once;   // once per process: changing a kernel attribute can wait for queued work
-  std::call_once(attr_once,
-                 [] { cudaFuncSetAttribute(k_xgemm<W>, cudaFuncAttributeMaxDynamicSharedMemorySize, XG_SMEM); });
+  static OncePerDevice attr;
+  attr([] { cudaFuncSetAttribute(k_xgemm<W>, cudaFuncAttributeMaxDynamicSharedMemorySize, XG_SMEM); });
   k_xgemm<W><<<(unsigned)std::min<int64_t>(g.units, xg_sms()), XG_THREADS, XG_SMEM, st>>>(g);
 }
 

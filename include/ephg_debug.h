@@ -73,6 +73,10 @@ int ephg_debug_group_tiles(int np, const int *mtiles, const int *ntiles, int *hi
  * lies outside, is taken twice or is left out. */
 int ephg_debug_epilogue_grid(int nstates, int nin, int64_t *grid);
 
+/* The guard that sets kernel attributes, with the current device given as devices[i] for
+ * call i (no device is touched): ran[i] = 1 where it sets them. */
+int ephg_debug_once_per_device(int n, const int *devices, int *ran);
+
 #ifdef __cplusplus
 }
 #endif
