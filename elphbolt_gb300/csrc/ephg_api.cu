@@ -14,6 +14,7 @@
 #include <vector>
 
 #include "../../include/ephg.h"
+#include "../../include/ephg_debug.h"
 #include "ephg_kernels.cuh"
 #include "ephg_tc.cuh"
 #include "ephg_ws.cuh"
@@ -1344,12 +1345,15 @@ int ephg::el_rates_view(ephg_handle *h, const ExecView &x, const ephg_rate_reque
   }
   if (!split) {
     // Each contraction is a Fourier sum of cells onto mesh points: one dimension at a
-    // time (launch_cells_fourier), or as a matrix product where that takes fewer FP64
-    // instructions (a wedge or a window of few rows; 4 per cell and row).  Both are
-    // bound by the FP64 pipe, so the counts decide: 12^3 and 279 cells, 1,479 rows,
-    // 468 ms as products and 14.7 ms as sums.
-    const bool sepA = cells_fourier_cost(h->cellk, mesh, nA) < 4.0 * nA * nwsk;
-    const bool sepB = cells_fourier_cost(h->cellq, mesh, nwv) < 4.0 * nwv * nwsq;
+    // time on the FP64 pipe (launch_cells_fourier), which forms whole mesh lines, or as a
+    // product with the rows' phases on the tensor cores (launch_xgemm), whose time grows
+    // with rows times cells.  Whichever is estimated shorter per column; of 300 measured
+    // contractions (6^3 to 24^3, 43 to 279 cells, 20 to 2,500 rows) the choice is within 5%
+    // of the better one in 285, the others being calls of a few columns (under 30 us).  Sums / products in ms, stage A: 12^3, 279 cells, 1,678 rows
+    // 8.8 / 14.4, 955 rows 7.8 / 8.0, 397 rows 6.5 / 3.5, 60 rows 5.6 / 0.6; 9x10x9, 93 cells,
+    // 756 rows 1.09 / 1.10; 24^3, 93 cells, 1,001 rows 4.0 / 1.4.
+    const bool sepA = cells_fourier_cycles(h->cellk, mesh, nA) < xgemm_cycles(nA, nwsk);
+    const bool sepB = cells_fourier_cycles(h->cellq, mesh, nwv) < xgemm_cycles(nwv, nwsq);
     const int64_t per = (int64_t)nw * nw, nper = (int64_t)nb * nwsq;   // columns of one (mode, Rp) block; blocks
     const int64_t bound = (int64_t)1 << 31;
     double2 *Pk = nullptr, *t1 = nullptr, *t2 = nullptr, *gk, *B, *Pq = nullptr, *Cb, *phk;
@@ -1530,4 +1534,54 @@ extern "C" int ephg_ph_rates(ephg_handle *h, const ephg_rate_request *req, int64
   const ExecView x{h->st, h->err, &h->ws, &h->timer_a, &h->timer_b, &h->launches};
   const PhOut ph{rates_phe, y, (double)spindeg};
   return el_rates_view(h, x, req, el_rates, indexlist, stats, g2, nullptr, nullptr, cap, &ph);
+}
+
+// The FP64 rate path's sums over cells on their own (include/ephg_debug.h).
+extern "C" int ephg_debug_cells_fourier(int64_t ncells, const int64_t *cells, const double *scale, const int64_t mesh[3],
+                                        int64_t nc, const double *in, int64_t nrows, const int64_t *rows, double *out) {
+  if (ncells <= 0 || !cells || !mesh || nc <= 0 || !in || nrows <= 0 || !rows || !out)
+    return fail(EPHG_ERR_ARG, "debug_cells_fourier: bad arguments");
+  const int m[3] = {(int)mesh[0], (int)mesh[1], (int)mesh[2]};
+  const int64_t N = mesh[0] * mesh[1] * mesh[2];
+  std::vector<int> r(3 * (size_t)ncells), rw(nrows), tab;
+  for (int64_t i = 0; i < ncells; ++i)
+    for (int c = 0; c < 3; ++c) r[3 * i + c] = (int)cells[i + ncells * c];
+  for (int64_t i = 0; i < nrows; ++i) {
+    if (rows[i] < 0 || rows[i] >= N) return fail(EPHG_ERR_ARG, "debug_cells_fourier: row outside the mesh");
+    rw[i] = (int)rows[i];
+  }
+  CellTab t;
+  size_t off[3];
+  if (!cell_tables(r, (int)ncells, t, tab, off)) return fail(EPHG_ERR_ARG, "debug_cells_fourier: cells");
+  t.ok = true;
+  if (std::isinf(cells_fourier_cost(t, m, nrows))) return fail(EPHG_ERR_ARG, "debug_cells_fourier: mesh");
+  const int L = lcm3(m);
+  Workspace ws;
+  int *td, *rd, *map, rc;
+  double *sd = nullptr;
+  double2 *roots, *t1, *t2, *a, *b;
+  if ((rc = wsget(ws, "tab", tab.size(), &td)) || (rc = wsget(ws, "rows", rw.size(), &rd)) ||
+      (rc = wsget(ws, "map", (size_t)N, &map)) || (rc = wsget(ws, "roots", (size_t)L, &roots)) ||
+      (scale && (rc = wsget(ws, "scale", (size_t)ncells, &sd))) ||
+      (rc = wsget(ws, "t1", (size_t)(cells_t1_rows(t, m) * nc), &t1)) ||
+      (rc = wsget(ws, "t2", (size_t)(cells_t2_rows(t, m) * nc), &t2)) ||
+      (rc = wsget(ws, "in", (size_t)(ncells * nc), &a)) || (rc = wsget(ws, "out", (size_t)(nrows * nc), &b))) {
+    ws.release();
+    return fail(rc, "%s", ws.msg.c_str());
+  }
+  t.tab1 = td + off[0];
+  t.tab2 = td + off[1];
+  t.tab3 = td + off[2];
+  cudaMemcpy(td, tab.data(), tab.size() * sizeof(int), cudaMemcpyHostToDevice);
+  cudaMemcpy(rd, rw.data(), rw.size() * sizeof(int), cudaMemcpyHostToDevice);
+  if (scale) cudaMemcpy(sd, scale, (size_t)ncells * sizeof(double), cudaMemcpyHostToDevice);
+  cudaMemcpy(a, in, (size_t)(ncells * nc) * sizeof(double2), cudaMemcpyHostToDevice);
+  launch_roots(L, roots, nullptr);
+  launch_row_map((int)N, (int)nrows, rd, map, nullptr);
+  launch_cells_fourier(t, a, nc, sd, (int)nc, m, L, roots, t1, t2, map, b, nc, nullptr);
+  const cudaError_t e = cudaMemcpy(out, b, (size_t)(nrows * nc) * sizeof(double2), cudaMemcpyDeviceToHost);
+  ws.release();
+  return e == cudaSuccess && cudaGetLastError() == cudaSuccess
+             ? EPHG_OK
+             : fail(EPHG_ERR_CUDA, "debug_cells_fourier: %s", cudaGetErrorString(e));
 }

@@ -37,8 +37,12 @@ struct CellTab {
   int npair = 0, n1 = 0;
   const int *tab1 = nullptr, *tab2 = nullptr, *tab3 = nullptr;
 };
-// FP64 operations per column of launch_cells_fourier, in multiply-adds; infinity where it cannot run
+// FP64 instructions per column of launch_cells_fourier; infinity where it cannot run
 double cells_fourier_cost(const CellTab &t, const int mesh[3], int64_t rows);
+// Cycles of one SM for 128 columns: four warps' FP64 instructions at 16 cycles each, as measured
+inline double cells_fourier_cycles(const CellTab &t, const int mesh[3], int64_t rows) {
+  return 60.0 * cells_fourier_cost(t, mesh, rows);
+}
 // work rows (double2 per column) of t1 and t2
 inline int64_t cells_t1_rows(const CellTab &t, const int mesh[3]) { return (int64_t)t.npair * mesh[2]; }
 inline int64_t cells_t2_rows(const CellTab &t, const int mesh[3]) { return (int64_t)t.n1 * mesh[1] * mesh[2]; }

@@ -9,6 +9,9 @@ namespace ephg {
 // Returns 0, or an EPHG_ERR code with ws.msg set.
 int launch_xgemm(Workspace &ws, int M, int64_t N, int K, const double2 *A, int64_t lda, const double2 *B, int64_t ldb,
                  const int *cexp, double2 *C, int64_t ldc, int *err, cudaStream_t st);
+// Cycles of one SM for 128 columns of a product of M rows: chunks of up to 32 rows, each splitting
+// B's K values anew.  Fitted to launches that fill the chip (43 to 279 cells, 150 to 2,500 rows).
+inline double xgemm_cycles(int64_t M, int K) { return (double)((M + 31) / 32) * (25000.0 + 4000.0 * ((K + 15) / 16)); }
 // Rows of A against several right-hand sides in one launch: chunk c (device) is (first row, rows
 // <= most <= XG_CHUNK, right-hand side); right-hand side b is B + b bstride, [K][N] at row stride ldb.
 // cexp: the exponents of xgemm_colexp, ldb per right-hand side.  The phases' digits take

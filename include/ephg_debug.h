@@ -73,6 +73,14 @@ int ephg_debug_group_tiles(int np, const int *mtiles, const int *ntiles, int *hi
  * lies outside, is taken twice or is left out. */
 int ephg_debug_epilogue_grid(int nstates, int nin, int64_t *grid);
 
+/* The FP64 rate path's Fourier sums over cells, one dimension at a time:
+ * out (nrows,nc) = sum over cells of e^{2 pi i k.R} scale[R] in (ncells,nc), row-major
+ * interleaved complex, for the mesh points rows[] (0-based, distinct); cells
+ * (ncells,3) column-major, distinct; scale nullable.  On its own because small meshes
+ * take the product with the phases instead. */
+int ephg_debug_cells_fourier(int64_t ncells, const int64_t *cells, const double *scale, const int64_t mesh[3], int64_t nc,
+                             const double *in, int64_t nrows, const int64_t *rows, double *out);
+
 /* The guard that sets kernel attributes, with the current device given as devices[i] for
  * call i (no device is touched): ran[i] = 1 where it sets them. */
 int ephg_debug_once_per_device(int n, const int *devices, int *ran);
