@@ -29,6 +29,14 @@ class OncePerDevice {
   }
 };
 
+// SMs of the current device
+inline int num_sms() {
+  int dev = 0, n = 0;
+  cudaGetDevice(&dev);
+  cudaDeviceGetAttribute(&n, cudaDevAttrMultiProcessorCount, dev);
+  return n > 0 ? n : 1;
+}
+
 // ---- constants: src/params.f90:27-57 (same expressions, same doubles) ----
 constexpr double qe = 1.602176634e-19;
 constexpr double me = 9.1093837015e-31;

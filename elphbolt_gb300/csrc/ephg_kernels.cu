@@ -1,8 +1,8 @@
 // ephg_kernels.cu - FP64 set-up and drop-in kernels of the e-ph vertex path.
 //
-// Phase tables, H(k)/D(q) assembly, the batched warp-level Hermitian Jacobi
-// eigensolver, the FP64 complex GEMM used by the plain drop-in, and the
-// per-(k', state) epilogue that forms |g|^2, X+- and the RTA rate partials.
+// Phase tables, Fourier sums over cells, the batched Hermitian Jacobi eigensolver (one to
+// four matrices per block), the FP64 complex GEMM of the call that may not allocate, and
+// the per-(state, final states) epilogue that forms |g|^2, X+- and the RTA rate partials.
 // Each kernel names the reference lines it restates.
 #include <algorithm>
 #include <cstdio>
@@ -126,7 +126,7 @@ void launch_mesh_fourier(const double2 *box, const int lo[3], const int ext[3], 
 // instruction of a warp holds the pipe for 16 cycles, so the ~3 shared loads
 // per 4 FMA are hidden at any occupancy of a few warps.  Measured, 12^3, nw 8, nb 6,
 // 279 cells (both contractions): 14.7 ms, 0.95 of the FP64 rate for the instructions
-// counted by cells_fourier_cost; the matrix products took 468 ms at 1.23 TFLOP/s.
+// counted by cells_fourier_cost; matrix products on that pipe took 468 ms at 1.23 TFLOP/s.
 constexpr int CF_THREADS = 128;
 constexpr int CF_MAXM = 1024;                 // mesh points per dimension (shared root table)
 constexpr int CF_SMEM = 160 * 1024;
@@ -455,7 +455,6 @@ __device__ __forceinline__ unsigned inv_of(int d) { return d == 1 ? 0u : 0xfffff
 __device__ __forceinline__ int div_by(int x, unsigned inv) { return inv ? (int)__umulhi((unsigned)x, inv) : x; }
 
 constexpr int EIG_G = 4;       // matrices per block at most
-constexpr int EIG_SMS = 152;   // SMs
 
 // What a block's sweeps share: which matrices are done, their last off-diagonal norms.
 struct EigState {
@@ -869,7 +868,7 @@ static void heig_run(int batch, int n, int G, const double2 *A, int64_t stride, 
                      cudaStream_t st) {
   static OncePerDevice attr;
   attr([] { cudaFuncSetAttribute(k_heig<T>, cudaFuncAttributeMaxDynamicSharedMemorySize, 96 * 1024); });
-  const size_t smem = (size_t)G * (4 * (n | 1) * n + 3 * 16) * sizeof(double2);   // 77 KB at most
+  const size_t smem = (size_t)G * (4 * (n | 1) * n + 3 * 16) * sizeof(double2);   // 67 KB at most (n = 32)
   k_heig<T><<<(batch + G - 1) / G, T, smem, st>>>(batch, n, G, A, stride, w, V, err);
 }
 
@@ -881,7 +880,7 @@ void launch_heig(int batch, int n, const double2 *A, int64_t stride, double *w, 
   // together saves where one leaves lanes idle.  Microseconds at G = 1 / together:
   //   512 of n = 8:    90 / 103 (G = 4)      1,728 of n = 6:  133 / 100 (G = 4)
   //   2,197 of n = 12: 659 / 613 (G = 2)     2,197 of n = 16: 1,190 / 1,242 (G = 2)
-  const bool many = batch >= 8 * EIG_SMS;
+  const bool many = batch >= 8 * num_sms();
   if (n <= 8) {
     if (many) heig_run<128>(batch, n, 4, A, stride, w, V, err, st);
     else heig_run<64>(batch, n, 1, A, stride, w, V, err, st);
@@ -1159,8 +1158,9 @@ void launch_iota(int n, int *out, cudaStream_t st) {
 // phases from a table.  Lanes are states, so that the stores run along the states
 // (the epilogue's lanes); each warp stages its states' nw x nw blocks through
 // shared memory in whole rows, ROT64_V values of each state at a time.
-// 12^3, nw 8, nb 6, 279 cells, 1,679 states: 1.74 ms (1.1 at the FP64 rate; 2.96 with
-// per-output phase arithmetic, 2.63 with each lane reading its own block).
+// 12^3, nw 8, nb 6, 279 cells, 1,679 states: 1.74 ms (1.1 at the FP64 rate; 2.63 with each
+// lane reading its own block).  With the phases tabulated but one state's columns after the
+// other's it took 1.34; the epilogue, whose lanes are states, gained more from this order.
 constexpr int ROT64_THREADS = 64, ROT64_V = 32;
 
 // A thread's sums over the initial band, one per final one, stay in registers: CAP of them, the next

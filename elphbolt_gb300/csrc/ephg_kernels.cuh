@@ -59,7 +59,7 @@ void launch_zgemm(int M, int N, int K, const double2 *A, int64_t lda, const doub
                   int64_t ldb, double2 *C, int64_t ldc, cudaStream_t st);
 
 // ---- Hermitian eigensolver (batched, n <= 32) ----
-// A: batch matrices (n,n) column-major at stride n*n, upper triangle forced
+// A: batch matrices (n,n) column-major, `stride` values apart, upper triangle forced
 // Hermitian as in wannier.f90:481-486.  w: (batch, n) ascending;
 // V: (batch, n, n) column-major, columns = eigenvectors.
 void launch_heig(int batch, int n, const double2 *A, int64_t stride, double *w, double2 *V,

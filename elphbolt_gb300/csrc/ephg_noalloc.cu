@@ -6,8 +6,11 @@
 // memory the GPU reaches through the Grace C2C link), a process whose memory
 // budget is fixed by another framework's pool, or a time-critical loop in which
 // cudaMalloc's implicit synchronisation is not acceptable.  For them
-// ephg_el_wann_noalloc runs the same kernels as ephg_el_wann on caller-owned
-// inputs and outputs, with its scratch (the phase matrix, the batch of H(k)
+// ephg_el_wann_noalloc interpolates on caller-owned inputs and outputs with kernels that
+// need no workspace of their own: a sincos per phase (k_phase_frac) and FP64 multiply-adds
+// (k_zgemm) where ephg_el_wann has phase tables and the tensor-core product, whose digits
+// take a buffer; the eigensolver is the same.  The two agree to rounding, and bands that
+// are degenerate to rounding may come in another gauge.  Its scratch (the phase matrix, the batch of H(k)
 // matrices and the eigensolver output) in one fixed file-scope device array.
 //
 // The array is part of the library image: every GPU that loads the library

@@ -23,7 +23,8 @@
 // f p_a conj(p_b) per pair of atoms and z.  The tensor-core rates round the
 // eigenvectors to FP32 in the gauge that the eigensolver leaves them in, which the
 // last bit of D decides where an off-diagonal element is all rounding: sums in
-// another order move those rates by 1e-7, so here the order stays the loop's.
+// another order move those rates by 1e-7, so here the order stays the loop's.  D of a call
+// with velocities therefore differs from that of one without in its last bits.
 #include <algorithm>
 
 #include "ephg_common.cuh"

@@ -575,13 +575,6 @@ static int make_map(CUtensorMap *m, const float *base, int Kp, int64_t rows, int
   return 0;
 }
 
-static int num_sms() {
-  int dev = 0, n = 0;
-  cudaGetDevice(&dev);
-  cudaDeviceGetAttribute(&n, cudaDevAttrMultiProcessorCount, dev);
-  return n > 0 ? n : 1;
-}
-
 // ------------------------------------------------------ grouped launches
 // The GEMMs of rate requests running concurrently (one host thread and stream
 // each) are gathered into rounds: a member that reaches a GEMM submits it and

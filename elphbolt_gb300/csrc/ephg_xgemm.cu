@@ -153,7 +153,7 @@ __global__ void __launch_bounds__(256) k_xg_phases(const int4 *chunks, int M, in
     const int k = kc * XG_CELLS + 4 * q + c;
     double2 a = make_double2(0.0, 0.0);
     if ((r >> 1) < ch.y && k < K) a = A[(int64_t)m * lda + k];
-    // a mean of phases may round to a few units above 1; anything else beyond is no phase
+    // a product of three table entries may round to a few units above 1; anything else beyond is no phase
     // (a non-finite k) and the row's results are NaN
     constexpr long long ONE = 0x3ff0000000000000ll, ABS = 0x7fffffffffffffffll;
     const long long ax = __double_as_longlong(a.x) & ABS, ay = __double_as_longlong(a.y) & ABS;
@@ -449,18 +449,11 @@ void launch_colexp(int64_t N, int K, const double2 *B, int *e, cudaStream_t st) 
   col_exp(1, N, K, B, N, 0, e, st);
 }
 
-static int xg_sms() {
-  int dev = 0, n = 0;
-  cudaGetDevice(&dev);
-  cudaDeviceGetAttribute(&n, cudaDevAttrMultiProcessorCount, dev);
-  return n > 0 ? n : 1;
-}
-
 template <int W>
 static void xg_run(const XgArgs &g, cudaStream_t st) {
   static OncePerDevice attr;
   attr([] { cudaFuncSetAttribute(k_xgemm<W>, cudaFuncAttributeMaxDynamicSharedMemorySize, XG_SMEM); });
-  k_xgemm<W><<<(unsigned)std::min<int64_t>(g.units, xg_sms()), XG_THREADS, XG_SMEM, st>>>(g);
+  k_xgemm<W><<<(unsigned)std::min<int64_t>(g.units, num_sms()), XG_THREADS, XG_SMEM, st>>>(g);
 }
 
 // MMA columns of a level for chunks of up to `rows` rows

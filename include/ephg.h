@@ -165,9 +165,13 @@ int ephg_irred_wedge(const double *lattvecs, int64_t nsymm, const int64_t *rotat
 int ephg_el_wann(ephg_handle *h, int64_t nk, const double *kvecs, double *energies,
                  double *velocities, double *evecs, const double *scissor);
 
-/* ph_wann, non-polar (wannier.f90:585-782): qvecs (nq,3) -> energies (nq,nb) eV,
+/* ph_wann (wannier.f90:585-782): qvecs (nq,3) -> energies (nq,nb) eV,
  * optional evecs (nq,nb,nb) with evecs(q,s,:) the eigenvector of mode s,
- * velocities (nq,nb,3) km/s.  Returns EPHG_ERR_NEG_PHONON where the reference stops. */
+ * velocities (nq,nb,3) km/s.  Returns EPHG_ERR_NEG_PHONON where the reference stops.
+ * A point's results, here and in el_wann, gkRp and gReq, do not depend on the other points
+ * of its call.  The polar terms are summed in another order where velocities are asked
+ * for: energies then agree with a call without them to rounding, and modes that are
+ * degenerate to rounding may come in another gauge. */
 int ephg_ph_wann(ephg_handle *h, int64_t nq, const double *qvecs, double *energies,
                  double *evecs, double *velocities);
 
@@ -371,7 +375,9 @@ int ephg_el_rates_batch(int64_t n, ephg_handle *const *crystals, const ephg_rate
  * The kernels run on the handle's own stream, which does not wait for other
  * streams: kvecs must be complete before the call (synchronise the stream or
  * OpenACC queue that wrote it), and the call returns after the handle's stream
- * has finished, so energies and evecs are complete on return. */
+ * has finished, so energies and evecs are complete on return.  They agree with
+ * ephg_el_wann's to rounding (H(k) is summed by other kernels); degenerate bands may come
+ * in another gauge. */
 #define EPHG_NOALLOC_SCRATCH_BYTES (16ull << 20)
 int ephg_el_wann_noalloc(ephg_handle *h, int64_t nk, const double *kvecs, double *energies,
                          double *evecs);
