@@ -1535,9 +1535,9 @@ void launch_mode_tab(int n, const double *om, const double *bose, double T, doub
 // U_k' and the delta's table are read by broadcast, the sum over final states
 // stays in the thread (compensated), and the occupations need no exponential:
 // f(E + w) = 1 / (1 + e^x e^v) and 1 - f(E - w) = 1 / (1 + e^-x e^v), x = (E - mu) / kT
-// per state, v = w / kT per mode.  12^3, nw 8, nb 6 (2.8 M pairs): 4.3 ms (3.9 at the
-// FP64 rate for its ~850 instructions a pair; 5.06 with 16 final states per thread); one thread per (k', state) with a loop
-// over the bands took 15.1 ms.  Tetrahedra, 10x12x11 (1.8 M pairs): 3.1 ms + 0.32 ms for
+// per state, v = w / kT per mode.  12^3, nw 8, nb 6 (2.8 M pairs): 4.2 ms (3.9 at the
+// FP64 rate for its ~850 instructions a pair; 5.1 with 16 final states per thread); one thread per (k', state) with a loop
+// over the bands took 15.1 ms.  Tetrahedra, 10x12x11 (1.8 M pairs): 2.6 ms + 0.32 ms for
 // the tables; with every simplex's formula at every vertex 511 ms.
 template <bool F32>
 __device__ __forceinline__ double2 epf_load(const FinalIn &c, int64_t off) {
